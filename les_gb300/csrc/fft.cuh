@@ -44,6 +44,7 @@ struct FftPlanDev {
   const float4* twd;  // the same as float-float pairs (re.hi, re.lo, im.hi, im.lo)
   const float2* unitf;  // exp(-2 pi i m / n), m < n, in FP32 (fixed-length kernels)
   const float4* unitd;  // the same as float-float pairs
+  const int4* uniti;    // the same in 62 fractional bits (integer-pipe kernels): re hi, re lo, im hi, im lo
 };
 
 struct RealPlanDev {
@@ -53,6 +54,7 @@ struct RealPlanDev {
   const double2* w;   // exp(-2 pi i k / nx), k = 0..m
   const float2* wf;   // the same in FP32
   const float4* wd;   // the same as float-float pairs
+  const int4* wi;     // the same in 62 fractional bits
 };
 
 // ---- radix butterflies -----------------------------------------------------

@@ -186,30 +186,22 @@ void cols_fixed(const ColJob& J, const FftPlanDev& Pin, const FftPlanDev& Pout, 
 
 template <typename T, typename TIn>
 bool launch_rows_r2c_fixed(const RowJob& J, const RealPlanDev& P, int rpc, size_t sm, cudaStream_t s) {
-  if constexpr (std::is_same<T, double>::value) {
-    return false;
-  } else {
-    switch (P.nx / 2) {
+  switch (P.nx / 2) {
 #define LES_CASE(n) \
-  case n: r2c_fixed<T, TIn, n>(J, P, rpc, s); return true;
-      LES_ROW_SIZES(LES_CASE)
+case n: r2c_fixed<T, TIn, n>(J, P, rpc, s); return true;
+    LES_ROW_SIZES(LES_CASE)
 #undef LES_CASE
-      default: return false;
-    }
+    default: return false;
   }
 }
 template <typename T, typename TOut>
 bool launch_rows_c2r_fixed(const RowJob& J, const RealPlanDev& P, int rpc, size_t sm, cudaStream_t s) {
-  if constexpr (std::is_same<T, double>::value) {
-    return false;
-  } else {
-    switch (P.nx / 2) {
+  switch (P.nx / 2) {
 #define LES_CASE(n) \
-  case n: c2r_fixed<T, TOut, n>(J, P, rpc, s); return true;
-      LES_ROW_SIZES(LES_CASE)
+case n: c2r_fixed<T, TOut, n>(J, P, rpc, s); return true;
+    LES_ROW_SIZES(LES_CASE)
 #undef LES_CASE
-      default: return false;
-    }
+    default: return false;
   }
 }
 
@@ -274,10 +266,8 @@ bool launch_cols_fixed(const ColJob& J, const FftPlanDev& Pin, const FftPlanDev&
   }
 }
 
-template bool launch_rows_r2c_fixed<double, double>(const RowJob&, const RealPlanDev&, int, size_t, cudaStream_t);
 template bool launch_rows_r2c_fixed<float, float>(const RowJob&, const RealPlanDev&, int, size_t, cudaStream_t);
 template bool launch_rows_r2c_fixed<float, double>(const RowJob&, const RealPlanDev&, int, size_t, cudaStream_t);
-template bool launch_rows_c2r_fixed<double, double>(const RowJob&, const RealPlanDev&, int, size_t, cudaStream_t);
 template bool launch_rows_c2r_fixed<float, float>(const RowJob&, const RealPlanDev&, int, size_t, cudaStream_t);
 template bool launch_rows_c2r_fixed<float, double>(const RowJob&, const RealPlanDev&, int, size_t, cudaStream_t);
 template bool launch_rows_r2c_fixed<dfloat, double>(const RowJob&, const RealPlanDev&, int, size_t, cudaStream_t);
@@ -287,9 +277,6 @@ template bool launch_rows_c2r_fixed<dfloat, dfloat>(const RowJob&, const RealPla
 #define LES_INST_COLS(T, TX, CIn)                                                                   \
   template bool launch_cols_fixed<T, TX, CIn>(const ColJob&, const FftPlanDev&, const FftPlanDev&, \
                                               size_t, dim3, cudaStream_t);
-LES_INST_COLS(double, 2, double2)
-LES_INST_COLS(double, 4, double2)
-LES_INST_COLS(double, 8, double2)
 LES_INST_COLS(float, 4, float2)
 LES_INST_COLS(float, 8, float2)
 LES_INST_COLS(float, 16, float2)

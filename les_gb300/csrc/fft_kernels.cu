@@ -16,7 +16,10 @@ int launch_rows_r2c(const RowJob& J, const RealPlanDev& P, cudaStream_t s) {
   JJ.dnc = FastDiv((unsigned)J.ncols);
   dim3 grid((J.ny + rpc - 1) / rpc, J.nlev, J.nfield);
   const bool pr = g_prof && prof_mark(sizeof(T) == 8 ? PROF_ROWS64 : PROF_ROWS32, s);
-  if (!launch_rows_r2c_fixed<T, TIn>(JJ, P, rpc, sm, s)) {
+  bool done = false;
+  if constexpr (std::is_same<T, double>::value) done = launch_rows_r2c_int(JJ, P, s);
+  else done = launch_rows_r2c_fixed<T, TIn>(JJ, P, rpc, sm, s);
+  if (!done) {
     static size_t sm_set = 48 * 1024;  // opt-in raised once per instantiation (not during capture)
     if (sm > sm_set) {
       cudaFuncSetAttribute(k_rows_r2c<T, TIn, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -38,7 +41,10 @@ int launch_rows_c2r(const RowJob& J, const RealPlanDev& P, cudaStream_t s) {
   const size_t sm = (size_t)rpc * ((m + 1) + 2 * m) * sizeof(C);
   dim3 grid((J.ny + rpc - 1) / rpc, J.nlev, J.nfield);
   const bool pr = g_prof && prof_mark(sizeof(T) == 8 ? PROF_ROWS64 : PROF_ROWS32, s);
-  if (!launch_rows_c2r_fixed<T, TOut>(J, P, rpc, sm, s)) {
+  bool done = false;
+  if constexpr (std::is_same<T, double>::value) done = launch_rows_c2r_int(J, P, s);
+  else done = launch_rows_c2r_fixed<T, TOut>(J, P, rpc, sm, s);
+  if (!done) {
     static size_t sm_set = 48 * 1024;  // opt-in raised once per instantiation (not during capture)
     if (sm > sm_set) {
       cudaFuncSetAttribute(k_rows_c2r<T, TOut, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -59,7 +65,10 @@ static int launch_cols_tx(const ColJob& J, const FftPlanDev& Pin, const FftPlanD
   const size_t sm = (size_t)(J.nin * J.ny_in + 2 * nymax) * TX * sizeof(C);
   dim3 grid((J.ncols + TX - 1) / TX, J.nlev, J.nf > 0 ? J.nf : 1);
   const bool pr = g_prof && prof_mark(sizeof(T) == 8 ? PROF_COLS64 : PROF_COLS32, s);
-  if (!launch_cols_fixed<T, TX, CIn>(J, Pin, Pout, sm, grid, s)) {
+  bool done = false;
+  if constexpr (std::is_same<T, double>::value) done = launch_cols_int(J, Pin, Pout, s);
+  else done = launch_cols_fixed<T, TX, CIn>(J, Pin, Pout, sm, grid, s);
+  if (!done) {
     static size_t sm_set = 48 * 1024;  // opt-in raised once per instantiation (not during capture)
     if (sm > sm_set) {
       cudaFuncSetAttribute(k_cols<T, TX, CIn>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);

@@ -53,6 +53,13 @@ static float4 ff_pair(long double re, long double im) {
   const float rh = (float)re, ih = (float)im;
   return make_float4(rh, (float)(re - (long double)rh), ih, (float)(im - (long double)ih));
 }
+// (re, im) in 62 fractional bits, each as a signed high and a signed low word
+static int4 fix_pair(long double re, long double im) {
+  const long double one = 4611686018427387904.0L;
+  const long long r = llrintl(re * one), i = llrintl(im * one);
+  const int rl = (int)(unsigned)((unsigned long long)r & 0xffffffffull), il = (int)(unsigned)((unsigned long long)i & 0xffffffffull);
+  return make_int4((int)((r - rl) >> 32), rl, (int)((i - il) >> 32), il);
+}
 // Stockham plan for a complex FFT of length n: radix 4, then 2, then 3.
 // Twiddles exp(-2 pi i k r / (Ns R)) are evaluated in long double.
 static int make_plan(les_ctx* c, int n, HostPlan& hp) {
@@ -107,6 +114,18 @@ static int make_plan(les_ctx* c, int n, HostPlan& hp) {
     LES_CUDA_CHECK(cudaMemcpy(hp.devud, ud.data(), ud.size() * sizeof(float4), cudaMemcpyHostToDevice));
     P.unitf = static_cast<const float2*>(hp.devuf);
     P.unitd = static_cast<const float4*>(hp.devud);
+    // no table: the integer-pipe launchers decline (see ref_rounding)
+    if (!(c->cfg.model == 3 && ref_rounding_grid(c->g))) {
+      std::vector<int4> ui(n);
+      for (int mm = 0; mm < n; ++mm) {
+        const long double ang = -2.0L * 3.14159265358979323846264338327950288L * mm / (long double)n;
+        ui[mm] = fix_pair(cosl(ang), sinl(ang));
+      }
+      LES_CUDA_CHECK(cudaMalloc(&hp.devui, ui.size() * sizeof(int4)));
+      c->allocs.push_back(hp.devui);
+      LES_CUDA_CHECK(cudaMemcpy(hp.devui, ui.data(), ui.size() * sizeof(int4), cudaMemcpyHostToDevice));
+      P.uniti = static_cast<const int4*>(hp.devui);
+    }
   }
   LES_CUDA_CHECK(cudaMalloc(&hp.dev, tw.size() * sizeof(double2)));
   c->allocs.push_back(hp.dev);
@@ -131,11 +150,17 @@ static int make_real_plan(les_ctx* c, int nx, HostRealPlan& rp) {
   rp.r.dm1 = FastDiv((unsigned)(m + 1));
   std::vector<double2> w(m + 1);
   std::vector<float4> wd(m + 1);
+  std::vector<int4> wi(m + 1);
   for (int k = 0; k <= m; ++k) {
     const long double ang = -2.0L * 3.14159265358979323846264338327950288L * k / (long double)nx;
     w[k] = make_double2((double)cosl(ang), (double)sinl(ang));
     wd[k] = ff_pair(cosl(ang), sinl(ang));
+    wi[k] = fix_pair(cosl(ang), sinl(ang));
   }
+  LES_CUDA_CHECK(cudaMalloc(&rp.devi, wi.size() * sizeof(int4)));
+  c->allocs.push_back(rp.devi);
+  LES_CUDA_CHECK(cudaMemcpy(rp.devi, wi.data(), wi.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  rp.r.wi = static_cast<const int4*>(rp.devi);
   LES_CUDA_CHECK(cudaMalloc(&rp.devd, wd.size() * sizeof(float4)));
   c->allocs.push_back(rp.devd);
   LES_CUDA_CHECK(cudaMemcpy(rp.devd, wd.data(), wd.size() * sizeof(float4), cudaMemcpyHostToDevice));

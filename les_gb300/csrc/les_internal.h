@@ -15,6 +15,12 @@ int launch_rows_c2r(const RowJob& J, const RealPlanDev& P, cudaStream_t s);
 template <typename T, typename CIn>
 int launch_cols(const ColJob& J, const FftPlanDev& Pin, const FftPlanDev& Pout, cudaStream_t s);
 
+// FP64 transforms on the integer pipe (fft_int_rows.cu, fft_int_cols.cu):
+// false when the job's length has no instantiation
+bool launch_rows_r2c_int(const RowJob& J, const RealPlanDev& P, cudaStream_t s);
+bool launch_rows_c2r_int(const RowJob& J, const RealPlanDev& P, cudaStream_t s);
+bool launch_cols_int(const ColJob& J, const FftPlanDev& Pin, const FftPlanDev& Pout, cudaStream_t s);
+
 // Host-side FFT plan: owns the device twiddle table.
 struct HostPlan {
   FftPlanDev c{};
@@ -23,12 +29,14 @@ struct HostPlan {
   void* devd = nullptr;  // float-float twiddles (float4)
   void* devuf = nullptr;  // unit-circle tables (float2, float4)
   void* devud = nullptr;
+  void* devui = nullptr;  // 62-bit unit-circle table (int4)
 };
 struct HostRealPlan {
   RealPlanDev r{};
   double2* dev = nullptr;
   float2* devf = nullptr;
   void* devd = nullptr;
+  void* devi = nullptr;
 };
 
 // Grid constants computed once on the host in the reference's expression
@@ -40,6 +48,16 @@ struct Grid {
   size_t C, CB;  // complex entries of a small x-spectrum plane (ny*lh) and a
                  // big truncated one (ny2*(nx/2))
 };
+
+// Grids on which results that cancel down to rounding level are held to the
+// reference's own roundings (the routine press_stag_array on an already
+// projected velocity, model 2's plane-sum ratio, and model 3, whose quintic
+// amplifies rounding 10^7-fold): there the FP64 transform kernels run, which
+// round as the reference's transforms do.  The integer-pipe transforms are
+// closer to the exact result (32^3 pressure gradient: 1.3e-12 of it against
+// the reference's and the FP64 kernels' 3.1e-11; rmsdiv after the projection
+// 0.39 of theirs) and run everywhere else.
+inline bool ref_rounding_grid(const Grid& g) { return g.nx <= 32 && g.ny <= 32; }
 
 }  // namespace les
 
@@ -101,6 +119,7 @@ struct les_ctx {
   std::vector<void*> allocs;
   double rmsdiv_last = 0.0;
   int status_flags = 0;
+  bool fp64_kernels = false;    // the transforms of the op in progress run on the FP64 kernels
   // launch shapes chosen by the autotuner (0: built-in defaults)
   int tx64 = 0, tx32 = 0;       // kx columns per CTA of the y-pass kernels
   int rpc_scale = 0;            // rows per CTA of the x-pass kernels: default * 2^rpc_scale
@@ -114,6 +133,14 @@ struct les_ctx {
 };
 
 namespace les {
+// for the length of an op: FP64 transform kernels on ref_rounding_grid grids
+struct RefRounding {
+  les_ctx* c;
+  explicit RefRounding(les_ctx* c_) : c(c_) { c->fp64_kernels = ref_rounding_grid(c->g); }
+  ~RefRounding() { c->fp64_kernels = false; }
+  RefRounding(const RefRounding&) = delete;
+  RefRounding& operator=(const RefRounding&) = delete;
+};
 // An FP32-mixed context (precision 1) holds these SGS intermediates in FP32:
 // the horizontal velocity and theta gradients (FP32 transforms), S_ij, Nu_t
 // and tau_ij.  Each keeps its FP64 allocation and (ld, ny, nz) layout; the FP32

@@ -84,7 +84,9 @@ static int r2cT(les_ctx* c, int nf, int nlev, const TIn* const* in, long pstride
       J.div[f] = div ? div[f0 + f] : 0.0;
       J.off[f] = off ? off[f0 + f] : nullptr;
     }
-    launch_rows_r2c<T, TIn>(J, big ? c->rxb.r : c->rx.r, c->stream);
+    RealPlanDev P = big ? c->rxb.r : c->rx.r;
+    if (c->fp64_kernels) P.c.uniti = nullptr;
+    launch_rows_r2c<T, TIn>(J, P, c->stream);
   }
   return 0;
 }
@@ -111,7 +113,9 @@ static int c2rT(les_ctx* c, int nf, int nlev, void* ws, TOut* const* out, long p
       J.div[f] = 0.0;
       J.off[f] = off ? off[f0 + f] : nullptr;
     }
-    launch_rows_c2r<T, TOut>(J, big ? c->rxb.r : c->rx.r, c->stream);
+    RealPlanDev P = big ? c->rxb.r : c->rx.r;
+    if (c->fp64_kernels) P.c.uniti = nullptr;
+    launch_rows_c2r<T, TOut>(J, P, c->stream);
   }
   return 0;
 }
@@ -147,8 +151,9 @@ template <typename T, typename CIn>
 static int colsT(les_ctx* c, const ColJob& J0) {
   ColJob J = J0;
   J.tx = sizeof(T) == 8 ? c->tx64 : c->tx32;
-  const FftPlanDev& Pin = (J.ny_in == c->g.ny) ? c->cy.c : c->cyb.c;
-  const FftPlanDev& Pout = (J.ny_out == c->g.ny) ? c->cy.c : c->cyb.c;
+  FftPlanDev Pin = (J.ny_in == c->g.ny) ? c->cy.c : c->cyb.c;
+  FftPlanDev Pout = (J.ny_out == c->g.ny) ? c->cy.c : c->cyb.c;
+  if (c->fp64_kernels) Pin.uniti = Pout.uniti = nullptr;
   return launch_cols<T, CIn>(J, Pin, Pout, c->stream);
 }
 static int cols(les_ctx* c, const ColJob& J) { return colsT<double, double2>(c, J); }
@@ -1878,6 +1883,7 @@ int op_lagrange_ssim(les_ctx* c, const double* const* S) {
 // k_sd_prep G_test-filtered, then k_sd_final with beta = 1 and
 // delta = (dx dy dz)^(1/3) (std_dynamic.f90:28)
 int op_stddyn(les_ctx* c, double* cs_z, const double* const* S) {
+  const RefRounding scope(c);
   const Grid& g = c->g;
   Ptr6 Sp;
   for (int q = 0; q < 6; ++q) Sp.p[q] = S[q];
@@ -3141,7 +3147,10 @@ static int pressT(les_ctx* c, double* p, double* dpdx, double* dpdy, const float
   fill(c, p + (size_t)nz * g.nplane, g.nplane, LES_BOGUS);
   return 0;
 }
-int op_press(les_ctx* c, double* p, double* dpdx, double* dpdy) { return pressT<double>(c, p, dpdx, dpdy); }
+int op_press(les_ctx* c, double* p, double* dpdx, double* dpdy) {
+  const RefRounding scope(c);
+  return pressT<double>(c, p, dpdx, dpdy);
+}
 
 // tridag_array.f90:1-109 with caller-supplied coefficients (per-routine entry)
 __global__ void k_tridag_generic(const double* a, const double* b, const double* cc, const C2* r, C2* u,

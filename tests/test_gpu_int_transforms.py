@@ -1,0 +1,146 @@
+"""FP64 plane transforms on the integer pipe (fft_int_rows.cu, fft_int_cols.cu)
+at every length they are instantiated for, against the same transforms in
+extended precision.
+
+Tolerances, relative L2 over the planes, set before the first run: a pass
+rounds its result to FP64 once (2^-53 of each value at most) and carries an
+error of at most a few units of 2^-55 of the row's largest value, so one plane
+transform (two passes) stays below 4 x 2^-53 = 4.4e-16 and a round trip with
+its derivative below 8 x 2^-53.
+"""
+import numpy as np
+import pytest
+
+import les_gb300 as lg
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -53
+
+# (nx, ny): x half lengths 16..192 of the small and 3/2 grids, y lengths 16..384
+GRIDS = [(32, 16), (48, 24), (72, 36), (64, 32), (96, 48), (144, 72), (128, 64), (192, 96), (256, 128), (216, 108),
+         (32, 144), (36, 192), (144, 216), (64, 256), (256, 288), (128, 384)]
+
+
+def rel(a, b):
+    a, b = a.astype(np.clongdouble), b.astype(np.clongdouble)
+    return float(np.linalg.norm((a - b).ravel()) / np.linalg.norm(b.ravel()))
+
+
+@pytest.fixture(scope="module")
+def ctx_of(gpu_lib):
+    made = {}
+
+    def get(nx, ny):
+        if (nx, ny) not in made:
+            cfg = lg.make_config(nx, ny, 4, rmsdiv_every=0)
+            made[nx, ny] = lg.Context(cfg, lg.uniform_surface(cfg))
+        return made[nx, ny]
+    yield get
+    for c in made.values():
+        c.close()
+
+
+def planes(kind, n, ny, nx, seed):
+    """Values the path meets: a mean with small fluctuations, white noise, a single point, a steep field."""
+    g = np.random.default_rng(seed)
+    if kind == "wind":
+        return 13.0 + 0.1 * g.standard_normal((n, ny, nx))
+    if kind == "point":
+        f = np.zeros((n, ny, nx))
+        f[:, ny // 3, nx // 5] = 1.7
+        return f
+    if kind == "steep":
+        f = g.standard_normal((n, ny, nx))
+        return f * np.exp(-np.arange(nx) / 3.0)[None, None, :]
+    return g.standard_normal((n, ny, nx))
+
+
+@pytest.mark.parametrize("nx,ny", GRIDS)
+@pytest.mark.parametrize("kind", ["wind", "noise", "point", "steep"])
+def test_plane_transforms(ctx_of, nx, ny, kind):
+    c = ctx_of(nx, ny)
+    for big in (0, 1):
+        mx, my = (3 * nx // 2, 3 * ny // 2) if big else (nx, ny)
+        f = planes(kind, 3, my, mx, nx + ny)
+        want = np.fft.rfft2(f.astype(np.longdouble))
+        a = np.zeros((3, my, mx + 2))
+        a[:, :, :mx] = f
+        c.call("fft_r2c", a, ints=(3, big))
+        assert rel(a.view(np.complex128), want) < 4 * EPS
+        # back from the rounded spectrum: the exact inverse of what the routine is given
+        h = a.view(np.complex128).astype(np.clongdouble)
+        back = np.fft.irfft2(h, s=(my, mx)) * (mx * my)
+        c.call("fft_c2r", a, ints=(3, big))
+        assert rel(a[:, :, :mx], back) < 4 * EPS
+
+
+@pytest.mark.parametrize("nx,ny", GRIDS)
+def test_derivatives_and_filter(ctx_of, nx, ny):
+    c = ctx_of(nx, ny)
+    f = planes("wind", 2, ny, nx, 5 * nx + ny)
+    h = np.fft.rfft2(f.astype(np.longdouble))
+    h[:, ny // 2, :] = 0
+    h[:, :, -1] = 0
+    kx = np.arange(nx // 2 + 1).astype(np.longdouble)[None, None, :]
+    ky = (((np.arange(ny) + ny // 2) % ny) - ny // 2).astype(np.longdouble)[None, :, None]
+    a = np.zeros((2, ny, nx + 2))
+    a[:, :, :nx] = f
+    dx, dy = np.zeros_like(a), np.zeros_like(a)
+    c.call("filt_da", a, dx, dy, ints=(2,))
+    want = np.fft.irfft2(h, s=(ny, nx))
+    assert rel(a[:, :, :nx], want) < 8 * EPS
+    # derivatives of wind + noise: the error is that of the largest value transformed times the wavenumber
+    scale = np.linalg.norm(want) * float(max(nx, ny)) / 2
+    for got, k in ((dx, kx), (dy, ky)):
+        w = np.fft.irfft2(1j * k * h, s=(ny, nx))
+        assert np.linalg.norm((got[:, :, :nx].astype(np.longdouble) - w).ravel()) < 8 * EPS * scale
+        assert np.all(got[:, :, nx:] == 0.0)
+
+
+@pytest.mark.parametrize("nx,ny", [(32, 16), (48, 24), (64, 32), (96, 48), (144, 72), (128, 64), (192, 96), (256, 128),
+                                   (32, 144), (36, 192), (64, 256)])
+def test_padding_and_truncation(ctx_of, nx, ny):
+    c = ctx_of(nx, ny)
+    mx, my = 3 * nx // 2, 3 * ny // 2
+    f = planes("noise", 2, ny, nx, 7 * nx + ny)
+    h = np.fft.rfft2(f.astype(np.longdouble)) / (nx * ny)
+    h[:, ny // 2, :] = 0
+    h[:, :, -1] = 0
+    hb = np.zeros((2, my, mx // 2 + 1), dtype=np.clongdouble)
+    hb[:, :ny // 2, :nx // 2] = h[:, :ny // 2, :nx // 2]
+    hb[:, my - ny // 2 + 1:, :nx // 2] = h[:, ny // 2 + 1:, :nx // 2]
+    want = np.fft.irfft2(hb, s=(my, mx)) * (mx * my)
+    a, big, back = np.zeros((2, ny, nx + 2)), np.zeros((2, my, mx + 2)), np.zeros((2, ny, nx + 2))
+    a[:, :, :nx] = f
+    c.call("dealias1", a, big, ints=(2,))
+    assert rel(big[:, :, :mx], want) < 8 * EPS
+    c.call("dealias2", back, big, ints=(2,))
+    assert rel(back[:, :, :nx], np.fft.irfft2(h, s=(ny, nx)) * (nx * ny)) < 16 * EPS
+
+
+@pytest.mark.parametrize("nx,ny", [(64, 32), (96, 48), (256, 256)])
+def test_range_ends(ctx_of, nx, ny):
+    """Zero planes, values near both ends of the FP64 range, and not-a-number or infinity in one plane of several."""
+    c = ctx_of(nx, ny)
+    g = np.random.default_rng(3)
+    f = g.standard_normal((2, ny, nx))
+    want = np.fft.rfft2(f.astype(np.longdouble))
+    for scale in (2.0 ** -1010, 2.0 ** -900, 2.0 ** 900, 2.0 ** 1000):
+        a = np.zeros((2, ny, nx + 2))
+        a[:, :, :nx] = f * scale
+        c.call("fft_r2c", a, ints=(2, 0))
+        got = a.view(np.complex128).astype(np.clongdouble) / np.longdouble(scale)
+        # 2^-1010: sums of a few hundred such values; their last bits are subnormal units of 2^-1074
+        tol = 4 * EPS if scale > 2.0 ** -1000 else 2.0 ** -50
+        assert rel(got, want) < tol
+    a = np.zeros((3, ny, nx + 2))
+    c.call("fft_r2c", a, ints=(3, 0))
+    assert np.all(a == 0.0)
+    for bad in (np.nan, np.inf, -np.inf):
+        a = np.zeros((3, ny, nx + 2))
+        a[0, :, :nx], a[2, :, :nx] = f[0], f[1]
+        a[1, 3, 5] = bad
+        c.call("fft_r2c", a, ints=(3, 0))
+        s = a.view(np.complex128)
+        assert not np.any(np.isfinite(s[1].real)) and np.all(np.isfinite(s[[0, 2]]))
+        assert rel(s[[0, 2]], want) < 4 * EPS
