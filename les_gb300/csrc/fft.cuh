@@ -413,6 +413,8 @@ struct RowJob {
   const double* off[JOB_MAXF];  // per-plane offsets: r2c subtracts off[plane] before
                                 // scaling, c2r adds it to the output (null: none)
   int rpc;                      // rows per CTA (0: default for the size)
+  unsigned char deriv[JOB_MAXF];  // c2r, integer-pipe kernels: i kx times the spectrum (kx = 0 at nx/2)
+  double kunit;                 // unit of kx (deriv)
   FastDiv dnc;                  // ncols
 };
 

@@ -7,19 +7,23 @@
 // (58 per clock per SM measured), a product with a twiddle is three
 // 32 x 32 -> 64-bit multiply-adds per real product (27 per clock), and the
 // same butterfly costs 0.4 clocks.  The FP64 pipe only converts: one
-// instruction per value on the way in and one on the way out (1.9 per clock).
+// instruction per value on the way out (1.9 per clock).
 //
 // Measured against the FP64 kernels (256^2 planes): field and derivatives of
-// 64 planes (les_filt_da) 1122 -> 335 us, FP64 step at 256^3 89.1 -> 31.6 ms.
+// 64 planes (les_filt_da) 1122 -> 200 us, FP64 step at 256^3 89.1 -> 22.0 ms.
+// What bounds them is instruction issue at 16 warps per SM (128 registers):
+// 42 to 46 % of the issue slots and half of the integer pipe are busy.
 //
 // Precision.  A value is a multiple of 2^ex with |value / 2^ex| < 2^61, so a
 // row's largest elements carry 55 to 60 bits (an FP64 number: 53) and
 // all others the same absolute resolution; a transform's error is set by its
 // largest inputs in FP64 arithmetic as well.  The scale is chosen from the
-// data three times per transform: from the row's largest exponent at the
-// load, from a bound on the partial sums before the first butterflies of an
-// inverse, and from the largest value between the two steps; each choice
-// leaves the headroom the following step can need, so nothing overflows.
+// data: from the row's largest exponent at the load, for an inverse from the
+// sums of moduli of its first butterflies (a spectrum that one mode dominates
+// keeps its full width), and from the largest value between the two steps
+// (the inverse x pass instead takes the sum of all moduli, which bounds both
+// steps).  Each choice leaves the headroom that the following step can need,
+// so nothing overflows.
 // Twiddles are rounded to 62 fractional bits.  Against extended precision
 // (noise, and a mean wind of 170 times the noise, 32^2 to 256^2) the relative
 // error is 0.25 to 0.75 of the FP64 kernels' in the field, its derivatives and
@@ -238,38 +242,69 @@ __device__ __forceinline__ unsigned fix_mag(double x) { return (unsigned)__doubl
 // exponent of the scale that brings values of high-word magnitude up to m
 // below 2^bits (0 for a zero row, which stays zero)
 __device__ __forceinline__ int fix_shift(unsigned m, int bits) { return m ? bits + 1022 - (int)(m >> 20) : 0; }
-__device__ __forceinline__ i64 fix_of(double x, int s20) {  // x 2^s, s20 = s << 20
-  const int hi = __double2hiint(x);
-  const int e = max((hi & 0x7fffffff) + s20, 0);
-  return __double2ll_rn(__hiloint2double(e | (hi & (int)0x80000000), __double2loint(x)));
+// x 2^s, truncated, on the integer pipe (the FP64 pipe's conversion would
+// bound these kernels: 81 % busy with it).  c = 1082 - s; the scale keeps the
+// result below 2^60, and zeros and subnormals fall to zero by their exponent.
+__device__ __forceinline__ i64 fix_of(double x, int c) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const int d = min(c - (int)((hi >> 20) & 0x7ffu), 63);
+  unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32) | lo;
+  m = (m << 7) >> d;
+  const i64 sg = (i64)((int)hi >> 31);
+  return ((i64)m ^ sg) - sg;
+}
+// x k 2^s for an integer k < 2^8 (the product is exact before the
+// truncation); e1 = 1077 - s, the result below 2^56
+__device__ __forceinline__ i64 fix_times(double x, unsigned k, int e1) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const int d = min(e1 - (int)((hi >> 20) & 0x7ffu), 63);
+  unsigned long long m = (unsigned long long)mad_wu(lo, k, 0) +
+                         ((unsigned long long)(((hi & 0xfffffu) | 0x100000u) * k) << 32);
+  m = (m << 2) >> d;
+  const i64 sg = (i64)((int)hi >> 31);
+  return ((i64)m ^ sg) - sg;
 }
 __device__ __forceinline__ double fix_pow2(int e) {  // 2^e, -1022 <= e <= 1023
   return __hiloint2double((e + 1023) << 20, 0);
 }
-// v 2^ex factor: the exponent added to the converted value when the factor is
-// 1 (FP64 pipe: one operation), else one product (two outside the usual range)
-struct FixOut {
-  double f1, f2;
-  int e20;
-  bool plain, two;
-  __device__ __forceinline__ FixOut(int ex, double factor) {
-    const int e1 = min(max(ex, -960), 900);
-    plain = factor == 1.0 && e1 == ex;
-    two = e1 != ex;
-    e20 = e1 * (1 << 20);
-    f1 = factor * fix_pow2(e1);
-    f2 = two ? fix_pow2(min(max(ex - e1, -1022), 1023)) : 1.0;
+// v 2^ex factor for N pairs, in place of the integers.  A power of two joins
+// the exponent, so that the FP64 pipe has the conversion alone; any other
+// factor costs one product more (two near the ends of the FP64 range).
+template <int N, int NV>
+__device__ __forceinline__ void fix_out(const cfix (&v)[NV], double2 (&o)[N], int ex, double factor) {
+  const int fh = __double2hiint(factor);
+  if (__double2loint(factor) == 0 && (fh & 0x800fffff) == 0 && fh >= (1 << 20)) {
+    ex += (fh >> 20) - 1023;
+    factor = 1.0;
   }
-  __device__ __forceinline__ double operator()(i64 v) const {
-    double r = __ll2double_rn(v);
-    if (plain) {
-      const int hi = __double2hiint(r);
-      return __hiloint2double(hi ? hi + e20 : 0, __double2loint(r));
+  const int e1 = min(max(ex, -960), 900);
+  if (factor == 1.0 && e1 == ex) {
+    const int e20 = ex * (1 << 20);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      o[i].x = __ll2double_rn(v[i].x);
+      o[i].y = __ll2double_rn(v[i].y);
+      const int hx = __double2hiint(o[i].x), hy = __double2hiint(o[i].y);
+      o[i].x = __hiloint2double(hx ? hx + e20 : 0, __double2loint(o[i].x));
+      o[i].y = __hiloint2double(hy ? hy + e20 : 0, __double2loint(o[i].y));
     }
-    r *= f1;
-    return two ? r * f2 : r;
+  } else {
+    const double f1 = factor * fix_pow2(e1);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      o[i].x = __ll2double_rn(v[i].x) * f1;
+      o[i].y = __ll2double_rn(v[i].y) * f1;
+    }
+    if (e1 != ex) {
+      const double f2 = fix_pow2(min(max(ex - e1, -1022), 1023));
+#pragma unroll
+      for (int i = 0; i < N; ++i) { o[i].x *= f2; o[i].y *= f2; }
+    }
   }
-};
+}
+__device__ __forceinline__ double nan_if(bool bad, double f) {
+  return bad ? __longlong_as_double(0x7ff8000000000000ll) : f;
+}
 __device__ __forceinline__ i64 fix_shr(i64 v, int s, i64 rnd) { return (v + rnd) >> s; }
 __device__ __forceinline__ i64 fix_rnd(int s) { return (1ll << s) >> 1; }
 __device__ __forceinline__ unsigned fix_top(i64 v) {  // magnitude of the high word (one's complement)
@@ -278,9 +313,11 @@ __device__ __forceinline__ unsigned fix_top(i64 v) {  // magnitude of the high w
 }
 // right shift that brings values of high-word magnitude m below 2^bits
 __device__ __forceinline__ int fix_down(unsigned m, int bits) { return max(64 - __clz((int)m) - bits, 0); }
-// the same for a sum of moduli below sum 2^44, to below 2^60
-__device__ __forceinline__ int fix_down_sum(unsigned sum) { return max(32 - __clz((int)sum) - 16, 0); }
-// a bound on |x| + |y| in units of 2^44
-__device__ __forceinline__ unsigned fix_l1(cfix v) { return ((fix_top(v.x) + fix_top(v.y) + 2u) >> 12) + 1u; }
+// the same for a sum of moduli below sum 2^unit, to below 2^60
+__device__ __forceinline__ int fix_down_sum(unsigned sum, int unit) { return max(32 - __clz((int)sum) + unit - 60, 0); }
+// a bound on |x| + |y| in units of 2^(32 + SH)
+template <int SH> __device__ __forceinline__ unsigned fix_l1(cfix v) {
+  return ((fix_top(v.x) + fix_top(v.y) + 2u) >> SH) + 1u;
+}
 
 }  // namespace les

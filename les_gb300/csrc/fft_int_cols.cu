@@ -9,7 +9,8 @@
 //
 // Outputs that only drop the Nyquist row (filt_da's field) or multiply by
 // the column's kx need no transform at all in y: the field less its
-// alternating sum, sum_y (-1)^y f / ny, is what the round trip gives.
+// alternating sum, sum_y (-1)^y f / ny, is what the round trip gives.  They are
+// written last, from the input again (cached), so that no register holds it.
 #include <algorithm>
 #include "fft_int.cuh"
 #include "les_internal.h"
@@ -69,12 +70,12 @@ __device__ __forceinline__ int col_fix(double2 (&x)[NV], cfix (&v)[NV], unsigned
     for (int i = 0; i < CNT; ++i) m = max(m, max(fix_mag(x[i].x), fix_mag(x[i].y)));
     m = col_max<TX>(m, slots + TX, b);
   }
-  const int s = fix_shift(m, bits), s20 = s * (1 << 20);
+  const int s = fix_shift(m, bits), c = 1082 - s;
   bad = bad || m >= 0x7ff00000u;
 #pragma unroll
   for (int i = 0; i < CNT; ++i) {
-    v[i].x = fix_of(x[i].x, s20);
-    v[i].y = fix_of(x[i].y, s20);
+    v[i].x = fix_of(x[i].x, c);
+    v[i].y = fix_of(x[i].y, c);
   }
   return -s - pre;
 }
@@ -108,7 +109,9 @@ __device__ __forceinline__ void col_fwd(cfix (&v)[NV], cfix* S, unsigned* slot, 
   }
 }
 // inverse: v[k1] = X[q + N2 k1], sums of N1 moduli below 2^60, to
-// v[n2] = x[q + N1 n2]
+// v[n2] = x[q + N1 n2].  (One bound from the whole column's sum would save
+// the second shift, 2 % of a step, but leaves 256 to 384 values of noise four
+// bits fewer: 3/2 round trip at 256^2 4.2e-16 against 1.6e-16.)
 template <int N1, int N2, int TX, int NV>
 __device__ __forceinline__ void col_inv(cfix (&v)[NV], cfix* S, unsigned* slot, const int4* __restrict__ tw, int q, int b,
                                         int& ex) {
@@ -135,15 +138,16 @@ __device__ __forceinline__ void col_inv(cfix (&v)[NV], cfix* S, unsigned* slot, 
     fdft<N2, 1>(v);
   }
 }
-// the sums of moduli below 2^60 that col_inv needs
+// the sums of moduli below 2^60 that col_inv needs: a thread's values, up to
+// 24 with weights up to 192, stay below 2^31 units of 2^44
 template <int N1, int N2, int TX, int NV>
 __device__ __forceinline__ void col_room(cfix (&v)[NV], unsigned* slot, int q, int b, int& ex) {
   unsigned sum = 0;
   if (q < N2) {
 #pragma unroll
-    for (int i = 0; i < N1; ++i) sum += fix_l1(v[i]);
+    for (int i = 0; i < N1; ++i) sum += fix_l1<12>(v[i]);
   }
-  const int s = fix_down_sum(col_max<TX>(sum, slot, b));
+  const int s = fix_down_sum(col_max<TX>(sum, slot, b), 44);
   const i64 rnd = fix_rnd(s);
   ex += s;
 #pragma unroll
@@ -152,57 +156,69 @@ __device__ __forceinline__ void col_room(cfix (&v)[NV], unsigned* slot, int q, i
     v[i].y = fix_shr(v[i].y, s, rnd);
   }
 }
-// i ky X with ky = k - (k >= N/2) N as an integer (its unit is a factor of
-// the output), with the same bound; `neg`: -i ky.  The products are exact
-// 96-bit integers before the shift.
+// the same for w(k) v with integer weights: 0 or 1, or (sgn) |ky| as an
+// integer, negative wavenumbers (i >= N1/2) changing sign.  The products are
+// exact 96-bit integers before the shift.
 template <int N1, int N2, int TX, int NV>
-__device__ __forceinline__ void col_iky(cfix (&v)[NV], unsigned* slot, int q, int b, bool zero, bool neg, int& ex) {
-  constexpr int N = N1 * N2;
+__device__ __forceinline__ void col_weigh(cfix (&v)[NV], const unsigned (&w)[N1], bool sgn, unsigned* slot, int q, int b,
+                                          int& ex) {
   unsigned sum = 0;
-  if (q < N2 && !zero) {
 #pragma unroll
-    for (int i = 0; i < N1; ++i) {
-      const int k = q + N2 * i;
-      const unsigned m = i < N1 / 2 ? k : N - k;
-      if (k != N / 2) sum += fix_l1(v[i]) * m;
-    }
-  }
-  const int s = fix_down_sum(col_max<TX>(sum, slot, b));
+  for (int i = 0; i < N1; ++i)
+    if (w[i]) sum += fix_l1<12>(v[i]) * w[i];
+  const int s = fix_down_sum(col_max<TX>(sum, slot, b), 44);
   const i64 rnd = fix_rnd(s);
+  const i64 flip = sgn ? -1 : 0;
   ex += s;
 #pragma unroll
   for (int i = 0; i < N1; ++i) {
-    const int k = q + N2 * i;
-    unsigned m = i < N1 / 2 ? k : N - k;
-    if (k == N / 2 || zero || q >= N2) m = 0;
-    const i64 lx = mad_wu((unsigned)v[i].x, m, rnd), ly = mad_wu((unsigned)v[i].y, m, rnd);
-    const i64 hx = mad_w((int)(v[i].x >> 32), (int)m, (i64)((unsigned long long)lx >> 32));
-    const i64 hy = mad_w((int)(v[i].y >> 32), (int)m, (i64)((unsigned long long)ly >> 32));
+    const i64 lx = mad_wu((unsigned)v[i].x, w[i], rnd), ly = mad_wu((unsigned)v[i].y, w[i], rnd);
+    const i64 hx = mad_w((int)(v[i].x >> 32), (int)w[i], (i64)((unsigned long long)lx >> 32));
+    const i64 hy = mad_w((int)(v[i].y >> 32), (int)w[i], (i64)((unsigned long long)ly >> 32));
     // (h 2^32 + low word) >> s, s < 32
-    const i64 px = (i64)(((unsigned long long)__funnelshift_r((unsigned)hx, (unsigned)(hx >> 32), s) << 32) |
-                         __funnelshift_r((unsigned)lx, (unsigned)hx, s));
-    const i64 py = (i64)(((unsigned long long)__funnelshift_r((unsigned)hy, (unsigned)(hy >> 32), s) << 32) |
-                         __funnelshift_r((unsigned)ly, (unsigned)hy, s));
-    if ((i < N1 / 2) != neg) {  // +i
-      v[i].x = -py;
-      v[i].y = px;
-    } else {
-      v[i].x = py;
-      v[i].y = -px;
+    v[i].x = (i64)(((unsigned long long)__funnelshift_r((unsigned)hx, (unsigned)(hx >> 32), s) << 32) |
+                   __funnelshift_r((unsigned)lx, (unsigned)hx, s));
+    v[i].y = (i64)(((unsigned long long)__funnelshift_r((unsigned)hy, (unsigned)(hy >> 32), s) << 32) |
+                   __funnelshift_r((unsigned)ly, (unsigned)hy, s));
+    if (i >= N1 / 2) {
+      v[i].x = (v[i].x ^ flip) - flip;
+      v[i].y = (v[i].y ^ flip) - flip;
     }
   }
 }
+// weights of ky: |k| or N - |k|, none for the Nyquist row
+template <int N1, int N2> __device__ __forceinline__ void ky_weights(unsigned (&w)[N1], int q, bool zero) {
+  constexpr int N = N1 * N2;
+#pragma unroll
+  for (int i = 0; i < N1; ++i) {
+    const int k = q + N2 * i;
+    w[i] = zero || q >= N2 || k == N / 2 ? 0u : (unsigned)(i < N1 / 2 ? k : N - k);
+  }
+}
 
-__device__ __forceinline__ double nan_if(bool bad, double f) {
-  return bad ? __longlong_as_double(0x7ff8000000000000ll) : f;
+// outputs while the integers stay in use: converted four at a time
+template <int CNT, class V, class St>
+__device__ __forceinline__ void fix_groups(V&& val, St&& store, int ex, double factor) {
+#pragma unroll
+  for (int g = 0; g < CNT; g += 4) {
+    cfix t[4];
+    double2 r[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) t[i] = val(g + i < CNT ? g + i : CNT - 1);
+    fix_out(t, r, ex, factor);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (g + i < CNT) store(g + i, r[i]);
+  }
 }
 __device__ __forceinline__ bool col_direct(const ColJob& J, int o) {  // needs no y transform
   const int code = J.coef[o][0];
   return J.dir == DIR_BOTH && ((J.inv_mask >> o) & 1u) && (code == CC_ONE || code == CC_KILL || code == CC_IKX);
 }
 
-// One input, same length.  ngen: inverse outputs that need a transform.
-template <int N1, int N2, int MB>
+// One input, same length.  DIR: the job's direction; ngen: inverse outputs
+// that need a transform (MULTI: several, the spectrum waits in shared memory).
+template <int N1, int N2, int MB, int DIR, bool MULTI>
 __global__ void __launch_bounds__(ICOL_TX * (N1 > N2 ? N1 : N2), MB)
     k_icol(ColJob J, const int4* __restrict__ tw, int total, int ndirect, int nspec, int ngen) {
   constexpr int TX = ICOL_TX, N = N1 * N2, NV = N1 > N2 ? N1 : N2, NT = TX * NV;
@@ -221,120 +237,125 @@ __global__ void __launch_bounds__(ICOL_TX * (N1 > N2 ? N1 : N2), MB)
   const size_t in0 = (size_t)lev * J.ps_in + (size_t)blockIdx.y * J.fs_in + jx;
   const size_t out0 = (size_t)lev * J.ps_out + (size_t)blockIdx.y * J.fs_out + jx;
   const double2* src = reinterpret_cast<const double2*>(J.in[0]) + in0;
-  const bool fwd = (J.dir & DIR_FWD) != 0;
+  constexpr bool fwd = (DIR & DIR_FWD) != 0;
   const bool last = jx == J.lh - 1;  // kx = nx/2: removed by KILL and by the derivatives
   cfix v[NV];
   int ex;
   bool bad = false;
   {
     double2 x[NV];
-    const int r0 = q, step = fwd ? N1 : N2, cnt = fwd ? N2 : N1;
+    constexpr int step = fwd ? N1 : N2, cnt = fwd ? N2 : N1;
     const bool act = ok && q < step;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       x[i] = make_double2(0.0, 0.0);
-      if (act && i < cnt) x[i] = src[(size_t)(r0 + step * i) * J.wc_in];
+      if (act && i < cnt) x[i] = src[(size_t)(q + step * i) * J.wc_in];
     }
     __syncthreads();  // slots are zero
-    ex = col_fix<TX, NV>(x, v, slots, b, fwd ? fix_in(N2) : 60, bad);
+    ex = col_fix<TX, cnt>(x, v, slots, b, fwd ? fix_in(N2) : 60, bad);
   }
-  if (ndirect) {
-    double cx = 0.0, cy = 0.0;
-    {
-      i64 sx = 0, sy = 0;
+  double ax = 0.0, ay = 0.0;  // (-1)^row times the alternating sum
+  if (DIR == DIR_BOTH && ndirect) {
+    i64 sx = 0, sy = 0;
 #pragma unroll
-      for (int i = 0; i < N2; ++i) { sx += (v[i].x + 2) >> 2; sy += (v[i].y + 2) >> 2; }
-      if (q & 1) { sx = -sx; sy = -sy; }
-      col_sum<TX>(sx, sy, sums, b);
-      cx = (double)sx * (4.0 / N);
-      cy = (double)sy * (4.0 / N);
-    }
-    const i64 ax = __double2ll_rn(q & 1 ? -cx : cx), ay = __double2ll_rn(q & 1 ? -cy : cy);
-    if (ok && q < N1) {
-      for (int o = 0; o < J.nout; ++o) {
-        if (!col_direct(J, o)) continue;
-        const int code = J.coef[o][0];
-        const bool one = code == CC_ONE, ikx = code == CC_IKX;
-        double f = nan_if(bad, ikx ? J.kx[jx] * (double)N : (double)N);
-        if (!one && last) f = 0.0;
-        const FixOut out(ex, f);
-        const i64 bx = one ? 0 : ax, by = one ? 0 : ay;
-        double2* dst = reinterpret_cast<double2*>(J.out[o]) + out0;
+    for (int i = 0; i < N2; ++i) { sx += (v[i].x + 2) >> 2; sy += (v[i].y + 2) >> 2; }
+    if (q & 1) { sx = -sx; sy = -sy; }
+    col_sum<TX>(sx, sy, sums, b);
+    if (q & 1) { sx = -sx; sy = -sy; }
+    const cfix t[1] = {{sx, sy}};
+    double2 r[1];
+    fix_out(t, r, ex + 2, 1.0);
+    ax = nan_if(bad, r[0].x);
+    ay = nan_if(bad, r[0].y);
+  }
+  auto direct = [&]() {
+    if (DIR != DIR_BOTH || ndirect == 0 || !ok || q >= N1) return;
+    for (int o = 0; o < J.nout; ++o) {
+      if (!col_direct(J, o)) continue;
+      const int code = J.coef[o][0];
+      const bool one = code == CC_ONE, ikx = code == CC_IKX;
+      const double f = !one && last ? 0.0 : (ikx ? J.kx[jx] : 1.0);
+      const double fn = f * (double)N, bx = one ? 0.0 : f * ax, by = one ? 0.0 : f * ay;
+      double2* dst = reinterpret_cast<double2*>(J.out[o]) + out0;
 #pragma unroll
-        for (int i = 0; i < N2; ++i) {
-          const double rx = out(v[i].x - bx), ry = out(v[i].y - by);
-          dst[(size_t)(q + N1 * i) * J.wc_out] = ikx ? make_double2(-ry, rx) : make_double2(rx, ry);
-        }
+      for (int i = 0; i < N2; ++i) {  // N f - (-1)^row sum, from the input again
+        const size_t row = (size_t)(q + N1 * i);
+        const double2 a = src[row * J.wc_in];
+        const double rx = fma(fn, a.x, -bx), ry = fma(fn, a.y, -by);
+        dst[row * J.wc_out] = ikx ? make_double2(-ry, rx) : make_double2(rx, ry);
       }
     }
+  };
+  if (nspec + ngen == 0) {
+    direct();
+    return;
   }
-  if (nspec + ngen == 0) return;
-  if (fwd) col_fwd<N1, N2, TX>(v, S, slots + 2 * TX, tw, q, b, ex);
-  if (nspec && ok && q < N2) {
+  if constexpr (fwd) col_fwd<N1, N2, TX>(v, S, slots + 2 * TX, tw, q, b, ex);
+  if (DIR != DIR_INV && nspec && ok && q < N2) {
     for (int o = 0; o < J.nout; ++o) {
       if ((J.inv_mask >> o) & 1u) continue;
       const bool kill = J.coef[o][0] == CC_KILL;
-      const FixOut out(ex, kill && last ? 0.0 : nan_if(bad, 1.0));
       double2* dst = reinterpret_cast<double2*>(J.out[o]) + out0;
-#pragma unroll
-      for (int i = 0; i < N1; ++i) {
+      fix_groups<N1>([&](int i) { return v[i]; }, [&](int i, double2 r) {
         const int k = q + N2 * i;
-        double2 r = make_double2(out(v[i].x), out(v[i].y));
-        if (kill && k == N / 2) r = make_double2(0.0, 0.0);
-        dst[(size_t)k * J.wc_out] = r;
-      }
+        dst[(size_t)k * J.wc_out] = kill && k == N / 2 ? make_double2(0.0, 0.0) : r;
+      }, ex, kill && last ? 0.0 : nan_if(bad, 1.0));
     }
   }
-  if (ngen == 0) return;
-  if (ngen > 1) {
-#pragma unroll
-    for (int i = 0; i < NV; ++i) K[(i * NV + q) * TX + b] = v[i];
+  if (DIR == DIR_FWD || ngen == 0) {
+    direct();
+    return;
   }
   const int ex0 = ex;
-  int done = 0;
-  for (int o = 0; o < J.nout; ++o) {
-    if (!((J.inv_mask >> o) & 1u) || col_direct(J, o)) continue;
-    if (done++ > 0) {
-#pragma unroll
-      for (int i = 0; i < NV; ++i) v[i] = K[(i * NV + q) * TX + b];
-    }
-    ex = ex0;
+  auto output = [&](int o) {
     const int code = J.coef[o][0];
     unsigned* so = slots + (3 + 2 * o) * TX;
     double f = 1.0;
-    bool rot = false;
-    if (code == CC_IKY || code == CC_MIKY) {
-      f = J.ky[J.lh];  // row 1: the unit of ky
-      col_iky<N1, N2, TX>(v, so, q, b, last, code == CC_MIKY, ex);
-    } else {
-      if (code == CC_KILL || code == CC_IKX) {
-        if (code == CC_IKX) { f = J.kx[jx]; rot = true; }
+    const bool iky = code == CC_IKY || code == CC_MIKY, rot = iky || code == CC_IKX;
+    unsigned w[N1];
+    if (iky) {
+      f = code == CC_IKY ? J.ky[J.lh] : -J.ky[J.lh];  // row 1: the unit of ky
+      ky_weights<N1, N2>(w, q, last);
+    } else if (code == CC_ONE || code == CC_KILL || code == CC_IKX) {
+      if (code == CC_IKX) f = J.kx[jx];
 #pragma unroll
-        for (int i = 0; i < N1; ++i)
-          if (last || q + N2 * i == N / 2) v[i].x = v[i].y = 0;
-      } else if (code != CC_ONE) {  // cutoff filters: pass or drop, one common factor
-        const bool wide = code == CC_G || code == CC_MASK;
-        const float* T = wide ? J.Gf : J.GGf;
-        if (code == CC_G || code == CC_GG) f = (wide ? J.G : J.GG)[0];
+      for (int i = 0; i < N1; ++i) w[i] = q >= N2 || (code != CC_ONE && (last || q + N2 * i == N / 2)) ? 0u : 1u;
+    } else {  // cutoff filters: pass or drop, one common factor
+      const bool wide = code == CC_G || code == CC_MASK;
+      const float* T = wide ? J.Gf : J.GGf;
+      if (code == CC_G || code == CC_GG) f = (wide ? J.G : J.GG)[0];
 #pragma unroll
-        for (int i = 0; i < N1; ++i) {
-          const int k = q + N2 * i;
-          if (q < N2 && __ldg(&T[(size_t)J.lh * k + jx]) == 0.f) v[i].x = v[i].y = 0;
-        }
-      }
-      col_room<N1, N2, TX>(v, so, q, b, ex);
+      for (int i = 0; i < N1; ++i)
+        w[i] = q >= N2 || __ldg(&T[(size_t)J.lh * (q + N2 * i) + jx]) == 0.f ? 0u : 1u;
     }
+    col_weigh<N1, N2, TX>(v, w, iky, so, q, b, ex);
     col_inv<N1, N2, TX>(v, S, so + TX, tw, q, b, ex);
     if (ok && q < N1) {
-      const FixOut out(ex, nan_if(bad, f));
       double2* dst = reinterpret_cast<double2*>(J.out[o]) + out0;
+      double2 r[N2];
+      fix_out(v, r, ex, nan_if(bad, f));
 #pragma unroll
-      for (int i = 0; i < N2; ++i) {
-        const double rx = out(v[i].x), ry = out(v[i].y);
-        dst[(size_t)(q + N1 * i) * J.wc_out] = rot ? make_double2(-ry, rx) : make_double2(rx, ry);
-      }
+      for (int i = 0; i < N2; ++i)
+        dst[(size_t)(q + N1 * i) * J.wc_out] = make_double2(rot ? -r[i].y : r[i].x, rot ? r[i].x : r[i].y);
     }
+  };
+  auto general = [&](int o) { return ((J.inv_mask >> o) & 1u) && !col_direct(J, o); };
+  if constexpr (MULTI) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) K[(i * NV + q) * TX + b] = v[i];
+    for (int o = 0; o < J.nout; ++o) {
+      if (!general(o)) continue;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) v[i] = K[(i * NV + q) * TX + b];
+      ex = ex0;
+      output(o);
+    }
+  } else {
+    int o = 0;
+    while (o + 1 < J.nout && !general(o)) ++o;
+    output(o);
   }
+  direct();
 }
 
 // i kx in0 + i ky in1 (the horizontal divergences): in1 makes the round trip;
@@ -384,7 +405,11 @@ __global__ void __launch_bounds__(ICOL_TX * (N1 > N2 ? N1 : N2), MB)
   }
   col_fwd<N1, N2, TX>(v, S, slots + 2 * TX, tw, q, b, ex);
   const bool last = jx == J.lh - 1;
-  col_iky<N1, N2, TX>(v, slots + 3 * TX, q, b, last, false, ex);
+  {
+    unsigned w[N1];
+    ky_weights<N1, N2>(w, q, last);
+    col_weigh<N1, N2, TX>(v, w, true, slots + 3 * TX, q, b, ex);
+  }
   col_inv<N1, N2, TX>(v, S, slots + 4 * TX, tw, q, b, ex);
   if (!act) return;
   double cx = 0.0, cy = 0.0;
@@ -393,14 +418,15 @@ __global__ void __launch_bounds__(ICOL_TX * (N1 > N2 ? N1 : N2), MB)
   const double kx = last ? 0.0 : J.kx[jx], kn = kx * (double)N;
   cx *= q & 1 ? -kx : kx;
   cy *= q & 1 ? -kx : kx;
-  const FixOut out(ex, nan_if(bad, J.ky[J.lh]));
   double2* dst = reinterpret_cast<double2*>(J.out[0]) + (size_t)lev * J.ps_out + (size_t)blockIdx.y * J.fs_out + jx;
+  double2 r[N2];
+  fix_out(v, r, ex, nan_if(bad, J.ky[J.lh]));
 #pragma unroll
   for (int i = 0; i < N2; ++i) {
     const size_t row = (size_t)(q + N1 * i);
     const double2 a = sx[row * J.wc_in];
     // i kx N (a - (-1)^y c / N)
-    dst[row * J.wc_out] = make_double2(fma(-kn, a.y, out(v[i].x) + cy), fma(kn, a.x, out(v[i].y) - cx));
+    dst[row * J.wc_out] = make_double2(fma(-kn, a.y, cy - r[i].y), fma(kn, a.x, r[i].x - cx));
   }
 }
 
@@ -475,9 +501,10 @@ __global__ void __launch_bounds__(ICOL_TX * (PadT<A1, A2, B1, B2, MB>::nv), MB)
   col_room<B1, B2, TX>(v, slots + 3 * TX, q, b, ex);
   col_inv<B1, B2, TX>(v, S, slots + 4 * TX, twb, q, b, ex);
   if (ok && q < B1) {
-    const FixOut out(ex, nan_if(bad, 1.0));
+    double2 r[B2];
+    fix_out(v, r, ex, nan_if(bad, 1.0));
 #pragma unroll
-    for (int i = 0; i < B2; ++i) dst[(size_t)(q + B1 * i) * J.wc_out] = make_double2(out(v[i].x), out(v[i].y));
+    for (int i = 0; i < B2; ++i) dst[(size_t)(q + B1 * i) * J.wc_out] = r[i];
   }
 }
 
@@ -508,9 +535,17 @@ template <int N1, int N2, int MB> bool run_same(const ColJob& J, const FftPlanDe
       }
     }
     const size_t sm = (size_t)(N1 * N2 + (ng > 1 ? NV * NV : 0)) * TX * sizeof(cfix);
-    static size_t set = 40 * 1024;  // the static arrays count too
-    smem_of(k_icol<N1, N2, MB>, sm, set);
-    k_icol<N1, N2, MB><<<grid, NT, sm, s>>>(J, P.uniti, total, nd, ns, ng);
+    auto run = [&](auto kernel, size_t& set) {
+      smem_of(kernel, sm, set);
+      kernel<<<grid, NT, sm, s>>>(J, P.uniti, total, nd, ns, ng);
+    };
+    static size_t set[5] = {40 * 1024, 40 * 1024, 40 * 1024, 40 * 1024, 40 * 1024};  // the static arrays count too
+    if (J.dir == DIR_FWD && ng == 0) run(k_icol<N1, N2, MB, DIR_FWD, false>, set[0]);
+    else if (J.dir == DIR_INV && ns == 0 && ng == 1) run(k_icol<N1, N2, MB, DIR_INV, false>, set[1]);
+    else if (J.dir == DIR_INV && ns == 0) run(k_icol<N1, N2, MB, DIR_INV, true>, set[2]);
+    else if (J.dir == DIR_BOTH && ng <= 1) run(k_icol<N1, N2, MB, DIR_BOTH, false>, set[3]);
+    else if (J.dir == DIR_BOTH) run(k_icol<N1, N2, MB, DIR_BOTH, true>, set[4]);
+    else return false;
     return true;
   }
   // sums: every output i kx of one input plus i ky of another

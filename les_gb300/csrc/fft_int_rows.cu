@@ -5,7 +5,9 @@
 // the N2 second-step transforms dealt out to the lanes, one exchange through
 // shared memory between them.  The Hermitian post- and pre-processing works
 // on the pairs (k, M - k): one twiddle product serves both members and every
-// element is read and written once.
+// element is read and written once.  The blocks of one group of rows in all
+// fields of a job are neighbours, so that a field and its x derivative, which
+// the inverse pass makes from the same spectrum, read it from memory once.
 #include <algorithm>
 #include "fft_int.cuh"
 #include "les_internal.h"
@@ -16,6 +18,11 @@ namespace {
 template <int TT> __device__ __forceinline__ unsigned row_max(unsigned m) {
 #pragma unroll
   for (int o = 1; o < TT; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  return m;
+}
+template <int TT> __device__ __forceinline__ unsigned row_sum(unsigned m) {
+#pragma unroll
+  for (int o = 1; o < TT; o <<= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
   return m;
 }
 // the row's scale: x to integers below 2^bits; returns the exponent of one unit
@@ -39,14 +46,51 @@ __device__ __forceinline__ int row_fix(double2 (&x)[CNT], cfix (&v)[CNT], int bi
     for (int i = 0; i < CNT; ++i) m = max(m, max(fix_mag(x[i].x), fix_mag(x[i].y)));
     m = row_max<TT>(m);
   }
-  const int s = fix_shift(m, bits), s20 = s * (1 << 20);
+  const int s = fix_shift(m, bits), c = 1082 - s;
   bad = bad || m >= 0x7ff00000u;
 #pragma unroll
   for (int i = 0; i < CNT; ++i) {
-    v[i].x = fix_of(x[i].x, s20);
-    v[i].y = fix_of(x[i].y, s20);
+    v[i].x = fix_of(x[i].x, c);
+    v[i].y = fix_of(x[i].y, c);
   }
   return -s - pre;
+}
+
+// the same for i k x with the integers k(i) of the row's elements, below 2^56
+template <int TT, int CNT, class KF>
+__device__ __forceinline__ int row_fix_ik(double2 (&x)[CNT], cfix (&v)[CNT], bool& bad, KF&& kof) {
+  auto top = [&](int i) {  // exponent field bound of k x (x = 0: 0)
+    const unsigned m = max(fix_mag(x[i].x), fix_mag(x[i].y));
+    return m >= 0x7ff00000u ? 0x7fffffffu : (m ? (m >> 20) + 32u - __clz((int)kof(i)) : 0u);
+  };
+  unsigned m = 0;
+  bool low = false;
+#pragma unroll
+  for (int i = 0; i < CNT; ++i) m = max(m, top(i));
+  low = m != 0u && m < 72u;
+  m = row_max<TT>(m);
+  int pre = 0;
+  if (__any_sync(0xffffffffu, low)) {  // near the smallest FP64 exponents
+    if (m != 0u && m < 72u) {
+      pre = FIX_PRE;
+      const double f = fix_pow2(FIX_PRE);
+#pragma unroll
+      for (int i = 0; i < CNT; ++i) { x[i].x *= f; x[i].y *= f; }
+    }
+    m = 0;
+#pragma unroll
+    for (int i = 0; i < CNT; ++i) m = max(m, top(i));
+    m = row_max<TT>(m);
+  }
+  bad = bad || m == 0x7fffffffu;
+  const int e1 = m ? (int)min(m, 4000u) - 1 : 4000;
+#pragma unroll
+  for (int i = 0; i < CNT; ++i) {
+    const unsigned k = kof(i);
+    v[i].x = -fix_times(x[i].y, k, e1);
+    v[i].y = fix_times(x[i].x, k, e1);
+  }
+  return e1 - 1077 - pre;
 }
 
 template <int N1, int N2, int TT> struct RowShape {
@@ -66,7 +110,7 @@ __global__ void __launch_bounds__(128, MB) k_ir2c(RowJob J, const int4* __restri
   extern __shared__ __align__(16) unsigned char smraw[];
   const int q = threadIdx.x % TT, r = threadIdx.x / TT;
   cfix* S = reinterpret_cast<cfix*>(smraw) + r * R::MS;
-  const int f = blockIdx.y, row = blockIdx.x * R::RPB + r;
+  const int f = blockIdx.x % J.nfield, row = (blockIdx.x / J.nfield) * R::RPB + r;
   const bool ok = row < nrows;
   const int lev = ok ? row / J.ny : 0, y = ok ? row - lev * J.ny : 0;
   const double2* src = reinterpret_cast<const double2*>(reinterpret_cast<const double*>(J.phys[f]) +
@@ -133,30 +177,44 @@ __global__ void __launch_bounds__(128, MB) k_ir2c(RowJob J, const int4* __restri
   __syncwarp();
   if (!ok) return;
   const double sd = J.div[f] != 0.0 ? J.scale[f] / J.div[f] : J.scale[f];
-  const FixOut out(ex - 1, bad ? __longlong_as_double(0x7ff8000000000000ll) : sd);  // X = (E + O) / 2
+  // X[k] = (E + O) / 2, X[M - k] = conj(E - O) / 2; lane 0: X[0], X[M], X[M / 2]
   double2* dst = reinterpret_cast<double2*>(J.work[f]) + (size_t)lev * J.pstride_work + (size_t)y * J.wc;
   const int nc = J.ncols;
+  cfix g[2 * R::KP + 1];
 #pragma unroll
   for (int i = 0; i < R::KP; ++i) {
     const int k = q + TT * i;
-    if ((M / 2) % TT != 0 && k >= M / 2) break;
-    const cfix a = S[k];
-    if (k == 0) {
-      if (0 < nc) dst[0] = make_double2(out((a.x + a.y) << 1), 0.0);
-      if (M < nc) dst[M] = make_double2(out((a.x - a.y) << 1), 0.0);
-      const cfix h = S[M / 2];
-      if (M / 2 < nc) dst[M / 2] = make_double2(out(h.x << 1), out(-(h.y << 1)));
-    } else if (k < nc) {
-      const cfix c = S[M - k];
-      const int4 t = __ldg(&wr[k]);
-      cfix e, d;  // Z[k] +- conj(Z[M - k])
-      e.x = a.x + c.x; e.y = a.y - c.y;
-      d.x = a.x - c.x; d.y = a.y + c.y;
-      const cfix o = fcmul(d, t.z, t.w, -t.x, -t.y);  // -i w d
-      dst[k] = make_double2(out(e.x + o.x), out(e.y + o.y));
-      if (M - k < nc) dst[M - k] = make_double2(out(e.x - o.x), out(o.y - e.y));
+    g[2 * i].x = g[2 * i].y = g[2 * i + 1].x = g[2 * i + 1].y = 0;
+    if (k < nc && ((M / 2) % TT == 0 || k < M / 2)) {
+      const cfix a = S[k];
+      if (i == 0 && k == 0) {
+        g[0].x = (a.x + a.y) << 1;
+        g[1].x = (a.x - a.y) << 1;
+      } else {
+        const cfix c = S[M - k];
+        const int4 t = __ldg(&wr[k]);
+        cfix e, d;  // Z[k] +- conj(Z[M - k])
+        e.x = a.x + c.x; e.y = a.y - c.y;
+        d.x = a.x - c.x; d.y = a.y + c.y;
+        const cfix o = fcmul(d, t.z, t.w, -t.x, -t.y);  // -i w d
+        g[2 * i].x = e.x + o.x; g[2 * i].y = e.y + o.y;
+        g[2 * i + 1].x = e.x - o.x; g[2 * i + 1].y = o.y - e.y;
+      }
     }
   }
+  g[2 * R::KP].x = S[M / 2].x << 1;
+  g[2 * R::KP].y = -(S[M / 2].y << 1);
+  double2 o[2 * R::KP + 1];
+  fix_out(g, o, ex - 1, nan_if(bad, J.div[f] != 0.0 ? J.scale[f] / J.div[f] : J.scale[f]));
+#pragma unroll
+  for (int i = 0; i < R::KP; ++i) {
+    const int k = q + TT * i;
+    if ((M / 2) % TT == 0 || k < M / 2) {
+      if (k < nc) dst[k] = o[2 * i];
+      if (M - k < nc) dst[M - k] = o[2 * i + 1];
+    }
+  }
+  if (q == 0 && M / 2 < nc) dst[M / 2] = o[2 * R::KP];
 }
 
 template <int N1, int N2, int TT, int MB>
@@ -167,7 +225,7 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
   extern __shared__ __align__(16) unsigned char smraw[];
   const int q = threadIdx.x % TT, r = threadIdx.x / TT;
   cfix* S = reinterpret_cast<cfix*>(smraw) + r * R::MS;
-  const int f = blockIdx.y, row = blockIdx.x * R::RPB + r;
+  const int f = blockIdx.x % J.nfield, row = (blockIdx.x / J.nfield) * R::RPB + r;
   const bool ok = row < nrows;
   const int lev = ok ? row / J.ny : 0, y = ok ? row - lev * J.ny : 0;
   const double2* src = reinterpret_cast<const double2*>(J.work[f]) + (size_t)lev * J.pstride_work + (size_t)y * J.wc;
@@ -192,7 +250,15 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
       x[1].y = 0.0;
     }
     cfix g[2 * KP + 1];
-    ex = row_fix<TT, 2 * KP + 1>(x, g, 58, bad);
+    if (J.deriv[f]) {  // i kx X, kx = 0 at k = 0 and k = M; the unit of kx is a factor of the output
+      if (q == 0) x[1] = make_double2(0.0, 0.0);
+      ex = row_fix_ik<TT, 2 * KP + 1>(x, g, bad, [&](int i) {
+        const int k = q + TT * (i / 2);
+        return (unsigned)(i == 2 * KP ? M / 2 : (i & 1 ? M - k : k));
+      });
+    } else {
+      ex = row_fix<TT, 2 * KP + 1>(x, g, 58, bad);
+    }
 #pragma unroll
     for (int i = 0; i < KP; ++i) {
       const int k = q + TT * i;
@@ -229,20 +295,18 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
   for (int j = 0; j < J1; ++j) {
     const int k1 = q + TT * j;
     if (N1 % TT == 0 || k1 < N1) {
-      unsigned t = 0;
 #pragma unroll
       for (int i = 0; i < N2; ++i) {
         v[j * N2 + i] = S[k1 + N1 * i];
-        t += fix_l1(v[j * N2 + i]);
+        sum += fix_l1<4>(v[j * N2 + i]);
       }
-      sum = max(sum, t);
     }
   }
-  int s = fix_down_sum(row_max<TT>(sum));
-  i64 rnd = fix_rnd(s);
+  // at most 24 values a lane: below 2^31 units of 2^36; the row's in units of 2^40
+  const int s = fix_down_sum(row_sum<TT>((sum >> 4) + 1u), 40);
+  const i64 rnd = fix_rnd(s);
   ex += s;
   __syncwarp();
-  unsigned top = 0;
 #pragma unroll
   for (int j = 0; j < J1; ++j) {
     const int k1 = q + TT * j;
@@ -256,39 +320,33 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
 #pragma unroll
       for (int i = 0; i < N2; ++i) {
         if (i > 0) v[j * N2 + i] = ftwc(v[j * N2 + i], __ldg(&tw[k1 * i]));
-        top = max(top, max(fix_top(v[j * N2 + i].x), fix_top(v[j * N2 + i].y)));
         S[i * LD1 + k1] = v[j * N2 + i];
       }
     }
   }
-  s = fix_down(row_max<TT>(top), fix_in(N1));
-  rnd = fix_rnd(s);
-  ex += s;
   __syncwarp();
   if (!ok) return;
-  const FixOut out(ex, bad ? __longlong_as_double(0x7ff8000000000000ll) : 1.0);
+  const double factor = nan_if(bad, J.deriv[f] ? J.kunit : 1.0);
   double2* dst = reinterpret_cast<double2*>(reinterpret_cast<double*>(const_cast<void*>(J.phys[f])) +
                                             (size_t)lev * J.pstride_phys + (size_t)y * J.ld);
-  const double off = J.off[f] ? J.off[f][lev] : 0.0;
-  const bool hasoff = J.off[f] != nullptr;
+  const double* offs = J.off[f];
 #pragma unroll
   for (int j = 0; j < J2; ++j) {
     const int n2 = q + TT * j;
     if (N2 % TT == 0 || n2 < N2) {
       cfix w[N1];
 #pragma unroll
-      for (int i = 0; i < N1; ++i) {
-        const cfix a = S[n2 * LD1 + i];
-        w[i].x = fix_shr(a.x, s, rnd);
-        w[i].y = fix_shr(a.y, s, rnd);
-      }
+      for (int i = 0; i < N1; ++i) w[i] = S[n2 * LD1 + i];
       fdft<N1, 1>(w);  // over k1: z[n2 + N2 i]
+      double2 o[N1];
+      fix_out(w, o, ex, factor);
+      if (offs) {
+        const double off = offs[lev];
 #pragma unroll
-      for (int i = 0; i < N1; ++i) {
-        double2 o = make_double2(out(w[i].x), out(w[i].y));
-        if (hasoff) { o.x += off; o.y += off; }
-        dst[n2 + N2 * i] = o;
+        for (int i = 0; i < N1; ++i) { o[i].x += off; o[i].y += off; }
       }
+#pragma unroll
+      for (int i = 0; i < N1; ++i) dst[n2 + N2 * i] = o[i];
     }
   }
   if (q == 0) dst[M] = make_double2(0.0, 0.0);  // padding columns ld-1:ld
@@ -304,7 +362,7 @@ void run_r2c(const RowJob& J, const RealPlanDev& P, cudaStream_t s) {
     set = true;
   }
   const int nrows = J.ny * J.nlev;
-  k_ir2c<N1, N2, TT, MB><<<dim3((nrows + R::RPB - 1) / R::RPB, J.nfield), R::NT, R::smem, s>>>(J, P.c.uniti, P.wi, nrows);
+  k_ir2c<N1, N2, TT, MB><<<(nrows + R::RPB - 1) / R::RPB * J.nfield, R::NT, R::smem, s>>>(J, P.c.uniti, P.wi, nrows);
 }
 template <int N1, int N2, int TT, int MB>
 void run_c2r(const RowJob& J, const RealPlanDev& P, cudaStream_t s) {
@@ -316,7 +374,7 @@ void run_c2r(const RowJob& J, const RealPlanDev& P, cudaStream_t s) {
     set = true;
   }
   const int nrows = J.ny * J.nlev;
-  k_ic2r<N1, N2, TT, MB><<<dim3((nrows + R::RPB - 1) / R::RPB, J.nfield), R::NT, R::smem, s>>>(J, P.c.uniti, P.wi, nrows);
+  k_ic2r<N1, N2, TT, MB><<<(nrows + R::RPB - 1) / R::RPB * J.nfield, R::NT, R::smem, s>>>(J, P.c.uniti, P.wi, nrows);
 }
 
 }  // namespace
@@ -327,6 +385,15 @@ void run_c2r(const RowJob& J, const RealPlanDev& P, cudaStream_t s) {
   X(54, 6, 9, 4, 3) X(64, 8, 8, 8, 6) X(72, 12, 6, 4, 3) X(96, 12, 8, 8, 4) X(108, 12, 9, 16, 5)       \
   X(128, 16, 8, 8, 4) X(144, 12, 12, 16, 5) X(192, 16, 12, 16, 4)
 
+bool int_rows_length(int m) {
+  switch (m) {
+#define LES_CASE(m, a, b, t, mb) case m:
+    LES_IROWS(LES_CASE)
+#undef LES_CASE
+    return true;
+    default: return false;
+  }
+}
 bool launch_rows_r2c_int(const RowJob& J, const RealPlanDev& P, cudaStream_t s) {
   if (!P.c.uniti) return false;
   switch (P.nx / 2) {

@@ -119,6 +119,34 @@ static int c2rT(les_ctx* c, int nf, int nlev, void* ws, TOut* const* out, long p
   }
   return 0;
 }
+// The integer-pipe transforms cover the small grid: their x pass can form
+// d/dx from a field's own y-transformed spectrum (i kx on the way in), which
+// saves the y pass an output.
+static bool int_deriv(const les_ctx* c) {
+  return c->rx.r.c.uniti && !c->fp64_kernels && int_rows_length(c->g.nx / 2);
+}
+// inverse x pass of chosen work fields (src[f]: index in ws), deriv[f]: i kx
+// times its spectrum; small grid, int_deriv grids
+static int c2r_deriv(les_ctx* c, int nf, int nlev, void* ws, const int* src, const unsigned char* deriv,
+                     double* const* out, long pstride) {
+  const Grid& g = c->g;
+  for (int f0 = 0; f0 < nf; f0 += JOB_MAXF) {
+    const int n = std::min(JOB_MAXF, nf - f0);
+    RowJob J{};
+    J.nfield = n; J.nlev = nlev; J.ny = g.ny; J.ld = g.ld; J.wc = g.lh; J.ncols = g.lh;
+    J.pstride_phys = pstride;
+    J.pstride_work = (long)g.C;
+    J.kunit = 2.0 * LES_PI / c->cfg.l_x;
+    for (int f = 0; f < n; ++f) {
+      J.phys[f] = out[f0 + f];
+      J.work[f] = (C2*)ws + (size_t)src[f0 + f] * nlev * g.C;
+      J.scale[f] = 1.0;
+      J.deriv[f] = deriv[f0 + f];
+    }
+    launch_rows_c2r<double, double>(J, c->rx.r, c->stream);
+  }
+  return 0;
+}
 static int r2c(les_ctx* c, int nf, int nlev, const double* const* in, long pstride,
                const double* scale, const double* div, void* ws, bool big, int ncols) {
   return r2cT<double, double>(c, nf, nlev, in, pstride, scale, div, ws, big, ncols);
@@ -244,6 +272,33 @@ int op_ddz(les_ctx* c, double* dfdz, const double* f, int uv) {
 }
 
 // ---------------------------------------------------------------------------
+// y pass of a filt_da job (outputs: field, d/dx, d/dy, and more) and its
+// inverse x pass; d/dx from the filtered field's spectrum where the x pass can
+static int filt_da_inverse(les_ctx* c, ColJob J, double* const* f, double* const* dx, double* const* dy, int nf,
+                           int nlev) {
+  const Grid& g = c->g;
+  double* out[3 * JOB_MAXF];
+  if (int_deriv(c)) {
+    for (int o = 1; o + 1 < J.nout; ++o) {  // output 1 (i kx) drops out
+      J.out[o] = J.out[o + 1];
+      J.coef[o][0] = J.coef[o + 1][0];
+    }
+    J.inv_mask = (J.inv_mask & 1u) | ((J.inv_mask >> 1) & ~1u);
+    --J.nout;
+    cols(c, J);
+    int src[3 * JOB_MAXF];
+    unsigned char deriv[3 * JOB_MAXF];
+    for (int i = 0; i < nf; ++i) {
+      out[3 * i] = f[i]; src[3 * i] = i; deriv[3 * i] = 0;
+      out[3 * i + 1] = dx[i]; src[3 * i + 1] = i; deriv[3 * i + 1] = 1;
+      out[3 * i + 2] = dy[i]; src[3 * i + 2] = 2 * nf + i; deriv[3 * i + 2] = 0;
+    }
+    return c2r_deriv(c, 3 * nf, nlev, c->wsB, src, deriv, out, (long)g.nplane);
+  }
+  cols(c, J);
+  for (int i = 0; i < nf; ++i) { out[i] = f[i]; out[nf + i] = dx[i]; out[2 * nf + i] = dy[i]; }
+  return c2r(c, 3 * nf, nlev, c->wsB, out, (long)g.nplane, false, g.lh);
+}
 // filt_da.f90:3-42 for nf fields at once
 static int filt_da_multi(les_ctx* c, double* const* f, double* const* dx, double* const* dy, int nf,
                          int nlev) {
@@ -261,11 +316,7 @@ static int filt_da_multi(les_ctx* c, double* const* f, double* const* dx, double
   J.out[2] = (C2*)c->wsB + (size_t)2 * nf * nlev * g.C;
   J.fs_out = (long)nlev * g.C;
   J.coef[0][0] = CC_KILL; J.coef[1][0] = CC_IKX; J.coef[2][0] = CC_IKY;
-  cols(c, J);
-  double* out[3 * JOB_MAXF];
-  for (int i = 0; i < nf; ++i) { out[i] = f[i]; out[nf + i] = dx[i]; out[2 * nf + i] = dy[i]; }
-  c2r(c, 3 * nf, nlev, c->wsB, out, (long)g.nplane, false, g.lh);
-  return 0;
+  return filt_da_inverse(c, J, f, dx, dy, nf, nlev);
 }
 // filt_da with the Nyquist-filtered spectra F(f/(nx*ny)) also stored in
 // `spec` (field stride nlev*C) for reuse by the fused step
@@ -287,11 +338,7 @@ int filt_da_multi_spec(les_ctx* c, double* const* f, double* const* dx, double* 
   J.out[3] = spec;
   J.fs_out = (long)nlev * g.C;
   J.coef[0][0] = CC_KILL; J.coef[1][0] = CC_IKX; J.coef[2][0] = CC_IKY; J.coef[3][0] = CC_KILL;
-  cols(c, J);
-  double* out[3 * JOB_MAXF];
-  for (int i = 0; i < nf; ++i) { out[i] = f[i]; out[nf + i] = dx[i]; out[2 * nf + i] = dy[i]; }
-  c2r(c, 3 * nf, nlev, c->wsB, out, (long)g.nplane, false, g.lh);
-  return 0;
+  return filt_da_inverse(c, J, f, dx, dy, nf, nlev);
 }
 // filt_da.f90:3-42 Nyquist removal done in physical space, in FP64.  With
 // a(x) = (1/ny) sum_y (-1)^y f(x,y), b(y) = (1/nx) sum_x (-1)^x f(x,y) and
@@ -585,6 +632,19 @@ int op_ddxy(les_ctx* c, double* dfdx, double* dfdy, const double* f, int nlev) {
   J.nin = 1; J.nout = 0;
   J.in[0] = c->wsA;
   double* out[2]; int no = 0;
+  if (int_deriv(c)) {  // d/dx from the filtered field in the x pass
+    int src[2];
+    unsigned char deriv[2];
+    if (dfdx) {
+      J.out[J.nout] = c->wsB; J.coef[J.nout][0] = CC_KILL; src[no] = J.nout; deriv[no] = 1; out[no++] = dfdx; J.nout++;
+    }
+    if (dfdy) {
+      J.out[J.nout] = (C2*)c->wsB + (size_t)J.nout * nlev * g.C; J.coef[J.nout][0] = CC_IKY;
+      src[no] = J.nout; deriv[no] = 0; out[no++] = dfdy; J.nout++;
+    }
+    cols(c, J);
+    return c2r_deriv(c, no, nlev, c->wsB, src, deriv, out, (long)g.nplane);
+  }
   if (dfdx) { J.out[J.nout] = (C2*)c->wsB + (size_t)J.nout * nlev * g.C; J.coef[J.nout][0] = CC_IKX; out[no++] = dfdx; J.nout++; }
   if (dfdy) { J.out[J.nout] = (C2*)c->wsB + (size_t)J.nout * nlev * g.C; J.coef[J.nout][0] = CC_IKY; out[no++] = dfdy; J.nout++; }
   cols(c, J);
@@ -4326,6 +4386,10 @@ static int scalarT(les_ctx* c, typename PX<M>::S* const* bigf, const ScalarDesc&
     J.in[0] = c->wsA;
     J.out[0] = c->wsB; J.out[1] = (CX*)c->wsB + FS; J.out[2] = (CX*)c->wsB + 2 * FS; J.out[3] = specT;
     J.coef[0][0] = CC_KILL; J.coef[1][0] = CC_IKX; J.coef[2][0] = CC_IKY; J.coef[3][0] = CC_KILL;
+    if constexpr (M == 0) {
+      double *f1[1] = {c->f[d.s]}, *x1[1] = {c->f[d.dsdx]}, *y1[1] = {c->f[d.dsdy]};
+      filt_da_inverse(c, J, f1, x1, y1, 1, nz);
+    } else {
     colsT<T, CX>(c, J);
     if constexpr (MX) {  // theta in FP64 (plane mean added back), the gradients FP32-held
       double* o1[1] = {c->f[d.s]};
@@ -4337,6 +4401,7 @@ static int scalarT(les_ctx* c, typename PX<M>::S* const* bigf, const ScalarDesc&
       double* out[3] = {c->f[d.s], c->f[d.dsdx], c->f[d.dsdy]};
       const double* offo[3] = {th0, nullptr, nullptr};
       c2rT<T, double>(c, 3, nz, c->wsB, out, (long)g.nplane, false, g.lh, offo);
+    }
     }
   }
   op_ddz(c, c->f[d.dsdz], c->f[d.s], 1);
