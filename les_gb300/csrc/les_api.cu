@@ -114,8 +114,12 @@ static int make_plan(les_ctx* c, int n, HostPlan& hp) {
     LES_CUDA_CHECK(cudaMemcpy(hp.devud, ud.data(), ud.size() * sizeof(float4), cudaMemcpyHostToDevice));
     P.unitf = static_cast<const float2*>(hp.devuf);
     P.unitd = static_cast<const float4*>(hp.devud);
-    // no table: the integer-pipe launchers decline (see ref_rounding)
-    if (!(c->cfg.model == 3 && ref_rounding_grid(c->g))) {
+    // no table: the integer-pipe launchers decline.  Model 3 on small grids:
+    // see ref_rounding_grid.  FP32-mixed contexts: the surface planes are the
+    // only FP64 transforms of their step, and its FP32 roundings turn a last-bit
+    // difference there into one of 1e-8 in v and w within ten steps, so they
+    // keep the kernels their stated errors were measured with.
+    if (c->cfg.precision != 1 && !(c->cfg.model == 3 && ref_rounding_grid(c->g))) {
       std::vector<int4> ui(n);
       for (int mm = 0; mm < n; ++mm) {
         const long double ang = -2.0L * 3.14159265358979323846264338327950288L * mm / (long double)n;
