@@ -66,7 +66,9 @@ typedef struct les_config {
   int jt_total0;        /* total_time.dat (param.f90:203-214) step offset        */
   int precision;        /* 0 = FP64 throughout, 1 = FP32-mixed form,
                                           2 = FP64 state and arithmetic with
-                                              float-float (about 48-bit) transforms */
+                                              transforms of at least float-float
+                                              precision (about 48 bits): the FP64
+                                              form's where they are faster */
   int rmsdiv_every;     /* main.f90:451   rmsdiv/CFL diagnostic period (500)    */
   int q_flag;           /* main.f90:274   1 = humidity qmix (scalars_module_q.f90)
                                           advanced after theta; needs s_flag.

@@ -604,6 +604,15 @@ bool run_pad(const ColJob& J, const FftPlanDev& Pa, const FftPlanDev& Pb, cudaSt
   X(128, 16, 8, 192, 16, 12, 4) X(144, 12, 12, 216, 24, 9, 2) X(192, 16, 12, 288, 24, 12, 2)               \
   X(256, 16, 16, 384, 24, 16, 2)
 
+bool int_cols_length(int ny) {  // ny and its 3/2 padding
+  switch (ny) {
+#define LES_CASE(n, a, b, m, c, d, mb) case n:
+    LES_IPADS(LES_CASE)
+#undef LES_CASE
+    return true;
+    default: return false;
+  }
+}
 bool launch_cols_int(const ColJob& J, const FftPlanDev& Pin, const FftPlanDev& Pout, cudaStream_t s) {
   if (!Pin.uniti || !Pout.uniti) return false;
   if (J.map == MAP_SAME) {

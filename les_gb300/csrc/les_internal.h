@@ -17,8 +17,9 @@ int launch_cols(const ColJob& J, const FftPlanDev& Pin, const FftPlanDev& Pout, 
 
 // FP64 transforms on the integer pipe (fft_int_rows.cu, fft_int_cols.cu):
 // false when the job's length has no instantiation
-// half lengths that the x pass covers
+// lengths they cover: half lengths of the x pass; y lengths with their padding
 bool int_rows_length(int m);
+bool int_cols_length(int ny);
 bool launch_rows_r2c_int(const RowJob& J, const RealPlanDev& P, cudaStream_t s);
 bool launch_rows_c2r_int(const RowJob& J, const RealPlanDev& P, cudaStream_t s);
 bool launch_cols_int(const ColJob& J, const FftPlanDev& Pin, const FftPlanDev& Pout, cudaStream_t s);
