@@ -35,12 +35,6 @@ template <typename C, typename T> __device__ __forceinline__ C ik(C f, T k) {
   C r; r.x = -(k * f.y); r.y = k * f.x; return r;
 }
 
-// FP32 truncation max(real(a), real(b)) of the reference's default-real MAX.
-__device__ __forceinline__ double fmax32(double a, double b) {
-  float fa = __double2float_rn(a), fb = __double2float_rn(b);
-  return (double)(fa > fb ? fa : fb);
-}
-
 // IEEE-754 binary32 <-> binary64 conversions done with integer operations.
 // On this part a hardware float<->double conversion issues on the FP64 pipe,
 // which is as scarce as FP64 arithmetic; these run on the integer pipe for
@@ -73,6 +67,28 @@ __device__ __forceinline__ float cvt_d2f(double x) {
   unsigned r = sgn | ((unsigned)fe << 23) | m23;
   if (rem > 0x10000000u || (rem == 0x10000000u && (m23 & 1u))) r += 1u;  // a carry rounds into the exponent
   return __uint_as_float(r);
+}
+// FP32 truncation max(real(a), real(b)) of the reference's default-real MAX.
+__device__ __forceinline__ double fmax32(double a, double b) {
+  const float fa = cvt_d2f(a), fb = cvt_d2f(b);
+  return cvt_f2d(fa > fb ? fa : fb);
+}
+// x / 2 and -2 x through the exponent field: exact products with powers of
+// two need no operation of the FP64 pipe (about 1.7 per clock per SM, which
+// bounds the pointwise FP64 kernels).  Infinities and NaN pass; subnormals
+// are shifted (x / 2 drops the last unit of 2^-1074).
+__device__ __forceinline__ double half_of(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const unsigned hi = (unsigned)(b >> 32), e = (hi >> 20) & 0x7ffu;
+  if (e > 1u) return e == 0x7ffu ? x : __hiloint2double((int)(hi - (1u << 20)), (int)(unsigned)b);
+  return __longlong_as_double((long long)((b & 0x8000000000000000ull) | ((b << 1) >> 2)));
+}
+__device__ __forceinline__ double minus_twice(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x) ^ 0x8000000000000000ull;
+  const unsigned hi = (unsigned)(b >> 32), e = (hi >> 20) & 0x7ffu;
+  if (e - 1u < 0x7fdu) return __hiloint2double((int)(hi + (1u << 20)), (int)(unsigned)b);
+  if (e == 0u) return __longlong_as_double((long long)((b & 0x8000000000000000ull) | (b << 1)));
+  return __longlong_as_double((long long)(e == 0x7ffu ? b : (b & 0x8000000000000000ull) | 0x7ff0000000000000ull));
 }
 // Float-float number ("double-single"): value hi + lo with |lo| <= ulp(hi)/2,
 // about 48 significant bits, computed on the FP32 pipe with error-free

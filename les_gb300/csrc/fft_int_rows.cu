@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
   }
   __syncwarp();
   if (!ok) return;
-  const double factor = nan_if(bad, J.deriv[f] ? J.kunit : 1.0);
+  const double factor = nan_if(bad, J.deriv[f] ? J.scale[f] * J.kunit : J.scale[f]);
   double2* dst = reinterpret_cast<double2*>(reinterpret_cast<double*>(const_cast<void*>(J.phys[f])) +
                                             (size_t)lev * J.pstride_phys + (size_t)y * J.ld);
   const double* offs = J.off[f];

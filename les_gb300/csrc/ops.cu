@@ -92,7 +92,7 @@ static int r2cT(les_ctx* c, int nf, int nlev, const TIn* const* in, long pstride
 }
 template <typename T, typename TOut>
 static int c2rT(les_ctx* c, int nf, int nlev, void* ws, TOut* const* out, long pstride, bool big, int ncols,
-                const double* const* off = nullptr) {
+                const double* const* off = nullptr, double scale = 1.0) {
   typedef typename CT<T>::type CX;
   const Grid& g = c->g;
   for (int f0 = 0; f0 < nf; f0 += JOB_MAXF) {
@@ -109,7 +109,7 @@ static int c2rT(les_ctx* c, int nf, int nlev, void* ws, TOut* const* out, long p
     for (int f = 0; f < n; ++f) {
       J.phys[f] = out[f0 + f];
       J.work[f] = (CX*)ws + (size_t)(f0 + f) * nlev * J.pstride_work;
-      J.scale[f] = 1.0;
+      J.scale[f] = scale;  // integer-pipe kernels only
       J.div[f] = 0.0;
       J.off[f] = off ? off[f0 + f] : nullptr;
     }
@@ -718,8 +718,9 @@ int op_dealias1(les_ctx* c, const double* const* in, double* const* out, int nf,
 // by `scale` (1/(nx2*ny2) in dealias2, 1 when the caller folded it in)
 int op_dealias2(les_ctx* c, double* const* out, const double* const* in, int nf, int nlev, double scale) {
   const Grid& g = c->g;
+  const bool late = int_deriv(c);  // factor in the inverse x pass: 4/9 of the points
   double sc[JOB_MAXF];
-  for (int i = 0; i < nf; ++i) sc[i] = scale;
+  for (int i = 0; i < nf; ++i) sc[i] = late ? 1.0 : scale;
   r2c(c, nf, nlev, in, (long)g.nplane_big, sc, nullptr, c->wsA, true, g.nx / 2);
   ColJob J = coljob(c, MAP_UNPAD, DIR_BOTH, nlev);
   J.nin = 1; J.nout = 1; J.nf = nf;
@@ -727,7 +728,7 @@ int op_dealias2(les_ctx* c, double* const* out, const double* const* in, int nf,
   J.out[0] = c->wsB; J.fs_out = (long)nlev * g.C;
   J.coef[0][0] = CC_ONE;
   cols(c, J);
-  c2r(c, nf, nlev, c->wsB, out, (long)g.nplane, false, g.nx / 2);
+  c2rT<double, double>(c, nf, nlev, c->wsB, out, (long)g.nplane, false, g.nx / 2, nullptr, late ? scale : 1.0);
   return 0;
 }
 
@@ -890,43 +891,44 @@ int op_wallstress(les_ctx* c, const double* uv1) {
 // sgs_stag.f90:371-498 calc_Sij ('wall') fused with the Lagrangian velocity
 // accumulation of sgs_stag.f90:59-69 (uls, vls, wls: the scalar model's
 // second sum, u_lag_s, when it is carried, else null)
-__global__ void k_calc_sij(const double* __restrict__ dudx, const double* __restrict__ dudy,
-                           const double* __restrict__ dudz, const double* __restrict__ dvdx,
-                           const double* __restrict__ dvdy, const double* __restrict__ dvdz,
-                           const double* __restrict__ dwdx, const double* __restrict__ dwdy,
-                           const double* __restrict__ dwdz, double* S11, double* S12, double* S13,
-                           double* S22, double* S23, double* S33, const double* __restrict__ u,
-                           const double* __restrict__ v, const double* __restrict__ w, double* ul,
-                           double* vl, double* wl, double* uls, double* vls, double* wls, int ld, int nx,
-                           int ny, int nz, int lag) {
-  const size_t np = (size_t)ld * ny;
-  GSTRIDE(i, np * nz) {
-    const int jz = (int)(i / np) + 1;
-    const int jx = (int)((i - (size_t)(jz - 1) * np) % ld);
-    if (lag) { ul[i] += u[i]; vl[i] += v[i]; wl[i] += w[i]; }
-    if (uls) { uls[i] += u[i]; vls[i] += v[i]; wls[i] += w[i]; }
-    if (jx >= nx) continue;
-    double ux, uy, uz, vx, vy, vz, wx, wy, wz;
-    if (jz == 1) {
-      ux = dudx[i]; uy = dudy[i]; uz = dudz[i];
-      vx = dvdx[i]; vy = dvdy[i]; vz = dvdz[i];
-      wx = 0.5 * (dwdx[i] + dwdx[i + np]);
-      wy = 0.5 * (dwdy[i] + dwdy[i + np]);
-      wz = dwdz[i];
-    } else {
-      ux = 0.5 * (dudx[i] + dudx[i - np]);
-      uy = 0.5 * (dudy[i] + dudy[i - np]);
-      uz = dudz[i];
-      vx = 0.5 * (dvdx[i] + dvdx[i - np]);
-      vy = 0.5 * (dvdy[i] + dvdy[i - np]);
-      vz = dvdz[i];
-      wx = dwdx[i];
-      wy = dwdy[i];
-      wz = 0.5 * (dwdz[i] + dwdz[i - np]);
-    }
-    S11[i] = ux; S12[i] = 0.5 * (uy + vx); S13[i] = 0.5 * (uz + wx);
-    S22[i] = vy; S23[i] = 0.5 * (vz + wy); S33[i] = wz;
+// grid (plane points, levels).  256^3: 625 -> 485 us with the halvings in the
+// exponent field (11 FP64 operations per point instead of 19) and no 64-bit
+// index division.
+__global__ void __launch_bounds__(256) k_calc_sij(
+    const double* __restrict__ dudx, const double* __restrict__ dudy, const double* __restrict__ dudz,
+    const double* __restrict__ dvdx, const double* __restrict__ dvdy, const double* __restrict__ dvdz,
+    const double* __restrict__ dwdx, const double* __restrict__ dwdy, const double* __restrict__ dwdz, double* S11,
+    double* S12, double* S13, double* S22, double* S23, double* S33, const double* __restrict__ u,
+    const double* __restrict__ v, const double* __restrict__ w, double* ul, double* vl, double* wl, double* uls,
+    double* vls, double* wls, int ld, int nx, int ny, int nz, int lag) {
+  const unsigned np = (unsigned)ld * ny;
+  const unsigned r = blockIdx.x * 256u + threadIdx.x;
+  if (r >= np) return;
+  const int jz = blockIdx.y + 1;
+  const size_t i = (size_t)blockIdx.y * np + r;
+  if (lag) { ul[i] += u[i]; vl[i] += v[i]; wl[i] += w[i]; }
+  if (uls) { uls[i] += u[i]; vls[i] += v[i]; wls[i] += w[i]; }
+  if ((int)(r % (unsigned)ld) >= nx) return;
+  double ux, uy, uz, vx, vy, vz, wx, wy, wz;
+  if (jz == 1) {
+    ux = dudx[i]; uy = dudy[i]; uz = dudz[i];
+    vx = dvdx[i]; vy = dvdy[i]; vz = dvdz[i];
+    wx = half_of(dwdx[i] + dwdx[i + np]);
+    wy = half_of(dwdy[i] + dwdy[i + np]);
+    wz = dwdz[i];
+  } else {
+    ux = half_of(dudx[i] + dudx[i - np]);
+    uy = half_of(dudy[i] + dudy[i - np]);
+    uz = dudz[i];
+    vx = half_of(dvdx[i] + dvdx[i - np]);
+    vy = half_of(dvdy[i] + dvdy[i - np]);
+    vz = dvdz[i];
+    wx = dwdx[i];
+    wy = dwdy[i];
+    wz = half_of(dwdz[i] + dwdz[i - np]);
   }
+  S11[i] = ux; S12[i] = half_of(uy + vx); S13[i] = half_of(uz + wx);
+  S22[i] = vy; S23[i] = half_of(vz + wy); S33[i] = wz;
 }
 
 // Mixed form: the same strain in FP32 from the FP32-held horizontal
@@ -974,52 +976,58 @@ __device__ __forceinline__ double smag(double a11, double a22, double a33, doubl
 }
 
 // sgs_stag.f90:166-211 (Cs override and Nu_t)
-__global__ void k_nut(const double* __restrict__ S11, const double* __restrict__ S12,
-                      const double* __restrict__ S13, const double* __restrict__ S22,
-                      const double* __restrict__ S23, const double* __restrict__ S33, double* Cs,
-                      double* Nu_t, int ld, int nx, int ny, int nz, double l2, int override_cs, double cs_ov) {
-  const size_t np = (size_t)ld * ny;
-  GSTRIDE(i, np * nz) {
-    if (override_cs) Cs[i] = cs_ov;
-    const int jx = (int)(i % ld);
-    if (jx >= nx) continue;
-    const double S = smag(S11[i], S22[i], S33[i], S12[i], S13[i], S23[i]);
-    Nu_t[i] = S * Cs[i] * l2;
-  }
-}
-// sgs_stag.f90:218-364 (tau_ij, 'wall', molec = .false.)
-__global__ void k_tau(const double* __restrict__ S11, const double* __restrict__ S12,
-                      const double* __restrict__ S13, const double* __restrict__ S22,
-                      const double* __restrict__ S23, const double* __restrict__ S33,
-                      const double* __restrict__ Nu_t, double* txx, double* txy, double* tyy, double* txz,
-                      double* tyz, double* tzz, int ld, int nx, int ny, int nz) {
-  const size_t np = (size_t)ld * ny;
-  GSTRIDE(i, np * nz) {
-    const int jz = (int)(i / np) + 1;
-    const int jx = (int)((i - (size_t)(jz - 1) * np) % ld);
+// Nu_t and tau_ij in one pass: a thread walks KZ levels of one plane point
+// with the level below's S_ij and Nu_t in registers, so every S_ij is read and
+// every Nu_t formed once.  256^3: 1075 us (Nu_t, then tau) -> 1000 us, bound by
+// the FP64 pipe (square root, about 30 operations per point).
+template <int KZ>
+__global__ void __launch_bounds__(256) k_nut_tau(
+    const double* __restrict__ S11, const double* __restrict__ S12, const double* __restrict__ S13,
+    const double* __restrict__ S22, const double* __restrict__ S23, const double* __restrict__ S33, double* Cs,
+    double* Nu_t, double* txx, double* txy, double* tyy, double* txz, double* tyz, double* tzz, int ld, int nx, int ny,
+    int nz, double l2, int override_cs, double cs_ov) {
+  const unsigned np = (unsigned)ld * ny;
+  const unsigned r = blockIdx.x * 256u + threadIdx.x;
+  if (r >= np) return;
+  const bool inx = (int)(r % (unsigned)ld) < nx;
+  const int j0 = blockIdx.y * KZ + 1, j1 = min(j0 + KZ - 1, nz);  // this thread's levels
+  size_t i = (size_t)(j0 - 1) * np + r;
+  double a11 = 0, a12 = 0, a13 = 0, a22 = 0, a23 = 0, a33 = 0, nu = 0;
+  auto level = [&](size_t t, bool own) {  // S_ij and Nu_t of one level
+    const double cs = override_cs ? cs_ov : Cs[t];
+    if (own && override_cs) Cs[t] = cs_ov;
+    if (!inx) return;
+    a11 = S11[t]; a12 = S12[t]; a13 = S13[t]; a22 = S22[t]; a23 = S23[t]; a33 = S33[t];
+    nu = smag(a11, a22, a33, a12, a13, a23) * (cs * l2);
+    if (own) Nu_t[t] = nu;
+  };
+  level(i, true);
+  for (int jz = j0; jz <= j1; ++jz, i += np) {
     if (jz == nz) {
       txx[i] = LES_BOGUS; txy[i] = LES_BOGUS; tyy[i] = LES_BOGUS; tzz[i] = LES_BOGUS;
       txz[i] = 0.0; tyz[i] = 0.0;
-      continue;
+      return;
     }
-    if (jx >= nx) continue;
-    if (jz == 1) {
-      const double cst = Nu_t[i], nu = 0.0;
-      txx[i] = -2.0 * (cst + nu) * S11[i];
-      txy[i] = -2.0 * (cst + nu) * S12[i];
-      tyy[i] = -2.0 * (cst + nu) * S22[i];
-      tzz[i] = -2.0 * (cst + nu) * S33[i];
-      // txz, tyz at the wall come from wallstress
+    const double b11 = a11, b12 = a12, b13 = a13, b22 = a22, b23 = a23, b33 = a33, nb = nu;
+    const double m = minus_twice(nb);
+    if (jz > 1 && inx) {
+      txz[i] = m * b13;
+      tyz[i] = m * b23;
+    }
+    // the next level: read for this level's averages, or as the next one of this thread
+    if (jz > 1 || jz < j1) level(i + np, jz < j1);
+    if (!inx) continue;
+    if (jz == 1) {  // txz, tyz at the wall come from wallstress
+      txx[i] = m * b11;
+      txy[i] = m * b12;
+      tyy[i] = m * b22;
+      tzz[i] = m * b33;
     } else {
-      const size_t ip = i + np;
-      const double cst = 0.5 * (Nu_t[i] + Nu_t[ip]), nu = 0.0;
-      txx[i] = -2.0 * (cst + nu) * 0.5 * (S11[i] + S11[ip]);
-      txy[i] = -2.0 * (cst + nu) * 0.5 * (S12[i] + S12[ip]);
-      tyy[i] = -2.0 * (cst + nu) * 0.5 * (S22[i] + S22[ip]);
-      tzz[i] = -2.0 * (cst + nu) * 0.5 * (S33[i] + S33[ip]);
-      const double c2 = Nu_t[i];
-      txz[i] = -2.0 * (c2 + nu) * S13[i];
-      tyz[i] = -2.0 * (c2 + nu) * S23[i];
+      const double c = -half_of(nb + nu);
+      txx[i] = c * (b11 + a11);
+      txy[i] = c * (b12 + a12);
+      tyy[i] = c * (b22 + a22);
+      tzz[i] = c * (b33 + a33);
     }
   }
 }
@@ -1079,6 +1087,21 @@ __global__ void __launch_bounds__(256) k_nut_tau32(Ptr6f Sp, double* Cs, float* 
   }
 }
 
+static void nut_tau(les_ctx* c, const double* const* S, int ov, double csov) {
+  const Grid& g = c->g;
+  // eight levels a thread once that leaves four blocks per SM (the level above
+  // the last is then formed twice for one in eight), else one level a thread
+  const unsigned pb = (unsigned)((g.nplane + 255) / 256);
+  const bool deep = (size_t)pb * (g.nz / 8) >= 4 * 152;
+  auto run = [&](auto kernel, int kz) {
+    kernel<<<dim3(pb, (unsigned)((g.nz + kz - 1) / kz)), 256, 0, c->stream>>>(
+        S[0], S[1], S[2], S[3], S[4], S[5], c->f[LES_CS_OPT2], c->f[LES_NU_T], c->f[LES_TXX], c->f[LES_TXY],
+        c->f[LES_TYY], c->f[LES_TXZ], c->f[LES_TYZ], c->f[LES_TZZ], g.ld, g.nx, g.ny, g.nz, g.delta * g.delta, ov, csov);
+  };
+  if (deep) run(k_nut_tau<8>, 8);
+  else run(k_nut_tau<1>, 1);
+  LES_COUNT_LAUNCH();
+}
 __global__ void k_bcast_levels(double* dst, const double* lev, size_t np, size_t n) {
   GSTRIDE(i, n) dst[i] = lev[i / np];
 }
@@ -1087,7 +1110,7 @@ int op_sgs_stag(les_ctx* c) {
   const Grid& g = c->g;
   const les_config& k = c->cfg;
   const bool lag = (k.model == 4 || k.model == 5 || k.model == 7);
-  k_calc_sij<<<grid1(g.nfield), 256, 0, c->stream>>>(
+  k_calc_sij<<<dim3((unsigned)((g.nplane + 255) / 256), (unsigned)g.nz), 256, 0, c->stream>>>(
       c->f[LES_DUDX], c->f[LES_DUDY], c->f[LES_DUDZ], c->f[LES_DVDX], c->f[LES_DVDY], c->f[LES_DVDZ],
       c->f[LES_DWDX], c->f[LES_DWDY], c->f[LES_DWDZ], c->f[LES_S11], c->f[LES_S12], c->f[LES_S13],
       c->f[LES_S22], c->f[LES_S23], c->f[LES_S33], c->f[LES_U], c->f[LES_V], c->f[LES_W], c->f[LES_U_LAG],
@@ -1118,23 +1141,18 @@ int op_sgs_stag(les_ctx* c) {
     csov = (double)(c016 * c016);
     if (k.model == 7) fill(c, c->f[LES_PR_T], g.nfield, k.pr);  // Pr_t = Pr (:171)
   }
-  const double delta = g.delta;
-  k_nut<<<grid1(g.nfield), 256, 0, c->stream>>>(S[0], S[1], S[2], S[3], S[4], S[5], c->f[LES_CS_OPT2],
-                                               c->f[LES_NU_T], g.ld, g.nx, g.ny, g.nz, delta * delta, ov, csov); LES_COUNT_LAUNCH();
-  k_tau<<<grid1(g.nfield), 256, 0, c->stream>>>(S[0], S[1], S[2], S[3], S[4], S[5], c->f[LES_NU_T],
-                                               c->f[LES_TXX], c->f[LES_TXY], c->f[LES_TYY], c->f[LES_TXZ],
-                                               c->f[LES_TYZ], c->f[LES_TZZ], g.ld, g.nx, g.ny, g.nz); LES_COUNT_LAUNCH();
+  nut_tau(c, S, ov, csov);
   return 0;
 }
 
 // ---------------------------------------------------------------------------
 // interpolag_Sdep.f90:2-380 (non-MPI).  Reads the accumulated u/v/w_lag and
 // the old F_*, writes the interpolated F_* into Fn.
-__device__ __forceinline__ double lag_disp_u(const double* ul, size_t i, size_t np, int jz, double cs,
-                                             double dt, double dxx) {
-  const double a = ul[i] / cs;
-  const double ua = (jz >= 2) ? 0.5 * (a + ul[i - np] / cs) : a;
-  return -ua * dt * cs / dxx;
+// 256^3: interpolag 3955 -> 1810 us with this and eight shared weights.
+// Displacement -(mean of u over the cycle) dt cs / dx from the sums ul over cs
+// steps: cs cancels, one product with f = -dt/dx (level average: -dt/(2 dx))
+__device__ __forceinline__ double lag_disp_u(const double* ul, size_t i, size_t np, int jz, double f) {
+  return jz >= 2 ? (ul[i] + ul[i - np]) * half_of(f) : ul[i] * f;
 }
 // NF: F_* fields carried (4: interpolag_Sdep, 2: interpolag_Ssim, which
 // also lacks the near-wall clip of interpolag_Sdep.f90:290-293, so its level 1 keeps
@@ -1144,35 +1162,34 @@ __global__ void k_interpolag(const double* __restrict__ ul, const double* __rest
                              const double* __restrict__ wl, const double* __restrict__ FLM,
                              const double* __restrict__ FMM, const double* __restrict__ FQN,
                              const double* __restrict__ FNN, double* oLM, double* oMM, double* oQN,
-                             double* oNN, int ld, int nx, int ny, int nz, double cs, double dt, double dx,
-                             double dy, double dz) {
+                             double* oNN, int ld, int nx, int ny, int nz, double fx_, double fy_, double fz_) {
   const size_t np = (size_t)ld * ny;
   GSTRIDE(t, (size_t)nx * ny * nz) {
     const int jx = (int)(t % nx);
     const int jy = (int)((t / nx) % ny);
     const int jz = (int)(t / ((size_t)nx * ny)) + 1;
     const size_t i = (size_t)jx + (size_t)ld * jy + np * (jz - 1);
-    const double xp = lag_disp_u(ul, i, np, jz, cs, dt, dx);
-    const double yp = lag_disp_u(vl, i, np, jz, cs, dt, dy);
+    const double xp = lag_disp_u(ul, i, np, jz, fx_);
+    const double yp = lag_disp_u(vl, i, np, jz, fy_);
     double zp;
     {
       // level 2 after the near-wall doubling and clipping (:285-293);
       // level 1 takes level 2's final value
       const size_t i2 = (size_t)jx + (size_t)ld * jy + np;
       if (SDEP && jz <= 2) {
-        double z2 = -(wl[i2] / cs) * dt * cs / dz;
+        double z2 = wl[i2] * fz_;
         z2 = z2 + fmin(z2, 0.0);
         z2 = fmin(1.0, z2);
         z2 = fmax(-1.0, z2);
         zp = z2;
       } else if (!SDEP && jz == 2) {
-        const double z2 = -(wl[i2] / cs) * dt * cs / dz;
+        const double z2 = wl[i2] * fz_;
         zp = z2 + fmin(z2, 0.0);
       } else if (!SDEP && jz == 1) {
-        const double z1 = -(0.25 * (wl[i2] / cs)) * dt * cs / dz;
+        const double z1 = 0.25 * wl[i2] * fz_;
         zp = z1 + fmax(z1, 0.0);
       } else {
-        zp = -(wl[i] / cs) * dt * cs / dz;
+        zp = wl[i] * fz_;
       }
     }
     const int addx = (xp < 0.0) ? -1 : 1;  // int(sign(1,x)), sign(1,-0) = +1
@@ -1186,9 +1203,13 @@ __global__ void k_interpolag(const double* __restrict__ ul, const double* __rest
     const size_t z0 = np * (jz - 1), z1 = np * za;
     const size_t a00 = (size_t)jx + (size_t)ld * jy, a01 = (size_t)jx + (size_t)ld * ya;
     const size_t a10 = (size_t)xa + (size_t)ld * jy, a11 = (size_t)xa + (size_t)ld * ya;
-#define LAGI(F)                                                                      \
-  (fx * fy * (F[a00 + z0] * fz + F[a00 + z1] * cz) + fx * cy * (F[a01 + z0] * fz + F[a01 + z1] * cz) + \
-   cx * fy * (F[a10 + z0] * fz + F[a10 + z1] * cz) + cx * cy * (F[a11 + z0] * fz + F[a11 + z1] * cz))
+    // the eight trilinear weights, shared by the fields
+    const double w0 = fx * fy, w1 = fx * cy, w2 = cx * fy, w3 = cx * cy;
+    const double w00 = w0 * fz, w01 = w0 * cz, w10 = w1 * fz, w11 = w1 * cz;
+    const double w20 = w2 * fz, w21 = w2 * cz, w30 = w3 * fz, w31 = w3 * cz;
+#define LAGI(F)                                                                           \
+  fma(w00, F[a00 + z0], fma(w01, F[a00 + z1], fma(w10, F[a01 + z0], fma(w11, F[a01 + z1], \
+  fma(w20, F[a10 + z0], fma(w21, F[a10 + z1], fma(w30, F[a11 + z0], w31 * F[a11 + z1])))))))
     oLM[i] = LAGI(FLM);
     oMM[i] = LAGI(FMM);
     if constexpr (NF == 4) {
@@ -1296,12 +1317,12 @@ int op_interpolag_n(les_ctx* c, int nf) {
   if (nf == 4)
     k_interpolag<4, true><<<grid1((size_t)g.nx * g.ny * g.nz), 256, 0, c->stream>>>(
         c->f[LES_U_LAG], c->f[LES_V_LAG], c->f[LES_W_LAG], c->f[LES_F_LM], c->f[LES_F_MM], c->f[LES_F_QN],
-        c->f[LES_F_NN], Fn[0], Fn[1], Fn[2], Fn[3], g.ld, g.nx, g.ny, g.nz, (double)k.cs_count, k.dt, g.dx, g.dy,
-        g.dz);
+        c->f[LES_F_NN], Fn[0], Fn[1], Fn[2], Fn[3], g.ld, g.nx, g.ny, g.nz, -k.dt / g.dx, -k.dt / g.dy,
+        -k.dt / g.dz);
   else
     k_interpolag<2, false><<<grid1((size_t)g.nx * g.ny * g.nz), 256, 0, c->stream>>>(
         c->f[LES_U_LAG], c->f[LES_V_LAG], c->f[LES_W_LAG], c->f[LES_F_LM], c->f[LES_F_MM], nullptr, nullptr,
-        Fn[0], Fn[1], nullptr, nullptr, g.ld, g.nx, g.ny, g.nz, (double)k.cs_count, k.dt, g.dx, g.dy, g.dz);
+        Fn[0], Fn[1], nullptr, nullptr, g.ld, g.nx, g.ny, g.nz, -k.dt / g.dx, -k.dt / g.dy, -k.dt / g.dz);
   LES_COUNT_LAUNCH();
   // interior values changed; padding columns are never read
   for (int q = 0; q < nf; ++q)
@@ -1342,6 +1363,14 @@ __global__ void k_lag_prep(const double* __restrict__ u, const double* __restric
 __device__ __forceinline__ double pow_m18(double x) { return 1.0 / sqrt(sqrt(sqrt(x))); }
 __device__ __forceinline__ float pow_m18(float x) { return 1.0f / sqrtf(sqrtf(sqrtf(x))); }
 // max(real(a), real(b)) of the reference: FP32 comparison, result widened
+// (dt/T) / (1 + dt/T): one division in FP64 (the FP64 pipe bounds
+// k_lag_final: 256^3, 32 levels 886 -> 780 us with this and fmax32 on the
+// integer pipe); FP32 as the reference writes it
+__device__ __forceinline__ double lag_epsi(double dt, double T) { return dt / (T + dt); }
+__device__ __forceinline__ float lag_epsi(float dt, float T) {
+  const float d = dt / T;
+  return d / (1.0f + d);
+}
 __device__ __forceinline__ double fmax32r(double a, double b) { return fmax32(a, b); }
 __device__ __forceinline__ float fmax32r(float a, float b) { return a > b ? a : b; }
 template <typename R>
@@ -1400,8 +1429,7 @@ __global__ void k_lag_final(const S* __restrict__ flt, double* F_LM, double* F_M
     if (TnLM) TnLM[gi] = (double)Tn;  // lagrange_Sdep.f90:322, read by lagrange_scalar_Sdep
     Tn = opftdelta * pow_m18(Tn);
     Tn = fmax32r(e24, Tn);
-    R dumfac = lagran_dt / Tn;
-    R epsi = dumfac / ((R)1 + dumfac);
+    R epsi = lag_epsi(lagran_dt, Tn);
     flm = (epsi * LM + ((R)1 - epsi) * flm);
     fmm = (epsi * MM + ((R)1 - epsi) * fmm);
     flm = fmax32r(e24, flm);
@@ -1412,8 +1440,7 @@ __global__ void k_lag_final(const S* __restrict__ flt, double* F_LM, double* F_M
     if (TnQN) TnQN[gi] = (double)Tn;  // :363
     Tn = opftdelta * pow_m18(Tn);
     Tn = fmax32r(e24, Tn);
-    dumfac = lagran_dt / Tn;
-    epsi = dumfac / ((R)1 + dumfac);
+    epsi = lag_epsi(lagran_dt, Tn);
     fqn = (epsi * QN + ((R)1 - epsi) * fqn);
     fnn = (epsi * NN + ((R)1 - epsi) * fnn);
     fqn = fmax32r(e24, fqn);
@@ -1482,8 +1509,8 @@ int op_interpolag_scalar(les_ctx* c) {
   for (int q = 0; q < 4; ++q) Fn[q] = c->spare + (size_t)q * g.nfield;
   k_interpolag<4, true><<<grid1((size_t)g.nx * g.ny * g.nz), 256, 0, c->stream>>>(
       c->f[LES_U_LAG_S], c->f[LES_V_LAG_S], c->f[LES_W_LAG_S], c->f[LES_G_LM], c->f[LES_G_MM], c->f[LES_G_QN],
-      c->f[LES_G_NN], Fn[0], Fn[1], Fn[2], Fn[3], g.ld, g.nx, g.ny, g.nz, (double)k.cs_count, k.dt, g.dx, g.dy,
-      g.dz); LES_COUNT_LAUNCH();
+      c->f[LES_G_NN], Fn[0], Fn[1], Fn[2], Fn[3], g.ld, g.nx, g.ny, g.nz, -k.dt / g.dx, -k.dt / g.dy,
+      -k.dt / g.dz); LES_COUNT_LAUNCH();
   for (int q = 0; q < 4; ++q)
     cudaMemcpyAsync(c->f[LES_G_LM + q], Fn[q], g.nfield * sizeof(double), cudaMemcpyDeviceToDevice, c->stream);
   cudaMemsetAsync(c->f[LES_U_LAG_S], 0, g.nfield * sizeof(double), c->stream);
@@ -2143,6 +2170,48 @@ __global__ void k_convec_prod(const S* __restrict__ u1, const S* __restrict__ u2
     }
   }
 }
+// The same products in FP64, without the factor `cst` (the inverse x pass
+// applies it to the truncated result, 4/9 of the points).  A thread walks KZ
+// levels of one point with the products u3 w and the velocities of the level
+// below in registers: 10 FP64 operations per point instead of 19, which is
+// what bounds it.  256^3: 1061 -> 712 us.
+template <int KZ>
+__global__ void __launch_bounds__(256) k_convec_prod64(const double* __restrict__ u1, const double* __restrict__ u2,
+                                                       const double* __restrict__ u3, const double* __restrict__ w1,
+                                                       const double* __restrict__ w2, const double* __restrict__ w3,
+                                                       double* ccx, double* ccy, double* ccz, int ldb, int nx2, int ny2,
+                                                       int nz) {
+  const unsigned np = (unsigned)ldb * ny2;
+  const unsigned r = blockIdx.x * 256u + threadIdx.x;
+  if (r >= np || (int)(r % (unsigned)ldb) >= nx2) return;
+  const int j0 = blockIdx.y * KZ + 1, j1 = min(j0 + KZ - 1, nz - 1);
+  size_t i = (size_t)(j0 - 1) * np + r;
+  double a1 = w1[i], a2 = w2[i];                       // this level's vorticity
+  const double c3 = j0 > 1 ? u3[i] : 0.0;              // level 1 has no flux through the wall
+  double t1 = c3 * a2, t2 = c3 * a1;
+  double p1 = j0 > 1 ? u1[i - np] : 0.0, p2 = j0 > 1 ? u2[i - np] : 0.0;
+  for (int jz = j0; jz <= j1; ++jz, i += np) {
+    const size_t ip = i + np;
+    const double b1 = w1[ip], b2 = w2[ip], b3 = u3[ip], c1 = u1[i], c2 = u2[i], v3 = w3[i];
+    const double n1 = b3 * b2, n2 = b3 * b1;
+    ccx[i] = fma(-c2, v3, half_of(n1 + t1));
+    ccy[i] = fma(c1, v3, -half_of(n2 + t2));
+    ccz[i] = jz == 1 ? 0.0 : half_of(fma(c2 + p2, a1, -((c1 + p1) * a2)));
+    t1 = n1; t2 = n2; a1 = b1; a2 = b2; p1 = c1; p2 = c2;
+  }
+}
+static void convec_prod64(les_ctx* c, double* const* b) {
+  const Grid& g = c->g;
+  const unsigned pb = (unsigned)((g.nplane_big + 255) / 256);
+  auto run = [&](auto kernel, int kz) {
+    kernel<<<dim3(pb, (unsigned)((g.nz - 1 + kz - 1) / kz)), 256, 0, c->stream>>>(
+        b[0], b[1], b[2], b[3], b[4], b[5], b[6], b[7], b[8], g.ld_big, g.nx2, g.ny2, g.nz);
+  };
+  // eight levels a thread once that leaves four blocks per SM
+  if ((size_t)pb * (g.nz / 8) >= 4 * 152) run(k_convec_prod64<8>, 8);
+  else run(k_convec_prod64<1>, 1);
+  LES_COUNT_LAUNCH();
+}
 int op_convec(les_ctx* c, double* cx, double* cy, double* cz) {
   const Grid& g = c->g;
   const double cst = 1.0 / (double)(g.nx * g.ny);
@@ -2165,13 +2234,10 @@ int op_convec(les_ctx* c, double* cx, double* cy, double* cz) {
     cols(c, J);
     c2r(c, 6, g.nz, c->wsB, bigf, (long)g.nplane_big, true, g.nx / 2);
   }
-  const double cst2 = 1.0 / (double)(g.nx2 * g.ny2);
-  k_convec_prod<double><<<grid1(g.nplane_big * (g.nz - 1)), 256, 0, c->stream>>>(
-      bigf[0], bigf[1], bigf[2], bigf[3], bigf[4], bigf[5], bigf[6], bigf[7], bigf[8], g.ld_big, g.nx2, g.ny2,
-      g.nz, cst2); LES_COUNT_LAUNCH();
+  convec_prod64(c, bigf);
   double* outs[3] = {cx, cy, cz};
   const double* bins[3] = {bigf[6], bigf[7], bigf[8]};
-  op_dealias2(c, outs, bins, 3, g.nz - 1, 1.0);
+  op_dealias2(c, outs, bins, 3, g.nz - 1, 1.0 / (double)(g.nx2 * g.ny2));
   const size_t top = (size_t)(g.nz - 1) * g.nplane;
   fill(c, cx + top, g.nplane, LES_BOGUS);
   fill(c, cy + top, g.nplane, LES_BOGUS);
@@ -2387,43 +2453,44 @@ __global__ void __launch_bounds__(256) k_rhs_ab2_mx(
 // main.f90:403-410 + forcing.f90:128-219 project, one thread per point of
 // levels 1..nz-1; the thread of level nz-1 also sets the top level and the
 // thread of level 1 the wall value of w.
-__global__ void k_dpdz_project(double* u, double* v, double* w, double* Rx, double* Ry, double* Rz,
-                               const double* __restrict__ p, const double* __restrict__ dpdx,
-                               const double* __restrict__ dpdy, double* dpdz, int ld, int nx, int ny, int nz,
-                               double dz, double dt) {
-  const size_t np = (size_t)ld * ny;
-  GSTRIDE(i, np * (nz - 1)) {
-    const int jz = (int)(i / np) + 1;
-    const size_t r = i - (size_t)(jz - 1) * np;
-    const int jx = (int)(r % ld);
-    double pz = 0.0;
-    if (jx < nx) {
-      const double dp = p[r + (size_t)jz * np] - p[r + (size_t)(jz - 1) * np];
-      pz = dp / dz;
-      dpdz[i] = pz;
-    } else {
-      pz = dpdz[i];
-    }
-    Rx[i] = Rx[i] - dpdx[i];
-    Ry[i] = Ry[i] - dpdy[i];
-    Rz[i] = Rz[i] - pz;
-    double uu = u[i], vv = v[i], ww = w[i];
-    if (jx < nx) {
-      uu = (uu + dt * (-1.5 * dpdx[i] + 0.0));
-      vv = (vv + dt * (-1.5 * dpdy[i] + 0.0));
-      if (jz >= 2) ww = (ww + dt * (-1.5 * pz + 0.0));
-      u[i] = uu; v[i] = vv;
-      if (jz >= 2) w[i] = ww;
-    }
-    if (jz == nz - 1) {
-      const size_t top = i + np;
-      dpdz[top] = LES_BOGUS;
-      u[top] = uu;
-      v[top] = vv;
-      w[top] = 0.0;
-    }
-    if (jz == 1) w[i] = 0.0;
+// 256^3: 571 -> 340 us with the products of constants formed on the host
+// (8 FP64 operations per point and no division; 24 before).
+__global__ void __launch_bounds__(256) k_dpdz_project(double* u, double* v, double* w, double* Rx, double* Ry, double* Rz,
+                                                      const double* __restrict__ p, const double* __restrict__ dpdx,
+                                                      const double* __restrict__ dpdy, double* dpdz, int ld, int nx,
+                                                      int ny, int nz, double idz, double mdt15) {  // 1/dz, -1.5 dt
+  const unsigned np = (unsigned)ld * ny;
+  const unsigned r = blockIdx.x * 256u + threadIdx.x;
+  if (r >= np) return;
+  const int jz = blockIdx.y + 1;
+  const size_t i = (size_t)blockIdx.y * np + r;
+  const bool inx = (int)(r % (unsigned)ld) < nx;
+  const double gx = dpdx[i], gy = dpdy[i];
+  double pz;
+  if (inx) {
+    pz = (p[i + np] - p[i]) * idz;
+    dpdz[i] = pz;
+  } else {
+    pz = dpdz[i];
   }
+  Rx[i] = Rx[i] - gx;
+  Ry[i] = Ry[i] - gy;
+  Rz[i] = Rz[i] - pz;
+  double uu = u[i], vv = v[i];
+  if (inx) {
+    uu = fma(mdt15, gx, uu);
+    vv = fma(mdt15, gy, vv);
+    u[i] = uu; v[i] = vv;
+    if (jz >= 2) w[i] = fma(mdt15, pz, w[i]);
+  }
+  if (jz == nz - 1) {
+    const size_t top = i + np;
+    dpdz[top] = LES_BOGUS;
+    u[top] = uu;
+    v[top] = vv;
+    w[top] = 0.0;
+  }
+  if (jz == 1) w[i] = 0.0;
 }
 // Mixed form: dpdz and the projection in FP64 with the fused factor
 // -1.5 dt (the pressure comes from float-float transforms and the projection
@@ -3296,51 +3363,50 @@ __global__ void k_scalar_prod(const S* __restrict__ um, const S* __restrict__ vm
 }
 // scalars_module.f90:77-82 Pr_: the constant Pr, or the field Pr_t of
 // model 7 when prt is not null
-__device__ __forceinline__ double pr_at(const double* __restrict__ prt, double pr, size_t i) {
-  return prt ? prt[i] : pr;
+// 1/Pr at point i; the constant Pr's reciprocal `ipr` is formed on the host
+__device__ __forceinline__ double ipr_at(const double* __restrict__ prt, double ipr, size_t i) {
+  return prt ? 1.0 / prt[i] : ipr;
 }
 // scalars_module.f90:364-407 horizontal SGS fluxes
 template <typename NT>
-__global__ void k_scalar_temp_xy(const NT* __restrict__ nut, const double* __restrict__ dsx,
-                                 const double* __restrict__ dsy, double* tx, double* ty, int ld, int nx, int ny,
-                                 int nz, double pr, const double* __restrict__ prt) {
-  const size_t np = (size_t)ld * ny;
-  GSTRIDE(i, np * nz) {
-    const int jz = (int)(i / np) + 1;
-    const int jx = (int)((i - (size_t)(jz - 1) * np) % ld);
-    if (jx >= nx) continue;
-    if (jz == nz) { tx[i] = 0.0; ty[i] = 0.0; continue; }
-    const double nu = cvt<double, NT>(nut[i]);
-    if (jz == 1) {
-      const double p1 = pr_at(prt, pr, i);
-      tx[i] = (1.0 / p1) * nu * dsx[i];
-      ty[i] = (1.0 / p1) * nu * dsy[i];
-    } else {
-      const double f = (1.0 / (0.5 * (pr_at(prt, pr, i) + pr_at(prt, pr, i + np)))) * 0.5 *
-                       (nu + cvt<double, NT>(nut[i + np]));
-      tx[i] = f * dsx[i];
-      ty[i] = f * dsy[i];
-    }
+__global__ void __launch_bounds__(256) k_scalar_temp_xy(const NT* __restrict__ nut, const double* __restrict__ dsx,
+                                                        const double* __restrict__ dsy, double* tx, double* ty, int ld,
+                                                        int nx, int ny, int nz, double ipr,
+                                                        const double* __restrict__ prt) {
+  const unsigned np = (unsigned)ld * ny;
+  const unsigned r = blockIdx.x * 256u + threadIdx.x;
+  if (r >= np || (int)(r % (unsigned)ld) >= nx) return;
+  const int jz = blockIdx.y + 1;
+  const size_t i = (size_t)blockIdx.y * np + r;
+  if (jz == nz) { tx[i] = 0.0; ty[i] = 0.0; return; }
+  const double nu = cvt<double, NT>(nut[i]);
+  double f;
+  if (jz == 1) {
+    f = ipr_at(prt, ipr, i) * nu;
+  } else {
+    const double q = prt ? 1.0 / half_of(prt[i] + prt[i + np]) : ipr;
+    f = q * half_of(nu + cvt<double, NT>(nut[i + np]));
   }
+  tx[i] = f * dsx[i];
+  ty[i] = f * dsy[i];
 }
 // scalars_module.f90:385-452 RHS assembly with the SGS divergence
 template <typename NT>
-__global__ void k_scalar_rhs(double* R, const double* __restrict__ dxy, const NT* __restrict__ nut,
-                             const double* __restrict__ dsz, const double* __restrict__ sgs_t3, int ld, int nx,
-                             int ny, int nz, double pr, const double* __restrict__ prt, double cdz) {
-  const size_t np = (size_t)ld * ny;
-  GSTRIDE(i, np * (nz - 1)) {
-    const int jz = (int)(i / np) + 1;
-    const size_t r = i - (size_t)(jz - 1) * np;
-    const int jx = (int)(r % ld);
-    if (jx >= nx) continue;
-    const int jy = (int)(r / ld);
-    // temp(k) = Nu_t dsdz / Pr on w-nodes, temp(1) = -surf_flux
-    const double t0 = (jz == 1) ? -1.0 * sgs_t3[(size_t)jy * nx + jx]
-                                : (1.0 / pr_at(prt, pr, i)) * cvt<double, NT>(nut[i]) * dsz[i];
-    const double t1 = (1.0 / pr_at(prt, pr, i + np)) * cvt<double, NT>(nut[i + np]) * dsz[i + np];
-    R[i] = (-1.0 * R[i] + dxy[i]) + cdz * (t1 - t0);
-  }
+__global__ void __launch_bounds__(256) k_scalar_rhs(double* R, const double* __restrict__ dxy, const NT* __restrict__ nut,
+                                                    const double* __restrict__ dsz, const double* __restrict__ sgs_t3,
+                                                    int ld, int nx, int ny, int nz, double ipr,
+                                                    const double* __restrict__ prt, double cdz) {
+  const unsigned np = (unsigned)ld * ny;
+  const unsigned r = blockIdx.x * 256u + threadIdx.x;
+  if (r >= np) return;
+  const unsigned jy = r / (unsigned)ld, jx = r - jy * (unsigned)ld;
+  if ((int)jx >= nx) return;
+  const int jz = blockIdx.y + 1;
+  const size_t i = (size_t)blockIdx.y * np + r;
+  // temp(k) = Nu_t dsdz / Pr on w-nodes, temp(1) = -surf_flux
+  const double t0 = (jz == 1) ? -1.0 * sgs_t3[(size_t)jy * nx + jx] : ipr_at(prt, ipr, i) * cvt<double, NT>(nut[i]) * dsz[i];
+  const double t1 = ipr_at(prt, ipr, i + np) * cvt<double, NT>(nut[i + np]) * dsz[i + np];
+  R[i] = (-1.0 * R[i] + dxy[i]) + cdz * (t1 - t0);
 }
 // scalars_module.f90:175-228 calcbeta from per-level plane sums
 // per level: sb = plane mean of theta, 1/sb (the divisions once per level)
@@ -3538,8 +3604,9 @@ static int op_scalar(les_ctx* c, const ScalarDesc& d) {
   double* tx = c->tmp;
   double* ty = c->tmp + g.nfield;
   double* dxy = c->tmp + 2 * g.nfield;
-  k_scalar_temp_xy<double><<<grid1(g.nfield), 256, 0, c->stream>>>(c->f[LES_NU_T], c->f[d.dsdx], c->f[d.dsdy], tx, ty,
-                                                          g.ld, g.nx, g.ny, nz, k.pr, c->f[LES_PR_T]);
+  const dim3 gpl((unsigned)((g.nplane + 255) / 256), (unsigned)nz);
+  k_scalar_temp_xy<double><<<gpl, 256, 0, c->stream>>>(c->f[LES_NU_T], c->f[d.dsdx], c->f[d.dsdy], tx, ty, g.ld, g.nx,
+                                                       g.ny, nz, 1.0 / k.pr, c->f[LES_PR_T]);
   LES_COUNT_LAUNCH();
   {
     const double sc = 1.0 / (double)(g.nx * g.ny);
@@ -3552,9 +3619,9 @@ static int op_scalar(les_ctx* c, const ScalarDesc& d) {
     cols(c, J);
     c2r(c, 1, nz, c->wsB, &dxy, (long)g.nplane, false, g.lh);
   }
-  k_scalar_rhs<double><<<grid1(g.nplane * (nz - 1)), 256, 0, c->stream>>>(rt, dxy, c->f[LES_NU_T], c->f[d.dsdz],
-                                                                 c->f[d.sgs3], g.ld, g.nx, g.ny, nz, k.pr,
-                                                                 c->f[LES_PR_T], 1.0 / g.dz); LES_COUNT_LAUNCH();
+  k_scalar_rhs<double><<<dim3(gpl.x, (unsigned)(nz - 1)), 256, 0, c->stream>>>(
+      rt, dxy, c->f[LES_NU_T], c->f[d.dsdz], c->f[d.sgs3], g.ld, g.nx, g.ny, nz, 1.0 / k.pr, c->f[LES_PR_T], 1.0 / g.dz);
+  LES_COUNT_LAUNCH();
   // calcbeta on theta before the update
   if (d.buoyancy) calcbeta(c);
   if (c->jt == 1 && !k.initsc)
@@ -4171,7 +4238,7 @@ static int sgs_stagT(les_ctx* c) {
         f32(c, LES_S22), f32(c, LES_S23), f32(c, LES_S33), c->f[LES_U], c->f[LES_V], c->f[LES_W], c->f[LES_U_LAG],
         c->f[LES_V_LAG], c->f[LES_W_LAG], g.ld, g.nx, g.ny, lag ? 1 : 0);
   else
-    k_calc_sij<<<grid1(g.nfield), 256, 0, c->stream>>>(
+    k_calc_sij<<<dim3((unsigned)((g.nplane + 255) / 256), (unsigned)g.nz), 256, 0, c->stream>>>(
         c->f[LES_DUDX], c->f[LES_DUDY], c->f[LES_DUDZ], c->f[LES_DVDX], c->f[LES_DVDY], c->f[LES_DVDZ],
         c->f[LES_DWDX], c->f[LES_DWDY], c->f[LES_DWDZ], c->f[LES_S11], c->f[LES_S12], c->f[LES_S13],
         c->f[LES_S22], c->f[LES_S23], c->f[LES_S33], c->f[LES_U], c->f[LES_V], c->f[LES_W], c->f[LES_U_LAG],
@@ -4212,12 +4279,7 @@ static int sgs_stagT(les_ctx* c) {
                                             csov); LES_COUNT_LAUNCH();
     return 0;
   }
-  k_nut<<<grid1(g.nfield), 256, 0, c->stream>>>(S[0], S[1], S[2], S[3], S[4], S[5], c->f[LES_CS_OPT2],
-                                               c->f[LES_NU_T], g.ld, g.nx, g.ny, g.nz, g.delta * g.delta, ov, csov);
-  LES_COUNT_LAUNCH();
-  k_tau<<<grid1(g.nfield), 256, 0, c->stream>>>(S[0], S[1], S[2], S[3], S[4], S[5], c->f[LES_NU_T],
-                                               c->f[LES_TXX], c->f[LES_TXY], c->f[LES_TYY], c->f[LES_TXZ],
-                                               c->f[LES_TYZ], c->f[LES_TZZ], g.ld, g.nx, g.ny, g.nz); LES_COUNT_LAUNCH();
+  nut_tau(c, S, ov, csov);
   return 0;
 }
 
@@ -4241,8 +4303,9 @@ static void unpadT(les_ctx* c, typename PX<M>::S* const* in, TO* const* out, int
   typedef typename PX<M>::CX CX;
   typedef typename PX<M>::S S;
   const Grid& g = c->g;
+  const bool late = std::is_same<T, double>::value && int_deriv(c);  // factor in the inverse x pass: 4/9 of the points
   double sc[JOB_MAXF];
-  for (int i = 0; i < nf; ++i) sc[i] = scale;
+  for (int i = 0; i < nf; ++i) sc[i] = late ? 1.0 : scale;
   const S* ii[JOB_MAXF];
   for (int i = 0; i < nf; ++i) ii[i] = in[i];
   r2cT<T, S>(c, nf, nlev, ii, (long)g.nplane_big, sc, nullptr, c->wsA, true, g.nx / 2);
@@ -4252,7 +4315,7 @@ static void unpadT(les_ctx* c, typename PX<M>::S* const* in, TO* const* out, int
   J.out[0] = c->wsB; J.fs_out = (long)nlev * g.C;
   J.coef[0][0] = CC_ONE;
   colsT<T, CX>(c, J);
-  c2rT<T, TO>(c, nf, nlev, c->wsB, out, (long)g.nplane, false, g.nx / 2);
+  c2rT<T, TO>(c, nf, nlev, c->wsB, out, (long)g.nplane, false, g.nx / 2, nullptr, late ? scale : 1.0);
 }
 
 // ddx + ddy of two fields summed in spectral space (one inverse); TS: their
@@ -4462,14 +4525,13 @@ static int scalarT(les_ctx* c, typename PX<M>::S* const* bigf, const ScalarDesc&
     double* tx = c->tmp;
     double* ty = c->tmp + g.nfield;
     double* dxy = c->tmp + 2 * g.nfield;
-    k_scalar_temp_xy<double><<<grid1(g.nfield), 256, 0, c->stream>>>(c->f[LES_NU_T], c->f[d.dsdx],
-                                                                    c->f[d.dsdy], tx, ty, g.ld, g.nx, g.ny, nz,
-                                                                    k.pr, c->f[LES_PR_T]); LES_COUNT_LAUNCH();
+    const dim3 gpl((unsigned)((g.nplane + 255) / 256), (unsigned)nz);
+    k_scalar_temp_xy<double><<<gpl, 256, 0, c->stream>>>(c->f[LES_NU_T], c->f[d.dsdx], c->f[d.dsdy], tx, ty, g.ld,
+                                                         g.nx, g.ny, nz, 1.0 / k.pr, c->f[LES_PR_T]); LES_COUNT_LAUNCH();
     div_xyT<M>(c, tx, ty, dxy, nz);
-    k_scalar_rhs<double><<<grid1(g.nplane * (nz - 1)), 256, 0, c->stream>>>(rt, dxy, c->f[LES_NU_T],
-                                                                           c->f[d.dsdz], c->f[d.sgs3],
-                                                                           g.ld, g.nx, g.ny, nz, k.pr, c->f[LES_PR_T],
-                                                                           1.0 / g.dz);
+    k_scalar_rhs<double><<<dim3(gpl.x, (unsigned)(nz - 1)), 256, 0, c->stream>>>(
+        rt, dxy, c->f[LES_NU_T], c->f[d.dsdz], c->f[d.sgs3], g.ld, g.nx, g.ny, nz, 1.0 / k.pr, c->f[LES_PR_T],
+        1.0 / g.dz);
     LES_COUNT_LAUNCH();
   }
   if (d.buoyancy) calcbeta(c);
@@ -4503,14 +4565,18 @@ static int convecT(les_ctx* c, typename PX<M>::S* const* bigf, double* cx, doubl
     S* o3[3] = {bigf[3], bigf[4], bigf[5]};
     padT<M, CX>(c, vs, 3, o3);
   }
-  const S cst2 = (S)(1.0 / (double)(g.nx2 * g.ny2));
-  k_convec_prod<S><<<grid1(g.nplane_big * (g.nz - 1)), 256, 0, c->stream>>>(
-      bigf[0], bigf[1], bigf[2], bigf[3], bigf[4], bigf[5], bigf[6], bigf[7], bigf[8], g.ld_big, g.nx2, g.ny2,
-      g.nz, cst2); LES_COUNT_LAUNCH();
+  const double cst2 = 1.0 / (double)(g.nx2 * g.ny2);
+  if constexpr (MX) {
+    k_convec_prod<S><<<grid1(g.nplane_big * (g.nz - 1)), 256, 0, c->stream>>>(
+        bigf[0], bigf[1], bigf[2], bigf[3], bigf[4], bigf[5], bigf[6], bigf[7], bigf[8], g.ld_big, g.nx2, g.ny2,
+        g.nz, (S)cst2); LES_COUNT_LAUNCH();
+  } else {
+    convec_prod64(c, bigf);
+  }
   {
     S* bins[3] = {bigf[6], bigf[7], bigf[8]};
     double* outs[3] = {cx, cy, cz};
-    unpadT<M>(c, bins, outs, 3, g.nz - 1, 1.0);
+    unpadT<M>(c, bins, outs, 3, g.nz - 1, MX ? 1.0 : cst2);
   }
   const size_t top = (size_t)(g.nz - 1) * g.nplane;
   fill(c, cx + top, g.nplane, LES_BOGUS);
@@ -4724,9 +4790,9 @@ static int stepT(les_ctx* c) {
     pressT<double>(c, c->f[LES_P], c->f[LES_DPDX], c->f[LES_DPDY]);
   }
   if (!MX)
-    k_dpdz_project<<<grid1(g.nplane * (g.nz - 1)), 256, 0, c->stream>>>(
+    k_dpdz_project<<<dim3((unsigned)((g.nplane + 255) / 256), (unsigned)(g.nz - 1)), 256, 0, c->stream>>>(
         c->f[LES_U], c->f[LES_V], c->f[LES_W], c->f[LES_RHSX], c->f[LES_RHSY], c->f[LES_RHSZ], c->f[LES_P],
-        c->f[LES_DPDX], c->f[LES_DPDY], c->f[LES_DPDZ], g.ld, g.nx, g.ny, g.nz, g.dz, k.dt);
+        c->f[LES_DPDX], c->f[LES_DPDY], c->f[LES_DPDZ], g.ld, g.nx, g.ny, g.nz, 1.0 / g.dz, -1.5 * k.dt);
   LES_COUNT_LAUNCH();
   LES_CUDA_CHECK(cudaGetLastError());
   if (rms_step) {
