@@ -125,10 +125,10 @@ static int c2rT(les_ctx* c, int nf, int nlev, void* ws, TOut* const* out, long p
 static bool int_deriv(const les_ctx* c) {
   return c->rx.r.c.uniti && !c->fp64_kernels && int_rows_length(c->g.nx / 2);
 }
-// inverse x pass of chosen work fields (src[f]: index in ws), deriv[f]: i kx
-// times its spectrum; small grid, int_deriv grids
-static int c2r_deriv(les_ctx* c, int nf, int nlev, void* ws, const int* src, const unsigned char* deriv,
-                     double* const* out, long pstride) {
+// inverse x pass of chosen y-transformed spectra, deriv[f]: i kx times its
+// spectrum; small grid, int_deriv grids
+static int c2r_deriv(les_ctx* c, int nf, int nlev, C2* const* src, const unsigned char* deriv, double* const* out,
+                     long pstride) {
   const Grid& g = c->g;
   for (int f0 = 0; f0 < nf; f0 += JOB_MAXF) {
     const int n = std::min(JOB_MAXF, nf - f0);
@@ -139,7 +139,7 @@ static int c2r_deriv(les_ctx* c, int nf, int nlev, void* ws, const int* src, con
     J.kunit = 2.0 * LES_PI / c->cfg.l_x;
     for (int f = 0; f < n; ++f) {
       J.phys[f] = out[f0 + f];
-      J.work[f] = (C2*)ws + (size_t)src[f0 + f] * nlev * g.C;
+      J.work[f] = src[f0 + f];
       J.scale[f] = 1.0;
       J.deriv[f] = deriv[f0 + f];
     }
@@ -286,14 +286,16 @@ static int filt_da_inverse(les_ctx* c, ColJob J, double* const* f, double* const
     J.inv_mask = (J.inv_mask & 1u) | ((J.inv_mask >> 1) & ~1u);
     --J.nout;
     cols(c, J);
-    int src[3 * JOB_MAXF];
+    C2* src[3 * JOB_MAXF];
     unsigned char deriv[3 * JOB_MAXF];
+    C2* base = (C2*)c->wsB;
+    const size_t fs = (size_t)nlev * g.C;
     for (int i = 0; i < nf; ++i) {
-      out[3 * i] = f[i]; src[3 * i] = i; deriv[3 * i] = 0;
-      out[3 * i + 1] = dx[i]; src[3 * i + 1] = i; deriv[3 * i + 1] = 1;
-      out[3 * i + 2] = dy[i]; src[3 * i + 2] = 2 * nf + i; deriv[3 * i + 2] = 0;
+      out[3 * i] = f[i]; src[3 * i] = base + i * fs; deriv[3 * i] = 0;
+      out[3 * i + 1] = dx[i]; src[3 * i + 1] = base + i * fs; deriv[3 * i + 1] = 1;
+      out[3 * i + 2] = dy[i]; src[3 * i + 2] = base + (size_t)(2 * nf + i) * fs; deriv[3 * i + 2] = 0;
     }
-    return c2r_deriv(c, 3 * nf, nlev, c->wsB, src, deriv, out, (long)g.nplane);
+    return c2r_deriv(c, 3 * nf, nlev, src, deriv, out, (long)g.nplane);
   }
   cols(c, J);
   for (int i = 0; i < nf; ++i) { out[i] = f[i]; out[nf + i] = dx[i]; out[2 * nf + i] = dy[i]; }
@@ -633,17 +635,17 @@ int op_ddxy(les_ctx* c, double* dfdx, double* dfdy, const double* f, int nlev) {
   J.in[0] = c->wsA;
   double* out[2]; int no = 0;
   if (int_deriv(c)) {  // d/dx from the filtered field in the x pass
-    int src[2];
+    C2* src[2];
     unsigned char deriv[2];
     if (dfdx) {
-      J.out[J.nout] = c->wsB; J.coef[J.nout][0] = CC_KILL; src[no] = J.nout; deriv[no] = 1; out[no++] = dfdx; J.nout++;
+      J.out[J.nout] = c->wsB; J.coef[J.nout][0] = CC_KILL; src[no] = (C2*)c->wsB; deriv[no] = 1; out[no++] = dfdx; J.nout++;
     }
     if (dfdy) {
       J.out[J.nout] = (C2*)c->wsB + (size_t)J.nout * nlev * g.C; J.coef[J.nout][0] = CC_IKY;
-      src[no] = J.nout; deriv[no] = 0; out[no++] = dfdy; J.nout++;
+      src[no] = (C2*)J.out[J.nout]; deriv[no] = 0; out[no++] = dfdy; J.nout++;
     }
     cols(c, J);
-    return c2r_deriv(c, no, nlev, c->wsB, src, deriv, out, (long)g.nplane);
+    return c2r_deriv(c, no, nlev, src, deriv, out, (long)g.nplane);
   }
   if (dfdx) { J.out[J.nout] = (C2*)c->wsB + (size_t)J.nout * nlev * g.C; J.coef[J.nout][0] = CC_IKX; out[no++] = dfdx; J.nout++; }
   if (dfdy) { J.out[J.nout] = (C2*)c->wsB + (size_t)J.nout * nlev * g.C; J.coef[J.nout][0] = CC_IKY; out[no++] = dfdy; J.nout++; }
@@ -2847,6 +2849,100 @@ __global__ void __launch_bounds__(128) k_tridiag2(const HC* __restrict__ Hx, con
   }
 }
 
+// The FP64 solve without its division: (Hz(k) - Hz(k-1)) times 1/dz, and the
+// forward recurrence as one fused multiply-add on the dependent path,
+// u = r ib - (a ib) u_below.  Eight FP64 operations per level and part instead
+// of about 24 bound it (the FP64 pipe): 256^2 x 128 pressure solve 972 -> 835 us.  Used with
+// the integer-pipe transforms; with the FP64 kernels k_tridiag2 rounds as the
+// reference does.  Loads run TRI64_D levels ahead.
+constexpr int TRI64_D = 4;
+__global__ void __launch_bounds__(128) k_tridiag64(const C2* __restrict__ Hx, const C2* __restrict__ Hy,
+                                                   const C2* __restrict__ Hz, const C2* __restrict__ bot,
+                                                   const C2* __restrict__ top, C2* P, const double* __restrict__ ibet,
+                                                   const double* __restrict__ gam, const double* __restrict__ kx,
+                                                   const double* __restrict__ ky, int lh, int ny, int nz, double dz,
+                                                   double idz) {
+  constexpr int D = TRI64_D;
+  const int nk = lh * ny;
+  const int g2 = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = g2 >> 1, part = g2 & 1;
+  if (t >= nk) return;
+  const int jx = t % lh, jy = t / lh;
+  if (t == 0 || jy == ny / 2 || jx == lh - 1) {
+    if (part == 0) tridiag_mode<C2, C2>(t, Hx, Hy, Hz, bot, top, P, ibet, gam, kx, ky, lh, ny, nz, dz);
+    return;
+  }
+  const size_t NK = (size_t)nk;
+  const int n = nz + 1;
+  // r = -+(kx hx + ky hy) + dh: the sign goes with the wavenumbers
+  const double k_x = part == 0 ? -kx[t] : kx[t], k_y = part == 0 ? -ky[t] : ky[t];
+  const double idz2 = idz * idz;
+  const double* hxp = reinterpret_cast<const double*>(Hx + t) + (part == 0 ? 1 : 0);
+  const double* hyp = reinterpret_cast<const double*>(Hy + t) + (part == 0 ? 1 : 0);
+  const double* hzp = reinterpret_cast<const double*>(Hz + t) + part;
+  const double* ibp = ibet + t;
+  double* pp = reinterpret_cast<double*>(P + t) + part;
+  const C2 b1 = bot[t], tp = top[t];
+  double up = (-dz * (part == 0 ? b1.x : b1.y)) * ibp[0];
+  pp[0] = up;
+  double hz0 = hzp[0];
+  double bx[D], by[D], bz[D], bi[D];  // row j's inputs in slot (j - 2) % D
+  auto load = [&](int j, int q) {
+    if (j <= n) bi[q] = ibp[(size_t)(j - 1) * NK];
+    if (j <= nz) {
+      bx[q] = hxp[(size_t)(j - 2) * 2 * NK];
+      by[q] = hyp[(size_t)(j - 2) * 2 * NK];
+    }
+    bz[q] = j <= nz - 1 ? hzp[(size_t)(j - 1) * 2 * NK] : 0.0;
+  };
+#pragma unroll
+  for (int q = 0; q < D; ++q) load(2 + q, q);
+  for (int jb = 2; jb <= n; jb += D) {
+#pragma unroll
+    for (int q = 0; q < D; ++q) {
+      const int j = jb + q;
+      if (j <= n) {
+        const double hx = bx[q], hy = by[q], hz1 = bz[q], ib = bi[q];
+        load(j + D, q);
+        double r, al;
+        if (j <= nz) {
+          r = fma(hz1 - hz0, idz, fma(k_x, hx, k_y * hy)) * ib;
+          al = -idz2 * ib;
+          hz0 = hz1;
+        } else {
+          r = -(part == 0 ? tp.x : tp.y) * dz * ib;
+          al = ib;
+        }
+        up = fma(al, up, r);
+        pp[(size_t)(j - 1) * 2 * NK] = up;
+      }
+    }
+  }
+  // back substitution, row j's gamma and forward value in slot (n-1-j) % D
+  const double* gp = gam + t;
+  double bg[D], bp[D];
+  auto loadb = [&](int j, int q) {
+    if (j >= 1) {
+      bg[q] = gp[(size_t)j * NK];
+      bp[q] = pp[(size_t)(j - 1) * 2 * NK];
+    }
+  };
+#pragma unroll
+  for (int q = 0; q < D; ++q) loadb(n - 1 - q, q);
+  for (int jb = n - 1; jb >= 1; jb -= D) {
+#pragma unroll
+    for (int q = 0; q < D; ++q) {
+      const int j = jb - q;
+      if (j >= 1) {
+        const double gm = bg[q], pv = bp[q];
+        loadb(j - D, q);
+        up = fma(-gm, up, pv);
+        pp[(size_t)(j - 1) * 2 * NK] = up;
+      }
+    }
+  }
+}
+
 // Mixed form: press_stag_array.f90:192-264 + tridag_array.f90:41-101 as a
 // chunked Thomas solve, the batched hybrid for many short-latency systems:
 // the z-recurrences of 16 modes (32 systems: real and imaginary parts; a, b,
@@ -3242,6 +3338,9 @@ static int pressT(les_ctx* c, double* p, double* dpdx, double* dpdy, const float
     A.dz = g.dz;
     k_tridiag_chunk<<<1 + (g.lh * g.ny + TRI_M - 1) / TRI_M, TRI_W * 32, sm, c->stream>>>(A, TRI_K2LOW);
     LES_COUNT_LAUNCH();
+  } else if (int_deriv(c)) {
+    k_tridiag64<<<(2 * g.lh * g.ny + 127) / 128, 128, 0, c->stream>>>(
+        Hx, Hy, Hz, BT, BT + g.C, P, c->ibet, c->gamt, c->kx, c->ky, g.lh, g.ny, nz, g.dz, 1.0 / g.dz); LES_COUNT_LAUNCH();
   } else {
     k_tridiag2<CX, PCX><<<(2 * g.lh * g.ny + 127) / 128, 128, 0, c->stream>>>(
         Hx, Hy, Hz, BT, BT + g.C, P, c->ibet, c->gamt, c->kx, c->ky, c->kxd, c->kyd, g.lh, g.ny, nz, g.dz,
@@ -3263,11 +3362,22 @@ static int pressT(les_ctx* c, double* p, double* dpdx, double* dpdy, const float
     ColJob L = coljob(c, MAP_SAME, DIR_INV, nz - 1);
     L.nin = 1; L.nout = 1; L.in[0] = P + g.C; L.out[0] = Yy; L.coef[0][0] = CC_IKY;
     colsT<T, PCX>(c, L);
-    k_ikx_rows<CX><<<grid1(L1), 256, 0, c->stream>>>(Y + g.C, Yx, c->kxd, c->kx, g.lh, L1, 0); LES_COUNT_LAUNCH();
     double* o0 = p;
-    c2rT<T, double>(c, 1, nz, Y, &o0, (long)g.nplane, false, g.lh);
     double* o1[2] = {dpdx, dpdy};
-    c2rT<T, double>(c, 2, nz - 1, Yx, o1, (long)g.nplane, false, g.lh);
+    c2rT<T, double>(c, 1, nz, Y, &o0, (long)g.nplane, false, g.lh);
+    bool done = false;
+    if constexpr (std::is_same<T, double>::value) {
+      if (int_deriv(c)) {  // i kx on the way into the inverse x pass
+        C2* src[2] = {Y + g.C, Yy};
+        const unsigned char deriv[2] = {1, 0};
+        c2r_deriv(c, 2, nz - 1, src, deriv, o1, (long)g.nplane);
+        done = true;
+      }
+    }
+    if (!done) {
+      k_ikx_rows<CX><<<grid1(L1), 256, 0, c->stream>>>(Y + g.C, Yx, c->kxd, c->kx, g.lh, L1, 0); LES_COUNT_LAUNCH();
+      c2rT<T, double>(c, 2, nz - 1, Yx, o1, (long)g.nplane, false, g.lh);
+    }
   }
   fill(c, dpdx + (size_t)(nz - 1) * g.nplane, g.nplane, LES_BOGUS);
   fill(c, dpdy + (size_t)(nz - 1) * g.nplane, g.nplane, LES_BOGUS);
