@@ -232,6 +232,7 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
   const int nc = ok ? J.ncols : 0;
   int ex;
   bool bad = false;
+  unsigned sum = 0;
   {
     double2 x[2 * KP + 1];  // X[k], X[M - k], and lane 0's X[M / 2]
 #pragma unroll
@@ -259,6 +260,10 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
     } else {
       ex = row_fix<TT, 2 * KP + 1>(x, g, 58, bad);
     }
+    auto put = [&](int k, cfix u) {  // element k = k1 + N1 k2 at k2 LD1 + k1
+      S[(k / N1) * LD1 + k % N1] = u;
+      sum += fix_l1<4>(u);
+    };
 #pragma unroll
     for (int i = 0; i < KP; ++i) {
       const int k = q + TT * i;
@@ -274,10 +279,10 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
         }
         cfix u;  // A[k] = E + i D, A[M - k] = conj(E - i D)
         u.x = e.x - o.y; u.y = e.y + o.x;
-        S[k] = u;
+        put(k, u);
         if (!(i == 0 && k == 0)) {
           u.x = e.x + o.y; u.y = o.x - e.y;
-          S[M - k] = u;
+          put(M - k, u);
         }
       }
     }
@@ -285,42 +290,32 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
       cfix u;
       u.x = g[2 * KP].x << 1;
       u.y = -(g[2 * KP].y << 1);
-      S[M / 2] = u;
+      put(M / 2, u);
     }
   }
-  __syncwarp();
-  cfix v[J1 * N2];
-  unsigned sum = 0;
-#pragma unroll
-  for (int j = 0; j < J1; ++j) {
-    const int k1 = q + TT * j;
-    if (N1 % TT == 0 || k1 < N1) {
-#pragma unroll
-      for (int i = 0; i < N2; ++i) {
-        v[j * N2 + i] = S[k1 + N1 * i];
-        sum += fix_l1<4>(v[j * N2 + i]);
-      }
-    }
-  }
-  // at most 24 values a lane: below 2^31 units of 2^36; the row's in units of 2^40
+  // at most 25 values a lane: below 2^31 units of 2^36; the row's in units of 2^40
   const int s = fix_down_sum(row_sum<TT>((sum >> 4) + 1u), 40);
   const i64 rnd = fix_rnd(s);
   ex += s;
   __syncwarp();
-#pragma unroll
+  // first step in place: a lane's transforms read and write their own slots,
+  // so the loop needs no registers for the others (and half the code)
+#pragma unroll 1
   for (int j = 0; j < J1; ++j) {
     const int k1 = q + TT * j;
     if (N1 % TT == 0 || k1 < N1) {
+      cfix v[N2];
 #pragma unroll
       for (int i = 0; i < N2; ++i) {
-        v[j * N2 + i].x = fix_shr(v[j * N2 + i].x, s, rnd);
-        v[j * N2 + i].y = fix_shr(v[j * N2 + i].y, s, rnd);
+        const cfix a = S[i * LD1 + k1];
+        v[i].x = fix_shr(a.x, s, rnd);
+        v[i].y = fix_shr(a.y, s, rnd);
       }
-      fdft<N2, 1>(v + j * N2);  // over k2
+      fdft<N2, 1>(v);  // over k2
 #pragma unroll
       for (int i = 0; i < N2; ++i) {
-        if (i > 0) v[j * N2 + i] = ftwc(v[j * N2 + i], __ldg(&tw[k1 * i]));
-        S[i * LD1 + k1] = v[j * N2 + i];
+        if (i > 0) v[i] = ftwc(v[i], __ldg(&tw[k1 * i]));
+        S[i * LD1 + k1] = v[i];
       }
     }
   }
