@@ -7,10 +7,23 @@ namespace les {
 // ---------------------------------------------------------------------------
 // host launchers
 
+// rows per CTA of a job.  An FP64 job of one or two planes takes single rows,
+// so that it reaches every SM (two planes of 96 x 64: 8 CTAs of 16 rows, 10 us;
+// 128 of one row, 8 us), in CTAs of two warps.
+template <typename T> inline int rows_of(const RowJob& J, int nx) {
+  int r = J.rpc > 0 ? J.rpc : rows_pc<T>(nx);
+  if (std::is_same<T, double>::value)
+    while (r > 1 && (long)((J.ny + r - 1) / r) * J.nlev * J.nfield < 2 * 152) r = (r + 1) / 2;
+  return r;
+}
+template <typename T> inline int threads_of(int work) {  // of the runtime-length kernels
+  return std::is_same<T, double>::value && work <= 256 ? 64 : 256;
+}
+
 template <typename T, typename TIn>
 int launch_rows_r2c(const RowJob& J, const RealPlanDev& P, cudaStream_t s) {
   typedef typename CT<T>::type C;
-  const int rpc = J.rpc > 0 ? J.rpc : rows_pc<T>(P.nx);
+  const int rpc = rows_of<T>(J, P.nx);
   const size_t sm = (size_t)2 * rpc * (P.nx / 2) * sizeof(C);
   RowJob JJ = J;
   JJ.dnc = FastDiv((unsigned)J.ncols);
@@ -25,7 +38,7 @@ int launch_rows_r2c(const RowJob& J, const RealPlanDev& P, cudaStream_t s) {
       cudaFuncSetAttribute(k_rows_r2c<T, TIn, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       sm_set = sm;
     }
-    k_rows_r2c<T, TIn, 0><<<grid, 256, sm, s>>>(JJ, P, rpc);
+    k_rows_r2c<T, TIn, 0><<<grid, threads_of<T>(rpc * P.nx / 2), sm, s>>>(JJ, P, rpc);
   }
   LES_COUNT_LAUNCH();
   if (pr)
@@ -36,7 +49,7 @@ int launch_rows_r2c(const RowJob& J, const RealPlanDev& P, cudaStream_t s) {
 template <typename T, typename TOut>
 int launch_rows_c2r(const RowJob& J, const RealPlanDev& P, cudaStream_t s) {
   typedef typename CT<T>::type C;
-  const int rpc = J.rpc > 0 ? J.rpc : rows_pc<T>(P.nx);
+  const int rpc = rows_of<T>(J, P.nx);
   const int m = P.nx / 2;
   const size_t sm = (size_t)rpc * ((m + 1) + 2 * m) * sizeof(C);
   dim3 grid((J.ny + rpc - 1) / rpc, J.nlev, J.nfield);
@@ -50,7 +63,7 @@ int launch_rows_c2r(const RowJob& J, const RealPlanDev& P, cudaStream_t s) {
       cudaFuncSetAttribute(k_rows_c2r<T, TOut, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       sm_set = sm;
     }
-    k_rows_c2r<T, TOut, 0><<<grid, 256, sm, s>>>(J, P, rpc);
+    k_rows_c2r<T, TOut, 0><<<grid, threads_of<T>(rpc * m), sm, s>>>(J, P, rpc);
   }
   LES_COUNT_LAUNCH();
   if (pr)
@@ -74,7 +87,7 @@ static int launch_cols_tx(const ColJob& J, const FftPlanDev& Pin, const FftPlanD
       cudaFuncSetAttribute(k_cols<T, TX, CIn>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       sm_set = sm;
     }
-    k_cols<T, TX, CIn><<<grid, 256, sm, s>>>(J, Pin, Pout);
+    k_cols<T, TX, CIn><<<grid, threads_of<T>(nymax * TX), sm, s>>>(J, Pin, Pout);
   }
   LES_COUNT_LAUNCH();
   if (pr) {
@@ -90,6 +103,11 @@ static int launch_cols_tx(const ColJob& J, const FftPlanDev& Pin, const FftPlanD
 template <typename T, typename CIn>
 int launch_cols(const ColJob& J, const FftPlanDev& Pin, const FftPlanDev& Pout, cudaStream_t s) {
   if (sizeof(T) == 8) {
+    if constexpr (std::is_same<T, double>::value) {
+      // one or two planes: single columns reach every SM
+      const long tiles = (long)((J.ncols + 3) / 4) * J.nlev * (J.nf > 0 ? J.nf : 1);
+      if (tiles < 152) return launch_cols_tx<T, 1, CIn>(J, Pin, Pout, s);
+    }
     switch (J.tx) {
       case 2: return launch_cols_tx<T, 2, CIn>(J, Pin, Pout, s);
       case 8: return launch_cols_tx<T, 8, CIn>(J, Pin, Pout, s);

@@ -101,10 +101,13 @@ static int make_plan(les_ctx* c, int n, HostPlan& hp) {
   {  // unit-circle tables exp(-2 pi i m / n), m < n
     std::vector<float2> uf(n);
     std::vector<float4> ud(n);
+    std::vector<int4> ui(n);
     for (int mm = 0; mm < n; ++mm) {
       const long double ang = -2.0L * 3.14159265358979323846264338327950288L * mm / (long double)n;
-      uf[mm] = make_float2((float)cosl(ang), (float)sinl(ang));
-      ud[mm] = ff_pair(cosl(ang), sinl(ang));
+      const long double cr = cosl(ang), ci = sinl(ang);
+      uf[mm] = make_float2((float)cr, (float)ci);
+      ud[mm] = ff_pair(cr, ci);
+      ui[mm] = fix_pair(cr, ci);
     }
     LES_CUDA_CHECK(cudaMalloc(&hp.devuf, uf.size() * sizeof(float2)));
     c->allocs.push_back(hp.devuf);
@@ -120,11 +123,6 @@ static int make_plan(les_ctx* c, int n, HostPlan& hp) {
     // difference there into one of 1e-8 in v and w within ten steps, so they
     // keep the kernels their stated errors were measured with.
     if (c->cfg.precision != 1 && !(c->cfg.model == 3 && ref_rounding_grid(c->g))) {
-      std::vector<int4> ui(n);
-      for (int mm = 0; mm < n; ++mm) {
-        const long double ang = -2.0L * 3.14159265358979323846264338327950288L * mm / (long double)n;
-        ui[mm] = fix_pair(cosl(ang), sinl(ang));
-      }
       LES_CUDA_CHECK(cudaMalloc(&hp.devui, ui.size() * sizeof(int4)));
       c->allocs.push_back(hp.devui);
       LES_CUDA_CHECK(cudaMemcpy(hp.devui, ui.data(), ui.size() * sizeof(int4), cudaMemcpyHostToDevice));
@@ -157,9 +155,10 @@ static int make_real_plan(les_ctx* c, int nx, HostRealPlan& rp) {
   std::vector<int4> wi(m + 1);
   for (int k = 0; k <= m; ++k) {
     const long double ang = -2.0L * 3.14159265358979323846264338327950288L * k / (long double)nx;
-    w[k] = make_double2((double)cosl(ang), (double)sinl(ang));
-    wd[k] = ff_pair(cosl(ang), sinl(ang));
-    wi[k] = fix_pair(cosl(ang), sinl(ang));
+    const long double cr = cosl(ang), ci = sinl(ang);
+    w[k] = make_double2((double)cr, (double)ci);
+    wd[k] = ff_pair(cr, ci);
+    wi[k] = fix_pair(cr, ci);
   }
   LES_CUDA_CHECK(cudaMalloc(&rp.devi, wi.size() * sizeof(int4)));
   c->allocs.push_back(rp.devi);
@@ -233,8 +232,8 @@ static Sizes sizes_of(const Grid& g, bool q, bool m7) {
   s.spare = 4 * g.nfield * sizeof(double) + (4 * nz + 4) * C * sizeof(double2) + 2 * (nz + 1) * C * sizeof(double);
   // saved spectra, wall-plane spectra, Thomas tables, reductions, wavenumber
   // and filter tables (FP64 + FP32)
-  s.aux = 4 * nz * C * sizeof(double2) + 4 * C * sizeof(double2) + 2 * (nz + 1) * C * sizeof(double) +
-          (36 * (nz + 8) + 64) * sizeof(double) + 5 * C * sizeof(double) + 4 * C * sizeof(float) +
+  s.aux = 4 * nz * C * sizeof(double2) + 8 * C * sizeof(double2) + 2 * (nz + 1) * C * sizeof(double) +
+          (45 * (nz + 8) + 96) * sizeof(double) + 5 * C * sizeof(double) + 4 * C * sizeof(float) +
           2 * C * sizeof(float2);
   return s;
 }
@@ -339,6 +338,12 @@ int les_ctx_create(const les_config* cfg, les_ctx** out) {
     les_set_error("stream creation failed"); delete c; return LES_ERR_CUDA;
   }
   c->own_stream = true;
+  if (cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->side_fork, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->side_done, cudaEventDisableTiming) != cudaSuccess) {
+    les_set_error("stream creation failed");
+    return fail(LES_ERR_CUDA);
+  }
   for (int f = 0; f < LES_NUM_FIELDS; ++f) {
     c->fsize[f] = felems(c, f);
     if (c->fsize[f] == 0) continue;  // not stored in this configuration (null pointer)
@@ -410,6 +415,11 @@ int les_ctx_create(const les_config* cfg, les_ctx** out) {
       (st = dalloc(c, (void**)&c->big, s.big)) || (st = dalloc(c, (void**)&c->tmp, s.tmp)) ||
       (st = dalloc(c, (void**)&c->spare, s.spare)) || (st = dalloc(c, (void**)&c->dscal, 64 * sizeof(double))) ||
       (st = dalloc(c, (void**)&c->dred, 36 * (size_t)(g.nz + 8) * sizeof(double))) ||
+      (st = dalloc(c, (void**)&c->psum, 8 * (size_t)(g.nz + 8) * sizeof(double))) ||
+      (st = dalloc(c, (void**)&c->pcount, 2 * (size_t)(g.nz + 8) * sizeof(unsigned))) ||
+      (st = dalloc(c, (void**)&c->psumS, 16 * sizeof(double))) ||
+      (st = dalloc(c, (void**)&c->pcountS, sizeof(unsigned))) ||
+      (st = dalloc(c, &c->wsS, 4 * g.C * sizeof(double2))) ||
       (st = dalloc(c, (void**)&c->spec, 4 * (size_t)g.nz * g.C * sizeof(double2))) ||
       (st = dalloc(c, (void**)&c->wspec, 4 * g.C * sizeof(double2))) ||
       (st = dalloc(c, (void**)&c->ibet, (size_t)(g.nz + 1) * g.C * sizeof(double))) ||
@@ -439,6 +449,10 @@ int les_ctx_destroy(les_ctx* c) {
         if (c->gexec[a][b][p]) cudaGraphExecDestroy(c->gexec[a][b][p]);
   for (void* p : c->allocs) cudaFree(p);
   if (c->host_scal) cudaFreeHost(c->host_scal);
+  if (c->side) cudaStreamSynchronize(c->side);
+  if (c->side_fork) cudaEventDestroy(c->side_fork);
+  if (c->side_done) cudaEventDestroy(c->side_done);
+  if (c->side) cudaStreamDestroy(c->side);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return LES_OK;
@@ -456,15 +470,19 @@ int les_ctx_set_priority(les_ctx* c, int priority) {
   int lo = 0, hi = 0;
   LES_CUDA_CHECK(cudaDeviceGetStreamPriorityRange(&lo, &hi));  // lo least urgent, hi most urgent
   const int p = std::max(hi, std::min(lo, priority));
-  cudaStream_t s = nullptr;
+  cudaStream_t s = nullptr, sd = nullptr;
   LES_CUDA_CHECK(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, p));
-  if (cudaStreamSynchronize(c->stream) != cudaSuccess) {
+  if (cudaStreamCreateWithPriority(&sd, cudaStreamNonBlocking, p) != cudaSuccess ||
+      cudaStreamSynchronize(c->stream) != cudaSuccess) {
     cudaStreamDestroy(s);
+    if (sd) cudaStreamDestroy(sd);
     les_set_error("%s", cudaGetErrorString(cudaGetLastError()));
     return LES_ERR_CUDA;
   }
   cudaStreamDestroy(c->stream);
+  cudaStreamDestroy(c->side);  // its work is joined into the stream within each step
   c->stream = s;
+  c->side = sd;
   return LES_OK;
 }
 size_t les_ctx_device_bytes(const les_ctx* c) { return c ? c->bytes : 0; }

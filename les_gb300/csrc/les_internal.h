@@ -69,6 +69,14 @@ struct les_ctx {
   les::Grid g;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
+  // A second stream for the step's chains on one or two planes (surface filter
+  // and obukhov, wall-plane spectra), which are too short to fill the GPU: they
+  // run beside the volume kernels, with workspaces of their own, and are joined
+  // back into `stream` before their results are read and within the step.
+  cudaStream_t side = nullptr;
+  cudaEvent_t side_fork = nullptr, side_done = nullptr;
+  bool side_open = false;                      // side work not yet joined
+  void* wsS = nullptr;                         // plane spectra of the side stream: 4 C complex
   int device = 0;
   int ptr_mode = 0;  // 0 host pointers, 1 device pointers
   int jt = 0, jt_total = 0;
@@ -110,10 +118,13 @@ struct les_ctx {
   // rmsdiv partials / model-3 Cs(z); 2..11 scaledep sums; 12..13
   // timestep_conditions partial maxima; 14 theta, 15 qmix plane means
   // (mixed); 16..18 u, v, w plane means (mixed filt_da); 20..21 the (virtual)
-  // theta level mean and its reciprocal (calcbeta); 24..27 partial plane sums;
-  // 28..33 the mixed form's per-level mean-wind factors (float-float);
+  // theta level mean and its reciprocal (calcbeta); 28..33 the mixed form's per-level mean-wind factors (float-float);
   // 34..35 the mixed form's txz, tyz plane means
   double* dred = nullptr;
+  double* psum = nullptr;                      // partial plane sums, 8 (nz + 8)
+  unsigned* pcount = nullptr;                  // finished parts per plane, 2 (nz + 8)
+  double* psumS = nullptr;                     // the same for one plane on the side stream
+  unsigned* pcountS = nullptr;
   // running statistics (MM_XYZ_Out): 133 accumulators of nx ny (nz-1)
   double* stats = nullptr;
   int stats_c = 0, stats_p = 0, stats_auto = 0;

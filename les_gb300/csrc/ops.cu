@@ -59,6 +59,19 @@ static void fill(les_ctx* c, double* p, size_t n, double v) {
   if (n) { k_fill<<<grid1(n), 256, 0, c->stream>>>(p, n, v); LES_COUNT_LAUNCH(); }
 }
 
+// one plane of three arrays at once
+__global__ void k_fill3(double* a, double* b, double* d, size_t n, double v) {
+  GSTRIDE(i, n) { a[i] = v; b[i] = v; d[i] = v; }
+}
+static void fill3(les_ctx* c, double* a, double* b, double* d, size_t n, double v) {
+  k_fill3<<<grid1(n), 256, 0, c->stream>>>(a, b, d, n, v);
+  LES_COUNT_LAUNCH();
+}
+// Kernels on one surface plane: blocks of one warp, so that a small plane
+// reaches every SM (FP64 logarithms and powers: 96 x 64 points in 24 blocks of
+// 256 took 48 us, in 192 of 32 25 us)
+constexpr int SFC_BS = 32;
+
 // ---------------------------------------------------------------------------
 // spectral pipeline helpers (T: transform precision; TIn/TOut: physical storage)
 template <typename T, typename TIn>
@@ -187,6 +200,42 @@ static int colsT(les_ctx* c, const ColJob& J0) {
 static int cols(les_ctx* c, const ColJob& J) { return colsT<double, double2>(c, J); }
 
 // ---------------------------------------------------------------------------
+// side stream: between side_begin and side_end every launch goes to it, with
+// the side workspaces in place of wsA, wsB and the plane-sum scratch; what it
+// reads must be complete on the stream at side_begin, and what it writes is
+// read after side_join only
+static void side_swap(les_ctx* c) {
+  std::swap(c->stream, c->side);
+  std::swap(c->psum, c->psumS);
+  std::swap(c->pcount, c->pcountS);
+}
+struct SideWork {
+  les_ctx* c;
+  void *a, *b;
+  explicit SideWork(les_ctx* c_) : c(c_), a(c_->wsA), b(c_->wsB) {
+    cudaEventRecord(c->side_fork, c->stream);
+    cudaStreamWaitEvent(c->side, c->side_fork, 0);
+    side_swap(c);
+    c->wsA = c->wsS;
+    c->wsB = (C2*)c->wsS + 2 * c->g.C;
+  }
+  ~SideWork() {
+    cudaEventRecord(c->side_done, c->stream);
+    side_swap(c);
+    c->wsA = a;
+    c->wsB = b;
+    c->side_open = true;
+  }
+  SideWork(const SideWork&) = delete;
+  SideWork& operator=(const SideWork&) = delete;
+};
+static void side_join(les_ctx* c) {
+  if (!c->side_open) return;
+  cudaStreamWaitEvent(c->stream, c->side_done, 0);
+  c->side_open = false;
+}
+
+// ---------------------------------------------------------------------------
 // deterministic reductions (fixed order, fixed tree)
 // Sum of f(1:nx, r0+1:r1) of one plane per block (512 threads): warp w takes
 // rows r0+w, r0+w+16, ..; lane l the columns l, l+32, ..; four independent
@@ -207,42 +256,61 @@ __device__ __forceinline__ double plane_sum_block(const TI* p, int ld, int nx, i
   }
   sh[threadIdx.x] = (a0 + a1) + (a2 + a3);
   __syncthreads();
-  for (int w = 256; w > 0; w >>= 1) {
+  for (int w = 256; w > 16; w >>= 1) {
     if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
     __syncthreads();
   }
-  return sh[0];
+  double t = sh[lane];  // the last five levels of the tree within the first warp
+  if (wid == 0) {
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) t += __shfl_down_sync(0xffffffffu, t, w);
+  }
+  return t;  // thread 0 holds the sum
 }
-// Row-split plane sums: block (q, j) sums rows [q rows, (q+1) rows) of plane
-// j into part[j nsplit + q]; k_plane_fin adds the nsplit partial sums of a
-// plane in order and divides by div (1: sums; nx*ny: means).  Several blocks
+// Row-split plane sums: block (q, j, f) sums rows [q rows, (q+1) rows) of plane
+// j of field f; the block that finishes a plane last adds the nsplit partial
+// sums in order and divides by div (1: sums; nx*ny: means).  Several blocks
 // per plane keep more loads in flight than one block per plane; the order
-// stays fixed, so the result is deterministic.
+// stays fixed, so the result is deterministic.  The counters wrap to zero.
+template <typename TI> struct PlaneSums {
+  const TI* f[2];
+  double* out[2];
+};
 template <typename TI>
-__global__ void __launch_bounds__(512) k_plane_part(const TI* f, long pstride, int ld, int nx, int ny, int rows,
-                                                    double* part) {
+__global__ void __launch_bounds__(512) k_plane_sums(PlaneSums<TI> A, long pstride, int ld, int nx, int ny, int rows,
+                                                    double div, double* part, unsigned* count) {
   __shared__ double sh[512];
+  const int nsplit = gridDim.x, j = blockIdx.y, f = blockIdx.z;
   const int r0 = blockIdx.x * rows, r1 = min(r0 + rows, ny);
-  const double t = plane_sum_block(f + (size_t)blockIdx.y * pstride, ld, nx, r0, r1, sh);
-  if (threadIdx.x == 0) part[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = t;
-}
-__global__ void k_plane_fin(const double* __restrict__ part, int nsplit, int nplanes, double div, double* out) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < nplanes) {
-    double s = 0.0;
-    for (int q = 0; q < nsplit; ++q) s += part[(size_t)j * nsplit + q];
-    out[j] = s / div;
+  const double t = plane_sum_block(A.f[f] + (size_t)j * pstride, ld, nx, r0, r1, sh);
+  if (threadIdx.x == 0) {
+    const size_t pl = (size_t)f * gridDim.y + j;
+    volatile double* p = part + pl * nsplit;
+    p[blockIdx.x] = t;
+    __threadfence();
+    if (atomicInc(&count[pl], (unsigned)nsplit - 1u) == (unsigned)nsplit - 1u) {
+      __threadfence();
+      double s = 0.0;
+      for (int q = 0; q < nsplit; ++q) s += p[q];
+      A.out[f][j] = s / div;
+    }
   }
 }
-// sums (div 1) or means (div nx*ny) of f(1:nx,1:ny) over nplanes planes;
-// nsplit * nplanes <= 4 (nz + 8)
+// sums (div 1) or means (div nx*ny) of f(1:nx,1:ny) over nplanes planes of nf
+// fields; nf * nplanes <= 2 (nz + 8), nsplit * nf * nplanes <= 8 (nz + 8)
+template <typename TI>
+static void plane_sums(les_ctx* c, const TI* const* f, double* const* out, int nf, long pstride, int nplanes, int nsplit,
+                       double div) {
+  const Grid& g = c->g;
+  PlaneSums<TI> A{};
+  for (int q = 0; q < nf; ++q) { A.f[q] = f[q]; A.out[q] = out[q]; }
+  const int rows = (g.ny + nsplit - 1) / nsplit;
+  k_plane_sums<TI><<<dim3(nsplit, nplanes, nf), 512, 0, c->stream>>>(A, pstride, g.ld, g.nx, g.ny, rows, div, c->psum,
+                                                                     c->pcount); LES_COUNT_LAUNCH();
+}
 template <typename TI>
 static void plane_sums(les_ctx* c, const TI* f, long pstride, int nplanes, int nsplit, double div, double* out) {
-  const Grid& g = c->g;
-  double* part = c->dred + 24 * (size_t)(g.nz + 8);
-  const int rows = (g.ny + nsplit - 1) / nsplit;
-  k_plane_part<TI><<<dim3(nsplit, nplanes), 512, 0, c->stream>>>(f, pstride, g.ld, g.nx, g.ny, rows, part); LES_COUNT_LAUNCH();
-  k_plane_fin<<<(nplanes + 127) / 128, 128, 0, c->stream>>>(part, nsplit, nplanes, div, out); LES_COUNT_LAUNCH();
+  plane_sums<TI>(c, &f, &out, 1, pstride, nplanes, nsplit, div);
 }
 
 // ---------------------------------------------------------------------------
@@ -262,6 +330,31 @@ __global__ void __launch_bounds__(256) k_ddz(double* __restrict__ dfdz, const do
   } else {
     dfdz[i] = cst * (f[i + np] - f[i]);
   }
+}
+// the three velocity components' z derivatives in one launch (level planes of
+// small grids are short)
+__global__ void __launch_bounds__(256) k_ddz3(double* __restrict__ du, double* __restrict__ dv, double* __restrict__ dw,
+                                              const double* __restrict__ u, const double* __restrict__ v,
+                                              const double* __restrict__ w, int ld, int nx, int ny, int nz, double cst) {
+  const unsigned np = (unsigned)ld * ny;
+  const unsigned r = blockIdx.x * 256u + threadIdx.x;
+  if (r >= np) return;
+  const int jz = blockIdx.y + 1;
+  const size_t i = (size_t)(jz - 1) * np + r;
+  if (jz == nz) { du[i] = 0.0; dv[i] = 0.0; dw[i] = 0.0; return; }
+  if ((int)(r % (unsigned)ld) >= nx) return;
+  if (jz >= 2) {
+    du[i] = cst * (u[i] - u[i - np]);
+    dv[i] = cst * (v[i] - v[i - np]);
+  }
+  dw[i] = cst * (w[i + np] - w[i]);
+}
+static void op_ddz3(les_ctx* c) {
+  const Grid& g = c->g;
+  k_ddz3<<<dim3((unsigned)((g.nplane + 255) / 256), (unsigned)g.nz), 256, 0, c->stream>>>(
+      c->f[LES_DUDZ], c->f[LES_DVDZ], c->f[LES_DWDZ], c->f[LES_U], c->f[LES_V], c->f[LES_W], g.ld, g.nx, g.ny, g.nz,
+      1.0 / g.dz);
+  LES_COUNT_LAUNCH();
 }
 int op_ddz(les_ctx* c, double* dfdz, const double* f, int uv) {
   const Grid& g = c->g;
@@ -801,10 +894,13 @@ __global__ void k_obukhov_init(double* psi_m, double* psi_m0, double* psi_h, dou
 // G_test_test-filtered surface u, v (test_filtermodule.f90:13-30 on the
 // first level; obukhov and wallstress filter the same planes) as one
 // two-field job: u1 at uv1, v1 at uv1 + nplane
-static void surface_uv_filtered(les_ctx* c, double* uv1) {
+static void surface_uv_spectra(les_ctx* c, void* ws) {  // x pass of the surface u, v into ws
   const Grid& g = c->g;
   const double* in[2] = {c->f[LES_U], c->f[LES_V]};
-  r2c(c, 2, 1, in, (long)g.nplane, nullptr, nullptr, c->wsA, false, g.lh);
+  r2c(c, 2, 1, in, (long)g.nplane, nullptr, nullptr, ws, false, g.lh);
+}
+static void surface_uv_inverse(les_ctx* c, double* uv1) {  // the rest, from wsA
+  const Grid& g = c->g;
   ColJob J = coljob(c, MAP_SAME, DIR_BOTH, 1);
   J.nin = 1; J.nout = 1; J.nf = 2;
   J.in[0] = c->wsA; J.fs_in = (long)g.C;
@@ -814,6 +910,10 @@ static void surface_uv_filtered(les_ctx* c, double* uv1) {
   double* out[2] = {uv1, uv1 + g.nplane};
   c2r(c, 2, 1, c->wsB, out, (long)g.nplane, false, g.lh);
 }
+static void surface_uv_filtered(les_ctx* c, double* uv1) {
+  surface_uv_spectra(c, c->wsA);
+  surface_uv_inverse(c, uv1);
+}
 // uv1: the filtered surface planes when the caller already has them, else
 // null (filtered here into the first two temp planes)
 int op_obukhov(les_ctx* c, const double* uv1) {
@@ -821,7 +921,7 @@ int op_obukhov(les_ctx* c, const double* uv1) {
   const les_config& k = c->cfg;
   const size_t ns = (size_t)g.nx * g.ny;
   if (c->jt == 1) {  // SCAL_init = 1 (scalars_module.f90:525-542)
-    k_obukhov_init<<<grid1(ns), 256, 0, c->stream>>>(c->f[LES_PSI_M], c->f[LES_PSI_M0], c->f[LES_PSI_H],
+    k_obukhov_init<<<grid1(ns, SFC_BS), SFC_BS, 0, c->stream>>>(c->f[LES_PSI_M], c->f[LES_PSI_M0], c->f[LES_PSI_H],
                                                      c->f[LES_PSI_H0], c->f[LES_SGS_T3_SFC], c->f[LES_WT_S],
                                                      c->f[LES_SGS_Q3_SFC], c->f[LES_WQ_S], ns, k.initsc,
                                                      k.u_star * k.t_scale, k.u_star * k.q_scale); LES_COUNT_LAUNCH();
@@ -834,7 +934,7 @@ int op_obukhov(les_ctx* c, const double* uv1) {
   const double* u1 = uv1;
   const double* v1 = uv1 + g.nplane;
   const double g_ = (k.g * k.z_i) / (k.u_star * k.u_star);
-  k_obukhov<<<grid1(ns), 256, 0, c->stream>>>(u1, v1, c->f[LES_THETA], c->f[LES_ZO], c->z_os,
+  k_obukhov<<<grid1(ns, SFC_BS), SFC_BS, 0, c->stream>>>(u1, v1, c->f[LES_THETA], c->f[LES_ZO], c->z_os,
                                               c->f[LES_SGS_T3_SFC], c->f[LES_USTAR_AVG], c->f[LES_PSI_M],
                                               c->f[LES_PSI_M0], c->f[LES_PSI_H], c->f[LES_PSI_H0],
                                               c->f[LES_PHI_M], c->f[LES_PHI_H], c->dscal + 0,
@@ -876,12 +976,12 @@ int op_wallstress(les_ctx* c, const double* uv1) {
   const double* u1 = uv1;
   const double* v1 = uv1 + g.nplane;
   if (c->cfg.precision == 1)
-    k_wallstress<float><<<grid1((size_t)g.nx * g.ny), 256, 0, c->stream>>>(
+    k_wallstress<float><<<grid1((size_t)g.nx * g.ny, SFC_BS), SFC_BS, 0, c->stream>>>(
         c->f[LES_U], c->f[LES_V], u1, v1, c->f[LES_ZO], c->f[LES_PSI_M], c->f[LES_PSI_M0], c->f[LES_PHI_M],
         c->f[LES_USTAR_AVG], f32(c, LES_TXZ), f32(c, LES_TYZ), c->f[LES_DUDZ], c->f[LES_DVDZ], g.nx, g.ny, g.ld,
         g.dz, c->cfg.vonk);
   else
-    k_wallstress<double><<<grid1((size_t)g.nx * g.ny), 256, 0, c->stream>>>(
+    k_wallstress<double><<<grid1((size_t)g.nx * g.ny, SFC_BS), SFC_BS, 0, c->stream>>>(
         c->f[LES_U], c->f[LES_V], u1, v1, c->f[LES_ZO], c->f[LES_PSI_M], c->f[LES_PSI_M0], c->f[LES_PHI_M],
         c->f[LES_USTAR_AVG], c->f[LES_TXZ], c->f[LES_TYZ], c->f[LES_DUDZ], c->f[LES_DVDZ], g.nx, g.ny, g.ld,
         g.dz, c->cfg.vonk);
@@ -2241,9 +2341,7 @@ int op_convec(les_ctx* c, double* cx, double* cy, double* cz) {
   const double* bins[3] = {bigf[6], bigf[7], bigf[8]};
   op_dealias2(c, outs, bins, 3, g.nz - 1, 1.0 / (double)(g.nx2 * g.ny2));
   const size_t top = (size_t)(g.nz - 1) * g.nplane;
-  fill(c, cx + top, g.nplane, LES_BOGUS);
-  fill(c, cy + top, g.nplane, LES_BOGUS);
-  fill(c, cz + top, g.nplane, LES_BOGUS);
+  fill3(c, cx + top, cy + top, cz + top, g.nplane, LES_BOGUS);
   return 0;
 }
 
@@ -3259,9 +3357,27 @@ int thomas_tables(les_ctx* c) {
 
 // T: transform precision of the three field transforms and the spectra H,
 // p-hat (double: FP64 form and the per-routine entry; dfloat: mixed form).
-// The wall planes' spectra and the tridiagonal solve are FP64 in both.
+// The wall planes' spectra and the tridiagonal solve are FP64 in both; walls:
+// form those spectra here (the step has them from the side stream).
+static C2* press_wall_spectra(les_ctx* c) {  // bottom, top: behind the spectra H of u*, v*, w* (16-byte complex)
+  return (C2*)c->wsP + (size_t)3 * (c->g.nz - 1) * c->g.C;
+}
+// bottomw, topw from divtz(1), divtz(nz) scaled by 1/(nx*ny)
+static void press_walls(les_ctx* c) {
+  const Grid& g = c->g;
+  const double cst = 1.0 / (double)(g.nx * g.ny);
+  const double* bi[2] = {c->f[LES_DIVTZ], c->f[LES_DIVTZ] + (size_t)(g.nz - 1) * g.nplane};
+  const double sc2[2] = {cst, cst};
+  r2c(c, 2, 1, bi, (long)g.nplane, sc2, nullptr, (C2*)c->wsA, false, g.lh);
+  ColJob K = coljob(c, MAP_SAME, DIR_FWD, 1);
+  K.nin = 1; K.nout = 1; K.nf = 2;
+  K.in[0] = c->wsA; K.fs_in = (long)g.C;
+  K.out[0] = press_wall_spectra(c); K.fs_out = (long)g.C;
+  K.coef[0][0] = CC_KILL;
+  cols(c, K);
+}
 template <typename T>
-static int pressT(les_ctx* c, double* p, double* dpdx, double* dpdy, const float2* const* ustar = nullptr) {
+static int pressT(les_ctx* c, double* p, double* dpdx, double* dpdy, bool walls, const float2* const* ustar = nullptr) {
   typedef typename CT<T>::type CX;
   const Grid& g = c->g;
   const les_config& k = c->cfg;
@@ -3285,7 +3401,8 @@ static int pressT(les_ctx* c, double* p, double* dpdx, double* dpdy, const float
     r2cT<T, double>(c, 3, nz - 1, in, (long)g.nplane, sc3, dv3, c->wsA, false, g.lh);
   }
   CX* H = (CX*)c->wsP;                                       // 3*(nz-1)*C
-  C2* BT = reinterpret_cast<C2*>(H + (size_t)3 * (nz - 1) * g.C);  // bottom, top
+  static_assert(sizeof(CX) == sizeof(C2), "press_wall_spectra");
+  C2* BT = press_wall_spectra(c);                            // bottom, top
   // p-hat in the transform precision (float-float in the mixed form)
   typedef CX PCX;
   PCX* P = reinterpret_cast<PCX*>(BT + 2 * g.C);            // (nz+1)*C
@@ -3295,18 +3412,8 @@ static int pressT(les_ctx* c, double* p, double* dpdx, double* dpdy, const float
   J.out[0] = H; J.fs_out = (long)(nz - 1) * g.C;
   J.coef[0][0] = CC_KILL;
   colsT<T, CX>(c, J);
-  // bottomw, topw from divtz(1), divtz(nz) scaled by 1/(nx*ny)
-  {
-    const double* bi[2] = {c->f[LES_DIVTZ], c->f[LES_DIVTZ] + (size_t)(nz - 1) * g.nplane};
-    const double sc2[2] = {cst, cst};
-    r2c(c, 2, 1, bi, (long)g.nplane, sc2, nullptr, (C2*)c->wsA, false, g.lh);
-    ColJob K = coljob(c, MAP_SAME, DIR_FWD, 1);
-    K.nin = 1; K.nout = 1; K.nf = 2;
-    K.in[0] = c->wsA; K.fs_in = (long)g.C;
-    K.out[0] = BT; K.fs_out = (long)g.C;
-    K.coef[0][0] = CC_KILL;
-    cols(c, K);
-  }
+  if (walls) press_walls(c);
+  else side_join(c);
   const CX* Hx = H;
   const CX* Hy = H + (size_t)(nz - 1) * g.C;
   const CX* Hz = H + (size_t)2 * (nz - 1) * g.C;
@@ -3379,14 +3486,13 @@ static int pressT(les_ctx* c, double* p, double* dpdx, double* dpdy, const float
       c2rT<T, double>(c, 2, nz - 1, Yx, o1, (long)g.nplane, false, g.lh);
     }
   }
-  fill(c, dpdx + (size_t)(nz - 1) * g.nplane, g.nplane, LES_BOGUS);
-  fill(c, dpdy + (size_t)(nz - 1) * g.nplane, g.nplane, LES_BOGUS);
-  fill(c, p + (size_t)nz * g.nplane, g.nplane, LES_BOGUS);
+  fill3(c, dpdx + (size_t)(nz - 1) * g.nplane, dpdy + (size_t)(nz - 1) * g.nplane, p + (size_t)nz * g.nplane, g.nplane,
+        LES_BOGUS);
   return 0;
 }
 int op_press(les_ctx* c, double* p, double* dpdx, double* dpdy) {
   const RefRounding scope(c);
-  return pressT<double>(c, p, dpdx, dpdy);
+  return pressT<double>(c, p, dpdx, dpdy, true);
 }
 
 // tridag_array.f90:1-109 with caller-supplied coefficients (per-routine entry)
@@ -3697,7 +3803,7 @@ static int op_scalar(les_ctx* c, const ScalarDesc& d) {
   fill(c, c->f[d.dsdz] + (size_t)(nz - 1) * g.nplane, g.nplane, d.top_grad);
   // RHS_Tf = RHS_T (RHS_T is fully rewritten below)
   cudaMemcpyAsync(c->f[d.rhsf], c->f[d.rhs], g.nfield * sizeof(double), cudaMemcpyDeviceToDevice, c->stream);
-  k_sflux<<<grid1((size_t)g.nx * g.ny), 256, 0, c->stream>>>(c->f[d.s], c->f[d.flux], c->f[LES_PHI_H],
+  k_sflux<<<grid1((size_t)g.nx * g.ny, SFC_BS), SFC_BS, 0, c->stream>>>(c->f[d.s], c->f[d.flux], c->f[LES_PHI_H],
                                                             c->f[LES_USTAR_AVG], c->f[d.dsdz],
                                                             c->f[d.sgs3], g.nx, g.ny, g.ld,
                                                             d.flux_scale, k.vonk, g.dz); LES_COUNT_LAUNCH();
@@ -4260,6 +4366,7 @@ static int lagrangeT(les_ctx* c) {
   const les_config& k = c->cfg;
   if (MX) op_interpolag32(c);
   else op_interpolag(c);
+  side_join(c);  // wall-plane spectra
   const double delta = g.delta;
   const double cst = 2.0 * (delta * delta);
   const double opftdelta = 1.5 * delta;
@@ -4493,8 +4600,8 @@ static int divstressT(les_ctx* c, double* divtx, double* divty, double* divtz) {
     const size_t ms = (size_t)g.nz + 8;
     double* m13 = c->dred + 34 * ms;
     double* m23 = c->dred + 35 * ms;
-    plane_sums(c, in[3], (long)g.nplane, g.nz, 4, (double)(g.nx * g.ny), m13);
-    plane_sums(c, in[4], (long)g.nplane, g.nz, 4, (double)(g.nx * g.ny), m23);
+    double* m[2] = {m13, m23};
+    plane_sums<TS>(c, in + 3, m, 2, (long)g.nplane, g.nz, 4, (double)(g.nx * g.ny));
     offs[3] = m13;
     offs[4] = m23;
   }
@@ -4580,7 +4687,7 @@ static int scalarT(les_ctx* c, typename PX<M>::S* const* bigf, const ScalarDesc&
   op_ddz(c, c->f[d.dsdz], c->f[d.s], 1);
   fill(c, c->f[d.dsdz] + (size_t)(nz - 1) * g.nplane, g.nplane, d.top_grad);
   // RHS_Tf = RHS_T: exchanged with the momentum RHS at the start of the step
-  k_sflux<<<grid1((size_t)g.nx * g.ny), 256, 0, c->stream>>>(c->f[d.s], c->f[d.flux], c->f[LES_PHI_H],
+  k_sflux<<<grid1((size_t)g.nx * g.ny, SFC_BS), SFC_BS, 0, c->stream>>>(c->f[d.s], c->f[d.flux], c->f[LES_PHI_H],
                                                             c->f[LES_USTAR_AVG], c->f[d.dsdz],
                                                             c->f[d.sgs3], g.nx, g.ny, g.ld,
                                                             d.flux_scale, k.vonk, g.dz); LES_COUNT_LAUNCH();
@@ -4689,9 +4796,7 @@ static int convecT(les_ctx* c, typename PX<M>::S* const* bigf, double* cx, doubl
     unpadT<M>(c, bins, outs, 3, g.nz - 1, MX ? 1.0 : cst2);
   }
   const size_t top = (size_t)(g.nz - 1) * g.nplane;
-  fill(c, cx + top, g.nplane, LES_BOGUS);
-  fill(c, cy + top, g.nplane, LES_BOGUS);
-  fill(c, cz + top, g.nplane, LES_BOGUS);
+  fill3(c, cx + top, cy + top, cz + top, g.nplane, LES_BOGUS);
   return 0;
 }
 
@@ -4827,8 +4932,14 @@ static int stepT(les_ctx* c) {
   // filtered surface u, v for obukhov and wallstress (u, v do not change in
   // between): the last two temp planes, which nothing before wallstress uses
   const double* uv1 = c->tmp + (size_t)(c->ntmp - 2) * g.nplane;
-  surface_uv_filtered(c, const_cast<double*>(uv1));
-  op_obukhov(c, uv1);
+  // beside filt_da: the x pass reads the unfiltered u, v here, the rest only its
+  // result and theta
+  surface_uv_spectra(c, c->wsS);
+  {
+    const SideWork side(c);
+    surface_uv_inverse(c, const_cast<double*>(uv1));
+    op_obukhov(c, uv1);
+  }
   if (M == 2) {
     filt_da_uvw_ff(c);
   } else if (!MX) {
@@ -4840,13 +4951,14 @@ static int stepT(les_ctx* c) {
     filt_da_uvw_mixed(c);
     meanflow_lin(c);
   }
-  op_ddz(c, c->f[LES_DUDZ], c->f[LES_U], 1);
-  op_ddz(c, c->f[LES_DVDZ], c->f[LES_V], 1);
-  op_ddz(c, c->f[LES_DWDZ], c->f[LES_W], 0);
+  op_ddz3(c);
   const bool rms_step = k.rmsdiv_every > 0 && c->jt % k.rmsdiv_every == 0;
   if (MX && rms_step) rmsdiv_mixed(c, c->tmp, c->f[LES_DWDZ], c->dscal + 1);
+  side_join(c);
   op_wallstress(c, uv1);
-  {  // spectra of the wall planes dudz(1), dvdz(1) set by wallstress
+  {  // spectra of the wall planes dudz(1), dvdz(1) set by wallstress, read by
+     // lagrangeT and convecT
+    const SideWork side(c);
     const double cs = 1.0 / (double)(g.nx * g.ny);
     const double* pl[2] = {c->f[LES_DUDZ], c->f[LES_DVDZ]};
     const double sc[2] = {cs, cs};
@@ -4867,6 +4979,11 @@ static int stepT(les_ctx* c) {
     fill(c, c->f[LES_BETA_SCAL], g.nfield, 0.0);
   }
   divstressT<M>(c, c->f[LES_DIVTX], c->f[LES_DIVTY], c->f[LES_DIVTZ]);
+  side_join(c);  // the wall-plane spectra, for convecT
+  {
+    const SideWork side(c);
+    press_walls(c);
+  }
   convecT<M>(c, bigf, c->f[LES_RHSX], c->f[LES_RHSY], c->f[LES_RHSZ]);
   const size_t nv = g.nplane * (g.nz - 1);
   const int euler = (c->jt == 1 && !k.initu) ? 1 : 0;
@@ -4888,7 +5005,7 @@ static int stepT(les_ctx* c) {
   if (MX) {
     const float2* ust = ustar_fields(c);
     const float2* u3[3] = {ust, ust + g.nfield, ust + 2 * g.nfield};
-    pressT<dfloat>(c, c->f[LES_P], c->f[LES_DPDX], c->f[LES_DPDY], u3);
+    pressT<dfloat>(c, c->f[LES_P], c->f[LES_DPDX], c->f[LES_DPDY], false, u3);
     k_dpdz_project32<<<dim3((unsigned)((g.nplane + 255) / 256), (unsigned)(g.nz - 1)), 256, 0, c->stream>>>(
         c->f[LES_U], c->f[LES_V], c->f[LES_W], u3[0], u3[1], u3[2], ff2(c, LES_RHSX), ff2(c, LES_RHSY),
         ff2(c, LES_RHSZ), c->f[LES_P], c->f[LES_DPDX], c->f[LES_DPDY], c->f[LES_DPDZ], g.ld, g.nx, g.ny, g.nz,
@@ -4897,7 +5014,7 @@ static int stepT(les_ctx* c) {
     // FP64 projection in the FP64 form and in the float-float transform form:
     // float-float transforms of the predictor would leave its rounding times
     // the wavenumber in the divergence (rmsdiv 4e-12 instead of 1e-13 at 128^3)
-    pressT<double>(c, c->f[LES_P], c->f[LES_DPDX], c->f[LES_DPDY]);
+    pressT<double>(c, c->f[LES_P], c->f[LES_DPDX], c->f[LES_DPDY], false);
   }
   if (!MX)
     k_dpdz_project<<<dim3((unsigned)((g.nplane + 255) / 256), (unsigned)(g.nz - 1)), 256, 0, c->stream>>>(
