@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cstdio>
+#include <utility>
 
 #define LES_PI 3.1415926535897932384626433   /* param.f90:51 */
 #define LES_BOGUS (-1234567890.0)              /* param.f90:50 */
@@ -179,6 +180,38 @@ extern unsigned long long g_les_launches;
 #define LES_COUNT_LAUNCH() (++g_les_launches)
 
 namespace les {
+// Launches with programmatic stream serialization: a kernel may be scheduled
+// while the one before it in its stream drains, and its first statement,
+// pdl_wait(), holds it until that kernel has finished and its writes are
+// visible.  Kernel to kernel in a graph 1.0 to 1.15 -> 0.76 to 0.9 us (8 to 304
+// blocks), in a stream 3.1 to 4.1 -> 1.6 us.  Every kernel launched this way
+// begins with pdl_wait(), also one that needs nothing from its predecessor:
+// the order of all earlier work rests on it.
+template <class... P> struct PdlCall {
+  void (*kernel)(P...);
+  dim3 grid, block;
+  size_t smem;
+  cudaStream_t stream;
+  template <class... A> void operator()(A&&... args) const {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kernel, P(std::forward<A>(args))...);
+  }
+};
+template <class... P>
+PdlCall<P...> pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem = 0, cudaStream_t stream = 0) {
+  return PdlCall<P...>{kernel, grid, block, smem, stream};
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Measurement hook (les_profile_begin/end): while a session is open, every
 // launch of one kernel family on the session's stream is bracketed by CUDA
 // events and its algorithmic bytes (inputs read once + outputs written once)

@@ -51,7 +51,7 @@ void r2c_fixed(const RowJob& J, const RealPlanDev& P, int rpc, cudaStream_t s) {
     static size_t set2 = 48 * 1024;
     raise_smem(k_r2c_reg2<T, TIn, A1, A2, AT, G::NT>, G::smem(), set2);
     const dim3 grid((J.ny + G::RPB - 1) / G::RPB, J.nlev, J.nfield);
-    k_r2c_reg2<T, TIn, A1, A2, AT, G::NT><<<grid, G::NT, G::smem(), s>>>(J, P);
+    pdl(k_r2c_reg2<T, TIn, A1, A2, AT, G::NT>, grid, G::NT, G::smem(), s)(J, P);
     return;
   }
   constexpr int N1 = RowSplit<NF>::n1, N2 = RowSplit<NF>::n2;
@@ -60,14 +60,14 @@ void r2c_fixed(const RowJob& J, const RealPlanDev& P, int rpc, cudaStream_t s) {
     static size_t set = 48 * 1024;
     raise_smem(k_r2c_reg<T, TIn, N1, N2, G::NT>, G::smem(), set);
     const dim3 grid((J.ny + G::RPB - 1) / G::RPB, J.nlev, J.nfield);
-    k_r2c_reg<T, TIn, N1, N2, G::NT><<<grid, G::NT, G::smem(), s>>>(J, P);
+    pdl(k_r2c_reg<T, TIn, N1, N2, G::NT>, grid, G::NT, G::smem(), s)(J, P);
     return;
   }
   const size_t smf = ((size_t)2 * rpc * skn(NF) + 2 * NF + 1) * sizeof(C);
   static size_t set = 48 * 1024;
   raise_smem(k_rows_r2c<T, TIn, NF>, smf, set);
   const dim3 grid((J.ny + rpc - 1) / rpc, J.nlev, J.nfield);
-  k_rows_r2c<T, TIn, NF><<<grid, 256, smf, s>>>(J, P, rpc);
+  pdl(k_rows_r2c<T, TIn, NF>, grid, 256, smf, s)(J, P, rpc);
 }
 template <typename T, typename TOut, int NF>
 void c2r_fixed(const RowJob& J, const RealPlanDev& P, int rpc, cudaStream_t s) {
@@ -78,7 +78,7 @@ void c2r_fixed(const RowJob& J, const RealPlanDev& P, int rpc, cudaStream_t s) {
     static size_t set2 = 48 * 1024;
     raise_smem(k_c2r_reg2<T, TOut, A1, A2, AT, G::NT>, G::smem(), set2);
     const dim3 grid((J.ny + G::RPB - 1) / G::RPB, J.nlev, J.nfield);
-    k_c2r_reg2<T, TOut, A1, A2, AT, G::NT><<<grid, G::NT, G::smem(), s>>>(J, P);
+    pdl(k_c2r_reg2<T, TOut, A1, A2, AT, G::NT>, grid, G::NT, G::smem(), s)(J, P);
     return;
   }
   constexpr int N1 = RowSplit<NF>::n1, N2 = RowSplit<NF>::n2;
@@ -87,14 +87,14 @@ void c2r_fixed(const RowJob& J, const RealPlanDev& P, int rpc, cudaStream_t s) {
     static size_t set = 48 * 1024;
     raise_smem(k_c2r_reg<T, TOut, N1, N2, G::NT>, G::smem(), set);
     const dim3 grid((J.ny + G::RPB - 1) / G::RPB, J.nlev, J.nfield);
-    k_c2r_reg<T, TOut, N1, N2, G::NT><<<grid, G::NT, G::smem(), s>>>(J, P);
+    pdl(k_c2r_reg<T, TOut, N1, N2, G::NT>, grid, G::NT, G::smem(), s)(J, P);
     return;
   }
   const size_t smf = ((size_t)rpc * (NF + 1) + (size_t)2 * rpc * skn(NF) + 2 * NF + 1) * sizeof(C);
   static size_t set = 48 * 1024;
   raise_smem(k_rows_c2r<T, TOut, NF>, smf, set);
   const dim3 grid((J.ny + rpc - 1) / rpc, J.nlev, J.nfield);
-  k_rows_c2r<T, TOut, NF><<<grid, 256, smf, s>>>(J, P, rpc);
+  pdl(k_rows_c2r<T, TOut, NF>, grid, 256, smf, s)(J, P, rpc);
 }
 // register-resident y pass (FP32, one input, same length N = R * R), 16 kx
 // columns per CTA.  The float-float transforms keep the shared-memory
@@ -121,7 +121,7 @@ void cols_reg(const ColJob& J, const FftPlanDev& P, cudaStream_t s) {
   const int ntile = (J.ncols + TX - 1) / TX;
   const int nitems = ntile * J.nlev * (J.nf > 0 ? J.nf : 1);
   const int nblk = std::min(nitems, 3 * nsm);  // three resident CTAs per SM (registers, shared memory)
-  k_colsr<T, TX, CIn, R><<<nblk, TX * R, smf, s>>>(J, P, ntile, nitems);
+  pdl(k_colsr<T, TX, CIn, R>, nblk, TX * R, smf, s)(J, P, ntile, nitems);
 }
 
 // several inputs summed into at most two outputs, same length N = R * R
@@ -133,7 +133,7 @@ void cols_reg_sum(const ColJob& J, const FftPlanDev& P, cudaStream_t s) {
   static size_t set = 48 * 1024;
   raise_smem(k_colsr_sum<T, TX, CIn, R, 2>, smf, set);
   const dim3 grid((J.ncols + TX - 1) / TX, J.nlev, J.nf > 0 ? J.nf : 1);
-  k_colsr_sum<T, TX, CIn, R, 2><<<grid, TX * R, smf, s>>>(J, P);
+  pdl(k_colsr_sum<T, TX, CIn, R, 2>, grid, TX * R, smf, s)(J, P);
 }
 
 // register-resident 3/2 padding / truncation (FP32), 16 kx columns per CTA
@@ -146,7 +146,7 @@ void cols_pad(const ColJob& J, const FftPlanDev& Pin, const FftPlanDev& Pout, cu
   static size_t set = 48 * 1024;
   raise_smem(k_colsr_pad<T, TX, CIn, NIN, NOUT>, smf, set);
   const dim3 grid((J.ncols + TX - 1) / TX, J.nlev, J.nf > 0 ? J.nf : 1);
-  k_colsr_pad<T, TX, CIn, NIN, NOUT><<<grid, TX * PS::tt, smf, s>>>(J, Pin, Pout);
+  pdl(k_colsr_pad<T, TX, CIn, NIN, NOUT>, grid, TX * PS::tt, smf, s)(J, Pin, Pout);
 }
 
 template <typename T, int TX, typename CIn, int NIN, int NOUT>
@@ -175,7 +175,7 @@ void cols_fixed(const ColJob& J, const FftPlanDev& Pin, const FftPlanDev& Pout, 
   const size_t smf = ((size_t)(J.nin * skn(NIN) + 2 * PMAX) * TX + NIN + NOUT) * sizeof(C);
   static size_t set = 48 * 1024;
   raise_smem(k_colsf<T, TX, CIn, NIN, NOUT>, smf, set);
-  k_colsf<T, TX, CIn, NIN, NOUT><<<grid, 256, smf, s>>>(J, Pin, Pout);
+  pdl(k_colsf<T, TX, CIn, NIN, NOUT>, grid, 256, smf, s)(J, Pin, Pout);
 }
 
 }  // namespace

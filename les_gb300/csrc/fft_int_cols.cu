@@ -221,6 +221,7 @@ __device__ __forceinline__ bool col_direct(const ColJob& J, int o) {  // needs n
 template <int N1, int N2, int MB, int DIR, bool MULTI>
 __global__ void __launch_bounds__(ICOL_TX * (N1 > N2 ? N1 : N2), MB)
     k_icol(ColJob J, const int4* __restrict__ tw, int total, int ndirect, int nspec, int ngen) {
+  pdl_wait();
   constexpr int TX = ICOL_TX, N = N1 * N2, NV = N1 > N2 ? N1 : N2, NT = TX * NV;
   static_assert(NT % 32 == 0 && N1 % 2 == 0, "whole warps; row parity by thread");
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -363,6 +364,7 @@ __global__ void __launch_bounds__(ICOL_TX * (N1 > N2 ? N1 : N2), MB)
 template <int N1, int N2, int MB>
 __global__ void __launch_bounds__(ICOL_TX * (N1 > N2 ? N1 : N2), MB)
     k_icol_div(ColJob J, const int4* __restrict__ tw, int total) {
+  pdl_wait();
   constexpr int TX = ICOL_TX, N = N1 * N2, NV = N1 > N2 ? N1 : N2, NT = TX * NV, NW = NT / 32;
   static_assert(NT % 32 == 0 && N1 % 2 == 0, "whole warps; row parity by thread");
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -440,6 +442,7 @@ template <int A1, int A2, int B1, int B2, int MB> struct PadT {
 template <int A1, int A2, int B1, int B2, int MB>
 __global__ void __launch_bounds__(ICOL_TX * (PadT<A1, A2, B1, B2, MB>::nv), MB)
     k_icol_pad(ColJob J, const int4* __restrict__ twa, const int4* __restrict__ twb, int total) {
+  pdl_wait();
   typedef PadT<A1, A2, B1, B2, MB> PT;
   constexpr int TX = ICOL_TX, NA = PT::NA, NB = PT::NB, NV = PT::nv, NT = TX * NV;
   constexpr bool PAD = NB > NA;
@@ -537,7 +540,7 @@ template <int N1, int N2, int MB> bool run_same(const ColJob& J, const FftPlanDe
     const size_t sm = (size_t)(N1 * N2 + (ng > 1 ? NV * NV : 0)) * TX * sizeof(cfix);
     auto run = [&](auto kernel, size_t& set) {
       smem_of(kernel, sm, set);
-      kernel<<<grid, NT, sm, s>>>(J, P.uniti, total, nd, ns, ng);
+      pdl(kernel, grid, NT, sm, s)(J, P.uniti, total, nd, ns, ng);
     };
     static size_t set[5] = {40 * 1024, 40 * 1024, 40 * 1024, 40 * 1024, 40 * 1024};  // the static arrays count too
     if (J.dir == DIR_FWD && ng == 0) run(k_icol<N1, N2, MB, DIR_FWD, false>, set[0]);
@@ -569,7 +572,7 @@ template <int N1, int N2, int MB> bool run_same(const ColJob& J, const FftPlanDe
     K.in[0] = J.in[a[o]];
     K.in[1] = J.in[c[o]];
     K.out[0] = J.out[o];
-    k_icol_div<N1, N2, MB><<<grid, NT, sm, s>>>(K, P.uniti, total);
+    pdl(k_icol_div<N1, N2, MB>, grid, NT, sm, s)(K, P.uniti, total);
     if (o > 0) LES_COUNT_LAUNCH();  // the caller counts one
   }
   return true;
@@ -586,7 +589,7 @@ bool run_pad(const ColJob& J, const FftPlanDev& Pa, const FftPlanDev& Pb, cudaSt
   const size_t sm = (size_t)std::max(PT::NA, PT::NB) * TX * sizeof(cfix);
   static size_t set = 40 * 1024;  // the static arrays count too
   smem_of(k_icol_pad<A1, A2, B1, B2, MB>, sm, set);
-  k_icol_pad<A1, A2, B1, B2, MB><<<dim3((total + TX - 1) / TX, J.nf > 0 ? J.nf : 1), TX * PT::nv, sm, s>>>(
+  pdl(k_icol_pad<A1, A2, B1, B2, MB>, dim3((total + TX - 1) / TX, J.nf > 0 ? J.nf : 1), TX * PT::nv, sm, s)(
       J, Pa.uniti, Pb.uniti, total);
   return true;
 }

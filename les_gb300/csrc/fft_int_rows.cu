@@ -105,6 +105,7 @@ template <int N1, int N2, int TT> struct RowShape {
 template <int N1, int N2, int TT, int MB>
 __global__ void __launch_bounds__(128, MB) k_ir2c(RowJob J, const int4* __restrict__ tw, const int4* __restrict__ wr,
                                                   int nrows) {
+  pdl_wait();
   typedef RowShape<N1, N2, TT> R;
   constexpr int M = R::M, J1 = R::J1, J2 = R::J2, LD1 = R::LD1;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -220,6 +221,7 @@ __global__ void __launch_bounds__(128, MB) k_ir2c(RowJob J, const int4* __restri
 template <int N1, int N2, int TT, int MB>
 __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restrict__ tw, const int4* __restrict__ wr,
                                                   int nrows) {
+  pdl_wait();
   typedef RowShape<N1, N2, TT> R;
   constexpr int M = R::M, J1 = R::J1, J2 = R::J2, LD1 = R::LD1, KP = R::KP;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -357,7 +359,7 @@ void run_r2c(const RowJob& J, const RealPlanDev& P, cudaStream_t s) {
     set = true;
   }
   const int nrows = J.ny * J.nlev;
-  k_ir2c<N1, N2, TT, MB><<<(nrows + R::RPB - 1) / R::RPB * J.nfield, R::NT, R::smem, s>>>(J, P.c.uniti, P.wi, nrows);
+  pdl(k_ir2c<N1, N2, TT, MB>, (nrows + R::RPB - 1) / R::RPB * J.nfield, R::NT, R::smem, s)(J, P.c.uniti, P.wi, nrows);
 }
 template <int N1, int N2, int TT, int MB>
 void run_c2r(const RowJob& J, const RealPlanDev& P, cudaStream_t s) {
@@ -369,7 +371,7 @@ void run_c2r(const RowJob& J, const RealPlanDev& P, cudaStream_t s) {
     set = true;
   }
   const int nrows = J.ny * J.nlev;
-  k_ic2r<N1, N2, TT, MB><<<(nrows + R::RPB - 1) / R::RPB * J.nfield, R::NT, R::smem, s>>>(J, P.c.uniti, P.wi, nrows);
+  pdl(k_ic2r<N1, N2, TT, MB>, (nrows + R::RPB - 1) / R::RPB * J.nfield, R::NT, R::smem, s)(J, P.c.uniti, P.wi, nrows);
 }
 
 }  // namespace

@@ -38,7 +38,7 @@ int launch_rows_r2c(const RowJob& J, const RealPlanDev& P, cudaStream_t s) {
       cudaFuncSetAttribute(k_rows_r2c<T, TIn, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       sm_set = sm;
     }
-    k_rows_r2c<T, TIn, 0><<<grid, threads_of<T>(rpc * P.nx / 2), sm, s>>>(JJ, P, rpc);
+    pdl(k_rows_r2c<T, TIn, 0>, grid, threads_of<T>(rpc * P.nx / 2), sm, s)(JJ, P, rpc);
   }
   LES_COUNT_LAUNCH();
   if (pr)
@@ -63,7 +63,7 @@ int launch_rows_c2r(const RowJob& J, const RealPlanDev& P, cudaStream_t s) {
       cudaFuncSetAttribute(k_rows_c2r<T, TOut, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       sm_set = sm;
     }
-    k_rows_c2r<T, TOut, 0><<<grid, threads_of<T>(rpc * m), sm, s>>>(J, P, rpc);
+    pdl(k_rows_c2r<T, TOut, 0>, grid, threads_of<T>(rpc * m), sm, s)(J, P, rpc);
   }
   LES_COUNT_LAUNCH();
   if (pr)
@@ -87,7 +87,7 @@ static int launch_cols_tx(const ColJob& J, const FftPlanDev& Pin, const FftPlanD
       cudaFuncSetAttribute(k_cols<T, TX, CIn>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       sm_set = sm;
     }
-    k_cols<T, TX, CIn><<<grid, threads_of<T>(nymax * TX), sm, s>>>(J, Pin, Pout);
+    pdl(k_cols<T, TX, CIn>, grid, threads_of<T>(nymax * TX), sm, s)(J, Pin, Pout);
   }
   LES_COUNT_LAUNCH();
   if (pr) {

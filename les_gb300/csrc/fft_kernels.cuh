@@ -54,6 +54,7 @@ template <typename T, typename TIn> __device__ __forceinline__ T sub_off(TIn x, 
 // transform, twiddles staged in shared memory after the work buffers).
 template <typename T, typename TIn, int NF>
 __global__ void __launch_bounds__(256) k_rows_r2c(RowJob J, RealPlanDev P, int rpc) {
+  pdl_wait();
   typedef typename CT<T>::type C;
   extern __shared__ __align__(16) unsigned char smraw[];
   C* A = reinterpret_cast<C*>(smraw);
@@ -120,6 +121,7 @@ __global__ void __launch_bounds__(256) k_rows_r2c(RowJob J, RealPlanDev P, int r
 // rows_c2r: inverse x-transform.  Reads J.ncols complex columns (rest zero).
 template <typename T, typename TOut, int NF>
 __global__ void __launch_bounds__(256) k_rows_c2r(RowJob J, RealPlanDev P, int rpc) {
+  pdl_wait();
   typedef typename CT<T>::type C;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int m = NF > 0 ? NF : P.nx / 2;
@@ -229,6 +231,7 @@ __device__ __forceinline__ void stage_rows_warp(C* S, const C* base, size_t wc, 
 // writes the real pairs n2 + N2 n1 of the row.
 template <typename T, typename TIn, int N1, int N2, int NT>
 __global__ void __launch_bounds__(NT) k_r2c_reg(RowJob J, RealPlanDev P) {
+  pdl_wait();
   typedef typename CT<T>::type C;
   typedef typename CT<TIn>::type CI;
   constexpr int M = N1 * N2, TT = N1 > N2 ? N1 : N2, RPB = NT / TT, MS = N2 * (N1 + 1);
@@ -320,6 +323,7 @@ __global__ void __launch_bounds__(NT) k_r2c_reg(RowJob J, RealPlanDev P) {
 
 template <typename T, typename TOut, int N1, int N2, int NT>
 __global__ void __launch_bounds__(NT) k_c2r_reg(RowJob J, RealPlanDev P) {
+  pdl_wait();
   typedef typename CT<T>::type C;
   typedef typename CT<TOut>::type CO;
   constexpr int M = N1 * N2, TT = N1 > N2 ? N1 : N2, RPB = NT / TT, MS = N2 * (N1 + 1);
@@ -402,6 +406,7 @@ __global__ void __launch_bounds__(NT) k_c2r_reg(RowJob J, RealPlanDev P) {
 // eight threads per row).
 template <typename T, typename TIn, int N1, int N2, int TT, int NT>
 __global__ void __launch_bounds__(NT, 5) k_r2c_reg2(RowJob J, RealPlanDev P) {
+  pdl_wait();
   typedef typename CT<T>::type C;
   typedef typename CT<TIn>::type CI;
   static_assert(N1 % TT == 0 && N2 % TT == 0 && NT % TT == 0, "thread split");
@@ -497,6 +502,7 @@ __global__ void __launch_bounds__(NT, 5) k_r2c_reg2(RowJob J, RealPlanDev P) {
 
 template <typename T, typename TOut, int N1, int N2, int TT, int NT>
 __global__ void __launch_bounds__(NT, 5) k_c2r_reg2(RowJob J, RealPlanDev P) {
+  pdl_wait();
   typedef typename CT<T>::type C;
   typedef typename CT<TOut>::type CO;
   static_assert(N1 % TT == 0 && N2 % TT == 0 && NT % TT == 0, "thread split");
@@ -626,6 +632,7 @@ __device__ __forceinline__ typename CT<T>::type apply_coef_k(int code, typename 
 // the lengths the workloads use.
 template <typename T, int TX, typename CIn>
 __global__ void __launch_bounds__(256) k_cols(ColJob J, FftPlanDev Pin, FftPlanDev Pout) {
+  pdl_wait();
   typedef typename CT<T>::type C;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int ny_in = J.ny_in, ny_out = J.ny_out;
@@ -755,6 +762,7 @@ __device__ __forceinline__ void coef_rows(const typename CT<T>::type* __restrict
 }
 template <typename T, int TX, typename CIn, int NIN, int NOUT>
 __global__ void __launch_bounds__(256) k_colsf(ColJob J, FftPlanDev Pin, FftPlanDev Pout) {
+  pdl_wait();
   typedef typename CT<T>::type C;
   static_assert(256 % TX == 0, "tile width divides the block");
   constexpr int RS = 256 / TX;
@@ -869,6 +877,7 @@ __device__ __forceinline__ void dft_r(typename CT<T>::type* v, int sign) {
 // staging needs no barrier.  8-byte elements (FP32 complex).
 template <typename T, int TX, typename CIn, int R>
 __global__ void __launch_bounds__(TX * R, 3) k_colsr(ColJob J, FftPlanDev P, int ntile, int nitems) {
+  pdl_wait();
   typedef typename CT<T>::type C;
   static_assert(sizeof(CIn) == 8 && sizeof(C) == 8, "8-byte complex elements");
   constexpr int N = R * R;
@@ -1010,6 +1019,7 @@ template <int NIN, int NOUT> struct PadShape {
 template <typename T, int TX, typename CIn, int NIN, int NOUT>
 __global__ void __launch_bounds__(TX * PadShape<NIN, NOUT>::tt, 2) k_colsr_pad(ColJob J, FftPlanDev Pin,
                                                                                  FftPlanDev Pout) {
+  pdl_wait();
   typedef typename CT<T>::type C;
   typedef PadShape<NIN, NOUT> PS;
   constexpr int A = PS::a, B = PS::b, NS = PS::ns, NB = PS::nb, TT = PS::tt;
@@ -1098,6 +1108,7 @@ __global__ void __launch_bounds__(TX * PadShape<NIN, NOUT>::tt, 2) k_colsr_pad(C
 // memory.  Same four-step split and exchange as k_colsr.
 template <typename T, int TX, typename CIn, int R, int NO>
 __global__ void __launch_bounds__(TX * R, 2) k_colsr_sum(ColJob J, FftPlanDev P) {
+  pdl_wait();
   typedef typename CT<T>::type C;
   constexpr int N = R * R;
   extern __shared__ __align__(16) unsigned char smraw[];

@@ -1447,6 +1447,7 @@ int les_test_filter_init(les_ctx* c, double alpha, double* G) {
 
 namespace les {
 __global__ void k_padd(double2* ub, const double2* us, int lh, int ny, int lhb, int ny2, int nx, int np) {
+  pdl_wait();
   const size_t tot = (size_t)lhb * ny2 * np;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < tot; i += (size_t)gridDim.x * blockDim.x) {
     const int p = (int)(i / ((size_t)lhb * ny2));
@@ -1463,6 +1464,7 @@ __global__ void k_padd(double2* ub, const double2* us, int lh, int ny, int lhb, 
   }
 }
 __global__ void k_unpadd(double2* cc, const double2* cb, int lh, int ny, int lhb, int ny2, int nx, int np) {
+  pdl_wait();
   const size_t tot = (size_t)lh * ny * np;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < tot; i += (size_t)gridDim.x * blockDim.x) {
     const int p = (int)(i / ((size_t)lh * ny));
@@ -1484,7 +1486,7 @@ int les_padd(les_ctx* c, double* u_big, const double* u, int nplanes) {
   const Grid& g = c->g;
   Arg B(c, u_big, g.nplane_big * nplanes), S(c, u, g.nplane * nplanes);
   CHK(B.alloc()); CHK(S.in());
-  k_padd<<<256, 256, 0, c->stream>>>((double2*)B.dev, (const double2*)S.dev, g.lh, g.ny, g.lh_big, g.ny2, g.nx, nplanes); LES_COUNT_LAUNCH();
+  pdl(k_padd, 256, 256, 0, c->stream)((double2*)B.dev, (const double2*)S.dev, g.lh, g.ny, g.lh_big, g.ny2, g.nx, nplanes); LES_COUNT_LAUNCH();
   CHK(B.out());
   return finish(c);
 }
@@ -1493,7 +1495,7 @@ int les_unpadd(les_ctx* c, double* cc, const double* cc_big, int nplanes) {
   const Grid& g = c->g;
   Arg S(c, cc, g.nplane * nplanes), B(c, cc_big, g.nplane_big * nplanes);
   CHK(S.alloc()); CHK(B.in());
-  k_unpadd<<<256, 256, 0, c->stream>>>((double2*)S.dev, (const double2*)B.dev, g.lh, g.ny, g.lh_big, g.ny2, g.nx, nplanes); LES_COUNT_LAUNCH();
+  pdl(k_unpadd, 256, 256, 0, c->stream)((double2*)S.dev, (const double2*)B.dev, g.lh, g.ny, g.lh_big, g.ny2, g.nx, nplanes); LES_COUNT_LAUNCH();
   CHK(S.out());
   return finish(c);
 }

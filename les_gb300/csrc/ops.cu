@@ -22,6 +22,7 @@ __device__ __forceinline__ unsigned long long splitmix64(unsigned long long x) {
   return x ^ (x >> 31);
 }
 __global__ void k_cvt_selftest(size_t n, unsigned long long seed, unsigned long long* bad) {
+  pdl_wait();
   unsigned long long nb = 0;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const unsigned long long r = splitmix64(seed + i);
@@ -40,7 +41,7 @@ __global__ void k_cvt_selftest(size_t n, unsigned long long seed, unsigned long 
   if (nb) atomicAdd(bad, nb);
 }
 int op_cvt_selftest(size_t n, unsigned long long seed, unsigned long long* bad_dev, cudaStream_t s) {
-  k_cvt_selftest<<<152 * 4, 256, 0, s>>>(n, seed, bad_dev); LES_COUNT_LAUNCH();
+  pdl(k_cvt_selftest, 152 * 4, 256, 0, s)(n, seed, bad_dev); LES_COUNT_LAUNCH();
   return 0;
 }
 
@@ -54,17 +55,18 @@ static inline dim3 grid1(size_t n, int bs = 256) {
 }
 #define GSTRIDE(i, n) for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (n); i += (size_t)gridDim.x * blockDim.x)
 
-__global__ void k_fill(double* p, size_t n, double v) { GSTRIDE(i, n) p[i] = v; }
+__global__ void k_fill(double* p, size_t n, double v) { pdl_wait(); GSTRIDE(i, n) p[i] = v; }
 static void fill(les_ctx* c, double* p, size_t n, double v) {
-  if (n) { k_fill<<<grid1(n), 256, 0, c->stream>>>(p, n, v); LES_COUNT_LAUNCH(); }
+  if (n) { pdl(k_fill, grid1(n), 256, 0, c->stream)(p, n, v); LES_COUNT_LAUNCH(); }
 }
 
 // one plane of three arrays at once
 __global__ void k_fill3(double* a, double* b, double* d, size_t n, double v) {
+  pdl_wait();
   GSTRIDE(i, n) { a[i] = v; b[i] = v; d[i] = v; }
 }
 static void fill3(les_ctx* c, double* a, double* b, double* d, size_t n, double v) {
-  k_fill3<<<grid1(n), 256, 0, c->stream>>>(a, b, d, n, v);
+  pdl(k_fill3, grid1(n), 256, 0, c->stream)(a, b, d, n, v);
   LES_COUNT_LAUNCH();
 }
 // Kernels on one surface plane: blocks of one warp, so that a small plane
@@ -279,6 +281,7 @@ template <typename TI> struct PlaneSums {
 template <typename TI>
 __global__ void __launch_bounds__(512) k_plane_sums(PlaneSums<TI> A, long pstride, int ld, int nx, int ny, int rows,
                                                     double div, double* part, unsigned* count) {
+  pdl_wait();
   __shared__ double sh[512];
   const int nsplit = gridDim.x, j = blockIdx.y, f = blockIdx.z;
   const int r0 = blockIdx.x * rows, r1 = min(r0 + rows, ny);
@@ -305,7 +308,7 @@ static void plane_sums(les_ctx* c, const TI* const* f, double* const* out, int n
   PlaneSums<TI> A{};
   for (int q = 0; q < nf; ++q) { A.f[q] = f[q]; A.out[q] = out[q]; }
   const int rows = (g.ny + nsplit - 1) / nsplit;
-  k_plane_sums<TI><<<dim3(nsplit, nplanes, nf), 512, 0, c->stream>>>(A, pstride, g.ld, g.nx, g.ny, rows, div, c->psum,
+  pdl(k_plane_sums<TI>, dim3(nsplit, nplanes, nf), 512, 0, c->stream)(A, pstride, g.ld, g.nx, g.ny, rows, div, c->psum,
                                                                      c->pcount); LES_COUNT_LAUNCH();
 }
 template <typename TI>
@@ -318,6 +321,7 @@ static void plane_sums(les_ctx* c, const TI* f, long pstride, int nplanes, int n
 // grid (ceil(np/256), nz): no 64-bit index division
 __global__ void __launch_bounds__(256) k_ddz(double* __restrict__ dfdz, const double* __restrict__ f, int ld,
                                              int nx, int ny, int nz, double cst, int uv) {
+  pdl_wait();
   const unsigned np = (unsigned)ld * ny;
   const unsigned r = blockIdx.x * 256u + threadIdx.x;
   if (r >= np) return;
@@ -336,6 +340,7 @@ __global__ void __launch_bounds__(256) k_ddz(double* __restrict__ dfdz, const do
 __global__ void __launch_bounds__(256) k_ddz3(double* __restrict__ du, double* __restrict__ dv, double* __restrict__ dw,
                                               const double* __restrict__ u, const double* __restrict__ v,
                                               const double* __restrict__ w, int ld, int nx, int ny, int nz, double cst) {
+  pdl_wait();
   const unsigned np = (unsigned)ld * ny;
   const unsigned r = blockIdx.x * 256u + threadIdx.x;
   if (r >= np) return;
@@ -351,14 +356,14 @@ __global__ void __launch_bounds__(256) k_ddz3(double* __restrict__ du, double* _
 }
 static void op_ddz3(les_ctx* c) {
   const Grid& g = c->g;
-  k_ddz3<<<dim3((unsigned)((g.nplane + 255) / 256), (unsigned)g.nz), 256, 0, c->stream>>>(
+  pdl(k_ddz3, dim3((unsigned)((g.nplane + 255) / 256), (unsigned)g.nz), 256, 0, c->stream)(
       c->f[LES_DUDZ], c->f[LES_DVDZ], c->f[LES_DWDZ], c->f[LES_U], c->f[LES_V], c->f[LES_W], g.ld, g.nx, g.ny, g.nz,
       1.0 / g.dz);
   LES_COUNT_LAUNCH();
 }
 int op_ddz(les_ctx* c, double* dfdz, const double* f, int uv) {
   const Grid& g = c->g;
-  k_ddz<<<dim3((unsigned)((g.nplane + 255) / 256), (unsigned)g.nz), 256, 0, c->stream>>>(dfdz, f, g.ld, g.nx, g.ny,
+  pdl(k_ddz, dim3((unsigned)((g.nplane + 255) / 256), (unsigned)g.nz), 256, 0, c->stream)(dfdz, f, g.ld, g.nx, g.ny,
                                                                                       g.nz, 1.0 / g.dz, uv);
   LES_COUNT_LAUNCH();
   return 0;
@@ -458,6 +463,7 @@ struct NyqScratch {
 template <int K>
 __global__ void k_nyq_part(const double* f0, const double* f1, const double* f2, NyqScratch S, int ld, int nx,
                            int ny, long ps, int nlev, int nch) {
+  pdl_wait();
   __shared__ double ws[8][NYQ_ROWS], wd[8][NYQ_ROWS];
   const int ch = blockIdx.x, lev = blockIdx.y, fld = blockIdx.z;
   const double* f = (fld == 0 ? f0 : fld == 1 ? f1 : f2) + (size_t)lev * ps;
@@ -518,6 +524,7 @@ template <int KP>
 __global__ void __launch_bounds__(128) k_nyq_part_rows(const double* f0, const double* f1, const double* f2,
                                                       NyqScratch S, int ld, int nx, int ny, long ps, int nlev,
                                                       int nch) {
+  pdl_wait();
   // per-lane partial row sums over even / odd x, summed once per row below
   // (31 adds per row instead of a 5-step warp reduction on every lane)
   __shared__ double pse[NYQ_ROWS][33], pso[NYQ_ROWS][33], ws[NYQ_ROWS];
@@ -576,6 +583,7 @@ __global__ void __launch_bounds__(128) k_nyq_part_rows(const double* f0, const d
 }
 __global__ void __launch_bounds__(256) k_nyq_comb(NyqScratch S, double* mean, int mstride, int nx, int ny, int nlev,
                                                   int nch) {
+  pdl_wait();
   __shared__ double red[256];
   const int lev = blockIdx.x, fld = blockIdx.y;
   const size_t pl = (size_t)fld * nlev + lev;
@@ -607,6 +615,7 @@ __global__ void __launch_bounds__(256) k_nyq_comb(NyqScratch S, double* mean, in
 // / 256), nf nlev).
 __global__ void __launch_bounds__(256) k_nyq_apply(double* f0, double* f1, double* f2, NyqScratch S, int ld,
                                                    int nx, int ny, long ps, int nlev) {
+  pdl_wait();
   const int np1 = nx / 2 + 1;  // pairs per row, the last one the padding columns
   const unsigned r = blockIdx.x * 256u + threadIdx.x;
   if (r >= (unsigned)ny * np1) return;
@@ -648,22 +657,22 @@ static void nyq_kill(les_ctx* c, double* const* f, int nf, int nlev, double* mea
   const size_t smr = (size_t)4 * np * sizeof(double2);
   if (KP <= 8) {
     switch (KP) {
-      case 1: k_nyq_part_rows<1><<<grid, 128, smr, c->stream>>>(f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev, nch); break;
-      case 2: k_nyq_part_rows<2><<<grid, 128, smr, c->stream>>>(f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev, nch); break;
-      case 3: case 4: k_nyq_part_rows<4><<<grid, 128, smr, c->stream>>>(f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev, nch); break;
-      default: k_nyq_part_rows<8><<<grid, 128, smr, c->stream>>>(f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev, nch); break;
+      case 1: pdl(k_nyq_part_rows<1>, grid, 128, smr, c->stream)(f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev, nch); break;
+      case 2: pdl(k_nyq_part_rows<2>, grid, 128, smr, c->stream)(f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev, nch); break;
+      case 3: case 4: pdl(k_nyq_part_rows<4>, grid, 128, smr, c->stream)(f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev, nch); break;
+      default: pdl(k_nyq_part_rows<8>, grid, 128, smr, c->stream)(f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev, nch); break;
     }
   } else switch (K) {
-    case 1: k_nyq_part<1><<<grid, bt, 0, c->stream>>>(f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev, nch); break;
-    case 2: k_nyq_part<2><<<grid, bt, 0, c->stream>>>(f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev, nch); break;
-    case 3: case 4: k_nyq_part<4><<<grid, bt, 0, c->stream>>>(f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev, nch); break;
+    case 1: pdl(k_nyq_part<1>, grid, bt, 0, c->stream)(f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev, nch); break;
+    case 2: pdl(k_nyq_part<2>, grid, bt, 0, c->stream)(f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev, nch); break;
+    case 3: case 4: pdl(k_nyq_part<4>, grid, bt, 0, c->stream)(f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev, nch); break;
     case 5: case 6: case 7: case 8:
-      k_nyq_part<8><<<grid, bt, 0, c->stream>>>(f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev, nch); break;
-    default: k_nyq_part<16><<<grid, bt, 0, c->stream>>>(f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev, nch); break;
+      pdl(k_nyq_part<8>, grid, bt, 0, c->stream)(f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev, nch); break;
+    default: pdl(k_nyq_part<16>, grid, bt, 0, c->stream)(f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev, nch); break;
   }
   LES_COUNT_LAUNCH();
-  k_nyq_comb<<<dim3(nlev, nf), 256, 0, c->stream>>>(S, mean, mstride, g.nx, g.ny, nlev, nch); LES_COUNT_LAUNCH();
-  k_nyq_apply<<<dim3((unsigned)((g.ny * (np + 1) + 255) / 256), (unsigned)npl), 256, 0, c->stream>>>(
+  pdl(k_nyq_comb, dim3(nlev, nf), 256, 0, c->stream)(S, mean, mstride, g.nx, g.ny, nlev, nch); LES_COUNT_LAUNCH();
+  pdl(k_nyq_apply, dim3((unsigned)((g.ny * (np + 1) + 255) / 256), (unsigned)npl), 256, 0, c->stream)(
       f0, f1, f2, S, g.ld, g.nx, g.ny, ps, nlev);
   LES_COUNT_LAUNCH();
 }
@@ -672,6 +681,7 @@ static void nyq_kill(les_ctx* c, double* const* f, int nf, int nlev, double* mea
 // step reads: the (0,0) mode is the FP64 plane mean itself
 __global__ void k_spec_widen(const float2* __restrict__ s, double2* __restrict__ d, const double* __restrict__ mean,
                              int mstride, size_t fs, size_t nk, int nf) {
+  pdl_wait();
   GSTRIDE(t, fs * nf) {
     const size_t fld = t / fs, r = t - fld * fs;
     const size_t lev = r / nk, m = r - lev * nk;
@@ -706,7 +716,7 @@ static int filt_da_uvw_mixed(les_ctx* c) {
   J.out[0] = ob + 6 * FS; J.out[1] = ob; J.out[2] = ob + 3 * FS; J.fs_out = FS;
   J.coef[0][0] = CC_KILL; J.coef[1][0] = CC_IKX; J.coef[2][0] = CC_IKY;
   colsT<float, float2>(c, J);
-  k_spec_widen<<<grid1(3 * (size_t)FS), 256, 0, c->stream>>>(ob + 6 * FS, c->spec, mean, ms, (size_t)FS, g.C, 3);
+  pdl(k_spec_widen, grid1(3 * (size_t)FS), 256, 0, c->stream)(ob + 6 * FS, c->spec, mean, ms, (size_t)FS, g.C, 3);
   LES_COUNT_LAUNCH();
   float* o6[6] = {f32(c, LES_DUDX), f32(c, LES_DVDX), f32(c, LES_DWDX), f32(c, LES_DUDY), f32(c, LES_DVDY),
                   f32(c, LES_DWDY)};  // FP32-held in the mixed form
@@ -838,6 +848,7 @@ __global__ void k_obukhov(const double* __restrict__ u1, const double* __restric
                           double* psi_h0, double* phi_m, double* phi_h, const double* theta_sum,
                           const double* __restrict__ sgs_q3, double q_scale,
                           int nx, int ny, int ld, double dz, double vonk, double g_, double nxny_f) {
+  pdl_wait();
   GSTRIDE(s, (size_t)nx * ny) {
     const int jy = (int)(s / nx), jx = (int)(s - (size_t)jy * nx);
     const size_t i = (size_t)jy * ld + jx;
@@ -883,6 +894,7 @@ __global__ void k_obukhov(const double* __restrict__ u1, const double* __restric
 __global__ void k_obukhov_init(double* psi_m, double* psi_m0, double* psi_h, double* psi_h0,
                                double* sgs_t3, const double* wt_s, double* sgs_q3, const double* wq_s,
                                size_t n, int initsc, double div, double divq) {
+  pdl_wait();
   GSTRIDE(s, n) {
     psi_m[s] = 0.0; psi_m0[s] = 0.0; psi_h[s] = 0.0; psi_h0[s] = 0.0;
     if (!initsc) {
@@ -921,7 +933,7 @@ int op_obukhov(les_ctx* c, const double* uv1) {
   const les_config& k = c->cfg;
   const size_t ns = (size_t)g.nx * g.ny;
   if (c->jt == 1) {  // SCAL_init = 1 (scalars_module.f90:525-542)
-    k_obukhov_init<<<grid1(ns, SFC_BS), SFC_BS, 0, c->stream>>>(c->f[LES_PSI_M], c->f[LES_PSI_M0], c->f[LES_PSI_H],
+    pdl(k_obukhov_init, grid1(ns, SFC_BS), SFC_BS, 0, c->stream)(c->f[LES_PSI_M], c->f[LES_PSI_M0], c->f[LES_PSI_H],
                                                      c->f[LES_PSI_H0], c->f[LES_SGS_T3_SFC], c->f[LES_WT_S],
                                                      c->f[LES_SGS_Q3_SFC], c->f[LES_WQ_S], ns, k.initsc,
                                                      k.u_star * k.t_scale, k.u_star * k.q_scale); LES_COUNT_LAUNCH();
@@ -934,7 +946,7 @@ int op_obukhov(les_ctx* c, const double* uv1) {
   const double* u1 = uv1;
   const double* v1 = uv1 + g.nplane;
   const double g_ = (k.g * k.z_i) / (k.u_star * k.u_star);
-  k_obukhov<<<grid1(ns, SFC_BS), SFC_BS, 0, c->stream>>>(u1, v1, c->f[LES_THETA], c->f[LES_ZO], c->z_os,
+  pdl(k_obukhov, grid1(ns, SFC_BS), SFC_BS, 0, c->stream)(u1, v1, c->f[LES_THETA], c->f[LES_ZO], c->z_os,
                                               c->f[LES_SGS_T3_SFC], c->f[LES_USTAR_AVG], c->f[LES_PSI_M],
                                               c->f[LES_PSI_M0], c->f[LES_PSI_H], c->f[LES_PSI_H0],
                                               c->f[LES_PHI_M], c->f[LES_PHI_H], c->dscal + 0,
@@ -951,6 +963,7 @@ __global__ void k_wallstress(const double* __restrict__ u, const double* __restr
                              const double* __restrict__ psi_m0, const double* __restrict__ phi_m,
                              double* ustar_avg, TT* txz, TT* tyz, double* dudz, double* dvdz,
                              int nx, int ny, int ld, double dz, double vonk) {
+  pdl_wait();
   GSTRIDE(s, (size_t)nx * ny) {
     const int jy = (int)(s / nx), jx = (int)(s - (size_t)jy * nx);
     const size_t i = (size_t)jy * ld + jx;
@@ -976,12 +989,12 @@ int op_wallstress(les_ctx* c, const double* uv1) {
   const double* u1 = uv1;
   const double* v1 = uv1 + g.nplane;
   if (c->cfg.precision == 1)
-    k_wallstress<float><<<grid1((size_t)g.nx * g.ny, SFC_BS), SFC_BS, 0, c->stream>>>(
+    pdl(k_wallstress<float>, grid1((size_t)g.nx * g.ny, SFC_BS), SFC_BS, 0, c->stream)(
         c->f[LES_U], c->f[LES_V], u1, v1, c->f[LES_ZO], c->f[LES_PSI_M], c->f[LES_PSI_M0], c->f[LES_PHI_M],
         c->f[LES_USTAR_AVG], f32(c, LES_TXZ), f32(c, LES_TYZ), c->f[LES_DUDZ], c->f[LES_DVDZ], g.nx, g.ny, g.ld,
         g.dz, c->cfg.vonk);
   else
-    k_wallstress<double><<<grid1((size_t)g.nx * g.ny, SFC_BS), SFC_BS, 0, c->stream>>>(
+    pdl(k_wallstress<double>, grid1((size_t)g.nx * g.ny, SFC_BS), SFC_BS, 0, c->stream)(
         c->f[LES_U], c->f[LES_V], u1, v1, c->f[LES_ZO], c->f[LES_PSI_M], c->f[LES_PSI_M0], c->f[LES_PHI_M],
         c->f[LES_USTAR_AVG], c->f[LES_TXZ], c->f[LES_TYZ], c->f[LES_DUDZ], c->f[LES_DVDZ], g.nx, g.ny, g.ld,
         g.dz, c->cfg.vonk);
@@ -1003,6 +1016,7 @@ __global__ void __launch_bounds__(256) k_calc_sij(
     double* S12, double* S13, double* S22, double* S23, double* S33, const double* __restrict__ u,
     const double* __restrict__ v, const double* __restrict__ w, double* ul, double* vl, double* wl, double* uls,
     double* vls, double* wls, int ld, int nx, int ny, int nz, int lag) {
+  pdl_wait();
   const unsigned np = (unsigned)ld * ny;
   const unsigned r = blockIdx.x * 256u + threadIdx.x;
   if (r >= np) return;
@@ -1044,6 +1058,7 @@ __global__ void __launch_bounds__(256) k_calc_sij32(
     float* S12, float* S13, float* S22, float* S23, float* S33, const double* __restrict__ u,
     const double* __restrict__ v, const double* __restrict__ w, double* ul, double* vl, double* wl, int ld, int nx,
     int ny, int lag) {
+  pdl_wait();
   const unsigned np = (unsigned)ld * ny;
   const unsigned p = blockIdx.x * 256u + threadIdx.x;
   if (p >= np) return;
@@ -1088,6 +1103,7 @@ __global__ void __launch_bounds__(256) k_nut_tau(
     const double* __restrict__ S22, const double* __restrict__ S23, const double* __restrict__ S33, double* Cs,
     double* Nu_t, double* txx, double* txy, double* tyy, double* txz, double* tyz, double* tzz, int ld, int nx, int ny,
     int nz, double l2, int override_cs, double cs_ov) {
+  pdl_wait();
   const unsigned np = (unsigned)ld * ny;
   const unsigned r = blockIdx.x * 256u + threadIdx.x;
   if (r >= np) return;
@@ -1149,6 +1165,7 @@ struct Ptr6f { const float* p[6]; };
 __global__ void __launch_bounds__(256) k_nut_tau32(Ptr6f Sp, double* Cs, float* Nu_t, float* txx, float* txy,
                                                    float* tyy, float* txz, float* tyz, float* tzz, int ld,
                                                    int nx, int ny, int nz, float l2, int override_cs, double cs_ov) {
+  pdl_wait();
   const unsigned np = (unsigned)ld * ny;
   const unsigned p = blockIdx.x * 256u + threadIdx.x;
   if (p >= np) return;
@@ -1196,7 +1213,7 @@ static void nut_tau(les_ctx* c, const double* const* S, int ov, double csov) {
   const unsigned pb = (unsigned)((g.nplane + 255) / 256);
   const bool deep = (size_t)pb * (g.nz / 8) >= 4 * 152;
   auto run = [&](auto kernel, int kz) {
-    kernel<<<dim3(pb, (unsigned)((g.nz + kz - 1) / kz)), 256, 0, c->stream>>>(
+    pdl(kernel, dim3(pb, (unsigned)((g.nz + kz - 1) / kz)), 256, 0, c->stream)(
         S[0], S[1], S[2], S[3], S[4], S[5], c->f[LES_CS_OPT2], c->f[LES_NU_T], c->f[LES_TXX], c->f[LES_TXY],
         c->f[LES_TYY], c->f[LES_TXZ], c->f[LES_TYZ], c->f[LES_TZZ], g.ld, g.nx, g.ny, g.nz, g.delta * g.delta, ov, csov);
   };
@@ -1205,6 +1222,7 @@ static void nut_tau(les_ctx* c, const double* const* S, int ov, double csov) {
   LES_COUNT_LAUNCH();
 }
 __global__ void k_bcast_levels(double* dst, const double* lev, size_t np, size_t n) {
+  pdl_wait();
   GSTRIDE(i, n) dst[i] = lev[i / np];
 }
 
@@ -1212,7 +1230,7 @@ int op_sgs_stag(les_ctx* c) {
   const Grid& g = c->g;
   const les_config& k = c->cfg;
   const bool lag = (k.model == 4 || k.model == 5 || k.model == 7);
-  k_calc_sij<<<dim3((unsigned)((g.nplane + 255) / 256), (unsigned)g.nz), 256, 0, c->stream>>>(
+  pdl(k_calc_sij, dim3((unsigned)((g.nplane + 255) / 256), (unsigned)g.nz), 256, 0, c->stream)(
       c->f[LES_DUDX], c->f[LES_DUDY], c->f[LES_DUDZ], c->f[LES_DVDX], c->f[LES_DVDY], c->f[LES_DVDZ],
       c->f[LES_DWDX], c->f[LES_DWDY], c->f[LES_DWDZ], c->f[LES_S11], c->f[LES_S12], c->f[LES_S13],
       c->f[LES_S22], c->f[LES_S23], c->f[LES_S33], c->f[LES_U], c->f[LES_V], c->f[LES_W], c->f[LES_U_LAG],
@@ -1225,7 +1243,7 @@ int op_sgs_stag(les_ctx* c) {
       if (k.model == 2) op_stddyn(c, csz, S);
       else op_scaledep(c, csz, S);
       // Cs_opt2(:,:,jz) = ziko(jz)
-      k_bcast_levels<<<grid1(g.nfield), 256, 0, c->stream>>>(c->f[LES_CS_OPT2], csz, g.nplane, g.nfield); LES_COUNT_LAUNCH();
+      pdl(k_bcast_levels, grid1(g.nfield), 256, 0, c->stream)(c->f[LES_CS_OPT2], csz, g.nplane, g.nfield); LES_COUNT_LAUNCH();
     } else if (k.model == 4) {
       op_lagrange_ssim(c, S);
     } else if (k.model == 5) {
@@ -1265,6 +1283,7 @@ __global__ void k_interpolag(const double* __restrict__ ul, const double* __rest
                              const double* __restrict__ FMM, const double* __restrict__ FQN,
                              const double* __restrict__ FNN, double* oLM, double* oMM, double* oQN,
                              double* oNN, int ld, int nx, int ny, int nz, double fx_, double fy_, double fz_) {
+  pdl_wait();
   const size_t np = (size_t)ld * ny;
   GSTRIDE(t, (size_t)nx * ny * nz) {
     const int jx = (int)(t % nx);
@@ -1329,6 +1348,7 @@ __global__ void k_interpolag(const double* __restrict__ ul, const double* __rest
 // over the cs_count steps, so the displacement is -u_lag dt / dx.
 __global__ void k_to_f32x4(const double* __restrict__ a, const double* __restrict__ b, const double* __restrict__ c,
                            const double* __restrict__ d, float* o, size_t n) {
+  pdl_wait();
   GSTRIDE(i, n) {
     o[i] = cvt_d2f(a[i]);
     o[i + n] = cvt_d2f(b[i]);
@@ -1340,6 +1360,7 @@ __global__ void k_interpolag32(const double* __restrict__ ul, const double* __re
                                const double* __restrict__ wl, const float* __restrict__ F4, double* oLM,
                                double* oMM, double* oQN, double* oNN, int ld, int nx, int ny, int nz, size_t nf,
                                float sx, float sy, float sz) {
+  pdl_wait();
   const size_t np = (size_t)ld * ny;
   const float* FLM = F4;
   const float* FMM = F4 + nf;
@@ -1396,10 +1417,10 @@ static int op_interpolag32(les_ctx* c) {
   double* Fn[4];
   for (int q = 0; q < 4; ++q) Fn[q] = c->spare + (size_t)q * g.nfield;
   float* F4 = reinterpret_cast<float*>(c->tmp);  // 4 * nfield floats, free until the filtering below
-  k_to_f32x4<<<grid1(g.nfield), 256, 0, c->stream>>>(c->f[LES_F_LM], c->f[LES_F_MM], c->f[LES_F_QN], c->f[LES_F_NN],
+  pdl(k_to_f32x4, grid1(g.nfield), 256, 0, c->stream)(c->f[LES_F_LM], c->f[LES_F_MM], c->f[LES_F_QN], c->f[LES_F_NN],
                                                      F4, g.nfield); LES_COUNT_LAUNCH();
   // u_lag holds the sum over cs_count steps: (sum / cs_count) * (dt * cs_count) / dx
-  k_interpolag32<<<grid1((size_t)g.nx * g.ny * g.nz), 256, 0, c->stream>>>(
+  pdl(k_interpolag32, grid1((size_t)g.nx * g.ny * g.nz), 256, 0, c->stream)(
       c->f[LES_U_LAG], c->f[LES_V_LAG], c->f[LES_W_LAG], F4, Fn[0], Fn[1], Fn[2], Fn[3], g.ld, g.nx, g.ny, g.nz,
       g.nfield, (float)(k.dt / g.dx), (float)(k.dt / g.dy), (float)(k.dt / g.dz)); LES_COUNT_LAUNCH();
   for (int q = 0; q < 4; ++q)
@@ -1417,12 +1438,12 @@ int op_interpolag_n(les_ctx* c, int nf) {
   double* Fn[4];
   for (int q = 0; q < 4; ++q) Fn[q] = c->spare + (size_t)q * g.nfield;
   if (nf == 4)
-    k_interpolag<4, true><<<grid1((size_t)g.nx * g.ny * g.nz), 256, 0, c->stream>>>(
+    pdl(k_interpolag<4, true>, grid1((size_t)g.nx * g.ny * g.nz), 256, 0, c->stream)(
         c->f[LES_U_LAG], c->f[LES_V_LAG], c->f[LES_W_LAG], c->f[LES_F_LM], c->f[LES_F_MM], c->f[LES_F_QN],
         c->f[LES_F_NN], Fn[0], Fn[1], Fn[2], Fn[3], g.ld, g.nx, g.ny, g.nz, -k.dt / g.dx, -k.dt / g.dy,
         -k.dt / g.dz);
   else
-    k_interpolag<2, false><<<grid1((size_t)g.nx * g.ny * g.nz), 256, 0, c->stream>>>(
+    pdl(k_interpolag<2, false>, grid1((size_t)g.nx * g.ny * g.nz), 256, 0, c->stream)(
         c->f[LES_U_LAG], c->f[LES_V_LAG], c->f[LES_W_LAG], c->f[LES_F_LM], c->f[LES_F_MM], nullptr, nullptr,
         Fn[0], Fn[1], nullptr, nullptr, g.ld, g.nx, g.ny, g.nz, -k.dt / g.dx, -k.dt / g.dy, -k.dt / g.dz);
   LES_COUNT_LAUNCH();
@@ -1439,6 +1460,7 @@ int op_interpolag_n(les_ctx* c, int nf) {
 __global__ void k_lag_prep(const double* __restrict__ u, const double* __restrict__ v,
                            const double* __restrict__ w, Ptr6 Sp,
                            double* out, int ld, int nx, int ny, int jz0, int nlev, size_t np) {
+  pdl_wait();
   const size_t tot = np * nlev;
   GSTRIDE(t, tot) {
     const int lc = (int)(t / np);
@@ -1490,6 +1512,7 @@ __global__ void k_lag_final(const S* __restrict__ flt, double* F_LM, double* F_M
                             double* F_NN, double* Beta, double* Cs, double* TnLM, double* TnQN, int ld, int nx,
                             int ny, int nz, int jz0, int nlev, size_t np, R cst, R opftdelta, R lagran_dt,
                             int bexp_one, R bexp) {
+  pdl_wait();
   const size_t tot = np * nlev;
   GSTRIDE(t, tot) {
     const int lc = (int)(t / np);
@@ -1574,7 +1597,7 @@ int op_lagrange(les_ctx* c, const double* const* S) {
     const int nl = std::min(nch, g.nz - jz0 + 1);
     double* prep = c->tmp;                              // 21 * nl planes
     double* flt = c->tmp + (size_t)21 * nch * g.nplane;  // 42 * nl planes
-    k_lag_prep<<<grid1(g.nplane * nl), 256, 0, c->stream>>>(c->f[LES_U], c->f[LES_V], c->f[LES_W],
+    pdl(k_lag_prep, grid1(g.nplane * nl), 256, 0, c->stream)(c->f[LES_U], c->f[LES_V], c->f[LES_W],
                                                            Sp, prep, g.ld, g.nx,
                                                            g.ny, jz0, nl, g.nplane); LES_COUNT_LAUNCH();
     const double* in[21];
@@ -1589,7 +1612,7 @@ int op_lagrange(les_ctx* c, const double* const* S) {
     double* out[42];
     for (int q = 0; q < 42; ++q) out[q] = flt + (size_t)q * nl * g.nplane;
     c2r(c, 42, nl, c->wsB, out, (long)g.nplane, false, g.lh);
-    k_lag_final<double, double><<<grid1(g.nplane * nl), 256, 0, c->stream>>>(
+    pdl(k_lag_final<double, double>, grid1(g.nplane * nl), 256, 0, c->stream)(
         flt, c->f[LES_F_LM], c->f[LES_F_MM], c->f[LES_F_QN], c->f[LES_F_NN], c->f[LES_BETA],
         c->f[LES_CS_OPT2], c->f[LES_TN_LMMM], c->f[LES_TN_QNNN], g.ld, g.nx, g.ny, g.nz, jz0, nl, g.nplane, cst,
         opftdelta, lagran_dt, bone, bexp); LES_COUNT_LAUNCH();
@@ -1609,7 +1632,7 @@ int op_interpolag_scalar(les_ctx* c) {
   if (!c->f[LES_G_LM]) return LES_ERR_STATE;
   double* Fn[4];
   for (int q = 0; q < 4; ++q) Fn[q] = c->spare + (size_t)q * g.nfield;
-  k_interpolag<4, true><<<grid1((size_t)g.nx * g.ny * g.nz), 256, 0, c->stream>>>(
+  pdl(k_interpolag<4, true>, grid1((size_t)g.nx * g.ny * g.nz), 256, 0, c->stream)(
       c->f[LES_U_LAG_S], c->f[LES_V_LAG_S], c->f[LES_W_LAG_S], c->f[LES_G_LM], c->f[LES_G_MM], c->f[LES_G_QN],
       c->f[LES_G_NN], Fn[0], Fn[1], Fn[2], Fn[3], g.ld, g.nx, g.ny, g.nz, -k.dt / g.dx, -k.dt / g.dy,
       -k.dt / g.dz); LES_COUNT_LAUNCH();
@@ -1631,6 +1654,7 @@ __global__ void __launch_bounds__(1024) k_lag_s_surface(const double* __restrict
                                                         const double* __restrict__ phi_h, double* dTdz, int nx,
                                                         int ny, int ld, double dz, double vonk, double t_scale,
                                                         double u_star) {
+  pdl_wait();
   __shared__ double red[4][32];
   const int ns = nx * ny;
   double a[4] = {0.0, 0.0, 0.0, 0.0};
@@ -1678,6 +1702,7 @@ __global__ void k_lag_s_prep(const double* __restrict__ u, const double* __restr
                              const double* __restrict__ w, const double* __restrict__ th, Ptr6 Sp,
                              const double* __restrict__ dTx, const double* __restrict__ dTy,
                              const double* __restrict__ dTz, double* out, int jz0, int nlev, size_t np) {
+  pdl_wait();
   const size_t tot = np * nlev;
   GSTRIDE(t, tot) {
     const int lc = (int)(t / np);
@@ -1720,6 +1745,7 @@ __global__ void k_lag_s_final(const double* __restrict__ flt, double* G_LM, doub
                               const double* __restrict__ Cs, double* Beta, double* Pr_t, double* cs2_pr, int ld,
                               int nx, int nz, int jz0, int nlev, size_t np, double cst, double opftdelta,
                               double lagran_dt, int bexp_one, double bexp) {
+  pdl_wait();
   const size_t tot = np * nlev;
   const double e24 = (double)1e-24f;
   GSTRIDE(t, tot) {
@@ -1795,7 +1821,7 @@ int op_lagrange_scalar(les_ctx* c, const double* const* S, double* cs2_pr) {
   op_filt_da(c, theta, dTx, dTy, g.nz);  // :83-84
   op_ddz(c, dTz, theta, 1);
   fill(c, dTz + (size_t)(g.nz - 1) * g.nplane, g.nplane, k.dtdz_top / k.t_scale * k.z_i);  // :86
-  k_lag_s_surface<<<1, 1024, 0, c->stream>>>(c->f[LES_U], c->f[LES_V], c->f[LES_ZO], c->f[LES_WT_S],
+  pdl(k_lag_s_surface, 1, 1024, 0, c->stream)(c->f[LES_U], c->f[LES_V], c->f[LES_ZO], c->f[LES_WT_S],
                                              c->f[LES_PSI_M], c->f[LES_PHI_H], dTz, g.nx, g.ny, g.ld, g.dz, k.vonk,
                                              k.t_scale, k.u_star); LES_COUNT_LAUNCH();
   const double delta = g.delta;
@@ -1811,7 +1837,7 @@ int op_lagrange_scalar(les_ctx* c, const double* const* S, double* cs2_pr) {
     const int nl = std::min(nch, g.nz - jz0 + 1);
     double* prep = c->tmp;                               // 19 * nl planes
     double* flt = c->tmp + (size_t)19 * nch * g.nplane;  // 38 * nl planes
-    k_lag_s_prep<<<grid1(g.nplane * nl), 256, 0, c->stream>>>(c->f[LES_U], c->f[LES_V], c->f[LES_W], th0, Sp, dTx,
+    pdl(k_lag_s_prep, grid1(g.nplane * nl), 256, 0, c->stream)(c->f[LES_U], c->f[LES_V], c->f[LES_W], th0, Sp, dTx,
                                                              dTy, dTz, prep, jz0, nl, g.nplane); LES_COUNT_LAUNCH();
     const double* in[19];
     for (int q = 0; q < 19; ++q) in[q] = prep + (size_t)q * nl * g.nplane;
@@ -1825,7 +1851,7 @@ int op_lagrange_scalar(les_ctx* c, const double* const* S, double* cs2_pr) {
     double* out[38];
     for (int q = 0; q < 38; ++q) out[q] = flt + (size_t)q * nl * g.nplane;
     c2r(c, 38, nl, c->wsB, out, (long)g.nplane, false, g.lh);
-    k_lag_s_final<<<grid1(g.nplane * nl), 256, 0, c->stream>>>(
+    pdl(k_lag_s_final, grid1(g.nplane * nl), 256, 0, c->stream)(
         flt, c->f[LES_G_LM], c->f[LES_G_MM], c->f[LES_G_QN], c->f[LES_G_NN], c->f[LES_TN_LMMM], c->f[LES_TN_QNNN],
         c->f[LES_CS_OPT2], c->f[LES_BETA], c->f[LES_PR_T], cs2_pr, g.ld, g.nx, g.nz, jz0, nl, g.nplane, cst,
         opftdelta, lagran_dt, bone, bexp); LES_COUNT_LAUNCH();
@@ -1837,6 +1863,7 @@ int op_lagrange_scalar(les_ctx* c, const double* const* S, double* cs2_pr) {
 __global__ void k_sd_prep(const double* __restrict__ u, const double* __restrict__ v,
                           const double* __restrict__ w, Ptr6 Sp, double* out,
                           int ld, int nx, int ny, int jz0, int nlev, size_t np) {
+  pdl_wait();
   const size_t tot = np * nlev;
   GSTRIDE(t, tot) {
     const int lc = (int)(t / np);
@@ -1873,6 +1900,7 @@ __global__ void k_sd_prep(const double* __restrict__ u, const double* __restrict
 }
 // Second filtered set: Q_ij inputs are products of the G-filtered velocities.
 __global__ void k_sd_qprep(const double* __restrict__ flt, double* qin, int nlev, size_t np) {
+  pdl_wait();
   const size_t st = np * nlev;
   GSTRIDE(t, st) {
     const double ub = flt[t], vb = flt[t + st], wb = flt[t + 2 * st];
@@ -1883,6 +1911,7 @@ __global__ void k_sd_qprep(const double* __restrict__ flt, double* qin, int nlev
 // per-level sums a1..e2 (10 sums) -> sums[lev*10 + q]; one CTA per level, fixed order
 __global__ void __launch_bounds__(256) k_sd_sums(const double* __restrict__ flt, const double* __restrict__ qf,
                                                  double* sums, int ld, int nx, int ny, int nlev, size_t np, int jz0) {
+  pdl_wait();
   __shared__ double sh[10][256];
   const int lc = blockIdx.x;
   const size_t st = np * nlev;
@@ -1938,6 +1967,7 @@ __device__ double rtnewt_d(const double* A) {
 __global__ void __launch_bounds__(256) k_sd_final(const double* __restrict__ flt, const double* __restrict__ sums,
                                                   double* cs_z, int ld, int nx, int ny, int nlev, size_t np,
                                                   int jz0, double delta) {
+  pdl_wait();
   __shared__ double sn[256], sd[256];
   __shared__ double beta_s;
   const int lc = blockIdx.x;
@@ -1996,6 +2026,7 @@ __global__ void __launch_bounds__(256) k_sd_final(const double* __restrict__ flt
 __global__ void k_ssim_final(const double* __restrict__ flt, double* F_LM, double* F_MM, double* Cs,
                              int ld, int nx, int ny, int nlev, size_t np, int jz0, double cst, double opftdelta,
                              double lagran_dt) {
+  pdl_wait();
   const double eps = 1e-32;  // lagrange_Ssim.f90:25
   const size_t st = np * nlev;
   GSTRIDE(t, st) {
@@ -2046,7 +2077,7 @@ int op_lagrange_ssim(les_ctx* c, const double* const* S) {
     const int nl = std::min(nch, g.nz - jz0 + 1);
     double* prep = c->tmp;
     double* flt = c->tmp + (size_t)21 * nch * g.nplane;
-    k_sd_prep<<<grid1(g.nplane * nl), 256, 0, c->stream>>>(c->f[LES_U], c->f[LES_V], c->f[LES_W],
+    pdl(k_sd_prep, grid1(g.nplane * nl), 256, 0, c->stream)(c->f[LES_U], c->f[LES_V], c->f[LES_W],
                                                           Sp, prep, g.ld, g.nx, g.ny,
                                                           jz0, nl, g.nplane); LES_COUNT_LAUNCH();
     const double* in[21];
@@ -2061,7 +2092,7 @@ int op_lagrange_ssim(les_ctx* c, const double* const* S) {
     double* out[21];
     for (int q = 0; q < 21; ++q) out[q] = flt + (size_t)q * nl * g.nplane;
     c2r(c, 21, nl, c->wsB, out, (long)g.nplane, false, g.lh);
-    k_ssim_final<<<grid1(g.nplane * nl), 256, 0, c->stream>>>(flt, c->f[LES_F_LM], c->f[LES_F_MM],
+    pdl(k_ssim_final, grid1(g.nplane * nl), 256, 0, c->stream)(flt, c->f[LES_F_LM], c->f[LES_F_MM],
                                                              c->f[LES_CS_OPT2], g.ld, g.nx, g.ny, nl, g.nplane,
                                                              jz0, cst, opftdelta, lagran_dt); LES_COUNT_LAUNCH();
   }
@@ -2082,7 +2113,7 @@ int op_stddyn(les_ctx* c, double* cs_z, const double* const* S) {
     const int nl = std::min(nch, g.nz - jz0 + 1);
     double* prep = c->tmp;
     double* flt = c->tmp + (size_t)21 * nch * g.nplane;
-    k_sd_prep<<<grid1(g.nplane * nl), 256, 0, c->stream>>>(c->f[LES_U], c->f[LES_V], c->f[LES_W],
+    pdl(k_sd_prep, grid1(g.nplane * nl), 256, 0, c->stream)(c->f[LES_U], c->f[LES_V], c->f[LES_W],
                                                           Sp, prep, g.ld, g.nx, g.ny,
                                                           jz0, nl, g.nplane); LES_COUNT_LAUNCH();
     const double* in[21];
@@ -2097,7 +2128,7 @@ int op_stddyn(les_ctx* c, double* cs_z, const double* const* S) {
     double* out[21];
     for (int q = 0; q < 21; ++q) out[q] = flt + (size_t)q * nl * g.nplane;
     c2r(c, 21, nl, c->wsB, out, (long)g.nplane, false, g.lh);
-    k_sd_final<<<nl, 256, 0, c->stream>>>(flt, nullptr, cs_z, g.ld, g.nx, g.ny, nl, g.nplane, jz0, delta3); LES_COUNT_LAUNCH();
+    pdl(k_sd_final, nl, 256, 0, c->stream)(flt, nullptr, cs_z, g.ld, g.nx, g.ny, nl, g.nplane, jz0, delta3); LES_COUNT_LAUNCH();
   }
   return 0;
 }
@@ -2111,7 +2142,7 @@ int op_scaledep(les_ctx* c, double* cs_z, const double* const* S) {
     const int nl = std::min(nch, g.nz - jz0 + 1);
     double* prep = c->tmp;
     double* flt = c->tmp + (size_t)21 * nch * g.nplane;
-    k_sd_prep<<<grid1(g.nplane * nl), 256, 0, c->stream>>>(c->f[LES_U], c->f[LES_V], c->f[LES_W],
+    pdl(k_sd_prep, grid1(g.nplane * nl), 256, 0, c->stream)(c->f[LES_U], c->f[LES_V], c->f[LES_W],
                                                           Sp, prep, g.ld, g.nx, g.ny,
                                                           jz0, nl, g.nplane); LES_COUNT_LAUNCH();
     const double* in[21];
@@ -2128,7 +2159,7 @@ int op_scaledep(les_ctx* c, double* cs_z, const double* const* S) {
     c2r(c, 42, nl, c->wsB, out, (long)g.nplane, false, g.lh);
     // Q_ij inputs: products of the G-filtered velocities, then GG-filtered
     double* qin = prep;  // reuse: 6 * nl planes
-    k_sd_qprep<<<grid1(g.nplane * nl), 256, 0, c->stream>>>(flt, qin, nl, g.nplane); LES_COUNT_LAUNCH();
+    pdl(k_sd_qprep, grid1(g.nplane * nl), 256, 0, c->stream)(flt, qin, nl, g.nplane); LES_COUNT_LAUNCH();
     const double* qi[6];
     double* qo[6];
     for (int q = 0; q < 6; ++q) { qi[q] = qin + (size_t)q * nl * g.nplane; qo[q] = prep + (size_t)(6 + q) * nl * g.nplane; }
@@ -2138,9 +2169,9 @@ int op_scaledep(les_ctx* c, double* cs_z, const double* const* S) {
     K.out[0] = c->wsB; K.fs_out = (long)nl * g.C; K.coef[0][0] = CC_GG;
     cols(c, K);
     c2r(c, 6, nl, c->wsB, qo, (long)g.nplane, false, g.lh);
-    k_sd_sums<<<nl, 256, 0, c->stream>>>(flt, prep + (size_t)6 * nl * g.nplane, sums, g.ld, g.nx, g.ny, nl,
+    pdl(k_sd_sums, nl, 256, 0, c->stream)(flt, prep + (size_t)6 * nl * g.nplane, sums, g.ld, g.nx, g.ny, nl,
                                          g.nplane, jz0); LES_COUNT_LAUNCH();
-    k_sd_final<<<nl, 256, 0, c->stream>>>(flt, sums, cs_z, g.ld, g.nx, g.ny, nl, g.nplane, jz0, g.delta); LES_COUNT_LAUNCH();
+    pdl(k_sd_final, nl, 256, 0, c->stream)(flt, sums, cs_z, g.ld, g.nx, g.ny, nl, g.nplane, jz0, g.delta); LES_COUNT_LAUNCH();
   }
   return 0;
 }
@@ -2154,6 +2185,7 @@ __global__ void k_divstress_fin(double* __restrict__ divx, double* __restrict__ 
                                 const double* __restrict__ txz, const double* __restrict__ tyz,
                                 const double* __restrict__ tzz, int ld, int nx, int ny, int nz, double cdz,
                                 int want) {
+  pdl_wait();
   const size_t np = (size_t)ld * ny;
   GSTRIDE(i, np * nz) {
     const int jz = (int)(i / np) + 1;
@@ -2197,7 +2229,7 @@ int op_divstress(les_ctx* c, double* divtx, double* divty, double* divtz) {
   cols(c, K);
   double* h[3] = {c->tmp, c->tmp + g.nfield, c->tmp + 2 * g.nfield};
   c2r(c, 3, g.nz, c->wsB, h, (long)g.nplane, false, g.lh);
-  k_divstress_fin<<<grid1(g.nfield), 256, 0, c->stream>>>(divtx, divty, divtz, h[0], h[1], h[2], c->f[LES_TXZ],
+  pdl(k_divstress_fin, grid1(g.nfield), 256, 0, c->stream)(divtx, divty, divtz, h[0], h[1], h[2], c->f[LES_TXZ],
                                                          c->f[LES_TYZ], c->f[LES_TZZ], g.ld, g.nx, g.ny, g.nz,
                                                          1.0 / g.dz, 7); LES_COUNT_LAUNCH();
   return 0;
@@ -2219,10 +2251,10 @@ int op_divstress_one(les_ctx* c, double* divt, const double* tx, const double* t
   double* h = c->tmp;
   c2r(c, 1, g.nz, c->wsB, &h, (long)g.nplane, false, g.lh);
   if (!w_variant) {
-    k_divstress_fin<<<grid1(g.nfield), 256, 0, c->stream>>>(divt, nullptr, nullptr, h, nullptr, nullptr, tz, nullptr,
+    pdl(k_divstress_fin, grid1(g.nfield), 256, 0, c->stream)(divt, nullptr, nullptr, h, nullptr, nullptr, tz, nullptr,
                                                            nullptr, g.ld, g.nx, g.ny, g.nz, 1.0 / g.dz, 1); LES_COUNT_LAUNCH();
   } else {
-    k_divstress_fin<<<grid1(g.nfield), 256, 0, c->stream>>>(nullptr, nullptr, divt, nullptr, nullptr, h, nullptr,
+    pdl(k_divstress_fin, grid1(g.nfield), 256, 0, c->stream)(nullptr, nullptr, divt, nullptr, nullptr, h, nullptr,
                                                            nullptr, tz, g.ld, g.nx, g.ny, g.nz, 1.0 / g.dz, 4); LES_COUNT_LAUNCH();
   }
   return 0;
@@ -2234,6 +2266,7 @@ __global__ void k_vort(const double* __restrict__ dudy, const double* __restrict
                        const double* __restrict__ dvdx, const double* __restrict__ dvdz,
                        const double* __restrict__ dwdx, const double* __restrict__ dwdy, double* o1,
                        double* o2, double* o3, int ld, int ny, int nz, double cst) {
+  pdl_wait();
   const size_t np = (size_t)ld * ny;
   GSTRIDE(i, np * nz) {
     const int jz = (int)(i / np) + 1;
@@ -2253,6 +2286,7 @@ __global__ void k_convec_prod(const S* __restrict__ u1, const S* __restrict__ u2
                               const S* __restrict__ u3, const S* __restrict__ w1,
                               const S* __restrict__ w2, const S* __restrict__ w3, S* ccx,
                               S* ccy, S* ccz, int ldb, int nx2, int ny2, int nz, S cst) {
+  pdl_wait();
   const size_t np = (size_t)ldb * ny2;
   GSTRIDE(i, np * (nz - 1)) {
     const int jz = (int)(i / np) + 1;
@@ -2283,6 +2317,7 @@ __global__ void __launch_bounds__(256) k_convec_prod64(const double* __restrict_
                                                        const double* __restrict__ w2, const double* __restrict__ w3,
                                                        double* ccx, double* ccy, double* ccz, int ldb, int nx2, int ny2,
                                                        int nz) {
+  pdl_wait();
   const unsigned np = (unsigned)ldb * ny2;
   const unsigned r = blockIdx.x * 256u + threadIdx.x;
   if (r >= np || (int)(r % (unsigned)ldb) >= nx2) return;
@@ -2306,7 +2341,7 @@ static void convec_prod64(les_ctx* c, double* const* b) {
   const Grid& g = c->g;
   const unsigned pb = (unsigned)((g.nplane_big + 255) / 256);
   auto run = [&](auto kernel, int kz) {
-    kernel<<<dim3(pb, (unsigned)((g.nz - 1 + kz - 1) / kz)), 256, 0, c->stream>>>(
+    pdl(kernel, dim3(pb, (unsigned)((g.nz - 1 + kz - 1) / kz)), 256, 0, c->stream)(
         b[0], b[1], b[2], b[3], b[4], b[5], b[6], b[7], b[8], g.ld_big, g.nx2, g.ny2, g.nz);
   };
   // eight levels a thread once that leaves four blocks per SM
@@ -2318,7 +2353,7 @@ int op_convec(les_ctx* c, double* cx, double* cy, double* cz) {
   const Grid& g = c->g;
   const double cst = 1.0 / (double)(g.nx * g.ny);
   double* vort[3] = {c->tmp, c->tmp + g.nfield, c->tmp + 2 * g.nfield};
-  k_vort<<<grid1(g.nfield), 256, 0, c->stream>>>(c->f[LES_DUDY], c->f[LES_DUDZ], c->f[LES_DVDX], c->f[LES_DVDZ],
+  pdl(k_vort, grid1(g.nfield), 256, 0, c->stream)(c->f[LES_DUDY], c->f[LES_DUDZ], c->f[LES_DVDX], c->f[LES_DVDZ],
                                                 c->f[LES_DWDX], c->f[LES_DWDY], vort[0], vort[1], vort[2], g.ld,
                                                 g.ny, g.nz, cst); LES_COUNT_LAUNCH();
   const double* in[6] = {c->f[LES_U], c->f[LES_V], c->f[LES_W], vort[0], vort[1], vort[2]};
@@ -2351,6 +2386,7 @@ __global__ void k_rhs_ab2(double* u, double* v, double* w, double* Rx, double* R
                           double* Ryf, double* Rzf, const double* __restrict__ dx_, const double* __restrict__ dy_,
                           const double* __restrict__ dz_, const double* __restrict__ bs, size_t nv, size_t np,
                           double dt, int sflag, int euler) {
+  pdl_wait();
   GSTRIDE(i, nv + np) {
     if (i >= nv) { u[i] = LES_BOGUS; v[i] = LES_BOGUS; w[i] = LES_BOGUS; continue; }
     const double rx = -Rx[i] - dx_[i];
@@ -2415,6 +2451,7 @@ template <> struct KxCol<double2> {
 template <typename CX>
 __global__ void k_ikx_rows(const CX* __restrict__ in, CX* out, const float2* __restrict__ kxd,
                            const double* __restrict__ kx, int lh, size_t n, int acc) {
+  pdl_wait();
   GSTRIDE(e, n) {
     const int jx = (int)(e % lh);
     const auto k = KxCol<CX>::get(kxd, kx, jx);
@@ -2440,6 +2477,7 @@ __device__ __forceinline__ float2 df2(double x) {
   return make_float2(d.hi, d.lo);
 }
 __global__ void k_mean_tab(const double* __restrict__ mean, int ms, int nz, double dz, MeanTab T) {
+  pdl_wait();
   const int jz = blockIdx.x * blockDim.x + threadIdx.x + 1;  // 1..nz
   if (jz > nz) return;
   const double U = mean[jz - 1], V = mean[ms + jz - 1];
@@ -2493,6 +2531,7 @@ __global__ void __launch_bounds__(256) k_rhs_ab2_mx(
     const double* __restrict__ bs, const dfloat* __restrict__ wz, const dfloat* __restrict__ wx,
     const float* __restrict__ dwdy, MeanTab T, float2* __restrict__ us, float2* __restrict__ vs,
     float2* __restrict__ ws, int ld, int ny, int nz, float2 idz2, float2 dt2, int sflag, int euler) {
+  pdl_wait();
   const unsigned np = (unsigned)ld * ny;
   const unsigned p = blockIdx.x * 256u + threadIdx.x;
   if (p >= np) return;
@@ -2558,7 +2597,7 @@ __global__ void __launch_bounds__(256) k_rhs_ab2_mx(
 __global__ void __launch_bounds__(256) k_dpdz_project(double* u, double* v, double* w, double* Rx, double* Ry, double* Rz,
                                                       const double* __restrict__ p, const double* __restrict__ dpdx,
                                                       const double* __restrict__ dpdy, double* dpdz, int ld, int nx,
-                                                      int ny, int nz, double idz, double mdt15) {  // 1/dz, -1.5 dt
+                                                      int ny, int nz, double idz, double mdt15) { pdl_wait();  // 1/dz, -1.5 dt
   const unsigned np = (unsigned)ld * ny;
   const unsigned r = blockIdx.x * 256u + threadIdx.x;
   if (r >= np) return;
@@ -2606,6 +2645,7 @@ __global__ void __launch_bounds__(256) k_dpdz_project32(double* u, double* v, do
                                                         const double* __restrict__ dpdx,
                                                         const double* __restrict__ dpdy, double* dpdz, int ld,
                                                         int nx, int ny, int nz, double idz, double dt) {
+  pdl_wait();
   const unsigned np = (unsigned)ld * ny;
   const unsigned r = blockIdx.x * 256u + threadIdx.x;
   if (r >= np) return;
@@ -2645,6 +2685,7 @@ __global__ void __launch_bounds__(256) k_dpdz_project32(double* u, double* v, do
 
 __global__ void k_project_only(double* u, double* v, double* w, const double* dpdx, const double* dpdy,
                                const double* dpdz, int ld, int nx, int ny, int nz, double dt) {
+  pdl_wait();
   const size_t np = (size_t)ld * ny;
   GSTRIDE(r, np) {
     const int jx = (int)(r % ld);
@@ -2667,7 +2708,7 @@ __global__ void k_project_only(double* u, double* v, double* w, const double* dp
 int op_project(les_ctx* c) {
   // stand-alone project (forcing.f90:128-219): dpdz is taken as given
   const Grid& g = c->g;
-  k_project_only<<<grid1(g.nplane), 256, 0, c->stream>>>(c->f[LES_U], c->f[LES_V], c->f[LES_W], c->f[LES_DPDX],
+  pdl(k_project_only, grid1(g.nplane), 256, 0, c->stream)(c->f[LES_U], c->f[LES_V], c->f[LES_W], c->f[LES_DPDX],
                                                         c->f[LES_DPDY], c->f[LES_DPDZ], g.ld, g.nx, g.ny, g.nz,
                                                         c->cfg.dt); LES_COUNT_LAUNCH();
   return 0;
@@ -2788,6 +2829,7 @@ __global__ void __launch_bounds__(128) k_tridiag2(const HC* __restrict__ Hx, con
                                                   const double* __restrict__ ky, const float2* __restrict__ kxd,
                                                   const float2* __restrict__ kyd, int lh, int ny, int nz, double dz,
                                                   const int* __restrict__ modes, int nmodes) {
+  pdl_wait();
   const int nk = lh * ny;
   const int g2 = blockIdx.x * blockDim.x + threadIdx.x;
   int t = g2 >> 1;
@@ -2960,6 +3002,7 @@ __global__ void __launch_bounds__(128) k_tridiag64(const C2* __restrict__ Hx, co
                                                    const double* __restrict__ gam, const double* __restrict__ kx,
                                                    const double* __restrict__ ky, int lh, int ny, int nz, double dz,
                                                    double idz) {
+  pdl_wait();
   constexpr int D = TRI64_D;
   const int nk = lh * ny;
   const int g2 = blockIdx.x * blockDim.x + threadIdx.x;
@@ -3245,6 +3288,7 @@ __device__ __forceinline__ void tri_chunk(const TriArgs& A, int t, bool act, boo
 // grid 1 + ceil(nk / 16): CTA 0 the FP64 modes, CTA b > 0 the modes
 // 16 (b - 1) .. 16 b - 1 in float-float (skipping the FP64 ones)
 __global__ void __launch_bounds__(TRI_W * 32) k_tridiag_chunk(TriArgs A, int k2low) {
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char smraw[];
   const int lane = threadIdx.x & 31;
   if (blockIdx.x == 0) {
@@ -3443,13 +3487,13 @@ static int pressT(les_ctx* c, double* p, double* dpdx, double* dpdy, bool walls,
     A.nk = g.lh * g.ny; A.lh = g.lh; A.ny = g.ny; A.nz = nz;
     A.idz2 = make_float2(idz.hi, idz.lo); A.a2 = make_float2(a2.hi, a2.lo); A.dz2 = make_float2(dz2.hi, dz2.lo);
     A.dz = g.dz;
-    k_tridiag_chunk<<<1 + (g.lh * g.ny + TRI_M - 1) / TRI_M, TRI_W * 32, sm, c->stream>>>(A, TRI_K2LOW);
+    pdl(k_tridiag_chunk, 1 + (g.lh * g.ny + TRI_M - 1) / TRI_M, TRI_W * 32, sm, c->stream)(A, TRI_K2LOW);
     LES_COUNT_LAUNCH();
   } else if (int_deriv(c)) {
-    k_tridiag64<<<(2 * g.lh * g.ny + 127) / 128, 128, 0, c->stream>>>(
+    pdl(k_tridiag64, (2 * g.lh * g.ny + 127) / 128, 128, 0, c->stream)(
         Hx, Hy, Hz, BT, BT + g.C, P, c->ibet, c->gamt, c->kx, c->ky, g.lh, g.ny, nz, g.dz, 1.0 / g.dz); LES_COUNT_LAUNCH();
   } else {
-    k_tridiag2<CX, PCX><<<(2 * g.lh * g.ny + 127) / 128, 128, 0, c->stream>>>(
+    pdl(k_tridiag2<CX, PCX>, (2 * g.lh * g.ny + 127) / 128, 128, 0, c->stream)(
         Hx, Hy, Hz, BT, BT + g.C, P, c->ibet, c->gamt, c->kx, c->ky, c->kxd, c->kyd, g.lh, g.ny, nz, g.dz,
         nullptr, 0); LES_COUNT_LAUNCH();
   }
@@ -3482,7 +3526,7 @@ static int pressT(les_ctx* c, double* p, double* dpdx, double* dpdy, bool walls,
       }
     }
     if (!done) {
-      k_ikx_rows<CX><<<grid1(L1), 256, 0, c->stream>>>(Y + g.C, Yx, c->kxd, c->kx, g.lh, L1, 0); LES_COUNT_LAUNCH();
+      pdl(k_ikx_rows<CX>, grid1(L1), 256, 0, c->stream)(Y + g.C, Yx, c->kxd, c->kx, g.lh, L1, 0); LES_COUNT_LAUNCH();
       c2rT<T, double>(c, 2, nz - 1, Yx, o1, (long)g.nplane, false, g.lh);
     }
   }
@@ -3498,6 +3542,7 @@ int op_press(les_ctx* c, double* p, double* dpdx, double* dpdy) {
 // tridag_array.f90:1-109 with caller-supplied coefficients (per-routine entry)
 __global__ void k_tridag_generic(const double* a, const double* b, const double* cc, const C2* r, C2* u,
                                  double* gam, int lh, int ny, int n, int* flag) {
+  pdl_wait();
   const int nk = lh * ny;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nk) return;
@@ -3530,14 +3575,14 @@ int op_tridag(les_ctx* c, const double* a, const double* b, const double* cc, co
   const Grid& g = c->g;
   int* flag = reinterpret_cast<int*>(c->dscal + 8);
   double* gam = (double*)c->wsA;
-  k_tridag_generic<<<(g.lh * g.ny + 127) / 128, 128, 0, c->stream>>>(a, b, cc, (const C2*)r, (C2*)u, gam, g.lh, g.ny,
+  pdl(k_tridag_generic, (g.lh * g.ny + 127) / 128, 128, 0, c->stream)(a, b, cc, (const C2*)r, (C2*)u, gam, g.lh, g.ny,
                                                                     g.nz + 1, flag); LES_COUNT_LAUNCH();
   return 0;
 }
 // The same kernel with caller-supplied scratch (gam: lh*ny*n doubles, flag: one int).
 void launch_tridag_generic(const double* a, const double* b, const double* cc, const double* r, double* u,
                            double* gam, int lh, int ny, int n, int* flag, cudaStream_t s) {
-  k_tridag_generic<<<(lh * ny + 127) / 128, 128, 0, s>>>(a, b, cc, (const C2*)r, (C2*)u, gam, lh, ny, n, flag);
+  pdl(k_tridag_generic, (lh * ny + 127) / 128, 128, 0, s)(a, b, cc, (const C2*)r, (C2*)u, gam, lh, ny, n, flag);
   LES_COUNT_LAUNCH();
 }
 
@@ -3546,6 +3591,7 @@ void launch_tridag_generic(const double* a, const double* b, const double* cc, c
 __global__ void k_sflux(const double* __restrict__ theta, const double* __restrict__ wt_s,
                         const double* __restrict__ phi_h, const double* __restrict__ ustar, double* dTdz,
                         double* sgs_t3, int nx, int ny, int ld, double tsus, double vonk, double dz) {
+  pdl_wait();
   GSTRIDE(s, (size_t)nx * ny) {
     const int jy = (int)(s / nx), jx = (int)(s - (size_t)jy * nx);
     const double sf = (theta[0] < 2.0) ? wt_s[s] / tsus : 0.0;
@@ -3561,6 +3607,7 @@ __global__ void k_scalar_prod(const S* __restrict__ um, const S* __restrict__ vm
                               const S* __restrict__ wm, const S* __restrict__ sx,
                               const S* __restrict__ sy, const S* __restrict__ sz, S* R, int ldb,
                               int nx2, int ny2, int nz, const float2* __restrict__ uvm) {
+  pdl_wait();
   const size_t np = (size_t)ldb * ny2;
   GSTRIDE(i, np * nz) {
     const int jz = (int)(i / np) + 1;
@@ -3589,6 +3636,7 @@ __global__ void __launch_bounds__(256) k_scalar_temp_xy(const NT* __restrict__ n
                                                         const double* __restrict__ dsy, double* tx, double* ty, int ld,
                                                         int nx, int ny, int nz, double ipr,
                                                         const double* __restrict__ prt) {
+  pdl_wait();
   const unsigned np = (unsigned)ld * ny;
   const unsigned r = blockIdx.x * 256u + threadIdx.x;
   if (r >= np || (int)(r % (unsigned)ld) >= nx) return;
@@ -3612,6 +3660,7 @@ __global__ void __launch_bounds__(256) k_scalar_rhs(double* R, const double* __r
                                                     const double* __restrict__ dsz, const double* __restrict__ sgs_t3,
                                                     int ld, int nx, int ny, int nz, double ipr,
                                                     const double* __restrict__ prt, double cdz) {
+  pdl_wait();
   const unsigned np = (unsigned)ld * ny;
   const unsigned r = blockIdx.x * 256u + threadIdx.x;
   if (r >= np) return;
@@ -3637,6 +3686,7 @@ __global__ void __launch_bounds__(256) k_divstress_fin32(double* __restrict__ di
                                                          const float* __restrict__ tyz,
                                                          const float* __restrict__ tzz, int ld, int nx, int ny,
                                                          int nz, float cdz) {
+  pdl_wait();
   const unsigned np = (unsigned)ld * ny;
   const unsigned r = blockIdx.x * 256u + threadIdx.x;
   if (r >= np) return;
@@ -3663,6 +3713,7 @@ __global__ void __launch_bounds__(256) k_scalar_temp_xy32(const float* __restric
                                                           const float* __restrict__ dsx,
                                                           const float* __restrict__ dsy, float* tx, float* ty,
                                                           int ld, int nx, int ny, int nz, float ipr) {
+  pdl_wait();
   const unsigned np = (unsigned)ld * ny;
   const unsigned r = blockIdx.x * 256u + threadIdx.x;
   if (r >= np || (int)(r % (unsigned)ld) >= nx) return;
@@ -3678,6 +3729,7 @@ __global__ void __launch_bounds__(256) k_scalar_rhs32(double* R, const float* __
                                                       const double* __restrict__ dsz,
                                                       const double* __restrict__ sgs_t3, int ld, int nx, int ny,
                                                       float ipr, float cdz) {
+  pdl_wait();
   const unsigned np = (unsigned)ld * ny;
   const unsigned r = blockIdx.x * 256u + threadIdx.x;
   if (r >= np) return;
@@ -3691,6 +3743,7 @@ __global__ void __launch_bounds__(256) k_scalar_rhs32(double* R, const float* __
 }
 
 __global__ void k_calcbeta_levels(const double* __restrict__ sums, double* sbr, int nz, double nxny, double gh) {
+  pdl_wait();
   for (int j = threadIdx.x; j < nz; j += blockDim.x) {
     const double sb = sums[j] / nxny;
     sbr[2 * j] = sb;
@@ -3705,6 +3758,7 @@ __global__ void k_calcbeta_levels(const double* __restrict__ sums, double* sbr, 
 template <int KZ>
 __global__ void k_calcbeta(const double* __restrict__ theta, const double* __restrict__ sbr, double* __restrict__ bs,
                            int ld, int nx, int ny, int nz) {
+  pdl_wait();
   const int np = ld * ny;
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= np) return;
@@ -3728,6 +3782,7 @@ __global__ void k_calcbeta(const double* __restrict__ theta, const double* __res
 // (scalars_module.f90:203,221-222), padding columns zero
 __global__ void k_thetav(const double* __restrict__ theta, const double* __restrict__ q, double* __restrict__ tv,
                          size_t n, int ld, int nx, double q_scale) {
+  pdl_wait();
   GSTRIDE(i, n) {
     tv[i] = ((int)(i % ld) < nx) ? theta[i] * (1.0 + 0.61 * 0.001 * q[i] * q_scale) : 0.0;
   }
@@ -3741,14 +3796,14 @@ static void calcbeta(les_ctx* c) {
   double* sbr = c->dred + 20 * (size_t)(g.nz + 8);  // 2 * nz values
   const double* th = c->f[LES_THETA];
   if (k.q_flag) {
-    k_thetav<<<grid1(g.nfield), 256, 0, c->stream>>>(c->f[LES_THETA], c->f[LES_Q], c->tmp, g.nfield, g.ld, g.nx,
+    pdl(k_thetav, grid1(g.nfield), 256, 0, c->stream)(c->f[LES_THETA], c->f[LES_Q], c->tmp, g.nfield, g.ld, g.nx,
                                                      k.q_scale); LES_COUNT_LAUNCH();
     th = c->tmp;
   }
   plane_sums(c, th, (long)g.nplane, g.nz, 4, 1.0, c->dred);
   const double g_hat = k.g * (k.z_i / (k.u_star * k.u_star));
-  k_calcbeta_levels<<<1, 256, 0, c->stream>>>(c->dred, sbr, g.nz, (double)(g.nx * g.ny), 0.5 * g_hat); LES_COUNT_LAUNCH();
-  k_calcbeta<8><<<dim3((unsigned)((g.nplane + 255) / 256), (g.nz + 7) / 8), 256, 0, c->stream>>>(
+  pdl(k_calcbeta_levels, 1, 256, 0, c->stream)(c->dred, sbr, g.nz, (double)(g.nx * g.ny), 0.5 * g_hat); LES_COUNT_LAUNCH();
+  pdl(k_calcbeta<8>, dim3((unsigned)((g.nplane + 255) / 256), (g.nz + 7) / 8), 256, 0, c->stream)(
       th, sbr, c->f[LES_BETA_SCAL], g.ld, g.nx, g.ny, g.nz);
   LES_COUNT_LAUNCH();
 }
@@ -3780,6 +3835,7 @@ static ScalarDesc q_desc(const les_ctx* c) {
 __global__ void k_step_scalar(double* __restrict__ theta, const double* __restrict__ R,
                               const double* __restrict__ Rf, int ld, int nx, int ny, int nz, double dt,
                               int top_grad, double inc) {
+  pdl_wait();
   const int np = ld * ny;
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= np) return;
@@ -3803,7 +3859,7 @@ static int op_scalar(les_ctx* c, const ScalarDesc& d) {
   fill(c, c->f[d.dsdz] + (size_t)(nz - 1) * g.nplane, g.nplane, d.top_grad);
   // RHS_Tf = RHS_T (RHS_T is fully rewritten below)
   cudaMemcpyAsync(c->f[d.rhsf], c->f[d.rhs], g.nfield * sizeof(double), cudaMemcpyDeviceToDevice, c->stream);
-  k_sflux<<<grid1((size_t)g.nx * g.ny, SFC_BS), SFC_BS, 0, c->stream>>>(c->f[d.s], c->f[d.flux], c->f[LES_PHI_H],
+  pdl(k_sflux, grid1((size_t)g.nx * g.ny, SFC_BS), SFC_BS, 0, c->stream)(c->f[d.s], c->f[d.flux], c->f[LES_PHI_H],
                                                             c->f[LES_USTAR_AVG], c->f[d.dsdz],
                                                             c->f[d.sgs3], g.nx, g.ny, g.ld,
                                                             d.flux_scale, k.vonk, g.dz); LES_COUNT_LAUNCH();
@@ -3811,7 +3867,7 @@ static int op_scalar(les_ctx* c, const ScalarDesc& d) {
   for (int q = 0; q < 7; ++q) bigf[q] = c->big + (size_t)q * g.nfield_big;
   const double* in[6] = {c->f[LES_U], c->f[LES_V], c->f[LES_W], c->f[d.dsdx], c->f[d.dsdy], c->f[d.dsdz]};
   op_dealias1(c, in, bigf, 6, nz);
-  k_scalar_prod<double><<<grid1(g.nfield_big), 256, 0, c->stream>>>(bigf[0], bigf[1], bigf[2], bigf[3], bigf[4], bigf[5],
+  pdl(k_scalar_prod<double>, grid1(g.nfield_big), 256, 0, c->stream)(bigf[0], bigf[1], bigf[2], bigf[3], bigf[4], bigf[5],
                                                            bigf[6], g.ld_big, g.nx2, g.ny2, nz, nullptr); LES_COUNT_LAUNCH();
   double* rt = c->f[d.rhs];
   const double* b6 = bigf[6];
@@ -3821,7 +3877,7 @@ static int op_scalar(les_ctx* c, const ScalarDesc& d) {
   double* ty = c->tmp + g.nfield;
   double* dxy = c->tmp + 2 * g.nfield;
   const dim3 gpl((unsigned)((g.nplane + 255) / 256), (unsigned)nz);
-  k_scalar_temp_xy<double><<<gpl, 256, 0, c->stream>>>(c->f[LES_NU_T], c->f[d.dsdx], c->f[d.dsdy], tx, ty, g.ld, g.nx,
+  pdl(k_scalar_temp_xy<double>, gpl, 256, 0, c->stream)(c->f[LES_NU_T], c->f[d.dsdx], c->f[d.dsdy], tx, ty, g.ld, g.nx,
                                                        g.ny, nz, 1.0 / k.pr, c->f[LES_PR_T]);
   LES_COUNT_LAUNCH();
   {
@@ -3835,7 +3891,7 @@ static int op_scalar(les_ctx* c, const ScalarDesc& d) {
     cols(c, J);
     c2r(c, 1, nz, c->wsB, &dxy, (long)g.nplane, false, g.lh);
   }
-  k_scalar_rhs<double><<<dim3(gpl.x, (unsigned)(nz - 1)), 256, 0, c->stream>>>(
+  pdl(k_scalar_rhs<double>, dim3(gpl.x, (unsigned)(nz - 1)), 256, 0, c->stream)(
       rt, dxy, c->f[LES_NU_T], c->f[d.dsdz], c->f[d.sgs3], g.ld, g.nx, g.ny, nz, 1.0 / k.pr, c->f[LES_PR_T], 1.0 / g.dz);
   LES_COUNT_LAUNCH();
   // calcbeta on theta before the update
@@ -3844,7 +3900,7 @@ static int op_scalar(les_ctx* c, const ScalarDesc& d) {
     cudaMemcpyAsync(c->f[d.rhsf], c->f[d.rhs], g.nfield * sizeof(double), cudaMemcpyDeviceToDevice,
                     c->stream);
   const int topg = k.lz_over_zi > 1.0 ? 1 : 0;
-  k_step_scalar<<<dim3((unsigned)((g.nplane + 255) / 256), nz - 1), 256, 0, c->stream>>>(
+  pdl(k_step_scalar, dim3((unsigned)((g.nplane + 255) / 256), nz - 1), 256, 0, c->stream)(
       c->f[d.s], c->f[d.rhs], c->f[d.rhsf], g.ld, g.nx, g.ny, nz, k.dt, topg,
       d.top_grad * g.dz); LES_COUNT_LAUNCH();
   return 0;
@@ -3858,6 +3914,7 @@ __global__ void k_thermo(const double* __restrict__ theta, const double* __restr
                          double* svp, double* pa, double* vp, double* sq, double* rh, double* rhq, double* zl,
                          int ld, int nx, int ny, int nz, double dz, double z_i, double T_scale, double q_scale,
                          double g, double cp, double Rd, double pr_surf) {
+  pdl_wait();
   const size_t np = (size_t)ld * ny;
   GSTRIDE(i, np * (nz - 1)) {
     if ((int)(i % ld) >= nx) continue;
@@ -3883,7 +3940,7 @@ int op_thermo(les_ctx* c, double* const* o) {
   const les_config& k = c->cfg;
   // param.f90:90-96
   const double cp = 1005.0, Rd = 287.04, pr_surf = 100000.0;
-  k_thermo<<<grid1(g.nplane * (g.nz - 1)), 256, 0, c->stream>>>(
+  pdl(k_thermo, grid1(g.nplane * (g.nz - 1)), 256, 0, c->stream)(
       c->f[LES_THETA], c->f[LES_Q], o[0], o[1], o[2], o[3], o[4], o[5], o[6], o[7], o[8], g.ld, g.nx, g.ny, g.nz,
       g.dz, k.z_i, k.t_scale, k.q_scale, k.g, cp, Rd, pr_surf); LES_COUNT_LAUNCH();
   return 0;
@@ -3894,6 +3951,7 @@ int op_thermo(les_ctx* c, double* const* o) {
 __global__ void __launch_bounds__(512) k_rmsdiv_part(const double* __restrict__ du, const double* __restrict__ dv,
                                                      const double* __restrict__ dw, double* part, int ld, int nx,
                                                      int ny) {
+  pdl_wait();
   __shared__ double sh[512];
   const size_t o = (size_t)blockIdx.x * ld * ny;
   double s = 0.0;
@@ -3911,6 +3969,7 @@ __global__ void __launch_bounds__(512) k_rmsdiv_part(const double* __restrict__ 
   if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
 __global__ void k_rmsdiv_fin(const double* part, int n, double denom, double* out) {
+  pdl_wait();
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     double s = 0.0;
     for (int i = 0; i < n; ++i) s += part[i];
@@ -3920,9 +3979,9 @@ __global__ void k_rmsdiv_fin(const double* part, int n, double denom, double* ou
 int op_rmsdiv(les_ctx* c, double* out_dev) {
   const Grid& g = c->g;
   double* part = c->dred;
-  k_rmsdiv_part<<<g.nz - 1, 512, 0, c->stream>>>(c->f[LES_DUDX], c->f[LES_DVDY], c->f[LES_DWDZ], part, g.ld, g.nx,
+  pdl(k_rmsdiv_part, g.nz - 1, 512, 0, c->stream)(c->f[LES_DUDX], c->f[LES_DVDY], c->f[LES_DWDZ], part, g.ld, g.nx,
                                                 g.ny); LES_COUNT_LAUNCH();
-  k_rmsdiv_fin<<<1, 32, 0, c->stream>>>(part, g.nz - 1, (double)(g.nx * g.ny * (g.nz - 1)), out_dev); LES_COUNT_LAUNCH();
+  pdl(k_rmsdiv_fin, 1, 32, 0, c->stream)(part, g.nz - 1, (double)(g.nx * g.ny * (g.nz - 1)), out_dev); LES_COUNT_LAUNCH();
   return 0;
 }
 // timestep_conditions maxima: one block per level reduces max |u|^2 and
@@ -3931,6 +3990,7 @@ template <typename NT>
 __global__ void __launch_bounds__(512) k_tsc_part(const double* __restrict__ u, const double* __restrict__ v,
                                                   const double* __restrict__ w, const NT* __restrict__ nut,
                                                   double* part1, double* part2, int ld, int nx, int ny) {
+  pdl_wait();
   __shared__ double s1[16], s2[16];
   double m1 = -1e300, m2 = -1e300;
   const size_t base = (size_t)ld * ny * blockIdx.x;
@@ -3953,6 +4013,7 @@ __global__ void __launch_bounds__(512) k_tsc_part(const double* __restrict__ u, 
   }
 }
 __global__ void k_tsc_fin(const double* part1, const double* part2, int n, double* out) {
+  pdl_wait();
   double m1 = -1e300, m2 = -1e300;
   for (int k = threadIdx.x; k < n; k += 32) { m1 = fmax(m1, part1[k]); m2 = fmax(m2, part2[k]); }
   for (int o = 16; o > 0; o >>= 1) {
@@ -3966,13 +4027,13 @@ int op_tsc(les_ctx* c, double* cflu, double* visc) {
   double* p1 = c->dred + 12 * (size_t)(g.nz + 8);  // slots 12, 13
   double* p2 = c->dred + 13 * (size_t)(g.nz + 8);
   if (c->cfg.precision == 1)
-    k_tsc_part<float><<<g.nz - 1, 512, 0, c->stream>>>(c->f[LES_U], c->f[LES_V], c->f[LES_W], f32(c, LES_NU_T),
+    pdl(k_tsc_part<float>, g.nz - 1, 512, 0, c->stream)(c->f[LES_U], c->f[LES_V], c->f[LES_W], f32(c, LES_NU_T),
                                                        p1, p2, g.ld, g.nx, g.ny);
   else
-    k_tsc_part<double><<<g.nz - 1, 512, 0, c->stream>>>(c->f[LES_U], c->f[LES_V], c->f[LES_W], c->f[LES_NU_T],
+    pdl(k_tsc_part<double>, g.nz - 1, 512, 0, c->stream)(c->f[LES_U], c->f[LES_V], c->f[LES_W], c->f[LES_NU_T],
                                                         p1, p2, g.ld, g.nx, g.ny);
   LES_COUNT_LAUNCH();
-  k_tsc_fin<<<1, 32, 0, c->stream>>>(p1, p2, g.nz - 1, c->dscal + 2); LES_COUNT_LAUNCH();
+  pdl(k_tsc_fin, 1, 32, 0, c->stream)(p1, p2, g.nz - 1, c->dscal + 2); LES_COUNT_LAUNCH();
   LES_CUDA_CHECK(cudaMemcpyAsync(c->host_scal + 2, c->dscal + 2, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   LES_CUDA_CHECK(cudaStreamSynchronize(c->stream));
   const double delta = std::min(g.dx, g.dy);
@@ -4055,6 +4116,7 @@ template <typename CO, typename R>
 __global__ void k_vort_spec32(const C2* __restrict__ U, const C2* __restrict__ V, const C2* __restrict__ W,
                               const C2* __restrict__ D1, const C2* __restrict__ D2, CO* o1, CO* o2, CO* o3,
                               const R* __restrict__ kx, const R* __restrict__ ky, int nk, int nz, double idz) {
+  pdl_wait();
   GSTRIDE(t, (size_t)nk * nz) {
     const int jz = (int)(t / nk) + 1;
     const size_t m = t - (size_t)(jz - 1) * nk;
@@ -4076,6 +4138,7 @@ __global__ void k_vort_spec(const C2* __restrict__ U, const C2* __restrict__ V, 
                             const C2* __restrict__ D1, const C2* __restrict__ D2, CO* o1, CO* o2, CO* o3,
                             const double* __restrict__ kx, const double* __restrict__ ky, int nk, int nz,
                             double idz) {
+  pdl_wait();
   GSTRIDE(t, (size_t)nk * nz) {
     const int jz = (int)(t / nk) + 1;
     const size_t m = t - (size_t)(jz - 1) * nk;
@@ -4112,6 +4175,7 @@ __global__ void k_dtheta_spec(const CI* __restrict__ T, const C2* __restrict__ Z
                               CO* o1, CO* o2, CO* o3, const double* __restrict__ kx,
                               const double* __restrict__ ky, int nk, int nz, double idz,
                               const double* __restrict__ th0) {
+  pdl_wait();
   GSTRIDE(t, (size_t)nk * nz) {
     const int jz = (int)(t / nk) + 1;
     const size_t m = t - (size_t)(jz - 1) * nk;
@@ -4138,6 +4202,7 @@ __global__ void k_dtheta_spec32(const float2* __restrict__ T, const C2* __restri
                                 float2* o1, float2* o2, float2* o3, const float* __restrict__ kx,
                                 const float* __restrict__ ky, int nk, int nz, double idz,
                                 const double* __restrict__ th0) {
+  pdl_wait();
   GSTRIDE(t, (size_t)nk * nz) {
     const int jz = (int)(t / nk) + 1;
     const size_t m = t - (size_t)(jz - 1) * nk;
@@ -4166,6 +4231,7 @@ __global__ void k_lag_spec(const C2* __restrict__ U, const C2* __restrict__ V, c
                            const C2* __restrict__ D1, const C2* __restrict__ D2, CO* out,
                            const double* __restrict__ kx, const double* __restrict__ ky, int nk, int nz,
                            int jz0, int nl, double idz, int shift) {
+  pdl_wait();
   const size_t st = (size_t)nk * nl;
   GSTRIDE(t, st) {
     const int lc = (int)(t / nk);
@@ -4263,6 +4329,7 @@ __global__ void k_lag_spec32(const C2* __restrict__ U, const C2* __restrict__ V,
                              const C2* __restrict__ D1, const C2* __restrict__ D2, CO* out,
                              const R* __restrict__ kx, const R* __restrict__ ky, int nk, int nz, int jz0, int nl,
                              double idz, int shift) {
+  pdl_wait();
   const size_t st = (size_t)nk * nl;
   GSTRIDE(t, st) {
     const int lc = (int)(t / nk);
@@ -4288,6 +4355,7 @@ __global__ void k_lag_spec32(const C2* __restrict__ U, const C2* __restrict__ V,
 __global__ void k_lag_prod32(const double* __restrict__ u, const double* __restrict__ v,
                              const double* __restrict__ w, Ptr6f Sp, float* out, int ld, int jz0, int nlev,
                              size_t np, const C2* __restrict__ U, const C2* __restrict__ V, size_t nk) {
+  pdl_wait();
   const size_t tot = np * nlev;
   GSTRIDE(t, tot) {
     const int lc = (int)(t / np);
@@ -4318,6 +4386,7 @@ template <typename S>
 __global__ void k_lag_prod(const double* __restrict__ u, const double* __restrict__ v,
                            const double* __restrict__ w, Ptr6 Sp, S* out, int ld, int jz0, int nlev,
                            size_t np, const C2* __restrict__ U, const C2* __restrict__ V, size_t nk) {
+  pdl_wait();
   const size_t tot = np * nlev;
   GSTRIDE(t, tot) {
     const int lc = (int)(t / np);
@@ -4391,17 +4460,17 @@ static int lagrangeT(les_ctx* c) {
     CX* xs = (CX*)c->wsA;
     CX* sp = xs + (size_t)12 * FS;
     if (MX)
-      k_lag_spec32<CX, float><<<grid1((size_t)g.C * nl), 256, 0, c->stream>>>(
+      pdl(k_lag_spec32<CX, float>, grid1((size_t)g.C * nl), 256, 0, c->stream)(
           U, V, W, c->wspec, c->wspec + g.C, sp, c->kxf, c->kyf, (int)g.C, g.nz, jz0, nl, 1.0 / g.dz, 1);
     else
-      k_lag_spec<CX><<<grid1((size_t)g.C * nl), 256, 0, c->stream>>>(U, V, W, c->wspec, c->wspec + g.C, sp, c->kx,
+      pdl(k_lag_spec<CX>, grid1((size_t)g.C * nl), 256, 0, c->stream)(U, V, W, c->wspec, c->wspec + g.C, sp, c->kx,
                                                                   c->ky, (int)g.C, g.nz, jz0, nl, 1.0 / g.dz,
                                                                   M != 0 ? 1 : 0); LES_COUNT_LAUNCH();
     if constexpr (MX)
-      k_lag_prod32<<<grid1(g.nplane * nl), 256, 0, c->stream>>>(c->f[LES_U], c->f[LES_V], c->f[LES_W], Sf, prod,
+      pdl(k_lag_prod32, grid1(g.nplane * nl), 256, 0, c->stream)(c->f[LES_U], c->f[LES_V], c->f[LES_W], Sf, prod,
                                                                 g.ld, jz0, nl, g.nplane, U, V, g.C);
     else
-      k_lag_prod<S><<<grid1(g.nplane * nl), 256, 0, c->stream>>>(c->f[LES_U], c->f[LES_V], c->f[LES_W], Sp, prod, g.ld,
+      pdl(k_lag_prod<S>, grid1(g.nplane * nl), 256, 0, c->stream)(c->f[LES_U], c->f[LES_V], c->f[LES_W], Sp, prod, g.ld,
                                                               jz0, nl, g.nplane, M != 0 ? U : nullptr,
                                                               M != 0 ? V : nullptr, g.C); LES_COUNT_LAUNCH();
     const S* in[12];
@@ -4433,7 +4502,7 @@ static int lagrangeT(les_ctx* c) {
     for (int q = 0; q < 42; ++q) out[q] = flt + (size_t)q * nl * g.nplane;
     c2rT<T, S>(c, 21, nl, c->wsB, out, (long)g.nplane, false, nG);              // G_test outputs
     c2rT<T, S>(c, 21, nl, ob + (size_t)21 * FS, out + 21, (long)g.nplane, false, nGG);  // G_test_test
-    k_lag_final<S, S><<<grid1(g.nplane * nl), 256, 0, c->stream>>>(
+    pdl(k_lag_final<S, S>, grid1(g.nplane * nl), 256, 0, c->stream)(
         flt, c->f[LES_F_LM], c->f[LES_F_MM], c->f[LES_F_QN], c->f[LES_F_NN], c->f[LES_BETA],
         c->f[LES_CS_OPT2], MX ? nullptr : c->f[LES_TN_LMMM], MX ? nullptr : c->f[LES_TN_QNNN], g.ld, g.nx, g.ny,
         g.nz, jz0, nl, g.nplane, (S)cst, (S)opftdelta, (S)lagran_dt, bone, (S)bexp); LES_COUNT_LAUNCH();
@@ -4449,13 +4518,13 @@ static int sgs_stagT(les_ctx* c) {
   const bool lag = (k.model == 4 || k.model == 5 || k.model == 7);
   const dim3 gpl((unsigned)((g.nplane + 255) / 256), (unsigned)g.nz);
   if (MX)
-    k_calc_sij32<<<gpl, 256, 0, c->stream>>>(
+    pdl(k_calc_sij32, gpl, 256, 0, c->stream)(
         f32(c, LES_DUDX), f32(c, LES_DUDY), c->f[LES_DUDZ], f32(c, LES_DVDX), f32(c, LES_DVDY), c->f[LES_DVDZ],
         f32(c, LES_DWDX), f32(c, LES_DWDY), c->f[LES_DWDZ], f32(c, LES_S11), f32(c, LES_S12), f32(c, LES_S13),
         f32(c, LES_S22), f32(c, LES_S23), f32(c, LES_S33), c->f[LES_U], c->f[LES_V], c->f[LES_W], c->f[LES_U_LAG],
         c->f[LES_V_LAG], c->f[LES_W_LAG], g.ld, g.nx, g.ny, lag ? 1 : 0);
   else
-    k_calc_sij<<<dim3((unsigned)((g.nplane + 255) / 256), (unsigned)g.nz), 256, 0, c->stream>>>(
+    pdl(k_calc_sij, dim3((unsigned)((g.nplane + 255) / 256), (unsigned)g.nz), 256, 0, c->stream)(
         c->f[LES_DUDX], c->f[LES_DUDY], c->f[LES_DUDZ], c->f[LES_DVDX], c->f[LES_DVDY], c->f[LES_DVDZ],
         c->f[LES_DWDX], c->f[LES_DWDY], c->f[LES_DWDZ], c->f[LES_S11], c->f[LES_S12], c->f[LES_S13],
         c->f[LES_S22], c->f[LES_S23], c->f[LES_S33], c->f[LES_U], c->f[LES_V], c->f[LES_W], c->f[LES_U_LAG],
@@ -4468,7 +4537,7 @@ static int sgs_stagT(les_ctx* c) {
       double* csz = c->dred;
       if (k.model == 2) op_stddyn(c, csz, S);
       else op_scaledep(c, csz, S);
-      k_bcast_levels<<<grid1(g.nfield), 256, 0, c->stream>>>(c->f[LES_CS_OPT2], csz, g.nplane, g.nfield); LES_COUNT_LAUNCH();
+      pdl(k_bcast_levels, grid1(g.nfield), 256, 0, c->stream)(c->f[LES_CS_OPT2], csz, g.nplane, g.nfield); LES_COUNT_LAUNCH();
     } else if (k.model == 4) {
       op_lagrange_ssim(c, S);
     } else if (k.model == 5) {
@@ -4490,7 +4559,7 @@ static int sgs_stagT(les_ctx* c) {
     Ptr6f Sp;
     const int sid[6] = {LES_S11, LES_S12, LES_S13, LES_S22, LES_S23, LES_S33};
     for (int q = 0; q < 6; ++q) Sp.p[q] = f32(c, sid[q]);
-    k_nut_tau32<<<gpl, 256, 0, c->stream>>>(Sp, c->f[LES_CS_OPT2], f32(c, LES_NU_T), f32(c, LES_TXX),
+    pdl(k_nut_tau32, gpl, 256, 0, c->stream)(Sp, c->f[LES_CS_OPT2], f32(c, LES_NU_T), f32(c, LES_TXX),
                                             f32(c, LES_TXY), f32(c, LES_TYY), f32(c, LES_TXZ), f32(c, LES_TYZ),
                                             f32(c, LES_TZZ), g.ld, g.nx, g.ny, g.nz, (float)(g.delta * g.delta), ov,
                                             csov); LES_COUNT_LAUNCH();
@@ -4560,8 +4629,8 @@ static void rmsdiv_mixed(les_ctx* c, double* dh, const double* dwdz, double* out
   const Grid& g = c->g;
   div_xyT<0>(c, c->f[LES_U], c->f[LES_V], dh, g.nz);
   double* part = c->dred;
-  k_rmsdiv_part<<<g.nz - 1, 512, 0, c->stream>>>(dh, nullptr, dwdz, part, g.ld, g.nx, g.ny); LES_COUNT_LAUNCH();
-  k_rmsdiv_fin<<<1, 32, 0, c->stream>>>(part, g.nz - 1, (double)(g.nx * g.ny * (g.nz - 1)), out_dev); LES_COUNT_LAUNCH();
+  pdl(k_rmsdiv_part, g.nz - 1, 512, 0, c->stream)(dh, nullptr, dwdz, part, g.ld, g.nx, g.ny); LES_COUNT_LAUNCH();
+  pdl(k_rmsdiv_fin, 1, 32, 0, c->stream)(part, g.nz - 1, (double)(g.nx * g.ny * (g.nz - 1)), out_dev); LES_COUNT_LAUNCH();
 }
 // les_rmsdiv between steps in the mixed form: the FP64 divergence of the
 // current state as the next step's filt_da sees it (w Nyquist-filtered; the
@@ -4624,11 +4693,11 @@ static int divstressT(les_ctx* c, double* divtx, double* divty, double* divtz) {
   TS* h[3] = {tmpS, tmpS + g.nfield, tmpS + 2 * g.nfield};
   c2rT<T, TS>(c, 3, g.nz, c->wsB, h, (long)g.nplane, false, g.lh);
   if constexpr (MX)
-    k_divstress_fin32<<<dim3((unsigned)((g.nplane + 255) / 256), (unsigned)g.nz), 256, 0, c->stream>>>(
+    pdl(k_divstress_fin32, dim3((unsigned)((g.nplane + 255) / 256), (unsigned)g.nz), 256, 0, c->stream)(
         divtx, divty, divtz, h[0], h[1], h[2], f32(c, LES_TXZ), f32(c, LES_TYZ), f32(c, LES_TZZ), g.ld, g.nx, g.ny,
         g.nz, (float)(1.0 / g.dz));
   else
-    k_divstress_fin<<<grid1(g.nfield), 256, 0, c->stream>>>(divtx, divty, divtz, h[0], h[1], h[2], c->f[LES_TXZ],
+    pdl(k_divstress_fin, grid1(g.nfield), 256, 0, c->stream)(divtx, divty, divtz, h[0], h[1], h[2], c->f[LES_TXZ],
                                                            c->f[LES_TYZ], c->f[LES_TZZ], g.ld, g.nx, g.ny, g.nz,
                                                            1.0 / g.dz, 7);
   LES_COUNT_LAUNCH();
@@ -4687,7 +4756,7 @@ static int scalarT(les_ctx* c, typename PX<M>::S* const* bigf, const ScalarDesc&
   op_ddz(c, c->f[d.dsdz], c->f[d.s], 1);
   fill(c, c->f[d.dsdz] + (size_t)(nz - 1) * g.nplane, g.nplane, d.top_grad);
   // RHS_Tf = RHS_T: exchanged with the momentum RHS at the start of the step
-  k_sflux<<<grid1((size_t)g.nx * g.ny, SFC_BS), SFC_BS, 0, c->stream>>>(c->f[d.s], c->f[d.flux], c->f[LES_PHI_H],
+  pdl(k_sflux, grid1((size_t)g.nx * g.ny, SFC_BS), SFC_BS, 0, c->stream)(c->f[d.s], c->f[d.flux], c->f[LES_PHI_H],
                                                             c->f[LES_USTAR_AVG], c->f[d.dsdz],
                                                             c->f[d.sgs3], g.nx, g.ny, g.ld,
                                                             d.flux_scale, k.vonk, g.dz); LES_COUNT_LAUNCH();
@@ -4699,17 +4768,17 @@ static int scalarT(les_ctx* c, typename PX<M>::S* const* bigf, const ScalarDesc&
   }
   CX* ds = (CX*)c->wsA;
   if constexpr (MX)
-    k_dtheta_spec32<<<grid1(FS), 256, 0, c->stream>>>(specT, c->wspec + 2 * g.C, c->wspec + 3 * g.C, ds, ds + FS,
+    pdl(k_dtheta_spec32, grid1(FS), 256, 0, c->stream)(specT, c->wspec + 2 * g.C, c->wspec + 3 * g.C, ds, ds + FS,
                                                       ds + 2 * FS, c->kxf, c->kyf, (int)g.C, nz, 1.0 / g.dz, th0);
   else
-    k_dtheta_spec<CX, CX><<<grid1(FS), 256, 0, c->stream>>>(specT, c->wspec + 2 * g.C, c->wspec + 3 * g.C, ds, ds + FS,
+    pdl(k_dtheta_spec<CX, CX>, grid1(FS), 256, 0, c->stream)(specT, c->wspec + 2 * g.C, c->wspec + 3 * g.C, ds, ds + FS,
                                                          ds + 2 * FS, c->kx, c->ky, (int)g.C, nz, 1.0 / g.dz,
                                                          th0); LES_COUNT_LAUNCH();
   {
     S* o3[3] = {bigf[3], bigf[4], bigf[5]};
     padT<M, CX>(c, ds, 3, o3);
   }
-  k_scalar_prod<S><<<grid1(g.nfield_big), 256, 0, c->stream>>>(bigf[0], bigf[1], bigf[2], bigf[3], bigf[4], bigf[5],
+  pdl(k_scalar_prod<S>, grid1(g.nfield_big), 256, 0, c->stream)(bigf[0], bigf[1], bigf[2], bigf[3], bigf[4], bigf[5],
                                                               bigf[6], g.ld_big, g.nx2, g.ny2, nz,
                                                               MX ? mean_tab(c).UVf : nullptr); LES_COUNT_LAUNCH();
   if constexpr (MX) {
@@ -4726,10 +4795,10 @@ static int scalarT(les_ctx* c, typename PX<M>::S* const* bigf, const ScalarDesc&
       unpadT<M, float>(c, b6, o, 1, nz, 1.0 / (double)(g.nx2 * g.ny2));
     }
     const dim3 gpl((unsigned)((g.nplane + 255) / 256), (unsigned)nz);
-    k_scalar_temp_xy32<<<gpl, 256, 0, c->stream>>>(f32(c, LES_NU_T), f32(c, d.dsdx), f32(c, d.dsdy), tx, ty,
+    pdl(k_scalar_temp_xy32, gpl, 256, 0, c->stream)(f32(c, LES_NU_T), f32(c, d.dsdx), f32(c, d.dsdy), tx, ty,
                                                    g.ld, g.nx, g.ny, nz, (float)(1.0 / k.pr)); LES_COUNT_LAUNCH();
     div_xyT<M, float>(c, tx, ty, dxy, nz);
-    k_scalar_rhs32<<<dim3(gpl.x, (unsigned)(nz - 1)), 256, 0, c->stream>>>(
+    pdl(k_scalar_rhs32, dim3(gpl.x, (unsigned)(nz - 1)), 256, 0, c->stream)(
         c->f[d.rhs], rtf, dxy, f32(c, LES_NU_T), c->f[d.dsdz], c->f[d.sgs3], g.ld, g.nx, g.ny,
         (float)(1.0 / k.pr), (float)(1.0 / g.dz)); LES_COUNT_LAUNCH();
   } else {
@@ -4743,10 +4812,10 @@ static int scalarT(les_ctx* c, typename PX<M>::S* const* bigf, const ScalarDesc&
     double* ty = c->tmp + g.nfield;
     double* dxy = c->tmp + 2 * g.nfield;
     const dim3 gpl((unsigned)((g.nplane + 255) / 256), (unsigned)nz);
-    k_scalar_temp_xy<double><<<gpl, 256, 0, c->stream>>>(c->f[LES_NU_T], c->f[d.dsdx], c->f[d.dsdy], tx, ty, g.ld,
+    pdl(k_scalar_temp_xy<double>, gpl, 256, 0, c->stream)(c->f[LES_NU_T], c->f[d.dsdx], c->f[d.dsdy], tx, ty, g.ld,
                                                          g.nx, g.ny, nz, 1.0 / k.pr, c->f[LES_PR_T]); LES_COUNT_LAUNCH();
     div_xyT<M>(c, tx, ty, dxy, nz);
-    k_scalar_rhs<double><<<dim3(gpl.x, (unsigned)(nz - 1)), 256, 0, c->stream>>>(
+    pdl(k_scalar_rhs<double>, dim3(gpl.x, (unsigned)(nz - 1)), 256, 0, c->stream)(
         rt, dxy, c->f[LES_NU_T], c->f[d.dsdz], c->f[d.sgs3], g.ld, g.nx, g.ny, nz, 1.0 / k.pr, c->f[LES_PR_T],
         1.0 / g.dz);
     LES_COUNT_LAUNCH();
@@ -4756,7 +4825,7 @@ static int scalarT(les_ctx* c, typename PX<M>::S* const* bigf, const ScalarDesc&
     cudaMemcpyAsync(c->f[d.rhsf], c->f[d.rhs], g.nfield * sizeof(double), cudaMemcpyDeviceToDevice,
                     c->stream);
   const int topg = k.lz_over_zi > 1.0 ? 1 : 0;
-  k_step_scalar<<<dim3((unsigned)((g.nplane + 255) / 256), nz - 1), 256, 0, c->stream>>>(
+  pdl(k_step_scalar, dim3((unsigned)((g.nplane + 255) / 256), nz - 1), 256, 0, c->stream)(
       c->f[d.s], c->f[d.rhs], c->f[d.rhsf], g.ld, g.nx, g.ny, nz, k.dt, topg,
       d.top_grad * g.dz); LES_COUNT_LAUNCH();
   return 0;
@@ -4771,11 +4840,11 @@ static int convecT(les_ctx* c, typename PX<M>::S* const* bigf, double* cx, doubl
   const size_t FS = (size_t)g.nz * g.C;
   CX* vs = (CX*)c->wsA;
   if (MX)
-    k_vort_spec32<CX, float><<<grid1(FS), 256, 0, c->stream>>>(c->spec, c->spec + FS, c->spec + 2 * FS, c->wspec,
+    pdl(k_vort_spec32<CX, float>, grid1(FS), 256, 0, c->stream)(c->spec, c->spec + FS, c->spec + 2 * FS, c->wspec,
                                                               c->wspec + g.C, vs, vs + FS, vs + 2 * FS, c->kxf,
                                                               c->kyf, (int)g.C, g.nz, 1.0 / g.dz);
   else
-    k_vort_spec<CX><<<grid1(FS), 256, 0, c->stream>>>(c->spec, c->spec + FS, c->spec + 2 * FS, c->wspec, c->wspec + g.C,
+    pdl(k_vort_spec<CX>, grid1(FS), 256, 0, c->stream)(c->spec, c->spec + FS, c->spec + 2 * FS, c->wspec, c->wspec + g.C,
                                                    vs, vs + FS, vs + 2 * FS, c->kx, c->ky, (int)g.C, g.nz,
                                                    1.0 / g.dz); LES_COUNT_LAUNCH();
   {
@@ -4784,7 +4853,7 @@ static int convecT(les_ctx* c, typename PX<M>::S* const* bigf, double* cx, doubl
   }
   const double cst2 = 1.0 / (double)(g.nx2 * g.ny2);
   if constexpr (MX) {
-    k_convec_prod<S><<<grid1(g.nplane_big * (g.nz - 1)), 256, 0, c->stream>>>(
+    pdl(k_convec_prod<S>, grid1(g.nplane_big * (g.nz - 1)), 256, 0, c->stream)(
         bigf[0], bigf[1], bigf[2], bigf[3], bigf[4], bigf[5], bigf[6], bigf[7], bigf[8], g.ld_big, g.nx2, g.ny2,
         g.nz, (S)cst2); LES_COUNT_LAUNCH();
   } else {
@@ -4820,7 +4889,7 @@ static void meanflow_lin(les_ctx* c) {
   const int nz = g.nz;
   const int ms = nz + 8;
   const double* mean = c->dred + 16 * (size_t)ms;  // u, v, w plane means (filt_da_uvw_mixed)
-  k_mean_tab<<<(nz + 127) / 128, 128, 0, c->stream>>>(mean, ms, nz, g.dz, mean_tab(c)); LES_COUNT_LAUNCH();
+  pdl(k_mean_tab, (nz + 127) / 128, 128, 0, c->stream)(mean, ms, nz, g.dz, mean_tab(c)); LES_COUNT_LAUNCH();
   // the transforms are unnormalised: u's x and y round trips gain nx ny,
   // v's and w's x round trip alone gains nx
   const double sc = 1.0 / (double)(g.nx * g.ny), scx = 1.0 / (double)g.nx;
@@ -4839,9 +4908,9 @@ static void meanflow_lin(les_ctx* c) {
   colsT<dfloat, dcomplex>(c, J);
   const dcomplex* sa = (const dcomplex*)c->wsA;
   dcomplex* sb = (dcomplex*)c->wsB;
-  k_ikx_rows<dcomplex><<<grid1((size_t)FS), 256, 0, c->stream>>>(sa + FS, sb, c->kxd, c->kx, g.lh, (size_t)FS, 1);
+  pdl(k_ikx_rows<dcomplex>, grid1((size_t)FS), 256, 0, c->stream)(sa + FS, sb, c->kxd, c->kx, g.lh, (size_t)FS, 1);
   LES_COUNT_LAUNCH();
-  k_ikx_rows<dcomplex><<<grid1((size_t)FS), 256, 0, c->stream>>>(sa + 2 * FS, sb + FS, c->kxd, c->kx, g.lh,
+  pdl(k_ikx_rows<dcomplex>, grid1((size_t)FS), 256, 0, c->stream)(sa + 2 * FS, sb + FS, c->kxd, c->kx, g.lh,
                                                                  (size_t)FS, 0);
   LES_COUNT_LAUNCH();
   dfloat* ml = mlin_fields(c);
@@ -4851,6 +4920,7 @@ static void meanflow_lin(les_ctx* c) {
 // the (0,0) modes of the saved u, v spectra (the plane means) set to zero:
 // the 3/2-grid u', v' and the vorticity fluctuations are padded from them
 __global__ void k_zero_mean_modes(C2* spec, size_t fs, size_t nk, int nz) {
+  pdl_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 2 * nz) return;
   const int f = t / nz, lev = t - f * nz;
@@ -4860,6 +4930,7 @@ __global__ void k_zero_mean_modes(C2* spec, size_t fs, size_t nk, int nz) {
 // float-float spectra of f - plane mean widened to FP64 in place (hi + lo,
 // exact), the plane mean put back into each level's (0,0) mode
 __global__ void k_widen_dc(C2* p, size_t n, size_t nk, int nz, const double* __restrict__ mean, int ms) {
+  pdl_wait();
   GSTRIDE(i, n) {
     const dcomplex v = reinterpret_cast<const dcomplex*>(p)[i];
     double2 w = to_d2(v);
@@ -4899,7 +4970,7 @@ static int filt_da_uvw_ff(les_ctx* c) {
   J.fs_out = FS;
   J.coef[0][0] = CC_KILL; J.coef[1][0] = CC_IKX; J.coef[2][0] = CC_IKY; J.coef[3][0] = CC_KILL;
   colsT<dfloat, dcomplex>(c, J);
-  k_widen_dc<<<grid1(3 * (size_t)FS), 256, 0, c->stream>>>(c->spec, 3 * (size_t)FS, g.C, nz, mean, ms);
+  pdl(k_widen_dc, grid1(3 * (size_t)FS), 256, 0, c->stream)(c->spec, 3 * (size_t)FS, g.C, nz, mean, ms);
   LES_COUNT_LAUNCH();
   double* o9[9] = {f3[0], f3[1], f3[2], c->f[LES_DUDX], c->f[LES_DVDX], c->f[LES_DWDX],
                    c->f[LES_DUDY], c->f[LES_DVDY], c->f[LES_DWDY]};
@@ -4968,7 +5039,7 @@ static int stepT(les_ctx* c) {
   S* bigf[9];
   for (int q = 0; q < 9; ++q) bigf[q] = reinterpret_cast<S*>(c->big) + (size_t)q * g.nfield_big;
   if (MX) {  // the mixed form pads u', v' (its linear terms use the plane means)
-    k_zero_mean_modes<<<(2 * g.nz + 127) / 128, 128, 0, c->stream>>>(c->spec, (size_t)g.nz * g.C, g.C, g.nz);
+    pdl(k_zero_mean_modes, (2 * g.nz + 127) / 128, 128, 0, c->stream)(c->spec, (size_t)g.nz * g.C, g.C, g.nz);
     LES_COUNT_LAUNCH();
   }
   padT<M, C2>(c, c->spec, 3, bigf);  // padded u, v, w (convec.f90:45-65)
@@ -4990,14 +5061,14 @@ static int stepT(les_ctx* c) {
   if (MX) {
     const dfloat* ml = mlin_fields(c);
     const dfloat idz(1.0 / g.dz), dtd(k.dt);
-    k_rhs_ab2_mx<<<dim3((unsigned)((g.nplane + 255) / 256), (unsigned)g.nz), 256, 0, c->stream>>>(
+    pdl(k_rhs_ab2_mx, dim3((unsigned)((g.nplane + 255) / 256), (unsigned)g.nz), 256, 0, c->stream)(
         c->f[LES_U], c->f[LES_V], c->f[LES_W], c->f[LES_RHSX], c->f[LES_RHSY], c->f[LES_RHSZ], ff2(c, LES_RHSX_F),
         ff2(c, LES_RHSY_F), ff2(c, LES_RHSZ_F), c->f[LES_DIVTX], c->f[LES_DIVTY], c->f[LES_DIVTZ],
         c->f[LES_BETA_SCAL], ml, ml + g.nfield, f32(c, LES_DWDY), mean_tab(c), ustar_fields(c),
         ustar_fields(c) + g.nfield, ustar_fields(c) + 2 * g.nfield, g.ld, g.ny, g.nz, make_float2(idz.hi, idz.lo),
         make_float2(dtd.hi, dtd.lo), k.s_flag, euler);
   } else
-    k_rhs_ab2<<<grid1(nv + g.nplane), 256, 0, c->stream>>>(
+    pdl(k_rhs_ab2, grid1(nv + g.nplane), 256, 0, c->stream)(
         c->f[LES_U], c->f[LES_V], c->f[LES_W], c->f[LES_RHSX], c->f[LES_RHSY], c->f[LES_RHSZ], c->f[LES_RHSX_F],
         c->f[LES_RHSY_F], c->f[LES_RHSZ_F], c->f[LES_DIVTX], c->f[LES_DIVTY], c->f[LES_DIVTZ], c->f[LES_BETA_SCAL],
         nv, g.nplane, k.dt, k.s_flag, euler);
@@ -5006,7 +5077,7 @@ static int stepT(les_ctx* c) {
     const float2* ust = ustar_fields(c);
     const float2* u3[3] = {ust, ust + g.nfield, ust + 2 * g.nfield};
     pressT<dfloat>(c, c->f[LES_P], c->f[LES_DPDX], c->f[LES_DPDY], false, u3);
-    k_dpdz_project32<<<dim3((unsigned)((g.nplane + 255) / 256), (unsigned)(g.nz - 1)), 256, 0, c->stream>>>(
+    pdl(k_dpdz_project32, dim3((unsigned)((g.nplane + 255) / 256), (unsigned)(g.nz - 1)), 256, 0, c->stream)(
         c->f[LES_U], c->f[LES_V], c->f[LES_W], u3[0], u3[1], u3[2], ff2(c, LES_RHSX), ff2(c, LES_RHSY),
         ff2(c, LES_RHSZ), c->f[LES_P], c->f[LES_DPDX], c->f[LES_DPDY], c->f[LES_DPDZ], g.ld, g.nx, g.ny, g.nz,
         1.0 / g.dz, k.dt);
@@ -5017,7 +5088,7 @@ static int stepT(les_ctx* c) {
     pressT<double>(c, c->f[LES_P], c->f[LES_DPDX], c->f[LES_DPDY], false);
   }
   if (!MX)
-    k_dpdz_project<<<dim3((unsigned)((g.nplane + 255) / 256), (unsigned)(g.nz - 1)), 256, 0, c->stream>>>(
+    pdl(k_dpdz_project, dim3((unsigned)((g.nplane + 255) / 256), (unsigned)(g.nz - 1)), 256, 0, c->stream)(
         c->f[LES_U], c->f[LES_V], c->f[LES_W], c->f[LES_RHSX], c->f[LES_RHSY], c->f[LES_RHSZ], c->f[LES_P],
         c->f[LES_DPDX], c->f[LES_DPDY], c->f[LES_DPDZ], g.ld, g.nx, g.ny, g.nz, 1.0 / g.dz, -1.5 * k.dt);
   LES_COUNT_LAUNCH();

@@ -90,6 +90,7 @@ template <typename NT>
 __global__ void __launch_bounds__(256) k_stats(StatsIn<NT> in, double* __restrict__ acc, int ld_, int nx, int ny,
                                                int nz, double fr, double pr, double dz, double z_i, double T_scale,
                                                double q_scale, double g) {
+  pdl_wait();
   const unsigned np = (unsigned)ld_ * ny;
   const unsigned r = blockIdx.x * 256u + threadIdx.x;
   if (r >= np) return;
@@ -259,10 +260,10 @@ int op_stats(les_ctx* c) {
   const double fr = (1.0 / (double)c->stats_p) * (double)c->stats_c;  // io.f90:504
   const dim3 grid((unsigned)((g.nplane + 255) / 256), (unsigned)(g.nz - 1));
   if (k.precision == 1)
-    k_stats<float><<<grid, 256, 0, c->stream>>>(stats_in<float>(c), c->stats, g.ld, g.nx, g.ny, g.nz, fr, k.pr, g.dz,
+    pdl(k_stats<float>, grid, 256, 0, c->stream)(stats_in<float>(c), c->stats, g.ld, g.nx, g.ny, g.nz, fr, k.pr, g.dz,
                                                 k.z_i, k.t_scale, k.q_scale, k.g);
   else
-    k_stats<double><<<grid, 256, 0, c->stream>>>(stats_in<double>(c), c->stats, g.ld, g.nx, g.ny, g.nz, fr, k.pr,
+    pdl(k_stats<double>, grid, 256, 0, c->stream)(stats_in<double>(c), c->stats, g.ld, g.nx, g.ny, g.nz, fr, k.pr,
                                                  g.dz, k.z_i, k.t_scale, k.q_scale, k.g);
   LES_COUNT_LAUNCH();
   return 0;
