@@ -1,11 +1,15 @@
 // FP64 y pass (cols) on the integer pipe; see fft_int.cuh.
 //
-// TX columns per block; a column of N = N1 N2 rows is served by
-// max(N1, N2) threads.  Thread q holds the rows q + N1 n2 (n2 < N2) of the
-// physical side or the wavenumbers q + N2 k1 (k1 < N1) of the spectral side;
-// one exchange through shared memory turns one into the other, so a column
-// goes through the registers once per transform.  Columns are numbered
-// through all levels, so that only the last block of a launch has idle ones.
+// TX columns per block, a column of N = R1 R2 R3 rows served by TT threads.  Rows
+// n = n1 + (N / R1) n2: the thread of job n1 holds the R1 rows over n2 and makes
+// the first butterflies; then R1 transforms of N / R1 points are left, done in
+// one step (R3 = 1) or two (R2, then R3), with an exchange through shared memory
+// before each step (the middle step reads and writes its own slots).  The
+// spectral side holds k = j + J k1 the same way.  The inverse runs the steps
+// backwards.  With steps of at most 8 values a thread needs 64 registers and 32
+// warps fit an SM: three steps made the 256-point pass 1.6 times as fast as two
+// of 16 (128 registers, 16 warps).  Columns are numbered through all levels, so
+// that only the last block of a launch has idle ones.
 //
 // Outputs that only drop the Nyquist row (filt_da's field) or multiply by
 // the column's kx need no transform at all in y: the field less its
@@ -80,122 +84,193 @@ __device__ __forceinline__ int col_fix(double2 (&x)[NV], cfix (&v)[NV], unsigned
   return -s - pre;
 }
 
-// forward: v[n2] = x[q + N1 n2], components below 2^fix_in(N2), to
-// v[k1] = X[q + N2 k1]
-template <int N1, int N2, int TX, int NV>
+constexpr int cdiv(int a, int b) { return (a + b - 1) / b; }
+constexpr int clog2(int n) { int b = 0; while ((1 << b) < n) ++b; return b; }
+constexpr int cmax(int a, int b) { return a > b ? a : b; }
+template <int R1_, int R2_, int R3_, int TT_> struct ColShape {
+  static constexpr int R1 = R1_, R2 = R2_, R3 = R3_, TT = TT_, N = R1 * R2 * R3;
+  static constexpr int N1 = N / R1, JA = cdiv(N1, TT);                     // physical side: jobs, jobs a thread
+  static constexpr int NB = R1 * R3, JB = cdiv(NB, TT);                    // middle (or, R3 = 1, last) step
+  static constexpr int SJ = R3 > 1 ? R1 * R2 : R1, SR = R3 > 1 ? R3 : R2;  // spectral side: k = job + SJ i, i < SR
+  static constexpr int JS = cdiv(SJ, TT);
+  static constexpr int PE = JA * R1, SE = JS * SR, E = cmax(PE, cmax(SE, JB * R2));
+  static_assert(N1 % 2 == 0 && TT % 2 == 0 && SR % 2 == 0, "row parity by thread, sign of ky by element");
+  static constexpr int first2 = R3 > 1 ? R1 * R2 : R1;  // points summed before the scale is taken again
+};
+// slot of element p of the sub-transform k2
+template <class P, int TX> __device__ __forceinline__ int col_at(int k2, int p, int b) { return (k2 * P::N1 + p) * TX + b; }
+
+// forward: v[j R1 + i] = x[(q + TT j) + N1 i], components below
+// 2^fix_in(first2), to v[j SR + i] = X[(q + TT j) + SJ i]
+template <class P, int TX, int NV>
 __device__ __forceinline__ void col_fwd(cfix (&v)[NV], cfix* S, unsigned* slot, const int4* __restrict__ tw, int q, int b,
                                         int& ex) {
+  constexpr int R1 = P::R1, R2 = P::R2, R3 = P::R3, TT = P::TT;
   unsigned top = 0;
-  if (q < N1) {
-    fdft<N2, -1>(v);
 #pragma unroll
-    for (int i = 0; i < N2; ++i) {
-      if (i > 0) v[i] = ftw(v[i], __ldg(&tw[q * i]));
-      top = max(top, max(fix_top(v[i].x), fix_top(v[i].y)));
-      S[(i * N1 + q) * TX + b] = v[i];
+  for (int j = 0; j < P::JA; ++j) {
+    const int n1 = q + TT * j;
+    if (n1 < P::N1) {
+      fdft<R1, -1>(v + j * R1);
+#pragma unroll
+      for (int i = 0; i < R1; ++i) {
+        cfix a = v[j * R1 + i];
+        if (i > 0) a = ftw(a, __ldg(&tw[n1 * i]));
+        if (R3 == 1) top = max(top, max(fix_top(a.x), fix_top(a.y)));
+        S[col_at<P, TX>(i, n1, b)] = a;
+      }
     }
   }
-  const int s = fix_down(col_max<TX>(top, slot, b), fix_in(N1));
+  if constexpr (R3 > 1) {
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < P::JB; ++j) {
+      const int t = q + TT * j, k2 = t / R3, m1 = t - k2 * R3;
+      if (t < P::NB) {
+        cfix w[R2];
+#pragma unroll
+        for (int i = 0; i < R2; ++i) w[i] = S[col_at<P, TX>(k2, m1 + R3 * i, b)];
+        fdft<R2, -1>(w);
+#pragma unroll
+        for (int i = 0; i < R2; ++i) {
+          if (i > 0) w[i] = ftw(w[i], __ldg(&tw[m1 * i * R1]));
+          top = max(top, max(fix_top(w[i].x), fix_top(w[i].y)));
+          S[col_at<P, TX>(k2, m1 + R3 * i, b)] = w[i];
+        }
+      }
+    }
+  }
+  const int s = fix_down(col_max<TX>(top, slot, b), fix_in(P::SR));
   const i64 rnd = fix_rnd(s);
   ex += s;
-  if (q < N2) {
 #pragma unroll
-    for (int i = 0; i < N1; ++i) {
-      const cfix a = S[(q * N1 + i) * TX + b];
-      v[i].x = fix_shr(a.x, s, rnd);
-      v[i].y = fix_shr(a.y, s, rnd);
+  for (int j = 0; j < P::JS; ++j) {
+    const int t = q + TT * j;
+    if (t < P::SJ) {
+      const int k2 = R3 > 1 ? t % R1 : t, l2 = R3 > 1 ? t / R1 : 0;
+#pragma unroll
+      for (int i = 0; i < P::SR; ++i) {
+        const cfix a = S[col_at<P, TX>(k2, R3 * l2 + i, b)];
+        v[j * P::SR + i].x = fix_shr(a.x, s, rnd);
+        v[j * P::SR + i].y = fix_shr(a.y, s, rnd);
+      }
+      fdft<P::SR, -1>(v + j * P::SR);
     }
-    fdft<N1, -1>(v);
   }
 }
-// inverse: v[k1] = X[q + N2 k1], sums of N1 moduli below 2^60, to
-// v[n2] = x[q + N1 n2].  (One bound from the whole column's sum would save
-// the second shift, 2 % of a step, but leaves 256 to 384 values of noise four
-// bits fewer: 3/2 round trip at 256^2 4.2e-16 against 1.6e-16.)
-template <int N1, int N2, int TX, int NV>
+// inverse: from v[j SR + i] = X[(q + TT j) + SJ i] with sums of moduli that stay
+// below 2^60 up to the last step (col_weigh), to v[j R1 + i] = x[(q + TT j) + N1 i]
+template <class P, int TX, int NV>
 __device__ __forceinline__ void col_inv(cfix (&v)[NV], cfix* S, unsigned* slot, const int4* __restrict__ tw, int q, int b,
                                         int& ex) {
+  constexpr int R1 = P::R1, R2 = P::R2, R3 = P::R3, TT = P::TT;
   unsigned top = 0;
-  if (q < N2) {
-    fdft<N1, 1>(v);
 #pragma unroll
-    for (int i = 0; i < N1; ++i) {
-      if (i > 0) v[i] = ftwc(v[i], __ldg(&tw[q * i]));
-      top = max(top, max(fix_top(v[i].x), fix_top(v[i].y)));
-      S[(q * N1 + i) * TX + b] = v[i];
+  for (int j = 0; j < P::JS; ++j) {
+    const int t = q + TT * j;
+    if (t < P::SJ) {
+      const int k2 = R3 > 1 ? t % R1 : t, l2 = R3 > 1 ? t / R1 : 0;
+      fdft<P::SR, 1>(v + j * P::SR);
+#pragma unroll
+      for (int i = 0; i < P::SR; ++i) {
+        cfix a = v[j * P::SR + i];
+        if (i > 0) a = ftwc(a, __ldg(&tw[R3 > 1 ? i * l2 * R1 : i * k2]));
+        if (R3 == 1) top = max(top, max(fix_top(a.x), fix_top(a.y)));
+        S[col_at<P, TX>(k2, R3 * l2 + i, b)] = a;
+      }
     }
   }
-  const int s = fix_down(col_max<TX>(top, slot, b), fix_in(N2));
-  const i64 rnd = fix_rnd(s);
-  ex += s;
-  if (q < N1) {
+  if constexpr (R3 > 1) {
+    __syncthreads();
 #pragma unroll
-    for (int i = 0; i < N2; ++i) {
-      const cfix a = S[(i * N1 + q) * TX + b];
-      v[i].x = fix_shr(a.x, s, rnd);
-      v[i].y = fix_shr(a.y, s, rnd);
+    for (int j = 0; j < P::JB; ++j) {
+      const int t = q + TT * j, k2 = t / R3, m1 = t - k2 * R3;
+      if (t < P::NB) {
+        cfix w[R2];
+#pragma unroll
+        for (int i = 0; i < R2; ++i) w[i] = S[col_at<P, TX>(k2, m1 + R3 * i, b)];
+        fdft<R2, 1>(w);
+#pragma unroll
+        for (int i = 0; i < R2; ++i) {
+          w[i] = ftwc(w[i], __ldg(&tw[(m1 + R3 * i) * k2]));
+          top = max(top, max(fix_top(w[i].x), fix_top(w[i].y)));
+          S[col_at<P, TX>(k2, m1 + R3 * i, b)] = w[i];
+        }
+      }
     }
-    fdft<N2, 1>(v);
   }
-}
-// the sums of moduli below 2^60 that col_inv needs: a thread's values, up to
-// 24 with weights up to 192, stay below 2^31 units of 2^44
-template <int N1, int N2, int TX, int NV>
-__device__ __forceinline__ void col_room(cfix (&v)[NV], unsigned* slot, int q, int b, int& ex) {
-  unsigned sum = 0;
-  if (q < N2) {
-#pragma unroll
-    for (int i = 0; i < N1; ++i) sum += fix_l1<12>(v[i]);
-  }
-  const int s = fix_down_sum(col_max<TX>(sum, slot, b), 44);
+  const int s = fix_down(col_max<TX>(top, slot, b), fix_in(R1));
   const i64 rnd = fix_rnd(s);
   ex += s;
 #pragma unroll
-  for (int i = 0; i < N1; ++i) {
-    v[i].x = fix_shr(v[i].x, s, rnd);
-    v[i].y = fix_shr(v[i].y, s, rnd);
+  for (int j = 0; j < P::JA; ++j) {
+    const int n1 = q + TT * j;
+    if (n1 < P::N1) {
+#pragma unroll
+      for (int i = 0; i < R1; ++i) {
+        const cfix a = S[col_at<P, TX>(i, n1, b)];
+        v[j * R1 + i].x = fix_shr(a.x, s, rnd);
+        v[j * R1 + i].y = fix_shr(a.y, s, rnd);
+      }
+      fdft<R1, 1>(v + j * R1);
+    }
   }
 }
-// the same for w(k) v with integer weights: 0 or 1, or (sgn) |ky| as an
-// integer, negative wavenumbers (i >= N1/2) changing sign.  The products are
-// exact 96-bit integers before the shift.
-template <int N1, int N2, int TX, int NV>
-__device__ __forceinline__ void col_weigh(cfix (&v)[NV], const unsigned (&w)[N1], bool sgn, unsigned* slot, int q, int b,
+// w(k) v with integer weights, 0 or 1, or (sgn) |ky| as an integer, negative
+// wavenumbers (i >= SR/2) changing sign, scaled so that the sums of moduli of
+// col_inv's steps before its own scaling stay below 2^60: a job's sum (up to 24
+// values, weights up to 192: below 2^31 units of 2^44), times R2 where a second
+// step follows.  The products are exact 96-bit integers before the shift.
+template <class P, int TX, int NV>
+__device__ __forceinline__ void col_weigh(cfix (&v)[NV], const unsigned (&w)[P::SE], bool sgn, unsigned* slot, int b,
                                           int& ex) {
   unsigned sum = 0;
 #pragma unroll
-  for (int i = 0; i < N1; ++i)
-    if (w[i]) sum += fix_l1<12>(v[i]) * w[i];
-  const int s = fix_down_sum(col_max<TX>(sum, slot, b), 44);
+  for (int j = 0; j < P::JS; ++j) {
+    unsigned t = 0;
+#pragma unroll
+    for (int i = 0; i < P::SR; ++i)
+      if (w[j * P::SR + i]) t += fix_l1<12>(v[j * P::SR + i]) * w[j * P::SR + i];
+    sum = max(sum, t);
+  }
+  const int s = fix_down_sum(col_max<TX>(sum, slot, b), 44 + (P::R3 > 1 ? clog2(P::R2) : 0));
   const i64 rnd = fix_rnd(s);
   const i64 flip = sgn ? -1 : 0;
   ex += s;
 #pragma unroll
-  for (int i = 0; i < N1; ++i) {
-    const i64 lx = mad_wu((unsigned)v[i].x, w[i], rnd), ly = mad_wu((unsigned)v[i].y, w[i], rnd);
-    const i64 hx = mad_w((int)(v[i].x >> 32), (int)w[i], (i64)((unsigned long long)lx >> 32));
-    const i64 hy = mad_w((int)(v[i].y >> 32), (int)w[i], (i64)((unsigned long long)ly >> 32));
+  for (int e = 0; e < P::SE; ++e) {
+    const i64 lx = mad_wu((unsigned)v[e].x, w[e], rnd), ly = mad_wu((unsigned)v[e].y, w[e], rnd);
+    const i64 hx = mad_w((int)(v[e].x >> 32), (int)w[e], (i64)((unsigned long long)lx >> 32));
+    const i64 hy = mad_w((int)(v[e].y >> 32), (int)w[e], (i64)((unsigned long long)ly >> 32));
     // (h 2^32 + low word) >> s, s < 32
-    v[i].x = (i64)(((unsigned long long)__funnelshift_r((unsigned)hx, (unsigned)(hx >> 32), s) << 32) |
+    v[e].x = (i64)(((unsigned long long)__funnelshift_r((unsigned)hx, (unsigned)(hx >> 32), s) << 32) |
                    __funnelshift_r((unsigned)lx, (unsigned)hx, s));
-    v[i].y = (i64)(((unsigned long long)__funnelshift_r((unsigned)hy, (unsigned)(hy >> 32), s) << 32) |
+    v[e].y = (i64)(((unsigned long long)__funnelshift_r((unsigned)hy, (unsigned)(hy >> 32), s) << 32) |
                    __funnelshift_r((unsigned)ly, (unsigned)hy, s));
-    if (i >= N1 / 2) {
-      v[i].x = (v[i].x ^ flip) - flip;
-      v[i].y = (v[i].y ^ flip) - flip;
+    if (e % P::SR >= P::SR / 2) {
+      v[e].x = (v[e].x ^ flip) - flip;
+      v[e].y = (v[e].y ^ flip) - flip;
     }
   }
 }
+// wavenumber of element e of a thread's spectral side, N for none
+template <class P> __device__ __forceinline__ int col_k(int e, int q) {
+  const int job = q + P::TT * (e / P::SR);
+  return job < P::SJ ? job + P::SJ * (e % P::SR) : P::N;
+}
 // weights of ky: |k| or N - |k|, none for the Nyquist row
-template <int N1, int N2> __device__ __forceinline__ void ky_weights(unsigned (&w)[N1], int q, bool zero) {
-  constexpr int N = N1 * N2;
+template <class P> __device__ __forceinline__ void ky_weights(unsigned (&w)[P::SE], int q, bool zero) {
 #pragma unroll
-  for (int i = 0; i < N1; ++i) {
-    const int k = q + N2 * i;
-    w[i] = zero || q >= N2 || k == N / 2 ? 0u : (unsigned)(i < N1 / 2 ? k : N - k);
+  for (int e = 0; e < P::SE; ++e) {
+    const int k = col_k<P>(e, q);
+    w[e] = zero || k == P::N / 2 || k >= P::N ? 0u : (unsigned)(k < P::N / 2 ? k : P::N - k);
   }
 }
-
+// row of element e of a thread's physical side, negative for none
+template <class P> __device__ __forceinline__ int col_row(int e, int q) {
+  const int job = q + P::TT * (e / P::R1);
+  return job < P::N1 ? job + P::N1 * (e % P::R1) : -1;
+}
 // outputs while the integers stay in use: converted four at a time
 template <int CNT, class V, class St>
 __device__ __forceinline__ void fix_groups(V&& val, St&& store, int ex, double factor) {
@@ -218,15 +293,15 @@ __device__ __forceinline__ bool col_direct(const ColJob& J, int o) {  // needs n
 
 // One input, same length.  DIR: the job's direction; ngen: inverse outputs
 // that need a transform (MULTI: several, the spectrum waits in shared memory).
-template <int N1, int N2, int MB, int DIR, bool MULTI>
-__global__ void __launch_bounds__(ICOL_TX * (N1 > N2 ? N1 : N2), MB)
+template <class P, int MB, int DIR, bool MULTI>
+__global__ void __launch_bounds__(ICOL_TX * P::TT, MB)
     k_icol(ColJob J, const int4* __restrict__ tw, int total, int ndirect, int nspec, int ngen) {
   pdl_wait();
-  constexpr int TX = ICOL_TX, N = N1 * N2, NV = N1 > N2 ? N1 : N2, NT = TX * NV;
-  static_assert(NT % 32 == 0 && N1 % 2 == 0, "whole warps; row parity by thread");
+  constexpr int TX = ICOL_TX, N = P::N, NT = TX * P::TT;
+  static_assert(NT % 32 == 0, "whole warps");
   extern __shared__ __align__(16) unsigned char smraw[];
   cfix* S = reinterpret_cast<cfix*>(smraw);
-  cfix* K = S + N * TX;  // the spectrum, kept for later outputs (ngen > 1)
+  cfix* K = S + N * TX;  // the spectrum, kept for later outputs (MULTI)
   __shared__ unsigned slots[ICOL_SLOTS * TX];
   __shared__ i64 sums[2 * TX];
   for (int t = threadIdx.x; t < ICOL_SLOTS * TX; t += NT) slots[t] = 0;
@@ -240,26 +315,26 @@ __global__ void __launch_bounds__(ICOL_TX * (N1 > N2 ? N1 : N2), MB)
   const double2* src = reinterpret_cast<const double2*>(J.in[0]) + in0;
   constexpr bool fwd = (DIR & DIR_FWD) != 0;
   const bool last = jx == J.lh - 1;  // kx = nx/2: removed by KILL and by the derivatives
-  cfix v[NV];
+  cfix v[P::E];
   int ex;
   bool bad = false;
   {
-    double2 x[NV];
-    constexpr int step = fwd ? N1 : N2, cnt = fwd ? N2 : N1;
-    const bool act = ok && q < step;
+    double2 x[P::E];
+    constexpr int cnt = fwd ? P::PE : P::SE;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      x[i] = make_double2(0.0, 0.0);
-      if (act && i < cnt) x[i] = src[(size_t)(q + step * i) * J.wc_in];
+    for (int e = 0; e < cnt; ++e) {
+      const int row = fwd ? col_row<P>(e, q) : col_k<P>(e, q);
+      x[e] = make_double2(0.0, 0.0);
+      if (ok && row >= 0 && row < N) x[e] = src[(size_t)row * J.wc_in];
     }
     __syncthreads();  // slots are zero
-    ex = col_fix<TX, cnt>(x, v, slots, b, fwd ? fix_in(N2) : 60, bad);
+    ex = col_fix<TX, cnt>(x, v, slots, b, fwd ? fix_in(P::first2) : 60, bad);
   }
   double ax = 0.0, ay = 0.0;  // (-1)^row times the alternating sum
   if (DIR == DIR_BOTH && ndirect) {
     i64 sx = 0, sy = 0;
 #pragma unroll
-    for (int i = 0; i < N2; ++i) { sx += (v[i].x + 2) >> 2; sy += (v[i].y + 2) >> 2; }
+    for (int e = 0; e < P::PE; ++e) { sx += (v[e].x + 2) >> 2; sy += (v[e].y + 2) >> 2; }
     if (q & 1) { sx = -sx; sy = -sy; }
     col_sum<TX>(sx, sy, sums, b);
     if (q & 1) { sx = -sx; sy = -sy; }
@@ -270,7 +345,7 @@ __global__ void __launch_bounds__(ICOL_TX * (N1 > N2 ? N1 : N2), MB)
     ay = nan_if(bad, r[0].y);
   }
   auto direct = [&]() {
-    if (DIR != DIR_BOTH || ndirect == 0 || !ok || q >= N1) return;
+    if (DIR != DIR_BOTH || ndirect == 0 || !ok) return;
     for (int o = 0; o < J.nout; ++o) {
       if (!col_direct(J, o)) continue;
       const int code = J.coef[o][0];
@@ -279,11 +354,13 @@ __global__ void __launch_bounds__(ICOL_TX * (N1 > N2 ? N1 : N2), MB)
       const double fn = f * (double)N, bx = one ? 0.0 : f * ax, by = one ? 0.0 : f * ay;
       double2* dst = reinterpret_cast<double2*>(J.out[o]) + out0;
 #pragma unroll
-      for (int i = 0; i < N2; ++i) {  // N f - (-1)^row sum, from the input again
-        const size_t row = (size_t)(q + N1 * i);
-        const double2 a = src[row * J.wc_in];
-        const double rx = fma(fn, a.x, -bx), ry = fma(fn, a.y, -by);
-        dst[row * J.wc_out] = ikx ? make_double2(-ry, rx) : make_double2(rx, ry);
+      for (int e = 0; e < P::PE; ++e) {  // N f - (-1)^row sum, from the input again
+        const int row = col_row<P>(e, q);
+        if (row >= 0) {
+          const double2 a = src[(size_t)row * J.wc_in];
+          const double rx = fma(fn, a.x, -bx), ry = fma(fn, a.y, -by);
+          dst[(size_t)row * J.wc_out] = ikx ? make_double2(-ry, rx) : make_double2(rx, ry);
+        }
       }
     }
   };
@@ -291,15 +368,15 @@ __global__ void __launch_bounds__(ICOL_TX * (N1 > N2 ? N1 : N2), MB)
     direct();
     return;
   }
-  if constexpr (fwd) col_fwd<N1, N2, TX>(v, S, slots + 2 * TX, tw, q, b, ex);
-  if (DIR != DIR_INV && nspec && ok && q < N2) {
+  if constexpr (fwd) col_fwd<P, TX>(v, S, slots + 2 * TX, tw, q, b, ex);
+  if (DIR != DIR_INV && nspec && ok) {
     for (int o = 0; o < J.nout; ++o) {
       if ((J.inv_mask >> o) & 1u) continue;
       const bool kill = J.coef[o][0] == CC_KILL;
       double2* dst = reinterpret_cast<double2*>(J.out[o]) + out0;
-      fix_groups<N1>([&](int i) { return v[i]; }, [&](int i, double2 r) {
-        const int k = q + N2 * i;
-        dst[(size_t)k * J.wc_out] = kill && k == N / 2 ? make_double2(0.0, 0.0) : r;
+      fix_groups<P::SE>([&](int e) { return v[e]; }, [&](int e, double2 r) {
+        const int k = col_k<P>(e, q);
+        if (k < N) dst[(size_t)k * J.wc_out] = kill && k == N / 2 ? make_double2(0.0, 0.0) : r;
       }, ex, kill && last ? 0.0 : nan_if(bad, 1.0));
     }
   }
@@ -313,41 +390,48 @@ __global__ void __launch_bounds__(ICOL_TX * (N1 > N2 ? N1 : N2), MB)
     unsigned* so = slots + (3 + 2 * o) * TX;
     double f = 1.0;
     const bool iky = code == CC_IKY || code == CC_MIKY, rot = iky || code == CC_IKX;
-    unsigned w[N1];
+    unsigned w[P::SE];
     if (iky) {
       f = code == CC_IKY ? J.ky[J.lh] : -J.ky[J.lh];  // row 1: the unit of ky
-      ky_weights<N1, N2>(w, q, last);
+      ky_weights<P>(w, q, last);
     } else if (code == CC_ONE || code == CC_KILL || code == CC_IKX) {
       if (code == CC_IKX) f = J.kx[jx];
 #pragma unroll
-      for (int i = 0; i < N1; ++i) w[i] = q >= N2 || (code != CC_ONE && (last || q + N2 * i == N / 2)) ? 0u : 1u;
+      for (int e = 0; e < P::SE; ++e) {
+        const int k = col_k<P>(e, q);
+        w[e] = k >= N || (code != CC_ONE && (last || k == N / 2)) ? 0u : 1u;
+      }
     } else {  // cutoff filters: pass or drop, one common factor
       const bool wide = code == CC_G || code == CC_MASK;
       const float* T = wide ? J.Gf : J.GGf;
       if (code == CC_G || code == CC_GG) f = (wide ? J.G : J.GG)[0];
 #pragma unroll
-      for (int i = 0; i < N1; ++i)
-        w[i] = q >= N2 || __ldg(&T[(size_t)J.lh * (q + N2 * i) + jx]) == 0.f ? 0u : 1u;
+      for (int e = 0; e < P::SE; ++e) {
+        const int k = col_k<P>(e, q);
+        w[e] = k >= N || __ldg(&T[(size_t)J.lh * k + jx]) == 0.f ? 0u : 1u;
+      }
     }
-    col_weigh<N1, N2, TX>(v, w, iky, so, q, b, ex);
-    col_inv<N1, N2, TX>(v, S, so + TX, tw, q, b, ex);
-    if (ok && q < N1) {
+    col_weigh<P, TX>(v, w, iky, so, b, ex);
+    col_inv<P, TX>(v, S, so + TX, tw, q, b, ex);
+    if (ok) {
       double2* dst = reinterpret_cast<double2*>(J.out[o]) + out0;
-      double2 r[N2];
+      double2 r[P::PE];
       fix_out(v, r, ex, nan_if(bad, f));
 #pragma unroll
-      for (int i = 0; i < N2; ++i)
-        dst[(size_t)(q + N1 * i) * J.wc_out] = make_double2(rot ? -r[i].y : r[i].x, rot ? r[i].x : r[i].y);
+      for (int e = 0; e < P::PE; ++e) {
+        const int row = col_row<P>(e, q);
+        if (row >= 0) dst[(size_t)row * J.wc_out] = make_double2(rot ? -r[e].y : r[e].x, rot ? r[e].x : r[e].y);
+      }
     }
   };
   auto general = [&](int o) { return ((J.inv_mask >> o) & 1u) && !col_direct(J, o); };
   if constexpr (MULTI) {
 #pragma unroll
-    for (int i = 0; i < NV; ++i) K[(i * NV + q) * TX + b] = v[i];
+    for (int e = 0; e < P::SE; ++e) K[(e * P::TT + q) * TX + b] = v[e];
     for (int o = 0; o < J.nout; ++o) {
       if (!general(o)) continue;
 #pragma unroll
-      for (int i = 0; i < NV; ++i) v[i] = K[(i * NV + q) * TX + b];
+      for (int e = 0; e < P::SE; ++e) v[e] = K[(e * P::TT + q) * TX + b];
       ex = ex0;
       output(o);
     }
@@ -361,12 +445,11 @@ __global__ void __launch_bounds__(ICOL_TX * (N1 > N2 ? N1 : N2), MB)
 
 // i kx in0 + i ky in1 (the horizontal divergences): in1 makes the round trip;
 // in0 needs none, only its Nyquist row removed, and is added on the way out.
-template <int N1, int N2, int MB>
-__global__ void __launch_bounds__(ICOL_TX * (N1 > N2 ? N1 : N2), MB)
-    k_icol_div(ColJob J, const int4* __restrict__ tw, int total) {
+template <class P, int MB>
+__global__ void __launch_bounds__(ICOL_TX * P::TT, MB) k_icol_div(ColJob J, const int4* __restrict__ tw, int total) {
   pdl_wait();
-  constexpr int TX = ICOL_TX, N = N1 * N2, NV = N1 > N2 ? N1 : N2, NT = TX * NV, NW = NT / 32;
-  static_assert(NT % 32 == 0 && N1 % 2 == 0, "whole warps; row parity by thread");
+  constexpr int TX = ICOL_TX, N = P::N, NT = TX * P::TT, NW = NT / 32;
+  static_assert(NT % 32 == 0, "whole warps");
   extern __shared__ __align__(16) unsigned char smraw[];
   cfix* S = reinterpret_cast<cfix*>(smraw);
   __shared__ unsigned slots[5 * TX];
@@ -379,17 +462,19 @@ __global__ void __launch_bounds__(ICOL_TX * (N1 > N2 ? N1 : N2), MB)
   const size_t in0 = (size_t)lev * J.ps_in + (size_t)blockIdx.y * J.fs_in + jx;
   const double2* sx = reinterpret_cast<const double2*>(J.in[0]) + in0;
   const double2* sy = reinterpret_cast<const double2*>(J.in[1]) + in0;
-  const bool act = ok && q < N1;
-  cfix v[NV];
+  cfix v[P::E];
   int ex;
   bool bad = false;
   {
-    double2 x[NV];
+    double2 x[P::E];
     double ax = 0.0, ay = 0.0;  // alternating sum of in0
 #pragma unroll
-    for (int i = 0; i < N2; ++i) x[i] = act ? sx[(size_t)(q + N1 * i) * J.wc_in] : make_double2(0.0, 0.0);
+    for (int e = 0; e < P::PE; ++e) {
+      const int row = col_row<P>(e, q);
+      x[e] = ok && row >= 0 ? sx[(size_t)row * J.wc_in] : make_double2(0.0, 0.0);
+    }
 #pragma unroll
-    for (int i = 0; i < N2; ++i) { ax += x[i].x; ay += x[i].y; }
+    for (int e = 0; e < P::PE; ++e) { ax += x[e].x; ay += x[e].y; }
     if (q & 1) { ax = -ax; ay = -ay; }
 #pragma unroll
     for (int o = TX; o < 32; o <<= 1) {
@@ -398,22 +483,22 @@ __global__ void __launch_bounds__(ICOL_TX * (N1 > N2 ? N1 : N2), MB)
     }
     if ((threadIdx.x & 31) < TX) part[(threadIdx.x >> 5) * TX + b] = make_double2(ax, ay);
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      x[i] = make_double2(0.0, 0.0);
-      if (act && i < N2) x[i] = sy[(size_t)(q + N1 * i) * J.wc_in];
+    for (int e = 0; e < P::PE; ++e) {
+      const int row = col_row<P>(e, q);
+      x[e] = ok && row >= 0 ? sy[(size_t)row * J.wc_in] : make_double2(0.0, 0.0);
     }
     __syncthreads();  // slots are zero, partial sums are written
-    ex = col_fix<TX, NV>(x, v, slots, b, fix_in(N2), bad);
+    ex = col_fix<TX, P::PE>(x, v, slots, b, fix_in(P::first2), bad);
   }
-  col_fwd<N1, N2, TX>(v, S, slots + 2 * TX, tw, q, b, ex);
+  col_fwd<P, TX>(v, S, slots + 2 * TX, tw, q, b, ex);
   const bool last = jx == J.lh - 1;
   {
-    unsigned w[N1];
-    ky_weights<N1, N2>(w, q, last);
-    col_weigh<N1, N2, TX>(v, w, true, slots + 3 * TX, q, b, ex);
+    unsigned w[P::SE];
+    ky_weights<P>(w, q, last);
+    col_weigh<P, TX>(v, w, true, slots + 3 * TX, b, ex);
   }
-  col_inv<N1, N2, TX>(v, S, slots + 4 * TX, tw, q, b, ex);
-  if (!act) return;
+  col_inv<P, TX>(v, S, slots + 4 * TX, tw, q, b, ex);
+  if (!ok) return;
   double cx = 0.0, cy = 0.0;
 #pragma unroll
   for (int w = 0; w < NW; ++w) { cx += part[w * TX + b].x; cy += part[w * TX + b].y; }
@@ -421,30 +506,27 @@ __global__ void __launch_bounds__(ICOL_TX * (N1 > N2 ? N1 : N2), MB)
   cx *= q & 1 ? -kx : kx;
   cy *= q & 1 ? -kx : kx;
   double2* dst = reinterpret_cast<double2*>(J.out[0]) + (size_t)lev * J.ps_out + (size_t)blockIdx.y * J.fs_out + jx;
-  double2 r[N2];
+  double2 r[P::PE];
   fix_out(v, r, ex, nan_if(bad, J.ky[J.lh]));
 #pragma unroll
-  for (int i = 0; i < N2; ++i) {
-    const size_t row = (size_t)(q + N1 * i);
-    const double2 a = sx[row * J.wc_in];
-    // i kx N (a - (-1)^y c / N)
-    dst[row * J.wc_out] = make_double2(fma(-kn, a.y, cy - r[i].y), fma(kn, a.x, r[i].x - cx));
+  for (int e = 0; e < P::PE; ++e) {
+    const int row = col_row<P>(e, q);
+    if (row >= 0) {
+      const double2 a = sx[(size_t)row * J.wc_in];
+      // i kx N (a - (-1)^y c / N)
+      dst[(size_t)row * J.wc_out] = make_double2(fma(-kn, a.y, cy - r[e].y), fma(kn, a.x, r[e].x - cx));
+    }
   }
 }
 
-// 3/2 padding (padd.f90:123-133) and truncation (unpadd.f90:143-155): A1 A2
-// rows in, B1 B2 rows out, unit coefficient.  From a spectrum each thread
+// 3/2 padding (padd.f90:123-133) and truncation (unpadd.f90:143-155): PA::N
+// rows in, PB::N rows out, unit coefficient.  From a spectrum each thread
 // loads the rows it needs; otherwise the two layouts meet in shared memory.
-template <int A1, int A2, int B1, int B2, int MB> struct PadT {
-  static constexpr int NA = A1 * A2, NB = B1 * B2;
-  static constexpr int ta = A1 > A2 ? A1 : A2, tb = B1 > B2 ? B1 : B2, nv = ta > tb ? ta : tb;
-};
-template <int A1, int A2, int B1, int B2, int MB>
-__global__ void __launch_bounds__(ICOL_TX * (PadT<A1, A2, B1, B2, MB>::nv), MB)
+template <class PA, class PB, int MB>
+__global__ void __launch_bounds__(ICOL_TX * cmax(PA::TT, PB::TT), MB)
     k_icol_pad(ColJob J, const int4* __restrict__ twa, const int4* __restrict__ twb, int total) {
   pdl_wait();
-  typedef PadT<A1, A2, B1, B2, MB> PT;
-  constexpr int TX = ICOL_TX, NA = PT::NA, NB = PT::NB, NV = PT::nv, NT = TX * NV;
+  constexpr int TX = ICOL_TX, NA = PA::N, NB = PB::N, NT = TX * cmax(PA::TT, PB::TT), E = cmax(PA::E, PB::E);
   constexpr bool PAD = NB > NA;
   constexpr int NS = PAD ? NA : NB, NL = PAD ? NB : NA;
   static_assert(NT % 32 == 0, "whole warps");
@@ -452,62 +534,70 @@ __global__ void __launch_bounds__(ICOL_TX * (PadT<A1, A2, B1, B2, MB>::nv), MB)
   cfix* S = reinterpret_cast<cfix*>(smraw);
   __shared__ unsigned slots[5 * TX];
   for (int t = threadIdx.x; t < 5 * TX; t += NT) slots[t] = 0;
-  const int b = threadIdx.x % TX, q = threadIdx.x / TX;
+  const int b = threadIdx.x % TX, q0 = threadIdx.x / TX;
+  const int qa = q0 < PA::TT ? q0 : 1 << 20, qb = q0 < PB::TT ? q0 : 1 << 20;  // beyond a side's threads: no jobs
   const int col = blockIdx.x * TX + b;
   const bool ok = col < total;
   const int lev = ok ? col / J.ncols : 0, jx = ok ? col - lev * J.ncols : 0;
   const double2* src = reinterpret_cast<const double2*>(J.in[0]) + (size_t)lev * J.ps_in + (size_t)blockIdx.y * J.fs_in + jx;
   double2* dst = reinterpret_cast<double2*>(J.out[0]) + (size_t)lev * J.ps_out + (size_t)blockIdx.y * J.fs_out + jx;
   auto from = [](int k) {  // input wavenumber row of output row k (negative: none)
+    if (k >= NB) return -1;
     if (PAD) return k < NS / 2 ? k : (k > NL - NS / 2 ? k - (NL - NS) : -1);
     return k < NS / 2 ? k : (k == NS / 2 ? -1 : k + (NL - NS));
   };
-  cfix v[NV];
+  cfix v[E];
   int ex;
   bool bad = false;
-  double2 x[NV];
+  double2 x[E];
 #pragma unroll
-  for (int i = 0; i < NV; ++i) x[i] = make_double2(0.0, 0.0);
+  for (int e = 0; e < E; ++e) x[e] = make_double2(0.0, 0.0);
   if (J.dir & DIR_FWD) {
-    if (ok && q < A1) {
 #pragma unroll
-      for (int i = 0; i < A2; ++i) x[i] = src[(size_t)(q + A1 * i) * J.wc_in];
+    for (int e = 0; e < PA::PE; ++e) {
+      const int row = col_row<PA>(e, qa);
+      if (ok && row >= 0) x[e] = src[(size_t)row * J.wc_in];
     }
     __syncthreads();  // slots are zero
-    ex = col_fix<TX, A2>(x, v, slots, b, fix_in(A2), bad);
-    col_fwd<A1, A2, TX>(v, S, slots + 2 * TX, twa, q, b, ex);
+    ex = col_fix<TX, PA::PE>(x, v, slots, b, fix_in(PA::first2), bad);
+    col_fwd<PA, TX>(v, S, slots + 2 * TX, twa, qa, b, ex);
     __syncthreads();  // the exchange buffer is read
-    if (q < A2) {
 #pragma unroll
-      for (int i = 0; i < A1; ++i) S[(q + A2 * i) * TX + b] = v[i];
+    for (int e = 0; e < PA::SE; ++e) {
+      const int k = col_k<PA>(e, qa);
+      if (k < NA) S[k * TX + b] = v[e];
     }
     __syncthreads();
-    if (q < B2) {
 #pragma unroll
-      for (int i = 0; i < B1; ++i) {
-        const int k = from(q + B2 * i);
-        v[i].x = v[i].y = 0;
-        if (k >= 0) v[i] = S[k * TX + b];
-      }
+    for (int e = 0; e < PB::SE; ++e) {
+      const int k = from(col_k<PB>(e, qb));
+      v[e].x = v[e].y = 0;
+      if (k >= 0) v[e] = S[k * TX + b];
     }
   } else {
-    if (ok && q < B2) {
 #pragma unroll
-      for (int i = 0; i < B1; ++i) {
-        const int k = from(q + B2 * i);
-        if (k >= 0) x[i] = src[(size_t)k * J.wc_in];
-      }
+    for (int e = 0; e < PB::SE; ++e) {
+      const int k = from(col_k<PB>(e, qb));
+      if (ok && k >= 0) x[e] = src[(size_t)k * J.wc_in];
     }
     __syncthreads();  // slots are zero
-    ex = col_fix<TX, B1>(x, v, slots, b, 60, bad);
+    ex = col_fix<TX, PB::SE>(x, v, slots, b, 60, bad);
   }
-  col_room<B1, B2, TX>(v, slots + 3 * TX, q, b, ex);
-  col_inv<B1, B2, TX>(v, S, slots + 4 * TX, twb, q, b, ex);
-  if (ok && q < B1) {
-    double2 r[B2];
+  {
+    unsigned w[PB::SE];
+#pragma unroll
+    for (int e = 0; e < PB::SE; ++e) w[e] = 1u;
+    col_weigh<PB, TX>(v, w, false, slots + 3 * TX, b, ex);
+  }
+  col_inv<PB, TX>(v, S, slots + 4 * TX, twb, qb, b, ex);
+  if (ok) {
+    double2 r[PB::PE];
     fix_out(v, r, ex, nan_if(bad, 1.0));
 #pragma unroll
-    for (int i = 0; i < B2; ++i) dst[(size_t)(q + B1 * i) * J.wc_out] = r[i];
+    for (int e = 0; e < PB::PE; ++e) {
+      const int row = col_row<PB>(e, qb);
+      if (row >= 0) dst[(size_t)row * J.wc_out] = r[e];
+    }
   }
 }
 
@@ -518,8 +608,12 @@ template <typename K> void smem_of(K kernel, size_t sm, size_t& set) {
   }
 }
 
-template <int N1, int N2, int MB> bool run_same(const ColJob& J, const FftPlanDev& P, cudaStream_t s) {
-  constexpr int TX = ICOL_TX, NV = N1 > N2 ? N1 : N2, NT = TX * NV;
+// resident blocks for about 1024 threads (three steps, 64 registers) or 512
+template <class P> constexpr int icol_mb(int tt) {
+  return cmax(1, (P::E <= 8 ? 1024 : (P::E <= 12 ? 640 : 512)) / (ICOL_TX * tt));
+}
+template <class P> bool run_same(const ColJob& J, const FftPlanDev& F, cudaStream_t s) {
+  constexpr int TX = ICOL_TX, NT = TX * P::TT, MB = icol_mb<P>(P::TT);
   const int total = J.ncols * J.nlev;
   const dim3 grid((total + TX - 1) / TX, J.nf > 0 ? J.nf : 1);
   if (J.nin == 1) {
@@ -537,17 +631,17 @@ template <int N1, int N2, int MB> bool run_same(const ColJob& J, const FftPlanDe
         ++ng;
       }
     }
-    const size_t sm = (size_t)(N1 * N2 + (ng > 1 ? NV * NV : 0)) * TX * sizeof(cfix);
+    const size_t sm = (size_t)(P::N + (ng > 1 ? P::SE * P::TT : 0)) * TX * sizeof(cfix);
     auto run = [&](auto kernel, size_t& set) {
       smem_of(kernel, sm, set);
-      pdl(kernel, grid, NT, sm, s)(J, P.uniti, total, nd, ns, ng);
+      pdl(kernel, grid, NT, sm, s)(J, F.uniti, total, nd, ns, ng);
     };
     static size_t set[5] = {40 * 1024, 40 * 1024, 40 * 1024, 40 * 1024, 40 * 1024};  // the static arrays count too
-    if (J.dir == DIR_FWD && ng == 0) run(k_icol<N1, N2, MB, DIR_FWD, false>, set[0]);
-    else if (J.dir == DIR_INV && ns == 0 && ng == 1) run(k_icol<N1, N2, MB, DIR_INV, false>, set[1]);
-    else if (J.dir == DIR_INV && ns == 0) run(k_icol<N1, N2, MB, DIR_INV, true>, set[2]);
-    else if (J.dir == DIR_BOTH && ng <= 1) run(k_icol<N1, N2, MB, DIR_BOTH, false>, set[3]);
-    else if (J.dir == DIR_BOTH) run(k_icol<N1, N2, MB, DIR_BOTH, true>, set[4]);
+    if (J.dir == DIR_FWD && ng == 0) run(k_icol<P, MB, DIR_FWD, false>, set[0]);
+    else if (J.dir == DIR_INV && ns == 0 && ng == 1) run(k_icol<P, MB, DIR_INV, false>, set[1]);
+    else if (J.dir == DIR_INV && ns == 0) run(k_icol<P, MB, DIR_INV, true>, set[2]);
+    else if (J.dir == DIR_BOTH && ng <= 1) run(k_icol<P, MB, DIR_BOTH, false>, set[3]);
+    else if (J.dir == DIR_BOTH) run(k_icol<P, MB, DIR_BOTH, true>, set[4]);
     else return false;
     return true;
   }
@@ -564,52 +658,54 @@ template <int N1, int N2, int MB> bool run_same(const ColJob& J, const FftPlanDe
     }
     if (a[o] < 0 || c[o] < 0) return false;
   }
-  const size_t sm = (size_t)N1 * N2 * TX * sizeof(cfix);
+  const size_t sm = (size_t)P::N * TX * sizeof(cfix);
   static size_t set = 40 * 1024;  // the static arrays count too
-  smem_of(k_icol_div<N1, N2, MB>, sm, set);
+  smem_of(k_icol_div<P, MB>, sm, set);
   for (int o = 0; o < J.nout; ++o) {
     ColJob K = J;
     K.in[0] = J.in[a[o]];
     K.in[1] = J.in[c[o]];
     K.out[0] = J.out[o];
-    pdl(k_icol_div<N1, N2, MB>, grid, NT, sm, s)(K, P.uniti, total);
+    pdl(k_icol_div<P, MB>, grid, NT, sm, s)(K, F.uniti, total);
     if (o > 0) LES_COUNT_LAUNCH();  // the caller counts one
   }
   return true;
 }
-template <int A1, int A2, int B1, int B2, int MB>
-bool run_pad(const ColJob& J, const FftPlanDev& Pa, const FftPlanDev& Pb, cudaStream_t s) {
-  constexpr int TX = ICOL_TX;
-  typedef PadT<A1, A2, B1, B2, MB> PT;
-  constexpr bool pad = PT::NB > PT::NA;
+template <class PA, class PB> bool run_pad(const ColJob& J, const FftPlanDev& Fa, const FftPlanDev& Fb, cudaStream_t s) {
+  constexpr int TX = ICOL_TX, TT = cmax(PA::TT, PB::TT);
+  constexpr int MB = cmax(PA::E, PB::E) == PA::E ? icol_mb<PA>(TT) : icol_mb<PB>(TT);
+  constexpr bool pad = PB::N > PA::N;
   if (J.nin != 1 || J.nout != 1 || J.coef[0][0] != CC_ONE || !(J.inv_mask & 1u) ||
-      J.map != (pad ? MAP_PAD : MAP_UNPAD) || J.ny_small != (pad ? PT::NA : PT::NB) || (!pad && !(J.dir & DIR_FWD)))
+      J.map != (pad ? MAP_PAD : MAP_UNPAD) || J.ny_small != (pad ? PA::N : PB::N) || (!pad && !(J.dir & DIR_FWD)))
     return false;
   const int total = J.ncols * J.nlev;
-  const size_t sm = (size_t)std::max(PT::NA, PT::NB) * TX * sizeof(cfix);
+  const size_t sm = (size_t)std::max(PA::N, PB::N) * TX * sizeof(cfix);
   static size_t set = 40 * 1024;  // the static arrays count too
-  smem_of(k_icol_pad<A1, A2, B1, B2, MB>, sm, set);
-  pdl(k_icol_pad<A1, A2, B1, B2, MB>, dim3((total + TX - 1) / TX, J.nf > 0 ? J.nf : 1), TX * PT::nv, sm, s)(
-      J, Pa.uniti, Pb.uniti, total);
+  smem_of(k_icol_pad<PA, PB, MB>, sm, set);
+  pdl(k_icol_pad<PA, PB, MB>, dim3((total + TX - 1) / TX, J.nf > 0 ? J.nf : 1), TX * TT, sm, s)(J, Fa.uniti, Fb.uniti,
+                                                                                               total);
   return true;
 }
 
+// shapes (R1, R2, R3, threads per column)
+template <int N> struct ColOf;
+#define LES_ICOLS(X)                                                                                        \
+  X(16, 4, 4, 1, 4) X(24, 6, 4, 1, 8) X(32, 4, 8, 1, 8) X(36, 6, 6, 1, 8) X(48, 6, 8, 1, 8) X(64, 8, 8, 1, 8) \
+  X(72, 6, 6, 2, 12) X(96, 6, 4, 4, 16) X(108, 9, 12, 1, 12) X(128, 8, 4, 4, 16) X(144, 6, 6, 4, 24)        \
+  X(192, 6, 8, 4, 32) X(216, 6, 6, 6, 36) X(256, 8, 8, 4, 32) X(288, 6, 8, 6, 48) X(384, 6, 8, 8, 64)
+#define LES_DEF(n, a, b, c, t) \
+  template <> struct ColOf<n> { typedef ColShape<a, b, c, t> type; };
+LES_ICOLS(LES_DEF)
+#undef LES_DEF
 }  // namespace
 
-// length: (N1, N2, resident blocks per SM)
-#define LES_ICOLS(X)                                                                                        \
-  X(16, 4, 4, 8) X(24, 8, 3, 6) X(32, 8, 4, 6) X(36, 12, 3, 5) X(48, 12, 4, 5) X(64, 8, 8, 8) X(72, 12, 6, 5)  \
-  X(96, 12, 8, 5) X(108, 12, 9, 5) X(128, 16, 8, 4) X(144, 12, 12, 5) X(192, 16, 12, 4) X(216, 24, 9, 2)     \
-  X(256, 16, 16, 4) X(288, 24, 12, 2) X(384, 24, 16, 2)
-#define LES_IPADS(X)                                                                                       \
-  X(16, 4, 4, 24, 8, 3, 6) X(24, 8, 3, 36, 12, 3, 5) X(32, 8, 4, 48, 12, 4, 5) X(48, 12, 4, 72, 12, 6, 5)  \
-  X(64, 8, 8, 96, 12, 8, 5) X(72, 12, 6, 108, 12, 9, 5) X(96, 12, 8, 144, 12, 12, 5)                       \
-  X(128, 16, 8, 192, 16, 12, 4) X(144, 12, 12, 216, 24, 9, 2) X(192, 16, 12, 288, 24, 12, 2)               \
-  X(256, 16, 16, 384, 24, 16, 2)
+#define LES_IPADS(X)                                                                                  \
+  X(16, 24) X(24, 36) X(32, 48) X(48, 72) X(64, 96) X(72, 108) X(96, 144) X(128, 192) X(144, 216) X(192, 288) \
+  X(256, 384)
 
 bool int_cols_length(int ny) {  // ny and its 3/2 padding
   switch (ny) {
-#define LES_CASE(n, a, b, m, c, d, mb) case n:
+#define LES_CASE(n, m) case n:
     LES_IPADS(LES_CASE)
 #undef LES_CASE
     return true;
@@ -621,17 +717,17 @@ bool launch_cols_int(const ColJob& J, const FftPlanDev& Pin, const FftPlanDev& P
   if (J.map == MAP_SAME) {
     if (J.ny_in != J.ny_out || J.ny_small != J.ny_in) return false;
     switch (J.ny_in) {
-#define LES_CASE(n, a, b, mb) \
-  case n: return run_same<a, b, mb>(J, Pin, s);
+#define LES_CASE(n, a, b, c, t) \
+  case n: return run_same<ColOf<n>::type>(J, Pin, s);
       LES_ICOLS(LES_CASE)
 #undef LES_CASE
       default: return false;
     }
   }
   switch (J.ny_in * 10000 + J.ny_out) {
-#define LES_CASE(n, a, b, m, c, d, mb)                                                \
-  case n * 10000 + m: return run_pad<a, b, c, d, mb>(J, Pin, Pout, s);                \
-  case m * 10000 + n: return run_pad<c, d, a, b, mb>(J, Pin, Pout, s);
+#define LES_CASE(n, m)                                                                      \
+  case n * 10000 + m: return run_pad<ColOf<n>::type, ColOf<m>::type>(J, Pin, Pout, s);      \
+  case m * 10000 + n: return run_pad<ColOf<m>::type, ColOf<n>::type>(J, Pin, Pout, s);
     LES_IPADS(LES_CASE)
 #undef LES_CASE
     default: return false;
