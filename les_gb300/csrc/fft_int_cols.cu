@@ -6,10 +6,13 @@
 // one step (R3 = 1) or two (R2, then R3), with an exchange through shared memory
 // before each step (the middle step reads and writes its own slots).  The
 // spectral side holds k = j + J k1 the same way.  The inverse runs the steps
-// backwards.  With steps of at most 8 values a thread needs 64 registers and 32
-// warps fit an SM: three steps made the 256-point pass 1.6 times as fast as two
-// of 16 (128 registers, 16 warps).  Columns are numbered through all levels, so
-// that only the last block of a launch has idle ones.
+// backwards.  What bounds the pass is issue: with steps of at most 8 values a
+// thread needs 64 registers and 32 warps fit an SM, and the code of one kernel
+// fits the instruction cache.  Two steps of 16 (128 registers, 16 warps) against
+// three, les_filt_da on 64 planes of 256^2: 189 against 172 us; 3/2 round trip of
+// 32 planes of 192^2: 165 against 145 us; FP64 step at 256^3: 20.0 against
+// 19.5 ms.  24 warps instead of 32 (no spills) gave 20.6 ms.  Columns are numbered
+// through all levels, so that only the last block of a launch has idle ones.
 //
 // Outputs that only drop the Nyquist row (filt_da's field) or multiply by
 // the column's kx need no transform at all in y: the field less its
@@ -23,7 +26,7 @@ namespace les {
 namespace {
 
 constexpr int ICOL_TX = 8;
-constexpr int ICOL_SLOTS = 3 + 2 * COL_MAXO;
+constexpr int ICOL_SLOTS = 4 + 2 * COL_MAXO;
 
 // largest m of the column (all threads of the block take part)
 template <int TX> __device__ __forceinline__ unsigned col_max(unsigned m, unsigned* slot, int b) {
@@ -95,13 +98,14 @@ template <int R1_, int R2_, int R3_, int TT_> struct ColShape {
   static constexpr int JS = cdiv(SJ, TT);
   static constexpr int PE = JA * R1, SE = JS * SR, E = cmax(PE, cmax(SE, JB * R2));
   static_assert(N1 % 2 == 0 && TT % 2 == 0 && SR % 2 == 0, "row parity by thread, sign of ky by element");
-  static constexpr int first2 = R3 > 1 ? R1 * R2 : R1;  // points summed before the scale is taken again
 };
 // slot of element p of the sub-transform k2
 template <class P, int TX> __device__ __forceinline__ int col_at(int k2, int p, int b) { return (k2 * P::N1 + p) * TX + b; }
 
-// forward: v[j R1 + i] = x[(q + TT j) + N1 i], components below
-// 2^fix_in(first2), to v[j SR + i] = X[(q + TT j) + SJ i]
+// forward: v[j R1 + i] = x[(q + TT j) + N1 i], components below 2^fix_in(R1),
+// to v[j SR + i] = X[(q + TT j) + SJ i].  The scale is taken again before each
+// step: headroom for 64 points at once would cost a column that one row
+// dominates three bits.  slot: two rows of TX words.
 template <class P, int TX, int NV>
 __device__ __forceinline__ void col_fwd(cfix (&v)[NV], cfix* S, unsigned* slot, const int4* __restrict__ tw, int q, int b,
                                         int& ex) {
@@ -116,20 +120,28 @@ __device__ __forceinline__ void col_fwd(cfix (&v)[NV], cfix* S, unsigned* slot, 
       for (int i = 0; i < R1; ++i) {
         cfix a = v[j * R1 + i];
         if (i > 0) a = ftw(a, __ldg(&tw[n1 * i]));
-        if (R3 == 1) top = max(top, max(fix_top(a.x), fix_top(a.y)));
+        top = max(top, max(fix_top(a.x), fix_top(a.y)));
         S[col_at<P, TX>(i, n1, b)] = a;
       }
     }
   }
   if constexpr (R3 > 1) {
-    __syncthreads();
+    const int s1 = fix_down(col_max<TX>(top, slot, b), fix_in(R2));
+    const i64 rnd1 = fix_rnd(s1);
+    ex += s1;
+    slot += TX;
+    top = 0;
 #pragma unroll
     for (int j = 0; j < P::JB; ++j) {
       const int t = q + TT * j, k2 = t / R3, m1 = t - k2 * R3;
       if (t < P::NB) {
         cfix w[R2];
 #pragma unroll
-        for (int i = 0; i < R2; ++i) w[i] = S[col_at<P, TX>(k2, m1 + R3 * i, b)];
+        for (int i = 0; i < R2; ++i) {
+          const cfix a = S[col_at<P, TX>(k2, m1 + R3 * i, b)];
+          w[i].x = fix_shr(a.x, s1, rnd1);
+          w[i].y = fix_shr(a.y, s1, rnd1);
+        }
         fdft<R2, -1>(w);
 #pragma unroll
         for (int i = 0; i < R2; ++i) {
@@ -328,7 +340,7 @@ __global__ void __launch_bounds__(ICOL_TX * P::TT, MB)
       if (ok && row >= 0 && row < N) x[e] = src[(size_t)row * J.wc_in];
     }
     __syncthreads();  // slots are zero
-    ex = col_fix<TX, cnt>(x, v, slots, b, fwd ? fix_in(P::first2) : 60, bad);
+    ex = col_fix<TX, cnt>(x, v, slots, b, fwd ? fix_in(P::R1) : 60, bad);
   }
   double ax = 0.0, ay = 0.0;  // (-1)^row times the alternating sum
   if (DIR == DIR_BOTH && ndirect) {
@@ -387,7 +399,7 @@ __global__ void __launch_bounds__(ICOL_TX * P::TT, MB)
   const int ex0 = ex;
   auto output = [&](int o) {
     const int code = J.coef[o][0];
-    unsigned* so = slots + (3 + 2 * o) * TX;
+    unsigned* so = slots + (4 + 2 * o) * TX;
     double f = 1.0;
     const bool iky = code == CC_IKY || code == CC_MIKY, rot = iky || code == CC_IKX;
     unsigned w[P::SE];
@@ -452,9 +464,9 @@ __global__ void __launch_bounds__(ICOL_TX * P::TT, MB) k_icol_div(ColJob J, cons
   static_assert(NT % 32 == 0, "whole warps");
   extern __shared__ __align__(16) unsigned char smraw[];
   cfix* S = reinterpret_cast<cfix*>(smraw);
-  __shared__ unsigned slots[5 * TX];
+  __shared__ unsigned slots[6 * TX];
   __shared__ double2 part[NW * TX];
-  for (int t = threadIdx.x; t < 5 * TX; t += NT) slots[t] = 0;
+  for (int t = threadIdx.x; t < 6 * TX; t += NT) slots[t] = 0;
   const int b = threadIdx.x % TX, q = threadIdx.x / TX;
   const int col = blockIdx.x * TX + b;
   const bool ok = col < total;
@@ -488,16 +500,16 @@ __global__ void __launch_bounds__(ICOL_TX * P::TT, MB) k_icol_div(ColJob J, cons
       x[e] = ok && row >= 0 ? sy[(size_t)row * J.wc_in] : make_double2(0.0, 0.0);
     }
     __syncthreads();  // slots are zero, partial sums are written
-    ex = col_fix<TX, P::PE>(x, v, slots, b, fix_in(P::first2), bad);
+    ex = col_fix<TX, P::PE>(x, v, slots, b, fix_in(P::R1), bad);
   }
   col_fwd<P, TX>(v, S, slots + 2 * TX, tw, q, b, ex);
   const bool last = jx == J.lh - 1;
   {
     unsigned w[P::SE];
     ky_weights<P>(w, q, last);
-    col_weigh<P, TX>(v, w, true, slots + 3 * TX, b, ex);
+    col_weigh<P, TX>(v, w, true, slots + 4 * TX, b, ex);
   }
-  col_inv<P, TX>(v, S, slots + 4 * TX, tw, q, b, ex);
+  col_inv<P, TX>(v, S, slots + 5 * TX, tw, q, b, ex);
   if (!ok) return;
   double cx = 0.0, cy = 0.0;
 #pragma unroll
@@ -532,8 +544,8 @@ __global__ void __launch_bounds__(ICOL_TX * cmax(PA::TT, PB::TT), MB)
   static_assert(NT % 32 == 0, "whole warps");
   extern __shared__ __align__(16) unsigned char smraw[];
   cfix* S = reinterpret_cast<cfix*>(smraw);
-  __shared__ unsigned slots[5 * TX];
-  for (int t = threadIdx.x; t < 5 * TX; t += NT) slots[t] = 0;
+  __shared__ unsigned slots[6 * TX];
+  for (int t = threadIdx.x; t < 6 * TX; t += NT) slots[t] = 0;
   const int b = threadIdx.x % TX, q0 = threadIdx.x / TX;
   const int qa = q0 < PA::TT ? q0 : 1 << 20, qb = q0 < PB::TT ? q0 : 1 << 20;  // beyond a side's threads: no jobs
   const int col = blockIdx.x * TX + b;
@@ -559,7 +571,7 @@ __global__ void __launch_bounds__(ICOL_TX * cmax(PA::TT, PB::TT), MB)
       if (ok && row >= 0) x[e] = src[(size_t)row * J.wc_in];
     }
     __syncthreads();  // slots are zero
-    ex = col_fix<TX, PA::PE>(x, v, slots, b, fix_in(PA::first2), bad);
+    ex = col_fix<TX, PA::PE>(x, v, slots, b, fix_in(PA::R1), bad);
     col_fwd<PA, TX>(v, S, slots + 2 * TX, twa, qa, b, ex);
     __syncthreads();  // the exchange buffer is read
 #pragma unroll
@@ -587,9 +599,9 @@ __global__ void __launch_bounds__(ICOL_TX * cmax(PA::TT, PB::TT), MB)
     unsigned w[PB::SE];
 #pragma unroll
     for (int e = 0; e < PB::SE; ++e) w[e] = 1u;
-    col_weigh<PB, TX>(v, w, false, slots + 3 * TX, b, ex);
+    col_weigh<PB, TX>(v, w, false, slots + 4 * TX, b, ex);
   }
-  col_inv<PB, TX>(v, S, slots + 4 * TX, twb, qb, b, ex);
+  col_inv<PB, TX>(v, S, slots + 5 * TX, twb, qb, b, ex);
   if (ok) {
     double2 r[PB::PE];
     fix_out(v, r, ex, nan_if(bad, 1.0));

@@ -52,11 +52,14 @@ def planes(kind, n, ny, nx, seed):
     if kind == "steep":
         f = g.standard_normal((n, ny, nx))
         return f * np.exp(-np.arange(nx) / 3.0)[None, None, :]
+    if kind == "ridge":  # each column of the y pass is one row and little else
+        f = g.standard_normal((n, ny, nx))
+        return f * np.exp(-np.arange(ny) / 3.0)[None, :, None]
     return g.standard_normal((n, ny, nx))
 
 
 @pytest.mark.parametrize("nx,ny", GRIDS)
-@pytest.mark.parametrize("kind", ["wind", "noise", "point", "steep"])
+@pytest.mark.parametrize("kind", ["wind", "noise", "point", "steep", "ridge"])
 def test_plane_transforms(ctx_of, nx, ny, kind):
     c = ctx_of(nx, ny)
     for big in (0, 1):
