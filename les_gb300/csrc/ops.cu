@@ -21,6 +21,17 @@ __device__ __forceinline__ unsigned long long splitmix64(unsigned long long x) {
   x = (x ^ (x >> 27)) * 0x94d049bb133111ebull;
   return x ^ (x >> 31);
 }
+// x^(-1/8): from an FP32 value, one step of the binomial series of
+// (1 - e)^(-1/8) with e = 1 - x y^8 (third order, e < 1e-5: below 1 ulp), 8 FP64
+// operations instead of three square roots and a division.  Values whose FP32
+// form is not normal take those.
+__device__ __forceinline__ double pow_m18(double x) {
+  const float xf = cvt_d2f(x);
+  if (!(xf >= 1e-30f && xf <= 1e30f)) return 1.0 / sqrt(sqrt(sqrt(x)));
+  const double y = cvt_f2d(rsqrtf(sqrtf(sqrtf(xf)))), y2 = y * y, y4 = y2 * y2;
+  const double e = fma(-x, y4 * y4, 1.0);
+  return fma(y, e * fma(e, 9.0 / 128.0, 0.125), y);
+}
 __global__ void k_cvt_selftest(size_t n, unsigned long long seed, unsigned long long* bad) {
   pdl_wait();
   unsigned long long nb = 0;
@@ -35,6 +46,8 @@ __global__ void k_cvt_selftest(size_t n, unsigned long long seed, unsigned long 
       x = 0.5 * (lo + hi);
     }
     if (__float_as_uint(cvt_d2f(x)) != __float_as_uint((float)x) && !(x != x)) ++nb;
+    const double ax = fabs(x), want = 1.0 / sqrt(sqrt(sqrt(ax)));  // within 4 units of its last place
+    if (ax > 0.0 && ax < 1e300 && !(fabs(pow_m18(ax) - want) <= 8.9e-16 * want)) ++nb;
     const float f = __uint_as_float((unsigned)r);
     if (__double_as_longlong(cvt_f2d(f)) != __double_as_longlong((double)f) && !(f != f)) ++nb;
   }
@@ -1484,12 +1497,9 @@ __global__ void k_lag_prep(const double* __restrict__ u, const double* __restric
   }
 }
 
-__device__ __forceinline__ double pow_m18(double x) { return 1.0 / sqrt(sqrt(sqrt(x))); }
 __device__ __forceinline__ float pow_m18(float x) { return 1.0f / sqrtf(sqrtf(sqrtf(x))); }
 // max(real(a), real(b)) of the reference: FP32 comparison, result widened
-// (dt/T) / (1 + dt/T): one division in FP64 (the FP64 pipe bounds
-// k_lag_final: 256^3, 32 levels 886 -> 780 us with this and fmax32 on the
-// integer pipe); FP32 as the reference writes it
+// (dt/T) / (1 + dt/T): one division in FP64; FP32 as the reference writes it
 __device__ __forceinline__ double lag_epsi(double dt, double T) { return dt / (T + dt); }
 __device__ __forceinline__ float lag_epsi(float dt, float T) {
   const float d = dt / T;
@@ -1503,6 +1513,9 @@ __device__ __forceinline__ R smagR(R a11, R a22, R a33, R a12, R a13, R a23) {
 }
 
 // lagrange_Sdep.f90:268-421 from the 42 filtered planes (G: q, GG: 21+q).
+// The FP64 form is bound by the FP64 pipe (205 operations a point; memory would
+// take 140 us): 256^3, 32 levels 781 -> 590 us with pow_m18's series, the
+// common factors taken out of the tensors and the averages as f + epsi (x - f).
 // S: storage of the filtered planes; R: arithmetic (double in the FP64
 // form; float in the mixed form, where the planes are FP32 and the
 // reference truncates F_LM, F_QN and Cs^2 to FP32 itself).  The module
@@ -1513,6 +1526,7 @@ __global__ void k_lag_final(const S* __restrict__ flt, double* F_LM, double* F_M
                             int ny, int nz, int jz0, int nlev, size_t np, R cst, R opftdelta, R lagran_dt,
                             int bexp_one, R bexp) {
   pdl_wait();
+  constexpr bool wide = sizeof(R) == 8;  // FP64: common factors and averages in fewer operations
   const size_t tot = np * nlev;
   GSTRIDE(t, tot) {
     const int lc = (int)(t / np);
@@ -1541,13 +1555,15 @@ __global__ void k_lag_final(const S* __restrict__ flt, double* F_LM, double* F_M
     R M[6], N[6];
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
-      M[q] = cst * (SSb[q] - (R)4 * Sb * Sb_[q]);
-      N[q] = cst * (SSh[q] - (R)16 * Sh * Sh_[q]);
+      M[q] = SSb[q] - (R)4 * Sb * Sb_[q];
+      N[q] = SSh[q] - (R)16 * Sh * Sh_[q];
+      if (!wide) { M[q] = cst * M[q]; N[q] = cst * N[q]; }
     }
-    const R LM = Lq[0] * M[0] + Lq[3] * M[3] + Lq[5] * M[5] + (R)2 * (Lq[1] * M[1] + Lq[2] * M[2] + Lq[4] * M[4]);
-    const R MM = M[0] * M[0] + M[3] * M[3] + M[5] * M[5] + (R)2 * (M[1] * M[1] + M[2] * M[2] + M[4] * M[4]);
-    const R QN = Qq[0] * N[0] + Qq[3] * N[3] + Qq[5] * N[5] + (R)2 * (Qq[1] * N[1] + Qq[2] * N[2] + Qq[4] * N[4]);
-    const R NN = N[0] * N[0] + N[3] * N[3] + N[5] * N[5] + (R)2 * (N[1] * N[1] + N[2] * N[2] + N[4] * N[4]);
+    R LM = Lq[0] * M[0] + Lq[3] * M[3] + Lq[5] * M[5] + (R)2 * (Lq[1] * M[1] + Lq[2] * M[2] + Lq[4] * M[4]);
+    R MM = M[0] * M[0] + M[3] * M[3] + M[5] * M[5] + (R)2 * (M[1] * M[1] + M[2] * M[2] + M[4] * M[4]);
+    R QN = Qq[0] * N[0] + Qq[3] * N[3] + Qq[5] * N[5] + (R)2 * (Qq[1] * N[1] + Qq[2] * N[2] + Qq[4] * N[4]);
+    R NN = N[0] * N[0] + N[3] * N[3] + N[5] * N[5] + (R)2 * (N[1] * N[1] + N[2] * N[2] + N[4] * N[4]);
+    if (wide) { LM *= cst; MM *= cst * cst; QN *= cst; NN *= cst * cst; }
     const R e24 = (R)1e-24f;
     R flm = (R)F_LM[gi], fmm = (R)F_MM[gi];
     R Tn = fmax32r(flm * fmm, e24);
@@ -1555,8 +1571,8 @@ __global__ void k_lag_final(const S* __restrict__ flt, double* F_LM, double* F_M
     Tn = opftdelta * pow_m18(Tn);
     Tn = fmax32r(e24, Tn);
     R epsi = lag_epsi(lagran_dt, Tn);
-    flm = (epsi * LM + ((R)1 - epsi) * flm);
-    fmm = (epsi * MM + ((R)1 - epsi) * fmm);
+    flm = wide ? flm + epsi * (LM - flm) : (epsi * LM + ((R)1 - epsi) * flm);
+    fmm = wide ? fmm + epsi * (MM - fmm) : (epsi * MM + ((R)1 - epsi) * fmm);
     flm = fmax32r(e24, flm);
     R cs2d = fmax32r(e24, flm / fmm);
     F_LM[gi] = flm; F_MM[gi] = fmm;
@@ -1566,8 +1582,8 @@ __global__ void k_lag_final(const S* __restrict__ flt, double* F_LM, double* F_M
     Tn = opftdelta * pow_m18(Tn);
     Tn = fmax32r(e24, Tn);
     epsi = lag_epsi(lagran_dt, Tn);
-    fqn = (epsi * QN + ((R)1 - epsi) * fqn);
-    fnn = (epsi * NN + ((R)1 - epsi) * fnn);
+    fqn = wide ? fqn + epsi * (QN - fqn) : (epsi * QN + ((R)1 - epsi) * fqn);
+    fnn = wide ? fnn + epsi * (NN - fnn) : (epsi * NN + ((R)1 - epsi) * fnn);
     fqn = fmax32r(e24, fqn);
     R cs4d = fmax32r(e24, fqn / fnn);
     F_QN[gi] = fqn; F_NN[gi] = fnn;
