@@ -48,6 +48,10 @@ __global__ void k_cvt_selftest(size_t n, unsigned long long seed, unsigned long 
     if (__float_as_uint(cvt_d2f(x)) != __float_as_uint((float)x) && !(x != x)) ++nb;
     const double ax = fabs(x), want = 1.0 / sqrt(sqrt(sqrt(ax)));  // within 4 units of its last place
     if (ax > 0.0 && ax < 1e300 && !(fabs(pow_m18(ax) - want) <= 8.9e-16 * want)) ++nb;
+    const dfloat h = split_d(x);
+    const float rest = (float)(x - (double)(float)x);
+    if (!(rest != rest) && (__float_as_uint(h.hi) != __float_as_uint((float)x) || __float_as_uint(h.lo) != __float_as_uint(rest)))
+      ++nb;
     const float f = __uint_as_float((unsigned)r);
     if (__double_as_longlong(cvt_f2d(f)) != __double_as_longlong((double)f) && !(f != f)) ++nb;
   }
@@ -2539,8 +2543,10 @@ __device__ __forceinline__ dfloat ldf2(const float2* p, size_t i) {
 // per point (splitting u and w into float-float) instead of seventeen; the
 // projection forms the FP64 state from u* (k_dpdz_project32).  wz = w_z,
 // wx = dw/dx on the uvp / w levels (float-float transforms), dwdy the
-// FP32-held dw/dy.  grid (ceil(np/256), nz).
-__global__ void __launch_bounds__(256) k_rhs_ab2_mx(
+// FP32-held dw/dy.  172 bytes a point, 427 us at 256^3: 806 us with loads between
+// the stores that they might alias, 595 us with all loads first, the integer
+// split and 24 warps (80 registers; 112 without the bound).  grid (ceil(np/256), nz).
+__global__ void __launch_bounds__(256, 3) k_rhs_ab2_mx(
     const double* __restrict__ u, const double* __restrict__ v, const double* __restrict__ w, double* Rx,
     double* Ry, double* Rz, float2* Rxf, float2* Ryf, float2* Rzf,
     const double* __restrict__ dx_, const double* __restrict__ dy_, const double* __restrict__ dz_,
@@ -2560,45 +2566,49 @@ __global__ void __launch_bounds__(256) k_rhs_ab2_mx(
   }
   const dfloat h(0.5f, 0.f);
   const dfloat idz(idz2.x, idz2.y);  // 1/dz and dt as float-float pairs formed on the host
+  // every field of the point before the first use and the first store
+  const size_t im = jz >= 2 ? i - np : i;
+  const double w0 = w[i], w1 = w[i + np], u0 = u[i], v0 = v[i], um0 = u[im], vm0 = v[im];
+  const double Rx0 = Rx[i], Ry0 = Ry[i], Rz0 = Rz[i], dx0 = dx_[i], dy0 = dy_[i], dz0 = dz_[i];
+  const double bs0 = sflag ? bs[i] : 0.0;
+  const dfloat s1 = wz[i], wx0 = wx[i];
+  const float dwdy0 = dwdy[i];
+  dfloat fx, fy, fz;
+  if (!euler) { fx = ldf2(Rxf, i); fy = ldf2(Ryf, i); fz = ldf2(Rzf, i); }
   const dfloat U = ldt(T.U, jz), V = ldt(T.V, jz);
-  const dfloat wi = cvt<dfloat>(w[i]), wp = cvt<dfloat>(w[i + np]);
-  const dfloat s1 = wz[i];
+  const dfloat wi = cvt<dfloat>(w0), wp = cvt<dfloat>(w1);
   const dfloat oyp = ldt(T.Oy, jz + 1), oxp = ldt(T.Ox, jz + 1), oy = ldt(T.Oy, jz), ox = ldt(T.Ox, jz);
   const dfloat cxl = (-V) * s1 + h * (oyp * wp + oy * wi);
   const dfloat cyl = U * s1 - h * (oxp * wp + ox * wi);
   dfloat czl(0.f, 0.f);
-  const dfloat uf = cvt<dfloat>(u[i]);
+  const dfloat uf = cvt<dfloat>(u0);
   if (jz >= 2) {
-    const size_t im = i - np;
     const dfloat Um = ldt(T.U, jz - 1);
-    const dfloat up = uf - U, upm = cvt<dfloat>(u[im]) - Um;
-    const float vp = cvt_d2f(v[i]) - T.UVf[jz].y, vpm = cvt_d2f(v[im]) - T.UVf[jz - 1].y;
-    const dfloat wyp = (up - upm) * idz - wx[i];                          // w_y' at w-level jz
-    const float wxp = dwdy[i] - (vp - vpm) * idz2.x;                    // w_x' (FP32: its factor V is small)
+    const dfloat up = uf - U, upm = cvt<dfloat>(um0) - Um;
+    const float vp = cvt_d2f(v0) - T.UVf[jz].y, vpm = cvt_d2f(vm0) - T.UVf[jz - 1].y;
+    const dfloat wyp = (up - upm) * idz - wx0;                          // w_y' at w-level jz
+    const float wxp = dwdy0 - (vp - vpm) * idz2.x;                    // w_x' (FP32: its factor V is small)
     const dfloat Us = U + Um;
     const float Vs = T.UVf[jz].y + T.UVf[jz - 1].y;
     czl = h * ((-Us) * wyp - oy * (up + upm)) + dfs(0.5f * (Vs * wxp) + 0.5f * (ox.hi * (vp + vpm))) +
           ldt(T.Cz, jz);
   }
-  const dfloat rx = -(dfs(cvt_d2f(Rx[i])) + cxl) - dfs(cvt_d2f(dx_[i]));
-  const dfloat ry = -(dfs(cvt_d2f(Ry[i])) + cyl) - dfs(cvt_d2f(dy_[i]));
-  dfloat rz = -(dfs(cvt_d2f(Rz[i])) + czl) - dfs(cvt_d2f(dz_[i]));
-  if (sflag) rz = rz + cvt<dfloat>(bs[i]);
+  const dfloat rx = -(dfs(cvt_d2f(Rx0)) + cxl) - dfs(cvt_d2f(dx0));
+  const dfloat ry = -(dfs(cvt_d2f(Ry0)) + cyl) - dfs(cvt_d2f(dy0));
+  dfloat rz = -(dfs(cvt_d2f(Rz0)) + czl) - dfs(cvt_d2f(dz0));
+  if (sflag) rz = rz + cvt<dfloat>(bs0);
   const float2 rx2 = make_float2(rx.hi, rx.lo), ry2 = make_float2(ry.hi, ry.lo), rz2 = make_float2(rz.hi, rz.lo);
   reinterpret_cast<float2*>(Rx)[i] = rx2;  // the slot held c_nl in FP64 until now
   reinterpret_cast<float2*>(Ry)[i] = ry2;
   reinterpret_cast<float2*>(Rz)[i] = rz2;
-  dfloat fx, fy, fz;
   if (euler) {
     fx = rx; fy = ry; fz = rz;
     Rxf[i] = rx2; Ryf[i] = ry2; Rzf[i] = rz2;
-  } else {
-    fx = ldf2(Rxf, i); fy = ldf2(Ryf, i); fz = ldf2(Rzf, i);
   }
   const dfloat dtf(dt2.x, dt2.y);
   const dfloat a15(1.5f, 0.f), a05(0.5f, 0.f);
   const dfloat ux = uf + dtf * (a15 * rx - a05 * fx);
-  const dfloat vx = cvt<dfloat>(v[i]) + dtf * (a15 * ry - a05 * fy);
+  const dfloat vx = cvt<dfloat>(v0) + dtf * (a15 * ry - a05 * fy);
   const dfloat wx2 = wi + dtf * (a15 * rz - a05 * fz);
   us[i] = make_float2(ux.hi, ux.lo);
   vs[i] = make_float2(vx.hi, vx.lo);
@@ -2669,20 +2679,23 @@ __global__ void __launch_bounds__(256) k_dpdz_project32(double* u, double* v, do
   const size_t i = (size_t)(jz - 1) * np + r;
   const bool inx = (int)(r % (unsigned)ld) < nx;
   const double c = -1.5 * dt;
+  // every field of the point before the first store
+  const double gx = dpdx[i], gy = dpdy[i], p0 = p[i], p1 = p[i + np];
+  const dfloat Rx0 = ldf2(Rx, i), Ry0 = ldf2(Ry, i), Rz0 = ldf2(Rz, i);
+  const dfloat u0 = ldf2(us, i), v0 = ldf2(vs, i), w0 = ldf2(ws, i);
   double pz;
   if (inx) {
-    pz = (p[i + np] - p[i]) * idz;
+    pz = (p1 - p0) * idz;
     dpdz[i] = pz;
   } else {
     pz = dpdz[i];
   }
-  const double gx = dpdx[i], gy = dpdy[i];
-  const dfloat rx = ldf2(Rx, i) - cvt<dfloat>(gx), ry = ldf2(Ry, i) - cvt<dfloat>(gy);
-  const dfloat rz = ldf2(Rz, i) - cvt<dfloat>(pz);
+  const dfloat rx = Rx0 - cvt<dfloat>(gx), ry = Ry0 - cvt<dfloat>(gy);
+  const dfloat rz = Rz0 - cvt<dfloat>(pz);
   Rx[i] = make_float2(rx.hi, rx.lo);
   Ry[i] = make_float2(ry.hi, ry.lo);
   Rz[i] = make_float2(rz.hi, rz.lo);
-  double uu = cvt<double>(ldf2(us, i)), vv = cvt<double>(ldf2(vs, i)), ww = cvt<double>(ldf2(ws, i));
+  double uu = cvt<double>(u0), vv = cvt<double>(v0), ww = cvt<double>(w0);
   if (inx) {
     uu = fma(c, gx, uu);
     vv = fma(c, gy, vv);
