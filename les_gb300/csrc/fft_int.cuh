@@ -10,9 +10,11 @@
 // instruction per value on the way out (1.9 per clock).
 //
 // Measured against the FP64 kernels (256^2 planes): field and derivatives of
-// 64 planes (les_filt_da) 1122 -> 200 us, FP64 step at 256^3 89.1 -> 22.0 ms.
-// What bounds them is instruction issue at 16 warps per SM (128 registers):
-// 42 to 46 % of the issue slots and half of the integer pipe are busy.
+// 64 planes (les_filt_da) 1122 -> 173 us, FP64 step at 256^3 89.1 -> 19.2 ms.
+// What bounds them is instruction issue: the x pass runs 16 to 20 warps per SM
+// (96 to 128 registers, 46 % of the issue slots busy, half of the integer pipe),
+// the y pass 32.  The x pass in three steps of at most eight values (64
+// registers, 32 warps) was no faster at any length.
 //
 // Precision.  A value is a multiple of 2^ex with |value / 2^ex| < 2^61, so a
 // row's largest elements carry 55 to 60 bits (an FP64 number: 53) and
@@ -20,14 +22,16 @@
 // largest inputs in FP64 arithmetic as well.  The scale is chosen from the
 // data: from the row's largest exponent at the load, for an inverse from the
 // sums of moduli of its first butterflies (a spectrum that one mode dominates
-// keeps its full width), and from the largest value between the two steps
-// (the inverse x pass instead takes the sum of all moduli, which bounds both
-// steps).  Each choice leaves the headroom that the following step can need,
-// so nothing overflows.
+// keeps its full width), and from the largest value between the steps (the
+// inverse x pass instead takes the sum of all moduli, which bounds all of it).
+// Each choice leaves the headroom that the following step can need, so nothing
+// overflows.
 // Twiddles are rounded to 62 fractional bits.  Against extended precision
-// (noise, and a mean wind of 170 times the noise, 32^2 to 256^2) the relative
-// error is 0.25 to 0.75 of the FP64 kernels' in the field, its derivatives and
-// the 3/2 round trip.
+// (noise, a mean wind of 170 times the noise, a single point, fields that fall
+// off along x or along y; 32^2 to 256^2 and their 3/2 grids) the relative error is
+// 0.16 to 0.85 of the FP64 kernels' in the field, its derivatives, the plane
+// transforms and the 3/2 round trip; the inverse of a single point's flat spectrum
+// in rows of 384, where the sum of moduli costs most, is at 1.2 (2.2 eps).
 //
 // Not-a-number and infinity in a row or column make all of it NaN, as the
 // butterflies of an FP64 transform do.  Values below 2^-1042 count as zero.
