@@ -98,6 +98,10 @@ template <int R1_, int R2_, int R3_, int TT_> struct ColShape {
   static constexpr int JS = cdiv(SJ, TT);
   static constexpr int PE = JA * R1, SE = JS * SR, E = cmax(PE, cmax(SE, JB * R2));
   static_assert(N1 % 2 == 0 && TT % 2 == 0 && SR % 2 == 0, "row parity by thread, sign of ky by element");
+  // shift of the alternating sum's terms: N of them below 2^fix_in(R1) (strictly:
+  // multiples of 2^(fix_in(R1) - 53)) stay below 2^63.  3 for 288 and 384 rows, else 2.
+  static constexpr int ALT = cmax(2, clog2(N) + fix_in(R1) - 63);
+  static_assert(clog2(N) + fix_in(R1) - ALT <= 63, "alternating sum");
 };
 // slot of element p of the sub-transform k2
 template <class P, int TX> __device__ __forceinline__ int col_at(int k2, int p, int b) { return (k2 * P::N1 + p) * TX + b; }
@@ -344,15 +348,17 @@ __global__ void __launch_bounds__(ICOL_TX * P::TT, MB)
   }
   double ax = 0.0, ay = 0.0;  // (-1)^row times the alternating sum
   if (DIR == DIR_BOTH && ndirect) {
+    constexpr int SH = P::ALT;
+    constexpr i64 SR = 1ll << (SH - 1);
     i64 sx = 0, sy = 0;
 #pragma unroll
-    for (int e = 0; e < P::PE; ++e) { sx += (v[e].x + 2) >> 2; sy += (v[e].y + 2) >> 2; }
+    for (int e = 0; e < P::PE; ++e) { sx += fix_shr(v[e].x, SH, SR); sy += fix_shr(v[e].y, SH, SR); }
     if (q & 1) { sx = -sx; sy = -sy; }
     col_sum<TX>(sx, sy, sums, b);
     if (q & 1) { sx = -sx; sy = -sy; }
     const cfix t[1] = {{sx, sy}};
     double2 r[1];
-    fix_out(t, r, ex + 2, 1.0);
+    fix_out(t, r, ex + SH, 1.0);
     ax = nan_if(bad, r[0].x);
     ay = nan_if(bad, r[0].y);
   }
