@@ -343,6 +343,11 @@ __global__ void __launch_bounds__(ICOL_TX * P::TT, MB)
       x[e] = make_double2(0.0, 0.0);
       if (ok && row >= 0 && row < N) x[e] = src[(size_t)row * J.wc_in];
     }
+    if (DIR == DIR_INV && !MULTI && q == 0) {  // row 0 has no part in i ky: it must not set the scale
+      const int code = J.coef[0][0];
+      if ((code == CC_IKY || code == CC_MIKY) && max(fix_mag(x[0].x), fix_mag(x[0].y)) < 0x7ff00000u)
+        x[0] = make_double2(0.0, 0.0);
+    }
     __syncthreads();  // slots are zero
     ex = col_fix<TX, cnt>(x, v, slots, b, fwd ? fix_in(P::R1) : 60, bad);
   }

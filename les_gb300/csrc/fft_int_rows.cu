@@ -254,7 +254,12 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
     }
     cfix g[2 * KP + 1];
     if (J.deriv[f]) {  // i kx X, kx = 0 at k = 0 and k = M; the unit of kx is a factor of the output
-      if (q == 0) x[1] = make_double2(0.0, 0.0);
+      if (q == 0) {
+        x[1] = make_double2(0.0, 0.0);
+        // a mean adds nothing, so it must not set the scale either (p at 10^6 times
+        // its fluctuations: 20 bits); not-a-number and infinity stay
+        if (fix_mag(x[0].x) < 0x7ff00000u) x[0].x = 0.0;
+      }
       ex = row_fix_ik<TT, 2 * KP + 1>(x, g, bad, [&](int i) {
         const int k = q + TT * (i / 2);
         return (unsigned)(i == 2 * KP ? M / 2 : (i & 1 ? M - k : k));

@@ -179,3 +179,27 @@ def test_alternating_rows(ctx_of, nx, ny, amp):
     for got, k, s in ((a, 1, 1), (dx, 1j * kx, kmax), (dy, 1j * ky, kmax), (dx2, 1j * kx, kmax), (dy2, 1j * ky, kmax)):
         want = np.fft.irfft2(k * h, s=(ny, nx))
         assert np.linalg.norm((got[:, :, :nx] - want).astype(np.float64).ravel()) < 8 * EPS * s * norm
+
+
+@pytest.mark.parametrize("nx,ny", [(48, 64), (64, 48), (96, 72), (144, 128), (256, 36), (384, 16)])
+def test_pressure_gradient_of_a_large_mean(ctx_of, nx, ny):
+    """A uniform divtz at the lower wall moves the plane mean of p and nothing else: every other mode, and so the
+    gradient, keeps its bits, whatever the mean's size."""
+    c = ctx_of(nx, ny)
+    shape = lg.config.field_shape(c.cfg, "u")
+    g = np.random.default_rng(nx * ny)
+    for nm in ("u", "v", "w"):
+        f = np.zeros(shape)
+        f[:, :, :nx] = 0.1 * g.standard_normal((shape[0], ny, nx))
+        c.set(nm, f)
+    got = {}
+    for mean in (0.0, 2.0 ** 40):
+        d = np.zeros(shape)
+        d[0, :, :nx] = mean
+        c.set("divtz", d)
+        p, x, y = np.zeros(lg.config.field_shape(c.cfg, "p")), np.zeros(shape), np.zeros(shape)
+        c.call("press_stag_array", p, x, y)
+        got[mean] = (p[1:c.cfg.nz, :, :nx], x[:-1, :, :nx], y[:-1, :, :nx])
+    assert np.min(np.abs(got[2.0 ** 40][0])) > 2.0 ** 30 and np.max(np.abs(got[0.0][0])) < 2.0 ** 20
+    for a, b in zip(got[0.0][1:], got[2.0 ** 40][1:]):
+        assert np.any(a != 0.0) and np.array_equal(a, b)
