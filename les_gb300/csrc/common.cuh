@@ -3,7 +3,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cstdio>
-#include <utility>
+#include <type_traits>
 
 #define LES_PI 3.1415926535897932384626433   /* param.f90:51 */
 #define LES_BOGUS (-1234567890.0)              /* param.f90:50 */
@@ -209,7 +209,8 @@ template <class... P> struct PdlCall {
   dim3 grid, block;
   size_t smem;
   cudaStream_t stream;
-  template <class... A> void operator()(A&&... args) const {
+  // the kernel's own parameter types: arguments convert as in a call, never by a cast
+  void operator()(P... args) const {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -220,9 +221,13 @@ template <class... P> struct PdlCall {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    (void)cudaLaunchKernelEx(&cfg, kernel, P(std::forward<A>(args))...);
+    (void)cudaLaunchKernelEx(&cfg, kernel, args...);  // a failure stays for cudaGetLastError, as with <<<>>>
   }
 };
+static_assert(std::is_invocable<PdlCall<const double*, int>, double*, int>::value &&
+                  !std::is_invocable<PdlCall<double*, int>, float*, int>::value &&
+                  !std::is_invocable<PdlCall<double*, int>, const double*, int>::value,
+              "a launch takes its kernel's argument types");
 template <class... P>
 PdlCall<P...> pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem = 0, cudaStream_t stream = 0) {
   return PdlCall<P...>{kernel, grid, block, smem, stream};
