@@ -258,13 +258,13 @@ __device__ __forceinline__ i64 fix_of(double x, int c) {
   return ((i64)m ^ sg) - sg;
 }
 // x k 2^s for an integer k < 2^8 (the product is exact before the
-// truncation); e1 = 1077 - s, the result below 2^56
+// truncation); e1 = 1078 - s, the result below 2^57
 __device__ __forceinline__ i64 fix_times(double x, unsigned k, int e1) {
   const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
   const int d = min(e1 - (int)((hi >> 20) & 0x7ffu), 63);
   unsigned long long m = (unsigned long long)mad_wu(lo, k, 0) +
                          ((unsigned long long)(((hi & 0xfffffu) | 0x100000u) * k) << 32);
-  m = (m << 2) >> d;
+  m = (m << 3) >> d;
   const i64 sg = (i64)((int)hi >> 31);
   return ((i64)m ^ sg) - sg;
 }

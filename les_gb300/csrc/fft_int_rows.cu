@@ -56,7 +56,7 @@ __device__ __forceinline__ int row_fix(double2 (&x)[CNT], cfix (&v)[CNT], int bi
   return -s - pre;
 }
 
-// the same for i k x with the integers k(i) of the row's elements, below 2^56
+// the same for i k x with the integers k(i) of the row's elements, below 2^57
 template <int TT, int CNT, class KF>
 __device__ __forceinline__ int row_fix_ik(double2 (&x)[CNT], cfix (&v)[CNT], bool& bad, KF&& kof) {
   auto top = [&](int i) {  // exponent field bound of k x (x = 0: 0)
@@ -90,7 +90,7 @@ __device__ __forceinline__ int row_fix_ik(double2 (&x)[CNT], cfix (&v)[CNT], boo
     v[i].x = -fix_times(x[i].y, k, e1);
     v[i].y = fix_times(x[i].x, k, e1);
   }
-  return e1 - 1077 - pre;
+  return e1 - 1078 - pre;
 }
 
 template <int N1, int N2, int TT> struct RowShape {
