@@ -52,16 +52,6 @@ struct Grid {
                  // big truncated one (ny2*(nx/2))
 };
 
-// Grids on which results that cancel down to rounding level are held to the
-// reference's own roundings (the routine press_stag_array on an already
-// projected velocity, model 2's plane-sum ratio, and model 3, whose quintic
-// amplifies rounding 10^7-fold): there the FP64 transform kernels run, which
-// round as the reference's transforms do.  The integer-pipe transforms are
-// closer to the exact result (32^3 pressure gradient: 1.3e-12 of it against
-// the reference's and the FP64 kernels' 3.1e-11; rmsdiv after the projection
-// 0.39 of theirs) and run everywhere else.
-inline bool ref_rounding_grid(const Grid& g) { return g.nx <= 32 && g.ny <= 32; }
-
 }  // namespace les
 
 struct les_ctx {
@@ -147,10 +137,16 @@ struct les_ctx {
 };
 
 namespace les {
-// for the length of an op: FP64 transform kernels on ref_rounding_grid grids
+// For the length of an op: the FP64 transform kernels, which round as the
+// reference's transforms do, in place of the closer and faster integer-pipe
+// ones.  For the routine entries whose result is a ratio of plane sums that
+// cancel (les_std_dynamic, les_scaledep_dynamic): Cs^2(z) of one call agrees with
+// the reference's to 1e-12 with these (3e-13 to 8e-13, 32^2 to 96 x 64) and to
+// 2e-11 with the others.  In a step of model 2 the sums cancel less and both
+// agree alike (2e-12 and 2e-12), so the step keeps the integer-pipe ones.
 struct RefRounding {
   les_ctx* c;
-  explicit RefRounding(les_ctx* c_) : c(c_) { c->fp64_kernels = ref_rounding_grid(c->g); }
+  explicit RefRounding(les_ctx* c_, bool on = true) : c(c_) { c->fp64_kernels = on; }
   ~RefRounding() { c->fp64_kernels = false; }
   RefRounding(const RefRounding&) = delete;
   RefRounding& operator=(const RefRounding&) = delete;

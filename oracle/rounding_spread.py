@@ -20,8 +20,12 @@ each field is printed.  Two cases:
            (every 10 steps): the first level's explicit SGS diffusion number
            Nu_t dt / dz^2 is above the AB2 stability limit, so from about
            step 55 rounding differences at level 1 grow until they saturate.
+  model<M>-<nx>x<ny>
+           32 levels, theta, striped surface, jt_total0 = 500, model M, 10
+           steps on another horizontal grid; model 7 with theta perturbed on
+           every level.
 
-  python -m oracle.rounding_spread model3|humid0|humid500|model7|c2
+  python -m oracle.rounding_spread model3|humid0|humid500|model7|c2|model5-64x96
 """
 import json
 import os
@@ -63,6 +67,11 @@ def run_case(case, lib_path, out_path):
     elif case == "model7":
         cfg = lc.make_config(32, s_flag=1, q_flag=1, jt_total0=500, model=7, rmsdiv_every=1)
         seed, blocks, every = 41, 1, 10
+    elif "-" in case:
+        model, grid = case[5:].split("-")
+        nx, ny = (int(n) for n in grid.split("x"))
+        cfg = lc.make_config(nx, ny, 32, s_flag=1, jt_total0=500, model=int(model), rmsdiv_every=1)
+        seed, blocks, every = 11, 1, 10
     else:
         cfg = lc.make_config(128, s_flag=1, rmsdiv_every=10)
         seed, blocks, every = 21, 20, 10
@@ -70,7 +79,7 @@ def run_case(case, lib_path, out_path):
     o = oo.Oracle(cfg, surf)
     if getattr(cfg, "q_flag", 0):
         o.set("wq_s", lc.moisture_flux(cfg))
-    levels = {"theta_levels": cfg.nz} if case == "model7" else {}
+    levels = {"theta_levels": cfg.nz} if cfg.model == 7 else {}
     for k, v in lc.initial_state(cfg, surf, seed=seed, **levels).items():
         o.set(k, v)
     n = cfg.nx
