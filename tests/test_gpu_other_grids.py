@@ -15,8 +15,18 @@ TOL = 1e-12
 FIELDS = ("u", "v", "w", "theta")
 # (model, nx, ny): spread of u, v, w, theta, Cs_opt2, rmsdiv
 SPREAD = {
+    (2, 48, 48): (9.2e-16, 2.9e-14, 7.3e-14, 5.7e-16, 1.6e-12, 6.6e-3),
+    (2, 64, 96): (8.9e-16, 4.1e-14, 7.6e-14, 6.1e-16, 1.9e-12, 6.2e-3),
+    (2, 96, 64): (8.2e-16, 3.6e-14, 8.5e-14, 5.5e-16, 8.9e-12, 1.1e-2),
     (3, 48, 48): (1.36e-9, 1.28e-7, 7.9e-8, 5.5e-16, 2.5e-2, 1.5e-2),
     (3, 64, 96): (7.8e-10, 7.8e-8, 4.5e-8, 6.3e-16, 1.2e-3, 2.1e-3),
+    (4, 48, 48): (8.8e-16, 3.0e-14, 7.4e-14, 5.6e-16, 3.7e-11, 1.1e-2),
+    (4, 64, 96): (9.4e-16, 4.2e-14, 7.8e-14, 5.9e-16, 2.8e-11, 1.1e-2),
+    (5, 48, 48): (4.9e-15, 5.7e-13, 4.4e-13, 5.2e-16, 9.7e-11, 3.7e-3),
+    (5, 64, 96): (6.3e-15, 8.7e-13, 7.2e-13, 2.0e-15, 3.8e-10, 1.2e-4),
+    (5, 96, 64): (6.6e-15, 9.1e-13, 8.8e-13, 5.5e-16, 9.3e-10, 3.7e-3),
+    (7, 48, 48): (3.3e-15, 2.5e-12, 1.1e-12, 1.6e-14, 3.4e-10, 3.6e-3),
+    (7, 96, 64): (3.6e-15, 1.5e-12, 1.0e-12, 1.4e-14, 3.6e-10, 4.6e-3),
 }
 
 
@@ -70,4 +80,88 @@ def test_std_dynamic_routine(gpu_lib, oracle_lib, nx, ny):
     o.call("std_dynamic", co, *S)
     assert np.all(co >= 0) and np.any(co > 0)
     assert rel(cg, co) < TOL
+    g.close()
+
+
+LAG_STATE = ("u", "v", "w", "F_LM", "F_MM", "F_QN", "F_NN", "u_lag", "v_lag", "w_lag", "Beta", "Cs_opt2")
+S_NAMES = ("S11", "S12", "S13", "S22", "S23", "S33")
+
+
+@pytest.mark.parametrize("nx,ny", [(48, 72), (64, 96), (96, 64)])
+def test_lagrange_sdep_routine(gpu_lib, oracle_lib, nx, ny):
+    """One Lagrangian update from the same state, tolerances of the 32 x 32 case."""
+    cfg = lg.make_config(nx, ny, 12, s_flag=1, model=5, rmsdiv_every=0)
+    g, o = pair(cfg, lg.striped_surface(cfg), seed=17)
+    g.step(9)
+    assert o.step(9) == 0
+    for nm in LAG_STATE + S_NAMES:
+        o.set(nm, g.get(nm))
+    g.call("lagrange_sdep", *[g.get(nm) for nm in S_NAMES])
+    o.call("lagrange_sdep")
+    lev = slice(0, cfg.nz - 1)
+    for nm in ("F_LM", "F_MM", "F_QN", "F_NN", "Beta", "Cs_opt2"):
+        e = rel(g.get(nm)[lev, :, :nx], o.get(nm)[lev, :, :nx])
+        assert e < (1e-7 if nm == "Cs_opt2" else TOL), (nm, e)
+    g.close()
+
+
+def exact_press(cfg, u, v, w, divtz):
+    """press_stag_array.f90 in extended precision: p on levels 0..nz-1, dp/dx and dp/dy on 1..nz-1."""
+    L = np.longdouble
+    nx, ny, nz = cfg.nx, cfg.ny, cfg.nz
+    dz = L(cfg.lz_over_zi) / (nz - 1)
+    kx = np.arange(nx // 2 + 1).astype(L)[None, :].repeat(ny, 0) * (2 * L(np.pi) / L(cfg.l_x))
+    ky = (((np.arange(ny) + ny // 2) % ny) - ny // 2).astype(L)[:, None].repeat(nx // 2 + 1, 1) * (2 * L(np.pi) / L(cfg.l_y))
+    keep = np.ones((ny, nx // 2 + 1))
+    keep[ny // 2] = 0
+    keep[:, -1] = 0
+    kx, ky = kx * keep, ky * keep
+    hx, hy, hz, d = (np.fft.rfft2(a[:, :, :nx].astype(L)) / (nx * ny) * keep for a in (u, v, w, divtz))
+    hx, hy, hz = (h / (L(1.5) * L(cfg.dt)) for h in (hx, hy, hz))
+    hz[nz - 1] = 0
+    r = np.empty((nz + 1, ny, nx // 2 + 1), dtype=np.clongdouble)
+    r[0], r[nz] = -dz * d[0], -dz * d[nz - 1]
+    r[1:nz] = 1j * (kx * hx[:-1] + ky * hy[:-1]) + (hz[1:] - hz[:-1]) / dz
+    k2 = kx * kx + ky * ky
+    k2[k2 == 0] = 1
+    off, diag = 1 / (dz * dz), -(k2 + 2 / (dz * dz))
+    gam, p = [None] * (nz + 1), np.empty_like(r)
+    bet = -np.ones_like(k2)
+    p[0] = r[0] / bet
+    for j in range(1, nz + 1):
+        a, b, above = (off, diag, off if j > 1 else L(1)) if j < nz else (L(-1), L(1), off)
+        gam[j] = above / bet
+        bet = b - a * gam[j]
+        p[j] = (r[j] - a * p[j - 1]) / bet
+    for j in range(nz - 1, -1, -1):
+        p[j] -= gam[j + 1] * p[j + 1]
+    p *= keep
+    p[0, 0, 0] = 0
+    p[1, 0, 0] = -dz * d[0, 0, 0]
+    for j in range(2, nz + 1):
+        p[j, 0, 0] = p[j - 1, 0, 0] + hz[j - 1, 0, 0] * dz
+    back = lambda h: np.fft.irfft2(h, s=(ny, nx)) * (nx * ny)
+    return back(p[:nz]), back(1j * kx * p[1:nz]), back(1j * ky * p[1:nz])
+
+
+@pytest.mark.parametrize("nx,ny", [(32, 32), (48, 48), (64, 96), (96, 64), (128, 128)])
+def test_press_routine(gpu_lib, oracle_lib, nx, ny):
+    """The pressure of a projected state, where it cancels most: no further from the exact result than the oracle's
+    (whose own error is 1e-14 to 4e-11), on the small planes that keep its roundings up to 1e-12 of the result."""
+    cfg = lg.make_config(nx, ny, 24, s_flag=1, rmsdiv_every=0)
+    g, o = pair(cfg, lg.striped_surface(cfg), seed=17)
+    assert o.step(6) == 0
+    args = [o.get(nm) for nm in ("u", "v", "w", "divtz")]
+    for nm, a in zip(("u", "v", "w", "divtz"), args):
+        g.set(nm, a)
+    want = exact_press(cfg, *args)
+    shp = lg.field_shape(cfg, "u")
+    err = []
+    for c in (g, o):
+        p, x, y = np.zeros(lg.field_shape(cfg, "p")), np.zeros(shp), np.zeros(shp)
+        c.call("press_stag_array", p, x, y)
+        got = (p[:cfg.nz, :, :nx], x[:cfg.nz - 1, :, :nx], y[:cfg.nz - 1, :, :nx])
+        err.append([float(rel(a.astype(np.longdouble), b)) for a, b in zip(got, want)])
+    for eg, eo in zip(*err):
+        assert eg < (eo if max(nx, ny) > 32 else eo + TOL), err
     g.close()
