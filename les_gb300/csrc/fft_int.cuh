@@ -93,6 +93,9 @@ __device__ __forceinline__ cfix ftwc(cfix a, int4 w) { return fcmul(a, w.x, w.y,
 
 __device__ __forceinline__ cfix fadd(cfix a, cfix b) { a.x += b.x; a.y += b.y; return a; }
 __device__ __forceinline__ cfix fsub(cfix a, cfix b) { a.x -= b.x; a.y -= b.y; return a; }
+// a / 2, halves to the even neighbour: rounded up, they would give all rows of a
+// plane the same quarter unit, which its ky = 0 modes collect
+__device__ __forceinline__ i64 fhalf(i64 a) { return (a + (i64)(((unsigned)a >> 1) & 1u)) >> 1; }
 
 // ---- constants: cos(2 pi k / 144) in 62 fractional bits -----------------------
 __host__ __device__ constexpr i64 fix_cos144(int k) {
@@ -189,8 +192,8 @@ template <int N, int SIGN> __device__ __forceinline__ void fdft(cfix* v) {
     const cfix a = v[0], s = fadd(v[1], v[2]), d = fsub(v[1], v[2]);
     constexpr i64 S3 = FixSin<48>::v;  // sin(2 pi / 3)
     cfix m, r;
-    m.x = a.x - ((s.x + 1) >> 1);
-    m.y = a.y - ((s.y + 1) >> 1);
+    m.x = a.x - fhalf(s.x);
+    m.y = a.y - fhalf(s.y);
     const i64 rx = fmul(d.x, fix_hi(S3), fix_lo(S3)), ry = fmul(d.y, fix_hi(S3), fix_lo(S3));
     r.x = SIGN < 0 ? ry : -ry;   // SIGN i sin(..) d
     r.y = SIGN < 0 ? -rx : rx;

@@ -149,7 +149,10 @@ __global__ void __launch_bounds__(128, MB) k_ir2c(RowJob J, const int4* __restri
   }
   // one bit spare for the sums of the post-processing
   const int s = fix_down(row_max<TT>(top), fix_in(N1) - 1);
-  const i64 rnd = fix_rnd(s);
+  // halves up in even rows and down in odd ones: the same in all rows they would
+  // add up in the ky = 0 modes (rows of a mean wind and small fluctuations:
+  // nearly all of those modes' error)
+  const i64 rnd = fix_rnd(s) - (s > 0 ? y & 1 : 0);
   ex += s;
   __syncwarp();
   cfix w[J2 * N1];
