@@ -111,7 +111,7 @@ template <class P, int TX> __device__ __forceinline__ int col_at(int k2, int p, 
 // step: headroom for 64 points at once would cost a column that one row
 // dominates three bits.  slot: two rows of TX words.
 template <class P, int TX, int NV>
-__device__ __forceinline__ void col_fwd(cfix (&v)[NV], cfix* S, unsigned* slot, const int4* __restrict__ tw, int q, int b,
+__device__ __forceinline__ void col_fwd(cfix (&v)[NV], cfix* S, unsigned* slot, const int4* __restrict__ tw, int q, int b, bool coin,
                                         int& ex) {
   constexpr int R1 = P::R1, R2 = P::R2, R3 = P::R3, TT = P::TT;
   unsigned top = 0;
@@ -130,9 +130,8 @@ __device__ __forceinline__ void col_fwd(cfix (&v)[NV], cfix* S, unsigned* slot, 
     }
   }
   if constexpr (R3 > 1) {
-    const int s1 = fix_down(col_max<TX>(top, slot, b), fix_in(R2));
-    const i64 rnd1 = fix_rnd(s1);
-    ex += s1;
+    const FixShift s1(fix_down(col_max<TX>(top, slot, b), fix_in(R2)), coin);
+    ex += s1.s;
     slot += TX;
     top = 0;
 #pragma unroll
@@ -143,8 +142,8 @@ __device__ __forceinline__ void col_fwd(cfix (&v)[NV], cfix* S, unsigned* slot, 
 #pragma unroll
         for (int i = 0; i < R2; ++i) {
           const cfix a = S[col_at<P, TX>(k2, m1 + R3 * i, b)];
-          w[i].x = fix_shr(a.x, s1, rnd1);
-          w[i].y = fix_shr(a.y, s1, rnd1);
+          w[i].x = s1(a.x);
+          w[i].y = s1(a.y);
         }
         fdft<R2, -1>(w);
 #pragma unroll
@@ -156,9 +155,8 @@ __device__ __forceinline__ void col_fwd(cfix (&v)[NV], cfix* S, unsigned* slot, 
       }
     }
   }
-  const int s = fix_down(col_max<TX>(top, slot, b), fix_in(P::SR));
-  const i64 rnd = fix_rnd(s);
-  ex += s;
+  const FixShift s(fix_down(col_max<TX>(top, slot, b), fix_in(P::SR)), coin);
+  ex += s.s;
 #pragma unroll
   for (int j = 0; j < P::JS; ++j) {
     const int t = q + TT * j;
@@ -167,8 +165,8 @@ __device__ __forceinline__ void col_fwd(cfix (&v)[NV], cfix* S, unsigned* slot, 
 #pragma unroll
       for (int i = 0; i < P::SR; ++i) {
         const cfix a = S[col_at<P, TX>(k2, R3 * l2 + i, b)];
-        v[j * P::SR + i].x = fix_shr(a.x, s, rnd);
-        v[j * P::SR + i].y = fix_shr(a.y, s, rnd);
+        v[j * P::SR + i].x = s(a.x);
+        v[j * P::SR + i].y = s(a.y);
       }
       fdft<P::SR, -1>(v + j * P::SR);
     }
@@ -177,7 +175,7 @@ __device__ __forceinline__ void col_fwd(cfix (&v)[NV], cfix* S, unsigned* slot, 
 // inverse: from v[j SR + i] = X[(q + TT j) + SJ i] with sums of moduli that stay
 // below 2^60 up to the last step (col_weigh), to v[j R1 + i] = x[(q + TT j) + N1 i]
 template <class P, int TX, int NV>
-__device__ __forceinline__ void col_inv(cfix (&v)[NV], cfix* S, unsigned* slot, const int4* __restrict__ tw, int q, int b,
+__device__ __forceinline__ void col_inv(cfix (&v)[NV], cfix* S, unsigned* slot, const int4* __restrict__ tw, int q, int b, bool coin,
                                         int& ex) {
   constexpr int R1 = P::R1, R2 = P::R2, R3 = P::R3, TT = P::TT;
   unsigned top = 0;
@@ -215,9 +213,8 @@ __device__ __forceinline__ void col_inv(cfix (&v)[NV], cfix* S, unsigned* slot, 
       }
     }
   }
-  const int s = fix_down(col_max<TX>(top, slot, b), fix_in(R1));
-  const i64 rnd = fix_rnd(s);
-  ex += s;
+  const FixShift s(fix_down(col_max<TX>(top, slot, b), fix_in(R1)), coin);
+  ex += s.s;
 #pragma unroll
   for (int j = 0; j < P::JA; ++j) {
     const int n1 = q + TT * j;
@@ -225,20 +222,21 @@ __device__ __forceinline__ void col_inv(cfix (&v)[NV], cfix* S, unsigned* slot, 
 #pragma unroll
       for (int i = 0; i < R1; ++i) {
         const cfix a = S[col_at<P, TX>(i, n1, b)];
-        v[j * R1 + i].x = fix_shr(a.x, s, rnd);
-        v[j * R1 + i].y = fix_shr(a.y, s, rnd);
+        v[j * R1 + i].x = s(a.x);
+        v[j * R1 + i].y = s(a.y);
       }
       fdft<R1, 1>(v + j * R1);
     }
   }
 }
+// (coin: the direction of halves, see FixShift)
 // w(k) v with integer weights, 0 or 1, or (sgn) |ky| as an integer, negative
 // wavenumbers (i >= SR/2) changing sign, scaled so that the sums of moduli of
 // col_inv's steps before its own scaling stay below 2^60: a job's sum (up to 24
 // values, weights up to 192: below 2^31 units of 2^44), times R2 where a second
 // step follows.  The products are exact 96-bit integers before the shift.
 template <class P, int TX, int NV>
-__device__ __forceinline__ void col_weigh(cfix (&v)[NV], const unsigned (&w)[P::SE], bool sgn, unsigned* slot, int b,
+__device__ __forceinline__ void col_weigh(cfix (&v)[NV], const unsigned (&w)[P::SE], bool sgn, unsigned* slot, int b, bool coin,
                                           int& ex) {
   unsigned sum = 0;
 #pragma unroll
@@ -250,12 +248,14 @@ __device__ __forceinline__ void col_weigh(cfix (&v)[NV], const unsigned (&w)[P::
     sum = max(sum, t);
   }
   const int s = fix_down_sum(col_max<TX>(sum, slot, b), 44 + (P::R3 > 1 ? clog2(P::R2) : 0));
-  const i64 rnd = fix_rnd(s);
+  const FixShift f[2] = {FixShift(s, coin), FixShift(s, !coin)};  // of the elements: 0 1 1 0 1 0 0 1 ...
   const i64 flip = sgn ? -1 : 0;
   ex += s;
 #pragma unroll
   for (int e = 0; e < P::SE; ++e) {
-    const i64 lx = mad_wu((unsigned)v[e].x, w[e], rnd), ly = mad_wu((unsigned)v[e].y, w[e], rnd);
+    const int c = (e ^ (e >> 1) ^ (e >> 2) ^ (e >> 3)) & 1;
+    const i64 lx = mad_wu((unsigned)v[e].x, w[e], (i64)(unsigned long long)f[c].rnd);
+    const i64 ly = mad_wu((unsigned)v[e].y, w[e], (i64)(unsigned long long)f[1 - c].rnd);
     const i64 hx = mad_w((int)(v[e].x >> 32), (int)w[e], (i64)((unsigned long long)lx >> 32));
     const i64 hy = mad_w((int)(v[e].y >> 32), (int)w[e], (i64)((unsigned long long)ly >> 32));
     // (h 2^32 + low word) >> s, s < 32
@@ -331,6 +331,7 @@ __global__ void __launch_bounds__(ICOL_TX * P::TT, MB)
   const double2* src = reinterpret_cast<const double2*>(J.in[0]) + in0;
   constexpr bool fwd = (DIR & DIR_FWD) != 0;
   const bool last = jx == J.lh - 1;  // kx = nx/2: removed by KILL and by the derivatives
+  const bool coin = fix_coin((unsigned)(jx * P::TT + q));
   cfix v[P::E];
   int ex;
   bool bad = false;
@@ -357,7 +358,7 @@ __global__ void __launch_bounds__(ICOL_TX * P::TT, MB)
     constexpr i64 SR = 1ll << (SH - 1);
     i64 sx = 0, sy = 0;
 #pragma unroll
-    for (int e = 0; e < P::PE; ++e) { sx += fix_shr(v[e].x, SH, SR); sy += fix_shr(v[e].y, SH, SR); }
+    for (int e = 0; e < P::PE; ++e) { sx += (v[e].x + SR) >> SH; sy += (v[e].y + SR) >> SH; }
     if (q & 1) { sx = -sx; sy = -sy; }
     col_sum<TX>(sx, sy, sums, b);
     if (q & 1) { sx = -sx; sy = -sy; }
@@ -391,7 +392,7 @@ __global__ void __launch_bounds__(ICOL_TX * P::TT, MB)
     direct();
     return;
   }
-  if constexpr (fwd) col_fwd<P, TX>(v, S, slots + 2 * TX, tw, q, b, ex);
+  if constexpr (fwd) col_fwd<P, TX>(v, S, slots + 2 * TX, tw, q, b, coin, ex);
   if (DIR != DIR_INV && nspec && ok) {
     for (int o = 0; o < J.nout; ++o) {
       if ((J.inv_mask >> o) & 1u) continue;
@@ -434,8 +435,8 @@ __global__ void __launch_bounds__(ICOL_TX * P::TT, MB)
         w[e] = k >= N || __ldg(&T[(size_t)J.lh * k + jx]) == 0.f ? 0u : 1u;
       }
     }
-    col_weigh<P, TX>(v, w, iky, so, b, ex);
-    col_inv<P, TX>(v, S, so + TX, tw, q, b, ex);
+    col_weigh<P, TX>(v, w, iky, so, b, coin, ex);
+    col_inv<P, TX>(v, S, so + TX, tw, q, b, coin, ex);
     if (ok) {
       double2* dst = reinterpret_cast<double2*>(J.out[o]) + out0;
       double2 r[P::PE];
@@ -513,14 +514,15 @@ __global__ void __launch_bounds__(ICOL_TX * P::TT, MB) k_icol_div(ColJob J, cons
     __syncthreads();  // slots are zero, partial sums are written
     ex = col_fix<TX, P::PE>(x, v, slots, b, fix_in(P::R1), bad);
   }
-  col_fwd<P, TX>(v, S, slots + 2 * TX, tw, q, b, ex);
+  const bool coin = fix_coin((unsigned)(jx * P::TT + q));
+  col_fwd<P, TX>(v, S, slots + 2 * TX, tw, q, b, coin, ex);
   const bool last = jx == J.lh - 1;
   {
     unsigned w[P::SE];
     ky_weights<P>(w, q, last);
-    col_weigh<P, TX>(v, w, true, slots + 4 * TX, b, ex);
+    col_weigh<P, TX>(v, w, true, slots + 4 * TX, b, coin, ex);
   }
-  col_inv<P, TX>(v, S, slots + 5 * TX, tw, q, b, ex);
+  col_inv<P, TX>(v, S, slots + 5 * TX, tw, q, b, coin, ex);
   if (!ok) return;
   double cx = 0.0, cy = 0.0;
 #pragma unroll
@@ -569,6 +571,7 @@ __global__ void __launch_bounds__(ICOL_TX * cmax(PA::TT, PB::TT), MB)
     if (PAD) return k < NS / 2 ? k : (k > NL - NS / 2 ? k - (NL - NS) : -1);
     return k < NS / 2 ? k : (k == NS / 2 ? -1 : k + (NL - NS));
   };
+  const bool coin = fix_coin((unsigned)(jx * cmax(PA::TT, PB::TT) + q0));
   cfix v[E];
   int ex;
   bool bad = false;
@@ -583,7 +586,7 @@ __global__ void __launch_bounds__(ICOL_TX * cmax(PA::TT, PB::TT), MB)
     }
     __syncthreads();  // slots are zero
     ex = col_fix<TX, PA::PE>(x, v, slots, b, fix_in(PA::R1), bad);
-    col_fwd<PA, TX>(v, S, slots + 2 * TX, twa, qa, b, ex);
+    col_fwd<PA, TX>(v, S, slots + 2 * TX, twa, qa, b, coin, ex);
     __syncthreads();  // the exchange buffer is read
 #pragma unroll
     for (int e = 0; e < PA::SE; ++e) {
@@ -610,9 +613,9 @@ __global__ void __launch_bounds__(ICOL_TX * cmax(PA::TT, PB::TT), MB)
     unsigned w[PB::SE];
 #pragma unroll
     for (int e = 0; e < PB::SE; ++e) w[e] = 1u;
-    col_weigh<PB, TX>(v, w, false, slots + 4 * TX, b, ex);
+    col_weigh<PB, TX>(v, w, false, slots + 4 * TX, b, coin, ex);
   }
-  col_inv<PB, TX>(v, S, slots + 5 * TX, twb, qb, b, ex);
+  col_inv<PB, TX>(v, S, slots + 5 * TX, twb, qb, b, coin, ex);
   if (ok) {
     double2 r[PB::PE];
     fix_out(v, r, ex, nan_if(bad, 1.0));

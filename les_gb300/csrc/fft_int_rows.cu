@@ -148,12 +148,8 @@ __global__ void __launch_bounds__(128, MB) k_ir2c(RowJob J, const int4* __restri
     }
   }
   // one bit spare for the sums of the post-processing
-  const int s = fix_down(row_max<TT>(top), fix_in(N1) - 1);
-  // halves up in even rows and down in odd ones: the same in all rows they would
-  // add up in the ky = 0 modes (rows of a mean wind and small fluctuations:
-  // nearly all of those modes' error)
-  const i64 rnd = fix_rnd(s) - (s > 0 ? y & 1 : 0);
-  ex += s;
+  const FixShift s(fix_down(row_max<TT>(top), fix_in(N1) - 1), fix_coin((unsigned)y));
+  ex += s.s;
   __syncwarp();
   cfix w[J2 * N1];
 #pragma unroll
@@ -163,8 +159,8 @@ __global__ void __launch_bounds__(128, MB) k_ir2c(RowJob J, const int4* __restri
 #pragma unroll
       for (int i = 0; i < N1; ++i) {
         const cfix a = S[k2 * LD1 + i];
-        w[j * N1 + i].x = fix_shr(a.x, s, rnd);
-        w[j * N1 + i].y = fix_shr(a.y, s, rnd);
+        w[j * N1 + i].x = s(a.x);
+        w[j * N1 + i].y = s(a.y);
       }
       fdft<N1, -1>(w + j * N1);  // over n1: Z[k2 + N2 i]
     }
@@ -304,9 +300,8 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
     }
   }
   // at most 25 values a lane: below 2^31 units of 2^36; the row's in units of 2^40
-  const int s = fix_down_sum(row_sum<TT>((sum >> 4) + 1u), 40);
-  const i64 rnd = fix_rnd(s);
-  ex += s;
+  const FixShift s(fix_down_sum(row_sum<TT>((sum >> 4) + 1u), 40), fix_coin((unsigned)y));
+  ex += s.s;
   __syncwarp();
   // first step in place: a lane's transforms read and write their own slots,
   // so the loop needs no registers for the others (and half the code)
@@ -318,8 +313,8 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
 #pragma unroll
       for (int i = 0; i < N2; ++i) {
         const cfix a = S[i * LD1 + k1];
-        v[i].x = fix_shr(a.x, s, rnd);
-        v[i].y = fix_shr(a.y, s, rnd);
+        v[i].x = s(a.x);
+        v[i].y = s(a.y);
       }
       fdft<N2, 1>(v);  // over k2
 #pragma unroll

@@ -78,6 +78,28 @@ def test_plane_transforms(ctx_of, nx, ny, kind):
 
 
 @pytest.mark.parametrize("nx,ny", GRIDS)
+def test_roundings_do_not_meet(ctx_of, nx, ny):
+    """No point of a plane collects the others' roundings.  White noise: every error is a sum of many roundings, close
+    to normal, so that none of the up to 300,000 values lies beyond 6 of their deviations, 8 with the spread of the
+    scales from row to row; the values at zero, which all coherent errors reach, are among them."""
+    c = ctx_of(nx, ny)
+    for big in (0, 1):
+        mx, my = (3 * nx // 2, 3 * ny // 2) if big else (nx, ny)
+        f = planes("noise", 2, my, mx, 3 * nx + ny)
+        want = np.fft.rfft2(f.astype(np.longdouble))
+        a = np.zeros((2, my, mx + 2))
+        a[:, :, :mx] = f
+        c.call("fft_r2c", a, ints=(2, big))
+        h = a.view(np.complex128).astype(np.clongdouble)
+        err = np.abs(h - want).astype(np.float64)
+        assert err.max() < 8 * max(np.sqrt((err ** 2).mean()), EPS * np.sqrt((np.abs(want) ** 2).mean()))
+        back = np.fft.irfft2(h, s=(my, mx)) * (mx * my)
+        c.call("fft_c2r", a, ints=(2, big))
+        err = np.abs(a[:, :, :mx] - back).astype(np.float64)
+        assert err.max() < 8 * max(np.sqrt((err ** 2).mean()), EPS * float(np.sqrt((back ** 2).mean())))
+
+
+@pytest.mark.parametrize("nx,ny", GRIDS)
 def test_derivatives_and_filter(ctx_of, nx, ny):
     c = ctx_of(nx, ny)
     f = planes("wind", 2, ny, nx, 5 * nx + ny)
