@@ -99,6 +99,12 @@ template <int N1, int N2, int TT> struct RowShape {
   static constexpr int MS = N2 * LD1 > M + 1 ? N2 * LD1 : M + 1;
   static constexpr int NT = 128, RPB = NT / TT, KP = (M / 2 + TT - 1) / TT;
   static_assert(32 % TT == 0 && M % 2 == 0, "a row within one warp");
+  // Inverse pass, the scale taken twice.  Rows of 384: one sum of moduli for the
+  // whole row leaves a flat spectrum (a single point's) 52 bits, 2.2 x 2^-53 of error
+  // (the FP64 kernels 1.7); taken twice 0.3 to 0.8.  Shorter rows stay below the FP64 kernels with
+  // one (288 points 1.2 against 1.9) and are 2 % faster with it.
+  static constexpr bool MID = M > 144;
+  static_assert(!MID || TT == N1, "a lane's elements at k, and those at M - k, belong to one k1 each");
   static constexpr size_t smem = (size_t)RPB * MS * sizeof(cfix);
 };
 
@@ -233,7 +239,7 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
   const int nc = ok ? J.ncols : 0;
   int ex;
   bool bad = false;
-  unsigned sum = 0;
+  unsigned sum = 0, sum2 = 0;  // moduli of the elements at k and at M - k
   {
     double2 x[2 * KP + 1];  // X[k], X[M - k], and lane 0's X[M / 2]
 #pragma unroll
@@ -266,9 +272,9 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
     } else {
       ex = row_fix<TT, 2 * KP + 1>(x, g, 58, bad);
     }
-    auto put = [&](int k, cfix u) {  // element k = k1 + N1 k2 at k2 LD1 + k1
+    auto put = [&](int k, cfix u, unsigned& total) {  // element k = k1 + N1 k2 at k2 LD1 + k1
       S[(k / N1) * LD1 + k % N1] = u;
-      sum += fix_l1<4>(u);
+      total += fix_l1<4>(u);
     };
 #pragma unroll
     for (int i = 0; i < KP; ++i) {
@@ -285,10 +291,10 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
         }
         cfix u;  // A[k] = E + i D, A[M - k] = conj(E - i D)
         u.x = e.x - o.y; u.y = e.y + o.x;
-        put(k, u);
+        put(k, u, sum);
         if (!(i == 0 && k == 0)) {
           u.x = e.x + o.y; u.y = o.x - e.y;
-          put(M - k, u);
+          put(M - k, u, sum2);
         }
       }
     }
@@ -296,12 +302,17 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
       cfix u;
       u.x = g[2 * KP].x << 1;
       u.y = -(g[2 * KP].y << 1);
-      put(M / 2, u);
+      put(M / 2, u, sum);
     }
   }
-  // at most 25 values a lane: below 2^31 units of 2^36; the row's in units of 2^40
-  const FixShift s(fix_down_sum(row_sum<TT>((sum >> 4) + 1u), 40), fix_coin((unsigned)y));
+  // at most 25 values a lane: below 2^31 units of 2^36; the row's in units of 2^40.
+  // MID: lane q holds all of the first step's transform k1 = q, so the two largest
+  // halves bound each of them, and the scale is taken again before the second step.
+  const int s1 = R::MID ? fix_down_sum(row_max<TT>(sum) + row_max<TT>(sum2), 36)
+                        : fix_down_sum(row_sum<TT>(((sum + sum2) >> 4) + 1u), 40);
+  const FixShift s(s1, fix_coin((unsigned)y));
   ex += s.s;
+  unsigned top = 0;
   __syncwarp();
   // first step in place: a lane's transforms read and write their own slots,
   // so the loop needs no registers for the others (and half the code)
@@ -320,10 +331,13 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
 #pragma unroll
       for (int i = 0; i < N2; ++i) {
         if (i > 0) v[i] = ftwc(v[i], __ldg(&tw[k1 * i]));
+        if (R::MID) top = max(top, max(fix_top(v[i].x), fix_top(v[i].y)));
         S[i * LD1 + k1] = v[i];
       }
     }
   }
+  const FixShift s2(R::MID ? fix_down(row_max<TT>(top), fix_in(N1)) : 0, fix_coin(~(unsigned)y));
+  ex += s2.s;
   __syncwarp();
   if (!ok) return;
   const double factor = nan_if(bad, J.deriv[f] ? J.scale[f] * J.kunit : J.scale[f]);
@@ -336,7 +350,13 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
     if (N2 % TT == 0 || n2 < N2) {
       cfix w[N1];
 #pragma unroll
-      for (int i = 0; i < N1; ++i) w[i] = S[n2 * LD1 + i];
+      for (int i = 0; i < N1; ++i) {
+        w[i] = S[n2 * LD1 + i];
+        if (R::MID) {
+          w[i].x = s2(w[i].x);
+          w[i].y = s2(w[i].y);
+        }
+      }
       fdft<N1, 1>(w);  // over k1: z[n2 + N2 i]
       double2 o[N1];
       fix_out(w, o, ex, factor);
