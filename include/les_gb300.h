@@ -329,7 +329,8 @@ int les_fft_c2r(les_ctx* ctx, double* planes, int nplanes, int big);
  * integer-pipe float<->double conversions with the hardware conversions on n
  * generated values (random bit patterns, the float range, halfway cases);
  * *mismatches receives the number of results whose bits differ.  The split
- * into a float-float pair is compared too, and x^(-1/8) with its roots. */
+ * into a float-float pair and x / 2, -2 x by the exponent field are compared
+ * too, and x^(-1/8) with its roots. */
 int les_selftest_conversions(size_t n, unsigned long long seed, unsigned long long* mismatches);
 int les_profile_begin(les_ctx* ctx, int family, int max_launches);
 int les_profile_end(les_ctx* ctx, int* launches, double* ms, double* bytes);

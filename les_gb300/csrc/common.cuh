@@ -75,12 +75,14 @@ __device__ __forceinline__ double fmax32(double a, double b) {
 // x / 2 and -2 x through the exponent field: exact products with powers of
 // two need no operation of the FP64 pipe (about 1.7 per clock per SM, which
 // bounds the pointwise FP64 kernels).  Infinities and NaN pass; subnormals
-// are shifted (x / 2 drops the last unit of 2^-1074).
+// are shifted, x / 2 to the nearest with halves to the even one: the bits of the
+// products in every case.
 __device__ __forceinline__ double half_of(double x) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   const unsigned hi = (unsigned)(b >> 32), e = (hi >> 20) & 0x7ffu;
   if (e > 1u) return e == 0x7ffu ? x : __hiloint2double((int)(hi - (1u << 20)), (int)(unsigned)b);
-  return __longlong_as_double((long long)((b & 0x8000000000000000ull) | ((b << 1) >> 2)));
+  const unsigned long long m = b & 0x7fffffffffffffffull;
+  return __longlong_as_double((long long)((b & 0x8000000000000000ull) | ((m >> 1) + (m & (m >> 1) & 1ull))));
 }
 __device__ __forceinline__ double minus_twice(double x) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x) ^ 0x8000000000000000ull;

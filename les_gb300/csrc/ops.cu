@@ -46,6 +46,13 @@ __global__ void k_cvt_selftest(size_t n, unsigned long long seed, unsigned long 
       x = 0.5 * (lo + hi);
     }
     if (__float_as_uint(cvt_d2f(x)) != __float_as_uint((float)x) && !(x != x)) ++nb;
+    if (!(x != x) && (__double_as_longlong(half_of(x)) != __double_as_longlong(0.5 * x) ||
+                      __double_as_longlong(minus_twice(x)) != __double_as_longlong(-2.0 * x)))
+      ++nb;
+    const double tiny = __longlong_as_double((long long)(r & 0x803fffffffffffffull));  // subnormals and around
+    if (__double_as_longlong(half_of(tiny)) != __double_as_longlong(0.5 * tiny) ||
+        __double_as_longlong(minus_twice(tiny)) != __double_as_longlong(-2.0 * tiny))
+      ++nb;
     const double ax = fabs(x), want = 1.0 / sqrt(sqrt(sqrt(ax)));  // within 4 units of its last place
     if (ax > 0.0 && ax < 1e300 && !(fabs(pow_m18(ax) - want) <= 8.9e-16 * want)) ++nb;
     const dfloat h = split_d(x);
