@@ -803,7 +803,8 @@ static std::map<std::tuple<int, int, int, int>, std::tuple<int, int, int>> g_tun
 
 int les_autotune(les_ctx* c, int* tx64, int* tx32, int* rpc_scale) {
   if (!c) return LES_ERR_ARG;
-  const auto key = std::make_tuple(c->g.nx, c->g.ny, c->g.nz, c->cfg.precision);
+  const bool has64 = autotune_has64(c);
+  const auto key = std::make_tuple(c->g.nx, c->g.ny, c->g.nz, c->cfg.precision + (has64 ? 0 : 4));
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);
@@ -838,7 +839,7 @@ int les_autotune(les_ctx* c, int* tx64, int* tx32, int* rpc_scale) {
       int best[2][2] = {{4, 0}, {8, 0}};
       const int txs[2][3] = {{2, 4, 8}, {4, 8, 16}};
       for (int fp32 = 0; fp32 < 2; ++fp32) {
-        if (fp32 && c->cfg.precision != 1) continue;
+        if (fp32 ? c->cfg.precision != 1 : !has64) continue;
         float bt = 1e30f;
         for (int a = 0; a < 3; ++a)
           for (int sc = -1; sc <= 1; ++sc) {

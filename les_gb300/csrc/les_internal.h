@@ -221,4 +221,5 @@ int op_tsc(les_ctx* c, double* cflu, double* visc);  // Nu_t read in the context
 int op_ddz(les_ctx* c, double* dfdz, const double* f, int uv);
 int thomas_tables(les_ctx* c);
 void autotune_probe(les_ctx* c, int fp32);
+bool autotune_has64(const les_ctx* c);
 }  // namespace les

@@ -5173,6 +5173,14 @@ static void tune_probe(les_ctx* c) {
   double* bo[3] = {c->big + 3 * g.nfield_big, c->big + 4 * g.nfield_big, c->big + 5 * g.nfield_big};
   c2rT<T, double>(c, 3, nz, c->wsA, bo, (long)g.nplane_big, true, g.nx / 2);
 }
+// all transforms of the grid, 3/2 rows among them, on the integer pipe
+static bool int_grid(const les_ctx* c) {
+  const Grid& g = c->g;
+  return c->cy.c.uniti && int_rows_length(g.nx / 2) && int_rows_length(g.nx2 / 2) && int_cols_length(g.ny);
+}
+// whether the 8-byte-real knobs act on the step: not in the FP64 and float-float
+// forms on grids that the integer-pipe transforms cover, whose shapes are fixed
+bool autotune_has64(const les_ctx* c) { return c->cfg.precision == 1 || !int_grid(c); }
 // fp32: the FP32 transforms' knobs; else the 8-byte-real knobs, probed with
 // the kernels the form runs them with (FP64 in the FP64 form, float-float in
 // the mixed and float-float transform forms)
@@ -5187,10 +5195,6 @@ int step_mixed(les_ctx* c) { return stepT<1>(c); }
 // Precision 2: the FP64 step where the integer-pipe transforms cover the grid
 // (they are faster than float-float ones, 128^3 with theta 4.25 -> 2.9 ms a
 // step, and closer to the exact result), else float-float transforms.
-int step_ff(les_ctx* c) {
-  const Grid& g = c->g;
-  const bool covered = c->cy.c.uniti && int_rows_length(g.nx / 2) && int_rows_length(g.nx2 / 2) && int_cols_length(g.ny);
-  return covered ? stepT<0>(c) : stepT<2>(c);
-}
+int step_ff(les_ctx* c) { return int_grid(c) ? stepT<0>(c) : stepT<2>(c); }
 
 }  // namespace les
