@@ -239,3 +239,71 @@ def test_pressure_gradient_of_a_large_mean(ctx_of, nx, ny):
     assert np.min(np.abs(got[2.0 ** 40][0])) > 2.0 ** 30 and np.max(np.abs(got[0.0][0])) < 2.0 ** 20
     for a, b in zip(got[0.0][1:], got[2.0 ** 40][1:]):
         assert np.any(a != 0.0) and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("nx,ny", [(64, 32), (96, 48), (256, 256), (384, 16)])
+def test_range_ends_of_every_pass(ctx_of, nx, ny):
+    """Values near both ends of the FP64 range through the filter, the derivatives, the 3/2 round trip and a divergence:
+    every pass scales by powers of two, so the results are those at scale 1, times the scale."""
+    c = ctx_of(nx, ny)
+    nz = c.cfg.nz
+    g = np.random.default_rng(9)
+    f = g.standard_normal((nz, ny, nx))
+    t = g.standard_normal((nz, ny, nx))
+    mx, my = 3 * nx // 2, 3 * ny // 2
+
+    def run(scale):
+        pad = lambda a: np.concatenate([a * scale, np.zeros((nz, ny, 2))], axis=2)
+        a, b, z = pad(f), pad(t), np.zeros((nz, ny, nx + 2))
+        out = [a.copy()] + [np.zeros_like(a) for _ in range(6)]
+        c.call("filt_da", out[0], out[1], out[2], ints=(nz,))
+        c.call("ddxy", out[3], out[4], a, ints=(nz,))
+        c.call("divstress_uv", out[5], a, b, z)
+        big = np.zeros((nz, my, mx + 2))
+        c.call("dealias1", a, big, ints=(nz,))
+        c.call("dealias2", out[6], big, ints=(nz,))
+        # the top level of a divergence is a constant
+        return [q[:nz - 1, :, :nx].astype(np.longdouble) / np.longdouble(scale) for q in out] + \
+            [big[:nz - 1, :, :mx].astype(np.longdouble) / np.longdouble(scale)]
+
+    want = run(1.0)
+    for scale in (2.0 ** -1005, 2.0 ** -980, 2.0 ** -900, 2.0 ** 900, 2.0 ** 990):
+        for i, (a, b) in enumerate(zip(run(scale), want)):
+            # the spectra carry 1/(nx ny): at the smallest scales their last bits are subnormal units of 2^-1074
+            assert rel(a, b) < (8 * EPS if scale > 2.0 ** -1000 else 2.0 ** -46), (scale, i)
+
+
+@pytest.mark.parametrize("nx,ny", [(64, 32), (96, 48), (256, 256)])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_not_a_number_through_every_pass(ctx_of, nx, ny, bad):
+    """Not-a-number or infinity in one plane: none of that plane is finite, all other planes keep their bits."""
+    c = ctx_of(nx, ny)
+    nz = c.cfg.nz
+    g = np.random.default_rng(10)
+    f, t = np.zeros((nz, ny, nx + 2)), np.zeros((nz, ny, nx + 2))
+    f[:, :, :nx] = g.standard_normal((nz, ny, nx))
+    t[:, :, :nx] = g.standard_normal((nz, ny, nx))
+    mx, my = 3 * nx // 2, 3 * ny // 2
+
+    def run(a, b):
+        out = [a.copy()] + [np.zeros_like(a) for _ in range(6)]
+        c.call("filt_da", out[0], out[1], out[2], ints=(nz,))
+        c.call("ddxy", out[3], out[4], a, ints=(nz,))
+        c.call("divstress_uv", out[5], a, b, np.zeros_like(a))
+        big = np.zeros((nz, my, mx + 2))
+        c.call("dealias1", a, big, ints=(nz,))
+        c.call("dealias2", out[6], big, ints=(nz,))
+        return [q[:, :, :nx] for q in out] + [big[:, :, :mx]]
+
+    want = run(f, t)
+    for which in (0, 1):
+        a, b = f.copy(), t.copy()
+        (a, b)[which][1, 3, 5] = bad
+        got = run(a, b)
+        for i, (q, w) in enumerate(zip(got, want)):
+            others = [k for k in range(nz) if k != 1]
+            assert np.array_equal(q[others], w[others]), i
+            if which == 0 or i == 5:
+                assert not np.any(np.isfinite(q[1])), i
+            else:
+                assert np.array_equal(q[1], w[1]), i
