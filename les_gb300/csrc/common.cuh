@@ -237,15 +237,14 @@ PdlCall<P...> pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem = 0, 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Measurement hook (les_profile_begin/end): while a session is open, every
-// launch of one kernel family on the context's stream or its side stream is
-// bracketed by CUDA events (on the side stream the time is that of a kernel that
-// shares the GPU) and its algorithmic bytes (inputs read once + outputs written once)
+// launch of one kernel family on the session's stream is bracketed by CUDA
+// events and its algorithmic bytes (inputs read once + outputs written once)
 // are summed.  Families: 1 FP64 y-pass, 2 FP32 y-pass, 3 FP64 x-pass,
 // 4 FP32 x-pass (forward and inverse).
 enum ProfFamily { PROF_COLS64 = 1, PROF_COLS32 = 2, PROF_ROWS64 = 3, PROF_ROWS32 = 4 };
 struct ProfSession {
   int family = 0;
-  cudaStream_t stream = nullptr, side = nullptr;
+  cudaStream_t stream = nullptr;
   int n = 0, cap = 0;
   cudaEvent_t* ev = nullptr;
   double bytes = 0.0;

@@ -17,7 +17,7 @@ namespace les {
 ProfSession* g_prof = nullptr;
 bool prof_mark(int family, cudaStream_t s) {
   ProfSession* p = g_prof;
-  if (!p || p->family != family || (s != p->stream && s != p->side) || p->n >= p->cap) return false;
+  if (!p || p->family != family || p->stream != s || p->n >= p->cap) return false;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
   return cudaEventRecord(p->ev[2 * p->n], s) == cudaSuccess;
@@ -1006,7 +1006,6 @@ int les_profile_begin(les_ctx* c, int family, int max_launches) {
   ProfSession* p = new ProfSession();
   p->family = family;
   p->stream = c->stream;
-  p->side = c->side;
   p->cap = max_launches;
   p->ev = new cudaEvent_t[2 * (size_t)max_launches]();
   for (int i = 0; i < 2 * max_launches; ++i)
