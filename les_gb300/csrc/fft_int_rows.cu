@@ -99,12 +99,13 @@ template <int N1, int N2, int TT> struct RowShape {
   static constexpr int MS = N2 * LD1 > M + 1 ? N2 * LD1 : M + 1;
   static constexpr int NT = 128, RPB = NT / TT, KP = (M / 2 + TT - 1) / TT;
   static_assert(32 % TT == 0 && M % 2 == 0, "a row within one warp");
-  // Inverse pass, the scale taken twice.  Rows of 384: one sum of moduli for the
-  // whole row leaves a flat spectrum (a single point's) 52 bits, 2.2 x 2^-53 of error
-  // (the FP64 kernels 1.7); taken twice 0.3 to 0.8.  Shorter rows stay below the FP64 kernels with
-  // one (288 points 1.2 against 1.9) and are 2 % faster with it.
-  static constexpr bool MID = M > 144;
-  static_assert(!MID || TT == N1, "a lane's elements at k, and those at M - k, belong to one k1 each");
+  // Inverse pass, scaled by the largest sum of moduli of the first step's transforms
+  // (FINE) instead of the whole row's.  Rows of 384: the row's leaves a flat spectrum (a
+  // single point's) 52 bits, 2.2 x 2^-53 of error (the FP64 kernels 1.7); with the
+  // steps' 0.4 to 0.8.  Shorter rows stay below the FP64 kernels with the row's (288
+  // points 1.2 against 1.9), which takes one reduction less.
+  static constexpr bool FINE = M > 144;
+  static_assert(!FINE || (TT == N1 && N1 == 16), "a lane's elements at k, and those at M - k, belong to one k1 each");
   static constexpr size_t smem = (size_t)RPB * MS * sizeof(cfix);
 };
 
@@ -306,13 +307,13 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
     }
   }
   // at most 25 values a lane: below 2^31 units of 2^36; the row's in units of 2^40.
-  // MID: lane q holds all of the first step's transform k1 = q, so the two largest
-  // halves bound each of them, and the scale is taken again before the second step.
-  const int s1 = R::MID ? fix_down_sum(row_max<TT>(sum) + row_max<TT>(sum2), 36)
-                        : fix_down_sum(row_sum<TT>(((sum + sum2) >> 4) + 1u), 40);
+  // FINE: lane q holds all of the first step's transform k1 = q, so the two largest
+  // parts bound each of them.  Below 2^58, the second step's inner four-point
+  // transforms stay below 2^60 before its rotations and its results below 2^62.
+  const int s1 = R::FINE ? fix_down_sum(row_max<TT>(sum) + row_max<TT>(sum2), 36 + 2)
+                         : fix_down_sum(row_sum<TT>(((sum + sum2) >> 4) + 1u), 40);
   const FixShift s(s1, fix_coin((unsigned)y));
   ex += s.s;
-  unsigned top = 0;
   __syncwarp();
   // first step in place: a lane's transforms read and write their own slots,
   // so the loop needs no registers for the others (and half the code)
@@ -331,13 +332,10 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
 #pragma unroll
       for (int i = 0; i < N2; ++i) {
         if (i > 0) v[i] = ftwc(v[i], __ldg(&tw[k1 * i]));
-        if (R::MID) top = max(top, max(fix_top(v[i].x), fix_top(v[i].y)));
         S[i * LD1 + k1] = v[i];
       }
     }
   }
-  const FixShift s2(R::MID ? fix_down(row_max<TT>(top), fix_in(N1)) : 0, fix_coin(~(unsigned)y));
-  ex += s2.s;
   __syncwarp();
   if (!ok) return;
   const double factor = nan_if(bad, J.deriv[f] ? J.scale[f] * J.kunit : J.scale[f]);
@@ -350,13 +348,7 @@ __global__ void __launch_bounds__(128, MB) k_ic2r(RowJob J, const int4* __restri
     if (N2 % TT == 0 || n2 < N2) {
       cfix w[N1];
 #pragma unroll
-      for (int i = 0; i < N1; ++i) {
-        w[i] = S[n2 * LD1 + i];
-        if (R::MID) {
-          w[i].x = s2(w[i].x);
-          w[i].y = s2(w[i].y);
-        }
-      }
+      for (int i = 0; i < N1; ++i) w[i] = S[n2 * LD1 + i];
       fdft<N1, 1>(w);  // over k1: z[n2 + N2 i]
       double2 o[N1];
       fix_out(w, o, ex, factor);
