@@ -319,7 +319,8 @@ int les_fft_r2c(les_ctx* ctx, double* planes, int nplanes, int big);
 int les_fft_c2r(les_ctx* ctx, double* planes, int nplanes, int big);
 /* Measurement (no counterpart in the reference): between les_profile_begin
  * and les_profile_end, every launch of one transform-kernel family on the
- * context's stream (eager steps, not graph replays) is bracketed by CUDA
+ * context's stream (eager steps, not graph replays; not a step's few surface
+ * planes, which run beside the others on a second stream) is bracketed by CUDA
  * events.  family: 1 FP64 y-pass, 2 FP32 y-pass, 3 FP64 x-pass, 4 FP32
  * x-pass; at most max_launches launches are measured.  end returns the
  * launches measured, their summed device time (ms) and summed algorithmic

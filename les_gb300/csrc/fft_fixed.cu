@@ -188,7 +188,7 @@ template <typename T, typename TIn>
 bool launch_rows_r2c_fixed(const RowJob& J, const RealPlanDev& P, int rpc, size_t sm, cudaStream_t s) {
   switch (P.nx / 2) {
 #define LES_CASE(n) \
-case n: r2c_fixed<T, TIn, n>(J, P, rpc, s); return true;
+  case n: r2c_fixed<T, TIn, n>(J, P, rpc, s); return true;
     LES_ROW_SIZES(LES_CASE)
 #undef LES_CASE
     default: return false;
@@ -198,7 +198,7 @@ template <typename T, typename TOut>
 bool launch_rows_c2r_fixed(const RowJob& J, const RealPlanDev& P, int rpc, size_t sm, cudaStream_t s) {
   switch (P.nx / 2) {
 #define LES_CASE(n) \
-case n: c2r_fixed<T, TOut, n>(J, P, rpc, s); return true;
+  case n: c2r_fixed<T, TOut, n>(J, P, rpc, s); return true;
     LES_ROW_SIZES(LES_CASE)
 #undef LES_CASE
     default: return false;

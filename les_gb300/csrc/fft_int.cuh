@@ -10,11 +10,14 @@
 // instruction per value on the way out (1.9 per clock).
 //
 // Measured against the FP64 kernels (256^2 planes): field and derivatives of
-// 64 planes (les_filt_da) 1122 -> 173 us, FP64 step at 256^3 89.1 -> 19.2 ms.
-// What bounds them is instruction issue: the x pass runs 16 to 20 warps per SM
-// (96 to 128 registers, 46 % of the issue slots busy, half of the integer pipe),
-// the y pass 32.  The x pass in three steps of at most eight values (64
-// registers, 32 warps) was no faster at any length.
+// 64 planes (les_filt_da) 1122 -> 174 us, FP64 step at 256^3 89.0 -> 19.3 ms.
+// What bounds them is latency at the warps that fit, not a pipe: of the three
+// launches of that les_filt_da the x pass has 14 to 15 warps an SM (128 registers;
+// 80 to 96 and 20 warps on other lengths) and issues in 42 and 51 % of the cycles,
+// the y pass 27 warps (64 registers, 24 to 476 bytes spilled) and 51 %; the
+// integer pipe is 46 to 55 % busy, the FP64 pipe 31 to 42 %, DRAM 15 to 20 %.  The
+// x pass in three steps of at most eight values (64 registers, 32 warps) was no
+// faster at any length.
 //
 // Precision.  A value is a multiple of 2^ex with |value / 2^ex| < 2^61, so a
 // row's largest elements carry 55 to 60 bits (an FP64 number: 53) and
@@ -23,15 +26,17 @@
 // data: from the row's largest exponent at the load, for an inverse from the
 // sums of moduli of its first butterflies (a spectrum that one mode dominates
 // keeps its full width), and from the largest value between the steps (the
-// inverse x pass instead takes the sum of all moduli, which bounds all of it).
-// Each choice leaves the headroom that the following step can need, so nothing
-// overflows.
-// Twiddles are rounded to 62 fractional bits.  Against extended precision
-// (noise, a mean wind of 170 times the noise, a single point, fields that fall
-// off along x or along y; 32^2 to 256^2 and their 3/2 grids) the relative error is
-// 0.16 to 0.85 of the FP64 kernels' in the field, its derivatives, the plane
-// transforms and the 3/2 round trip; the inverse of a single point's flat spectrum
-// in rows of 384, where the sum of moduli costs most, is at 1.2 (2.2 eps).
+// inverse x pass instead takes the sum of all moduli, which bounds all of it; at
+// 384 points the first step's, see RowShape).  Each choice leaves the headroom
+// that the following step can need, so nothing overflows.
+// Twiddles are rounded to 62 fractional bits, halves in a direction of each row
+// and column (FixShift).  Against extended precision, as a share of the FP64
+// kernels' relative error, 16 x 64 to 64 x 256, 256^2 and 384 x 32 with their 3/2
+// grids: 0.07 to 0.83 in the plane transforms, the field, its derivatives and the
+// 3/2 round trip for noise, a mean wind of 130 and of 12000 times the noise,
+// smooth fields and fields that fall off along x or along y; a single point 0.17
+// to 1.03, its filtered field in rows of 64 by 24 rows 1.34 (2.2 x 2^-53).  The
+// largest error of a plane stays within 8 of its rms.
 //
 // Not-a-number and infinity in a row or column make all of it NaN, as the
 // butterflies of an FP64 transform do.  Values below 2^-1042 count as zero.

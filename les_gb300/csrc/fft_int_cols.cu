@@ -6,13 +6,15 @@
 // one step (R3 = 1) or two (R2, then R3), with an exchange through shared memory
 // before each step (the middle step reads and writes its own slots).  The
 // spectral side holds k = j + J k1 the same way.  The inverse runs the steps
-// backwards.  What bounds the pass is issue: with steps of at most 8 values a
-// thread needs 64 registers and 32 warps fit an SM, and the code of one kernel
-// fits the instruction cache.  Two steps of 16 (128 registers, 16 warps) against
-// three, les_filt_da on 64 planes of 256^2: 189 against 172 us; 3/2 round trip of
-// 32 planes of 192^2: 165 against 145 us; FP64 step at 256^3: 20.0 against
-// 19.5 ms.  24 warps instead of 32 (no spills) gave 20.6 ms.  Columns are numbered
-// through all levels, so that only the last block of a launch has idle ones.
+// backwards.  With steps of at most 8 values a thread makes do with 64 registers,
+// so that 32 warps fit an SM to hide the latency that bounds the pass, at the
+// price of spills: 24 to 476 bytes a thread at 256 rows, up to 512 at 192 and 384
+// (both directions) and 20 to 544 in the 3/2 passes.  Two steps of 16 (128
+// registers, 16 warps) against three, when the shapes were chosen: les_filt_da on
+// 64 planes of 256^2 189 against 172 us, 3/2 round trip of 32 planes of 192^2 165
+// against 145 us, FP64 step at 256^3 20.0 against 19.5 ms; 24 warps instead of 32
+// (no spills) 20.6 ms.  Columns are numbered through all levels, so that only the
+// last block of a launch has idle ones.
 //
 // Outputs that only drop the Nyquist row (filt_da's field) or multiply by
 // the column's kx need no transform at all in y: the field less its
@@ -229,15 +231,16 @@ __device__ __forceinline__ void col_inv(cfix (&v)[NV], cfix* S, unsigned* slot, 
     }
   }
 }
-// (coin: the direction of halves, see FixShift)
 // w(k) v with integer weights, 0 or 1, or (sgn) |ky| as an integer, negative
 // wavenumbers (i >= SR/2) changing sign, scaled so that the sums of moduli of
-// col_inv's steps before its own scaling stay below 2^60: a job's sum (up to 24
-// values, weights up to 192: below 2^31 units of 2^44), times R2 where a second
-// step follows.  The products are exact 96-bit integers before the shift.
+// col_inv's steps before its own scaling stay below 2^60: a job's sum (SR values of
+// at most 2^18 units of 2^44, weights up to N/2: below 2^31 units), times R2 where
+// a second step follows.  The products are exact 96-bit integers before the shift.
+// coin: the direction of halves (FixShift).
 template <class P, int TX, int NV>
 __device__ __forceinline__ void col_weigh(cfix (&v)[NV], const unsigned (&w)[P::SE], bool sgn, unsigned* slot, int b, bool coin,
                                           int& ex) {
+  static_assert(P::SR * (P::N / 2) < 1 << 13, "a job's sum of moduli");
   unsigned sum = 0;
 #pragma unroll
   for (int j = 0; j < P::JS; ++j) {

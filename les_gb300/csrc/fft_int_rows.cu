@@ -183,7 +183,6 @@ __global__ void __launch_bounds__(128, MB) k_ir2c(RowJob J, const int4* __restri
   }
   __syncwarp();
   if (!ok) return;
-  const double sd = J.div[f] != 0.0 ? J.scale[f] / J.div[f] : J.scale[f];
   // X[k] = (E + O) / 2, X[M - k] = conj(E - O) / 2; lane 0: X[0], X[M], X[M / 2]
   double2* dst = reinterpret_cast<double2*>(J.work[f]) + (size_t)lev * J.pstride_work + (size_t)y * J.wc;
   const int nc = J.ncols;

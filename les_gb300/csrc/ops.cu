@@ -1509,13 +1509,13 @@ __global__ void k_lag_prep(const double* __restrict__ u, const double* __restric
 }
 
 __device__ __forceinline__ float pow_m18(float x) { return 1.0f / sqrtf(sqrtf(sqrtf(x))); }
-// max(real(a), real(b)) of the reference: FP32 comparison, result widened
 // (dt/T) / (1 + dt/T): one division in FP64; FP32 as the reference writes it
 __device__ __forceinline__ double lag_epsi(double dt, double T) { return dt / (T + dt); }
 __device__ __forceinline__ float lag_epsi(float dt, float T) {
   const float d = dt / T;
   return d / (1.0f + d);
 }
+// max(real(a), real(b)) of the reference: FP32 comparison, result widened
 __device__ __forceinline__ double fmax32r(double a, double b) { return fmax32(a, b); }
 __device__ __forceinline__ float fmax32r(float a, float b) { return a > b ? a : b; }
 template <typename R>
@@ -2629,7 +2629,9 @@ __global__ void __launch_bounds__(256, 3) k_rhs_ab2_mx(
 __global__ void __launch_bounds__(256) k_dpdz_project(double* u, double* v, double* w, double* Rx, double* Ry, double* Rz,
                                                       const double* __restrict__ p, const double* __restrict__ dpdx,
                                                       const double* __restrict__ dpdy, double* dpdz, int ld, int nx,
-                                                      int ny, int nz, double idz, double mdt15) { pdl_wait();  // 1/dz, -1.5 dt
+                                                      int ny, int nz, double idz,    // 1/dz
+                                                      double mdt15) {                // -1.5 dt
+  pdl_wait();
   const unsigned np = (unsigned)ld * ny;
   const unsigned r = blockIdx.x * 256u + threadIdx.x;
   if (r >= np) return;
@@ -4780,18 +4782,18 @@ static int scalarT(les_ctx* c, typename PX<M>::S* const* bigf, const ScalarDesc&
       double *f1[1] = {c->f[d.s]}, *x1[1] = {c->f[d.dsdx]}, *y1[1] = {c->f[d.dsdy]};
       filt_da_inverse(c, J, f1, x1, y1, 1, nz);
     } else {
-    colsT<T, CX>(c, J);
-    if constexpr (MX) {  // theta in FP64 (plane mean added back), the gradients FP32-held
-      double* o1[1] = {c->f[d.s]};
-      const double* offo[1] = {th0};
-      c2rT<T, double>(c, 1, nz, c->wsB, o1, (long)g.nplane, false, g.lh, offo);
-      float* o2[2] = {f32(c, d.dsdx), f32(c, d.dsdy)};
-      c2rT<T, float>(c, 2, nz, (CX*)c->wsB + FS, o2, (long)g.nplane, false, g.lh);
-    } else {
-      double* out[3] = {c->f[d.s], c->f[d.dsdx], c->f[d.dsdy]};
-      const double* offo[3] = {th0, nullptr, nullptr};
-      c2rT<T, double>(c, 3, nz, c->wsB, out, (long)g.nplane, false, g.lh, offo);
-    }
+      colsT<T, CX>(c, J);
+      if constexpr (MX) {  // theta in FP64 (plane mean added back), the gradients FP32-held
+        double* o1[1] = {c->f[d.s]};
+        const double* offo[1] = {th0};
+        c2rT<T, double>(c, 1, nz, c->wsB, o1, (long)g.nplane, false, g.lh, offo);
+        float* o2[2] = {f32(c, d.dsdx), f32(c, d.dsdy)};
+        c2rT<T, float>(c, 2, nz, (CX*)c->wsB + FS, o2, (long)g.nplane, false, g.lh);
+      } else {
+        double* out[3] = {c->f[d.s], c->f[d.dsdx], c->f[d.dsdy]};
+        const double* offo[3] = {th0, nullptr, nullptr};
+        c2rT<T, double>(c, 3, nz, c->wsB, out, (long)g.nplane, false, g.lh, offo);
+      }
     }
   }
   op_ddz(c, c->f[d.dsdz], c->f[d.s], 1);
@@ -5193,7 +5195,7 @@ void autotune_probe(les_ctx* c, int fp32) {
 int step_fp64(les_ctx* c) { return stepT<0>(c); }
 int step_mixed(les_ctx* c) { return stepT<1>(c); }
 // Precision 2: the FP64 step where the integer-pipe transforms cover the grid
-// (they are faster than float-float ones, 128^3 with theta 4.25 -> 2.9 ms a
+// (they are faster than float-float ones, 128^3 with theta 4.25 -> 2.37 ms a
 // step, and closer to the exact result), else float-float transforms.
 int step_ff(les_ctx* c) { return int_grid(c) ? stepT<0>(c) : stepT<2>(c); }
 
