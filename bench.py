@@ -58,7 +58,8 @@ def parse():
     p.add_argument("--steps", type=int, default=10)  # multiple of cs_count (5)
     p.add_argument("--warmup", type=int, default=3)
     p.add_argument("--form", default="mixed", choices=["fp64", "mixed", "ff"],
-                   help="mixed: FP32-mixed step; fp64: FP64 step; ff: FP64 state with float-float transforms")
+                   help="mixed: FP32-mixed step; fp64: FP64 step; ff: precision 2, FP64 state with transforms of "
+                        "at least float-float precision (the FP64 form's where they cover the grid)")
     p.add_argument("--model", type=int, default=5, choices=[5, 4, 3, 2],
                    help="SGS model of the FP64 step (5 Lagrangian scale-dependent, 4 scale-invariant, "
                         "3 plane-averaged scale-dependent, 2 standard dynamic)")
@@ -409,7 +410,8 @@ def main():
                    "rmsdiv_mixed": ctx_m.rmsdiv(), "rmsdiv_fp64": ctx_d.rmsdiv(),
                    "fp64_step_ledger_frac": bpp_d * pts / (ms_d / args.steps / 1e3) / 1e9 / hbm}
         ctx_m.close()
-        # the FP64 state with float-float transforms (precision 2), same steps
+        # precision 2, same steps: the FP64 form's own step where the integer-pipe
+        # transforms cover the grid (this one), float-float transforms elsewhere
         cfg_f, ctx_f = new_member(lg, args.grid, "ff", 1234)
         for _ in range(warm):
             ctx_f.step(1)
@@ -445,7 +447,7 @@ def main():
         line = {"metric": METRIC, "value": value, "unit": "pt-steps/s", "n_gpus": world, "steps": args.steps,
                 "warmup": warm, "ms_per_step": ms_max / args.steps, "higher_is_better": True,
                 "scaling": "weak", "vs_baseline": None,
-                "dtype": {"fp64": "f64", "ff": "f64 (float-float transforms)"}.get(args.form, "f32/f64-mixed"),
+                "dtype": {"fp64": "f64", "ff": "f64 (transforms at least float-float)"}.get(args.form, "f32/f64-mixed"),
                 "data": "synthetic (seeded SplitMix64 initial state, x-striped surface)",
                 "config": {"workload": workload_name(cfg), "grid": [cfg.nx, cfg.ny, cfg.nz - 1],
                            "form": args.form, "dt": cfg.dt, "cflu": cflu, "visc_stab": visc,
