@@ -9,8 +9,9 @@ With --pert X a third member runs the FP64 step from the same state with
 every interior u, v, w value multiplied by (1 + X r), r uniform in [-1, 1]
 (X = 1e-15: a perturbation at the size of FP64 rounding), and its difference
 from the FP64 member is reported beside the mixed form's: it shows how the
-configuration itself amplifies a difference of rounding size.  With --ff the
-FP64 state with float-float transforms (precision 2) runs beside them too.
+configuration itself amplifies a difference of rounding size.  With --ff
+precision 2 runs beside them too: the FP64 step itself on grids that the
+integer-pipe transforms cover (256^3 among them), float-float transforms on others.
 
   python -m les_gb300.precision_study [--grid 256] [--steps 500] [--every 50]
                                       [--jt0 0] [--dt 2e-4] [--pert 1e-15] [--ff]
